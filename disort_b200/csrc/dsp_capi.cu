@@ -17,8 +17,7 @@
 #include "../../include/dsp.h"
 #include "dsp_device.cuh"
 #include "dsp_host.hpp"
-#include "flux_bvp_tile.cuh"
-#include "flux_bvp_reg.cuh"
+#include "flux_bvp.cuh"
 #include "flux_jac.cuh"
 #include "flux_layer.cuh"
 #include "flux_setup.cuh"
@@ -29,10 +28,8 @@ using namespace dsp_host;
 
 namespace {
 
-// One chunk of a flux solve.  JAC: the temperature-Jacobian forms of the layer
-// and boundary-value kernels (they also write the P/Q and multiplier records),
-// then flux_jac_kernel with the view `jv`.
-template <int N, bool JAC, bool SPH>
+// One chunk of a flux solve; with the Jacobian view `jv` flux_jac_kernel follows.
+template <int N, bool SPH>
 dsp_status launch_flux_chunk(dsp_context ctx, const FluxParams& p, cudaStream_t s, const JacView* jv) {
   {
     KernelTimer kt(ctx, "flux_setup_kernel", s);
@@ -45,16 +42,16 @@ dsp_status launch_flux_chunk(dsp_context ctx, const FluxParams& p, cudaStream_t 
   {
     static bool attr = false;
     if (!attr) {
-      flux_layer_set_attrs<N, JAC>();
+      flux_layer_set_attrs<N>();
       attr = true;
     }
     // the schedule for (N, L) may pick the layer stage's form and CTA size
     const dsp_schedule sch = find_schedule(ctx, N, p.L);
     const bool split = sch.layer_stage == 0 ? layer_split<N>() : sch.layer_stage == 1;
-    flux_layer_launch<N, JAC>(
-        p, ctx->host_tables.at(N).data(), s,
-        [&](const char* name, auto&& launch) {
-          KernelTimer kt(ctx, name, s);
+    flux_layer_launch<N>(
+        p, (long long)p.n * p.L, ctx->host_tables.at(N).data(), s,
+        [&](int kind, auto&& launch) {
+          KernelTimer kt(ctx, kind == 1 ? "flux_eigen_kernel" : "flux_layer_kernel", s);
           launch();
         },
         split, sch.layer_cta ? sch.layer_cta : 128);
@@ -72,24 +69,16 @@ dsp_status launch_flux_chunk(dsp_context ctx, const FluxParams& p, cudaStream_t 
     KernelTimer kt(ctx, "flux_sph_source_kernel", s);
     flux_sph_source_kernel<N><<<(unsigned)((tasks + C::WPC - 1) / C::WPC), 32 * C::WPC, C::smem_bytes(), s>>>(p);
   }
-  if constexpr (N <= 16) {
-    using C = RCfg<N>;
-    const size_t sm = C::smem_bytes();
-    const int grid = (p.n + C::TPC - 1) / C::TPC;
-    KernelTimer kt(ctx, "flux_bvp_kernel", s);
-    flux_bvp_reg_kernel<N, false, JAC, SPH><<<grid, C::CTA, sm, s>>>(p);
-  } else {
-    using C = TCfg<N>;
-    const size_t sm = C::smem_bytes();
+  {
+    using C = BCfg<N>;
     static bool attr = false;
     if (!attr) {
-      cudaFuncSetAttribute(flux_bvp_tile_kernel<N, false, JAC, SPH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)sm);
+      cudaFuncSetAttribute(flux_bvp_kernel<N, false, SPH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)C::smem_bytes());
       attr = true;
     }
-    const int grid = (p.n + C::TPC - 1) / C::TPC;
     KernelTimer kt(ctx, "flux_bvp_kernel", s);
-    flux_bvp_tile_kernel<N, false, JAC, SPH><<<grid, C::CTA, sm, s>>>(p);
+    flux_bvp_kernel<N, false, SPH><<<(p.n + C::TPW - 1) / C::TPW, 32, C::smem_bytes(), s>>>(p);
   }
   if (jv) {
     using C = JCfg<N>;
@@ -110,17 +99,11 @@ dsp_status launch_flux_chunk(dsp_context ctx, const FluxParams& p, cudaStream_t 
 // GPU at once (one wave).
 template <int N>
 int64_t bvp_wave_n(int sm_count) {
+  using C = BCfg<N>;
   int blocks = 0;
-  if constexpr (N <= 16) {
-    using C = RCfg<N>;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, flux_bvp_reg_kernel<N>, C::CTA, C::smem_bytes());
-    return (int64_t)std::max(blocks, 1) * C::TPC * sm_count;
-  } else {
-    using C = TCfg<N>;
-    cudaFuncSetAttribute(flux_bvp_tile_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem_bytes());
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, flux_bvp_tile_kernel<N>, C::CTA, C::smem_bytes());
-    return (int64_t)std::max(blocks, 1) * C::TPC * sm_count;
-  }
+  cudaFuncSetAttribute(flux_bvp_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem_bytes());
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, flux_bvp_kernel<N>, 32, C::smem_bytes());
+  return (int64_t)std::max(blocks, 1) * C::TPW * sm_count;
 }
 
 int64_t bvp_wave(int N, int sm_count) {
@@ -140,11 +123,8 @@ int64_t bvp_wave(int N, int sm_count) {
 
 template <int N>
 dsp_status launch_flux_n(dsp_context ctx, const FluxParams& p, cudaStream_t s, const JacView* jv) {
-  // Jacobian records are only needed when there is a thermal source to differentiate
-  const bool jac = jv && (p.flags & DSP_FLAG_THERMAL);
-  const bool sph = (p.flags & DSP_FLAG_SPHERICAL_BEAM) != 0;
-  if (sph) return jac ? launch_flux_chunk<N, true, true>(ctx, p, s, jv) : launch_flux_chunk<N, false, true>(ctx, p, s, jv);
-  return jac ? launch_flux_chunk<N, true, false>(ctx, p, s, jv) : launch_flux_chunk<N, false, false>(ctx, p, s, jv);
+  return (p.flags & DSP_FLAG_SPHERICAL_BEAM) ? launch_flux_chunk<N, true>(ctx, p, s, jv)
+                                             : launch_flux_chunk<N, false>(ctx, p, s, jv);
 }
 
 dsp_status launch_flux(dsp_context ctx, int N, const FluxParams& p, cudaStream_t s, const JacView* jv) {
@@ -499,15 +479,12 @@ dsp_status flux_solve(dsp_context ctx, const dsp_flux_batch* batch_in, const dsp
   const size_t hg_doubles = hg ? (size_t)round4(L * b.pmom_count) : 0;  // keeps the records 32-byte aligned
   Sizes sz = sizes_for(N, L);
   sz.inst += hg_doubles;
-  // with Jacobians of a thermal solve: P/Q and multiplier records, and the
-  // replayed right-hand side values [L][N][ndof]
+  // with Jacobians of a thermal solve: the vectors r of every degree of freedom [L][h][ndof]
   const bool jrecs = jac && thermal;
-  const size_t jpq_d = jrecs ? (size_t)L * jpq_stride(N) : 0;
-  const size_t jrec_d = jrecs ? (size_t)L * jrec_stride(N) : 0;
-  const size_t jcv_d = jrecs ? (size_t)L * N * ndof : 0;
+  const size_t jcv_d = jrecs ? (size_t)L * (N / 2) * ndof : 0;
   // with the pseudo-spherical beam: the spherical record of every layer
   const size_t sph_d = spherical ? (size_t)L * sph_stride(N) : 0;
-  sz.bvp += jpq_d + jrec_d + jcv_d + sph_d;
+  sz.bvp += jcv_d + sph_d;
   const size_t inst_doubles = sz.inst + sz.layer + sz.bvp;
   size_t budget = workspace_budget();
   size_t freeb = 0, totalb = 0;
@@ -548,14 +525,11 @@ dsp_status flux_solve(dsp_context ctx, const dsp_flux_batch* batch_in, const dsp
       for (int f = 0; f < 8; ++f) p.out[f] = dout[f] + off * nlev;
       p.status = dstatus + off;
       // the spherical and Jacobian areas follow the elimination records of the chunk
-      double* xbase = p.bvp_rec + (size_t)m * (sz.bvp - jpq_d - jrec_d - jcv_d - sph_d);
+      double* xbase = p.bvp_rec + (size_t)m * (sz.bvp - jcv_d - sph_d);
       p.sph = spherical ? xbase : nullptr;
       JacView jv;
       if (jac) {
-        double* jbase = xbase + (size_t)m * sph_d;
-        p.jac_pq = jrecs ? jbase : nullptr;
-        p.jac_rec = jrecs ? jbase + (size_t)m * jpq_d : nullptr;
-        jv.cv = jrecs ? jbase + (size_t)m * (jpq_d + jrec_d) : nullptr;
+        jv.cv = jrecs ? xbase + (size_t)m * sph_d : nullptr;
         jv.ndof = ndof;
         for (int f = 0; f < 6; ++f) jv.out[f] = djac[f] + off * nlev * ndof;
       }

@@ -91,47 +91,57 @@ struct GenLayout {
   }
 };
 
-// Layer record (doubles) written by the layer kernel:
-// G[N][N] | eig[N] | zb[N] | z0[N] | z1[N] | xr0 | xr1
-__host__ __device__ constexpr int lrec_G(int) { return 0; }
-__host__ __device__ constexpr int lrec_eig(int N) { return N * N; }
-__host__ __device__ constexpr int lrec_zb(int N) { return N * N + N; }
-__host__ __device__ constexpr int lrec_z0(int N) { return N * N + 2 * N; }
-__host__ __device__ constexpr int lrec_z1(int N) { return N * N + 3 * N; }
-__host__ __device__ constexpr int lrec_xr(int N) { return N * N + 4 * N; }
+// Layer record (doubles) written by the layer stage, h = N/2 (rows of HP, h rounded
+// up to even, pads zero):
+//   X^T [h][HP] | Y^T [h][HP] | k [HP] | beam c, d [HP] each | thermal c, d [HP]
+//   each | xr0 | xr1
+// With D = diag(sqrt(w_i mu_i)) and up/down the intensities at the h quadrature
+// angles, the layer's modes are phi = D (up + down) = X C, psi = D (up - down) =
+// Y D_, where C = E1 a + E2 b + c_p, D_ = E2 b - E1 a + d_p with
+// E1 = exp(-k (tau - tau_top)), E2 = exp(-k (tau_bot - tau)); X^T Y = I.  (Row c of
+// X^T is mode c.)  The particular solution (c_p, d_p) in these coordinates is
+// exp(-tau/mu0) (c, d) for the beam and ((xr0 + xr1 tau) c, xr1 d) for thermal
+// emission.  lrec_stride is the space allotted to a record.
+__host__ __device__ constexpr int mod_hp(int N) { return N / 2 + ((N / 2) & 1); }
+__host__ __device__ constexpr int mod_X(int) { return 0; }
+__host__ __device__ constexpr int mod_Y(int N) { return (N / 2) * mod_hp(N); }
+__host__ __device__ constexpr int mod_k(int N) { return 2 * (N / 2) * mod_hp(N); }
+__host__ __device__ constexpr int mod_cb(int N) { return mod_k(N) + mod_hp(N); }
+__host__ __device__ constexpr int mod_db(int N) { return mod_k(N) + 2 * mod_hp(N); }
+__host__ __device__ constexpr int mod_ct(int N) { return mod_k(N) + 3 * mod_hp(N); }
+__host__ __device__ constexpr int mod_dt(int N) { return mod_k(N) + 4 * mod_hp(N); }
+__host__ __device__ constexpr int mod_xr(int N) { return mod_k(N) + 5 * mod_hp(N); }
+__host__ __device__ constexpr int mod_size(int N) { return mod_xr(N) + 2; }
 __host__ __device__ constexpr int lrec_stride(int N) { return round4(N * N + 4 * N + 2); }
-// Elimination record (doubles) written by the BVP kernels, per layer: the N
-// pivot rows [U | V | c] of U x_l + V x_{l+1} = c and the pivot reciprocals.
-// N <= 16: rows of 2N + 2 ([U | V | c | 1/pivot]); N >= 32: rows of 2N + 1
-// ([U | V | c]), then 1 / pivot [N].
+// Boundary-value record (doubles) per layer: H [h][HP] | G [h][HP] | r [HP], and
+// in the last solved layer's record the downward intensities at the bottom [HP]
+// and the inverse [h][HP] of the surface system.  Before the boundary-value
+// kernel runs the area holds the hand-off of a split layer stage.  brec_stride is
+// the space allotted to a record.
+__host__ __device__ constexpr int brec_H(int) { return 0; }
+__host__ __device__ constexpr int brec_G(int N) { return (N / 2) * mod_hp(N); }
+__host__ __device__ constexpr int brec_r(int N) { return 2 * (N / 2) * mod_hp(N); }
+__host__ __device__ constexpr int brec_dn(int N) { return brec_r(N) + mod_hp(N); }
+__host__ __device__ constexpr int brec_inv(int N) { return brec_r(N) + 2 * mod_hp(N); }
 __host__ __device__ constexpr int brec_stride(int N) { return round4(N * (2 * N + 2)); }
+static_assert(mod_size(4) <= lrec_stride(4) && mod_size(6) <= lrec_stride(6) && mod_size(14) <= lrec_stride(14) &&
+                  mod_size(64) <= lrec_stride(64),
+              "layer record");
+static_assert(brec_inv(4) + 4 <= brec_stride(4) && brec_inv(6) + 12 <= brec_stride(6) &&
+                  brec_inv(64) + 1024 <= brec_stride(64),
+              "boundary-value record");
 
-// Pseudo-spherical beam record of the flux path, per layer: the slope Z1 of the
-// beam particular solution Z(tau) = exp(-xba tau) (Z0 + Z1 tau) (Z0 is the layer
-// record's zb), its attenuation xba, and the layer's Chapman factor
-// (computeBeamSourceSpherical, FluxSolver.cpp:650-738; :391-419).
+// Pseudo-spherical beam record, per layer: with the layer record's beam slots
+// (c0, d0), the beam's particular solution is exp(-xba tau) ((c0, d0) + tau (c1, d1))
+// in the layer's modes (computeBeamSourceSpherical, FluxSolver.cpp:650-738;
+// :391-419): c1 [h] | d1 [h] | xba | the layer's Chapman factor.
 __host__ __device__ constexpr int sph_stride(int N) { return round4(N + 2); }
 __host__ __device__ constexpr int sph_xba(int N) { return N; }
 __host__ __device__ constexpr int sph_ch(int N) { return N + 1; }
 
-// Temperature-Jacobian records of the flux path (compute_temperature_jacobian).
-// Per layer, written by the layer stage: P[NN] | Q[NN], the thermal particular
-// solution per unit Planck intercept and slope: with P and Q the solution of
-// computeIsotropicSource is Z1 = xr1 P / 2 in both hemispheres and
-// Z0 = (xr0 P +/- xr1 Q) / 2 (z0's upper / lower hemisphere order), so the
-// derivatives with respect to a layer's top and bottom level Planck values
-// (FluxSolver.cpp:789-829) follow from the derivatives of xr0 and xr1.
-__host__ __device__ constexpr int jpq_stride(int N) { return N; }
-// Per layer, written by the boundary-value kernels: the multiplier applied to
-// every panel slot at every pivot column, [N][3N/2] (0 where the slot was not a
-// candidate or the column was skipped as singular), then the pivot slot of each
-// column [N] (as doubles).  Together with the pivot rows of the elimination
-// record they replay the band LU on further right-hand sides.
-__host__ __device__ constexpr int jrec_stride(int N) { return round4(N * (3 * (N / 2)) + N); }
-
 // General-solver layer record: the flux layer record, then the eigenvectors
 // and sources at the user polar angles of the current mode:
-// GU[numu][N] | zbu[numu] | z0u[numu] | z1u[numu]
+// GU[numu][N] (columns b[h] | a[h]) | zbu[numu] | z0u[numu] | z1u[numu]
 __host__ __device__ constexpr int glrec_gu(int N) { return lrec_stride(N); }
 __host__ __device__ constexpr int glrec_stride(int N, int numu) { return round4(lrec_stride(N) + numu * (N + 3)); }
 
@@ -155,7 +165,8 @@ struct GenView {
   const double* zalt;          // level altitudes, laid out like temp (pseudo-spherical beam only)
   DArr utau, umu, phi, phi0;
   long long lstride;           // layer record stride (glrec_stride)
-  double* cc;                  // [layers][N] boundary-value solution of the mode
+  double* cc;                  // [layers][N] boundary-value solution of the mode (b[h] | a[h])
+  double* ptab;                // per slot: P_l^m(-mu0) [N], then P_l^m(mu_u) [numu][N], of the mode
   double* out_flux[8];         // [batch][ntau_out]
   double* out_int;             // [batch][ntau_out][numu_out][nphi]
   double* out_iavg;            // [batch][ntau_out][numu_out]
@@ -213,17 +224,15 @@ struct FluxParams {
   int32_t* status;
   GenView g;  // general-solver launches only
   double* sph = nullptr;      // [n][L][sph_stride], general: [layers][sph_stride] (pseudo-spherical beam only)
-  double* jac_pq = nullptr;   // [n][L][jpq_stride] (temperature-Jacobian launches only)
-  double* jac_rec = nullptr;  // [n][L][jrec_stride] (temperature-Jacobian launches only)
 };
 
-// The temperature-Jacobian launch of a flux chunk: the right-hand side values
-// of the replayed elimination, per instance [L][N][ndof], and the six outputs
-// [batch][L+1][ndof] (already offset to the chunk's first instance).
+// The temperature-Jacobian launch of a flux chunk: the vectors r of every degree
+// of freedom, per instance [L][h][ndof], and the six outputs [batch][L+1][ndof]
+// (already offset to the chunk's first instance).
 struct JacView {
   int ndof;         // flux path: L + 2 degrees of freedom (level temperatures 0..L,
                     // surface); general path: the largest L + 2 of the batch
-  double* cv;       // [n][L][N][ndof] (general path: [chunk layers][N][ndof])
+  double* cv;       // [n][L][h][ndof] (general path: [chunk layers][h][ndof])
   double* out[6];   // flux_up, flux_down, mean_intensity, _down, _up, flux_divergence
   int ndof_out;     // general path: column stride of out (>= L + 2 of every instance)
 };
@@ -283,44 +292,6 @@ __device__ __forceinline__ void team_sync() {
   }
 }
 
-// Arg-max of (v, i) over the team, ties to the smaller index; result to all.
-// `red` is team-private shared scratch of 2*(TEAM/32) doubles (unused for TEAM <= 32).
-template <int TEAM>
-__device__ __forceinline__ void team_argmax(double& v, int& idx, double* red) {
-  constexpr int W = TEAM < 32 ? TEAM : 32;
-  const unsigned m = team_mask<TEAM>();
-#pragma unroll
-  for (int off = W / 2; off > 0; off >>= 1) {
-    const double ov = __shfl_xor_sync(m, v, off, W);
-    const int oi = __shfl_xor_sync(m, idx, off, W);
-    if (ov > v || (ov == v && oi < idx)) { v = ov; idx = oi; }
-  }
-  if constexpr (TEAM > 32) {
-    constexpr int NW = TEAM / 32;
-    const int w = threadIdx.x >> 5;
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) {
-      red[w] = v;
-      reinterpret_cast<int*>(red + NW)[w] = idx;
-    }
-    __syncthreads();
-    v = red[0];
-    idx = reinterpret_cast<int*>(red + NW)[0];
-#pragma unroll
-    for (int k = 1; k < NW; ++k) {
-      const double ov = red[k];
-      const int oi = reinterpret_cast<int*>(red + NW)[k];
-      if (ov > v || (ov == v && oi < idx)) { v = ov; idx = oi; }
-    }
-    __syncthreads();
-  }
-}
-
-// Arg-max of a >= 0 over the candidate lanes of a full warp, ties to the lowest
-// lane; 32 when no lane is a candidate.  Non-negative doubles order like their
-// bit patterns, so the maximum is two 32-bit warp reductions (high words, then
-// the low words of the lanes that tie on the high word) and the winner is the
-// lowest lane of the ballot of exact matches.  `zero` reports a maximum of 0.
 // 1/x without branches: the hardware approximation (rcp.approx.ftz.f64)
 // refined by two Newton-Raphson steps y <- y + y (1 - x y), each about doubling
 // the correct bits (Muller et al., Handbook of Floating-Point Arithmetic, 2nd
@@ -334,18 +305,6 @@ __device__ __forceinline__ double rcp_newton(double x) {
   y = fma(y, e, y);
   e = fma(-x, y, 1.0);
   return fma(y, e, y);
-}
-
-__device__ __forceinline__ int warp_argmax_nonneg(double a, bool cand, bool& zero) {
-  const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(a));
-  const unsigned hi = cand ? static_cast<unsigned>(b >> 32) : 0u;
-  const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
-  const bool tie = cand && hi == mhi;
-  const unsigned lo = tie ? static_cast<unsigned>(b) : 0u;
-  const unsigned mlo = __reduce_max_sync(0xffffffffu, lo);
-  const unsigned win = __ballot_sync(0xffffffffu, tie && static_cast<unsigned>(b) == mlo);
-  zero = (mhi | mlo) == 0u;
-  return win ? __ffs(win) - 1 : 32;
 }
 
 // Team copy of nd doubles from global to shared memory: 16-byte cp.async

@@ -3,15 +3,14 @@
 //
 // Instances are grouped by stream count (one kernel instantiation per N), the
 // groups cut into chunks that fit the workspace, and each chunk runs
-//   gen_setup_kernel, then for every azimuth mode m the layer kernel (eigen-
-//   systems, particular solutions, user-angle interpolation), the boundary-
-//   value kernel (solution coefficients; fluxes at m = 0) and the intensity
-//   kernel (Fourier accumulation and the convergence test).
+//   gen_setup_kernel, then for every azimuth mode m the layer stage (eigen-
+//   systems, particular solutions), the user-angle kernel, the boundary-value
+//   kernel (solution coefficients; fluxes at m = 0) and the intensity kernel
+//   (Fourier accumulation and the convergence test).
 // Instances whose series has ended (last mode, or converged) skip the later
 // mode launches on the device.
 #include "dsp_host.hpp"
-#include "flux_bvp_tile.cuh"
-#include "flux_bvp_reg.cuh"
+#include "flux_bvp.cuh"
 #include "flux_jac.cuh"
 #include "flux_layer.cuh"
 #include "flux_sph.cuh"
@@ -74,6 +73,7 @@ dsp_status get_mode_tables(dsp_context ctx, int N, const double** out) {
   e = cudaMemcpy(d, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMemcpy(mode tables)");
   ctx->mode_tables[N] = d;
+  ctx->host_mode_tables[N] = std::move(tab);
   *out = d;
   return DSP_OK;
 }
@@ -123,10 +123,6 @@ dsp_status get_brdf_quadrature(dsp_context ctx, const double** out) {
   return DSP_OK;
 }
 
-// The mode-m layer and boundary-value launches of a chunk; JAC: their
-// temperature-Jacobian forms (mode 0 with Jacobians asked for); SPH: with the
-// pseudo-spherical beam, whose particular solution of the mode is formed
-// between the two.
 // Resident CTAs of a kernel on the whole GPU (persistent launches).
 template <class K>
 int resident_ctas(dsp_context ctx, K kernel, int threads, size_t smem) {
@@ -136,28 +132,43 @@ int resident_ctas(dsp_context ctx, K kernel, int threads, size_t smem) {
   return per_sm * ctx->sm_count;
 }
 
+// The mode-m layer, user-angle and boundary-value launches of a chunk; SPH: with
+// the pseudo-spherical beam, whose particular solution of the mode is formed
+// between them (after the user angles, which read its raw source).
 // `order`/`head` (persistent boundary-value launch): the chunk's slots by
-// descending layer count and this mode's queue counter; null: one CTA or team
-// per slot.
-template <int N, bool JAC, bool SPH>
+// descending layer count and this mode's queue counter; null: one team per slot.
+// `host_tab`: host copy of the mode's tables.
+template <int N, bool SPH>
 void launch_general_mode(dsp_context ctx, const FluxParams& p, long long layers, cudaStream_t s, const int* order,
-                         int* head) {
-  using LC = LCfg<N, true>;
+                         int* head, const double* host_tab) {
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(flux_layer_kernel<N, true, JAC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)LC::smem_bytes());
-    if constexpr (N > 16)
-      cudaFuncSetAttribute(flux_bvp_tile_kernel<N, true, JAC, SPH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)TCfg<N>::smem_bytes());
+    flux_layer_set_attrs<N, true>();
+    cudaFuncSetAttribute(flux_bvp_kernel<N, true, SPH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)BCfg<N>::smem_bytes());
+    cudaFuncSetAttribute(gen_bvp_persistent_kernel<N, SPH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)BCfg<N>::smem_bytes());
     if constexpr (SPH)
       cudaFuncSetAttribute(flux_sph_source_kernel<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)SCfg<N>::smem_bytes());
     attr = true;
   }
+  {
+    // P_l^m at -mu0 and at the user angles
+    const long long items = (long long)p.n * (1 + p.g.numu);
+    KernelTimer kt(ctx, "gen_setup_kernel");
+    gen_ptab_kernel<<<(unsigned)((items + 127) / 128), 128, 0, s>>>(p);
+  }
   if (layers > 0) {
-    KernelTimer kt(ctx, "gen_layer_kernel");
-    flux_layer_kernel<N, true, JAC><<<(unsigned)((layers + LC::TPC - 1) / LC::TPC), LC::CTA, LC::smem_bytes(), s>>>(p);
+    flux_layer_launch<N, true>(p, layers, host_tab, s, [&](int, auto&& launch) {
+      KernelTimer kt(ctx, "gen_layer_kernel");
+      launch();
+    });
+    if (p.g.numu > 0) {
+      using C = ACfg<N>;
+      KernelTimer kt(ctx, "gen_angle_kernel");
+      gen_angle_kernel<N><<<(unsigned)((layers + C::TPC - 1) / C::TPC), 128, 0, s>>>(p);
+    }
   }
   if constexpr (SPH) {
     if (layers > 0) {
@@ -166,33 +177,14 @@ void launch_general_mode(dsp_context ctx, const FluxParams& p, long long layers,
       flux_sph_source_kernel<N, true><<<(unsigned)((layers + C::WPC - 1) / C::WPC), 32 * C::WPC, C::smem_bytes(), s>>>(p);
     }
   }
-  if constexpr (N <= 16) {
-    using C = RCfg<N>;
-    KernelTimer kt(ctx, "gen_bvp_kernel");
-    const int slots = (p.n + C::TPC - 1) / C::TPC;
-    if (order) {
-      static const int cap = resident_ctas(ctx, gen_bvp_reg_persistent_kernel<N, JAC, SPH>, C::CTA, C::smem_bytes());
-      gen_bvp_reg_persistent_kernel<N, JAC, SPH><<<slots < cap ? slots : cap, C::CTA, C::smem_bytes(), s>>>(p, order,
-                                                                                                          head);
-    } else {
-      flux_bvp_reg_kernel<N, true, JAC, SPH><<<slots, C::CTA, C::smem_bytes(), s>>>(p);
-    }
+  using C = BCfg<N>;
+  KernelTimer kt(ctx, "gen_bvp_kernel");
+  const int warps = (p.n + C::TPW - 1) / C::TPW;
+  if (order) {
+    static const int cap = resident_ctas(ctx, gen_bvp_persistent_kernel<N, SPH>, 32, C::smem_bytes());
+    gen_bvp_persistent_kernel<N, SPH><<<warps < cap ? warps : cap, 32, C::smem_bytes(), s>>>(p, order, head);
   } else {
-    using C = TCfg<N>;
-    KernelTimer kt(ctx, "gen_bvp_kernel");
-    if (order) {
-      static bool pattr = false;
-      if (!pattr) {
-        cudaFuncSetAttribute(gen_bvp_tile_persistent_kernel<N, JAC, SPH>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem_bytes());
-        pattr = true;
-      }
-      static const int cap = resident_ctas(ctx, gen_bvp_tile_persistent_kernel<N, JAC, SPH>, C::CTA, C::smem_bytes());
-      gen_bvp_tile_persistent_kernel<N, JAC, SPH><<<p.n < cap ? p.n : cap, C::CTA, C::smem_bytes(), s>>>(p, order,
-                                                                                                        head);
-    } else {
-      flux_bvp_tile_kernel<N, true, JAC, SPH><<<p.n, C::CTA, C::smem_bytes(), s>>>(p);
-    }
+    flux_bvp_kernel<N, true, SPH><<<warps, 32, C::smem_bytes(), s>>>(p);
   }
 }
 
@@ -200,6 +192,7 @@ template <int N, bool SPH>
 dsp_status launch_general_chunk(dsp_context ctx, FluxParams p, long long layers, int maxm, const double* tabs,
                                 const JacView* jv, const int* order, int* heads) {
   cudaStream_t s = ctx->stream;
+  const double* const host_tabs = ctx->host_mode_tables.at(N).data();
   p.tables = tabs;
   {
     KernelTimer kt(ctx, "gen_setup_kernel");
@@ -210,8 +203,6 @@ dsp_status launch_general_chunk(dsp_context ctx, FluxParams p, long long layers,
     KernelTimer kt(ctx, "gen_sph_chapman_kernel");
     flux_sph_chapman_kernel<true><<<(p.n + 3) / 4, 128, 0, s>>>(p);
   }
-  // Jacobian records only when there is a thermal source to differentiate
-  const bool jrecs = jv && (p.flags & DSP_FLAG_THERMAL);
   for (int m = 0; m <= maxm; ++m) {
     p.g.m = m;
     p.tables = tabs + (size_t)m * tab_size(N);
@@ -221,10 +212,9 @@ dsp_status launch_general_chunk(dsp_context ctx, FluxParams p, long long layers,
       KernelTimer kt(ctx, "gen_brdf_kernel");
       gen_brdf_kernel<N><<<p.n, 128, 0, s>>>(p);
     }
-    if (m == 0 && jrecs) launch_general_mode<N, true, SPH>(ctx, p, layers, s, order, head);
-    else launch_general_mode<N, false, SPH>(ctx, p, layers, s, order, head);
+    launch_general_mode<N, SPH>(ctx, p, layers, s, order, head, host_tabs + (size_t)m * tab_size(N));
     if (m == 0 && jv) {
-      // the Jacobians use the mode-0 elimination before the next mode replaces it
+      // the Jacobians use the mode-0 matrices before the next mode replaces them
       using C = JCfg<N>;
       static bool attr = false;
       if (!attr) {
@@ -761,12 +751,12 @@ dsp_status general_solve(dsp_context ctx, const dsp_general_batch* bin, const ds
   const double* h_fbeam = (!dev && b.direct_beam_flux.ptr) ? b.direct_beam_flux.ptr : nullptr;
   const double* h_umu0 = (!dev && b.direct_beam_mu.ptr) ? b.direct_beam_mu.ptr : nullptr;
   const double* h_mu = (!dev && user_mu) ? b.mu_user.ptr : nullptr;
-  // with Jacobians of a thermal solve, per layer: P/Q, multiplier records and
-  // the replayed right-hand side values [N][jdof]
+  // with Jacobians of a thermal solve, per layer: the vectors r of every degree
+  // of freedom [h][jdof]
   const bool jrecs = jac && thermal;
-  auto jac_per_layer = [&](int N) -> int64_t {
-    return jrecs ? (int64_t)jpq_stride(N) + jrec_stride(N) + (int64_t)N * jdof : 0;
-  };
+  auto jac_per_layer = [&](int N) -> int64_t { return jrecs ? (int64_t)(N / 2) * jdof : 0; };
+  // per instance: P_l^m at -mu0 and at the user angles, of the current mode
+  auto ptab_doubles = [&](int N) -> int64_t { return (int64_t)N * (1 + numu_eff); };
   // with the pseudo-spherical beam: the spherical record of every layer
   auto sph_per_layer = [&](int N) -> int64_t { return spherical ? (int64_t)sph_stride(N) : 0; };
   for (int N : kSupported) {
@@ -788,7 +778,7 @@ dsp_status general_solve(dsp_context ctx, const dsp_general_batch* bin, const ds
       if (hN[i] != N) continue;
       const int L = hL[i] > 0 ? hL[i] : 0;
       const int NT = user_tau ? b.num_user_tau : L + 1;
-      const int64_t rec = GenLayout::make(L, N, NT).stride + (brdf ? brdf_stride(N, numu_eff) : 0) +
+      const int64_t rec = GenLayout::make(L, N, NT).stride + ptab_doubles(N) + (brdf ? brdf_stride(N, numu_eff) : 0) +
                           (becorr ? becor_stride(ntau_need, na) : 0);
       const size_t ib = (size_t)(rec + (int64_t)L * per_layer) * sizeof(double);
       if (!c.ids.empty() && bytes + ib > budget) flush();
@@ -828,7 +818,7 @@ dsp_status general_solve(dsp_context ctx, const dsp_general_batch* bin, const ds
                    align256(c.layers * 4) + align256(c.order.size() * 4) + align256((c.maxm + 1) * 4);
       const int64_t lstride = glrec_stride(c.N, numu_eff);
       const size_t w =
-          (size_t)(c.inst_doubles + c.surf_doubles + c.be_doubles +
+          (size_t)(c.inst_doubles + c.surf_doubles + c.be_doubles + (int64_t)c.ids.size() * ptab_doubles(c.N) +
                    c.layers * (lstride + brec_stride(c.N) + c.N + sph_per_layer(c.N) + jac_per_layer(c.N))) *
           sizeof(double);
       if (w > ws_need) ws_need = w;
@@ -934,11 +924,8 @@ dsp_status general_solve(dsp_context ctx, const dsp_general_batch* bin, const ds
       p.sph = spherical ? g.cc + c.layers * c.N : nullptr;
       JacView jv;
       if (jac) {
-        // then P/Q, multipliers, replayed values
-        double* jb = g.cc + c.layers * (c.N + sph_per_layer(c.N));
-        p.jac_pq = jrecs ? jb : nullptr;
-        p.jac_rec = jrecs ? jb + c.layers * jpq_stride(c.N) : nullptr;
-        jv.cv = jrecs ? p.jac_rec + c.layers * jrec_stride(c.N) : nullptr;
+        // then the Jacobians' vectors
+        jv.cv = jrecs ? g.cc + c.layers * (c.N + sph_per_layer(c.N)) : nullptr;
         jv.ndof = jdof;
         jv.ndof_out = (int)jdof_o;
         for (int f = 0; f < 6; ++f) jv.out[f] = djac[f];
@@ -948,10 +935,11 @@ dsp_status general_solve(dsp_context ctx, const dsp_general_batch* bin, const ds
                            c.layers * (g.lstride + brec_stride(c.N) + c.N + sph_per_layer(c.N) + jac_per_layer(c.N));
       g.brdf = brdf ? wend : nullptr;
       g.becor = becorr ? wend + c.surf_doubles : nullptr;
+      g.ptab = wend + c.surf_doubles + c.be_doubles;
       const double* tabs = nullptr;
       if ((st = get_mode_tables(ctx, c.N, &tabs)) != DSP_OK) return st;
       if (ctx->debug & DSP_DEBUG_POISON_SCRATCH) {
-        const size_t wb = (size_t)(c.inst_doubles + c.surf_doubles + c.be_doubles +
+        const size_t wb = (size_t)(c.inst_doubles + c.surf_doubles + c.be_doubles + (int64_t)nc * ptab_doubles(c.N) +
                                    c.layers * (g.lstride + brec_stride(c.N) + c.N + sph_per_layer(c.N) +
                                                jac_per_layer(c.N))) *
                           sizeof(double);

@@ -37,8 +37,7 @@
 
 #include "../../include/dsp.h"
 #include "dsp_device.cuh"
-#include "flux_bvp_tile.cuh"
-#include "flux_bvp_reg.cuh"
+#include "flux_bvp.cuh"
 #include "flux_layer.cuh"
 #include "flux_setup.cuh"
 
@@ -100,22 +99,15 @@ bool tables_for(int N, std::vector<double>& tab) {
 template <int N>
 void set_attrs() {
   flux_layer_set_attrs<N>();
-  if constexpr (N > 16)
-    cudaFuncSetAttribute(flux_bvp_tile_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)TCfg<N>::smem_bytes());
+  cudaFuncSetAttribute(flux_bvp_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BCfg<N>::smem_bytes());
 }
 
 template <int N>
 void launch(const FluxParams& p, const double* host_tab, cudaStream_t s) {
   flux_setup_kernel<<<(p.n + 3) / 4, 128, 0, s>>>(p);
-  flux_layer_launch<N>(p, host_tab, s, [](const char*, auto&& launch) { launch(); });
-  if constexpr (N <= 16) {
-    using C = RCfg<N>;
-    flux_bvp_reg_kernel<N><<<(p.n + C::TPC - 1) / C::TPC, C::CTA, C::smem_bytes(), s>>>(p);
-  } else {
-    using C = TCfg<N>;
-    flux_bvp_tile_kernel<N><<<(p.n + C::TPC - 1) / C::TPC, C::CTA, C::smem_bytes(), s>>>(p);
-  }
+  flux_layer_launch<N>(p, (long long)p.n * p.L, host_tab, s, [](int, auto&& launch) { launch(); });
+  using C = BCfg<N>;
+  flux_bvp_kernel<N><<<(p.n + C::TPW - 1) / C::TPW, 32, C::smem_bytes(), s>>>(p);
 }
 
 template <int N>

@@ -1,0 +1,798 @@
+// flux_bvp.cuh — boundary-value problem and fluxes of one instance, all stream
+// counts, on a team of pow2ceil(N/2) lanes of one warp.
+//
+// Replaces setMatrix (FluxSolver.cpp:838-959), solve0 (:966-1131) and
+// computeFluxes (:1138-1287), and their DisortSolver counterparts
+// (DisortSolver.cpp:1153-1317, 1669-1920, 1980-2124): the same linear system
+// (continuity at every interface, the two boundary conditions), solved without
+// forming it.
+//
+// With h = N/2, D = diag(sqrt(w mu)), phi = D (up + down), psi = D (up - down),
+// a layer's modes are phi = X C, psi = Y D_ with X^T Y = I (layer stage) and
+//   C = E1 a + E2 b + c_p,   D_ = E2 b - E1 a + d_p,
+// E1 = exp(-k (tau - tau_top)), E2 = exp(-k (tau_bot - tau)), c_p and d_p the
+// particular solution.  The layers above a depth reflect: psi = A phi + g with a
+// symmetric A (reciprocity), A = I, g = -2 D (incoming) at the top.  Through a
+// layer, with E = exp(-k dtau):
+//   M  = X^T A X,  H = (I + M)^{-1},  Z = (1 - E^2) + 2 E H E,  G = Z^{-1},
+//   A' = Y (2 G - I) Y^T,
+//   r  = c_t + H (X^T g - d_t - c_t),  q = E r,
+//   g' = Y (c_b + d_b + 2 G (q - c_b))            (c, d: particular at top, bottom)
+// and back up, from phi at the bottom of the layer:
+//   b = G (Y^T phi_b - c_b + q),  c = 2 H E b - r,  a = c - E b,
+//   phi_t = X (c + c_t).
+// I + M and Z are symmetric positive definite whatever the layer (M is a
+// congruence of A, and Z < 2), so both are inverted without pivoting, and no
+// growing exponential is formed.  Two h x h inverses and four h^3 products per
+// layer take the place of the N-column elimination of a 3h-row panel, about a
+// tenth of its operations; near omega' = 1 (k -> 0) nothing cancels, because
+// 1 - E^2 comes from expm1.
+//
+// Mapping: lane j of a team owns column j; products read the other operand from
+// shared memory as broadcasts (one 16-byte word of each team per instruction),
+// the inverses are symmetric sweeps whose pivot row is exchanged through shared
+// memory.  A warp holds 32/TEAM instances and runs them in lockstep over its
+// deepest column.  The layer record of the next layer is brought in with
+// cp.async as soon as the current one's matrices are used up.
+#pragma once
+
+#include "dsp_device.cuh"
+
+namespace dsp {
+
+template <int N>
+struct BCfg {
+  static constexpr int H = N / 2;
+  static constexpr int HP = mod_hp(N);          // row length of the records, even
+  static constexpr int TEAM = pow2ceil(H);
+  static constexpr int TPW = 32 / TEAM;         // instances per warp (= per CTA)
+  // row stride of the matrices in shared memory: an odd number of 16-byte words,
+  // so that 8 lanes reading one row each with 16-byte loads meet no conflict
+  static constexpr int LDM = HP % 4 == 2 ? HP : HP + 2;
+  static constexpr int MAT = H * LDM;
+  static constexpr int NV = 5 * HP + 2;         // vectors of a layer record
+  static constexpr int SB = 2 * HP + 4;         // pivot-row buffer of a sweep
+  // team shared memory (doubles)
+  static constexpr int O_X = 0;                 // X^T: row c = column c of X
+  static constexpr int O_Y = O_X + MAT;         // Y^T
+  static constexpr int O_A = O_Y + MAT;         // admittance A; up: H
+  static constexpr int O_W = O_A + MAT;         // work; up: G
+  static constexpr int O_V = O_W + MAT;         // layer-record vectors
+  static constexpr int O_S = O_V + NV;          // 2 pivot-row buffers
+  static constexpr int O_G = O_S + 2 * SB;      // gathered vectors, HP each:
+  static constexpr int NG = 7;                  // g, w1, w2, gamma, scale, E / phi, D
+  static constexpr int SIZE = O_G + NG * HP;
+  // teams of a warp start 4 banks apart: their broadcasts are conflict-free
+  static constexpr int STRIDE = TPW == 1 ? SIZE : SIZE + ((2 - SIZE) % 16 + 16) % 16;
+  static_assert(STRIDE % 2 == 0 && NV % 2 == 0 && SB % 2 == 0, "16-byte alignment");
+  static constexpr size_t smem_bytes() { return sizeof(double) * (size_t)(TPW * STRIDE); }
+  // resident warps per SM: as many as shared memory admits (228 KB, 1 KB reserved
+  // per CTA), within 128 registers a thread at 16 warps and 255 at 8
+  static constexpr int MINB_SMEM = (int)((228u * 1024u) / (smem_bytes() + 1024u));
+  static constexpr int MINB_REGS = H <= 8 ? 16 : (H <= 16 ? 12 : 8);
+  static constexpr int MINB = MINB_SMEM < MINB_REGS ? MINB_SMEM : MINB_REGS;
+  static constexpr bool ROLL = H > 16;          // 64 streams: rolled outer loops
+};
+
+// Negative inverse of a symmetric positive definite matrix with unit diagonal
+// (the caller scales), columns held by the lanes: symmetric sweeps (Goodnight
+// 1979, The American Statistician 33) of pivots 0..H-1.  In step k lane j's a[i]
+// is row (k + i) mod H of its column: the update shifts it by one row, so every
+// register index is a constant.  By symmetry the pivot column is the pivot row,
+// one element per lane, exchanged through `buf` (twice, so that the rotated
+// reads are contiguous; one double further in odd steps, to keep 16-byte
+// alignment).  With a unit diagonal every pivot is <= 1, so the pivot lane can
+// take the common update with 1 - 1/pivot in the place of the multiplier
+// without losing digits: v - v (1 - p) = v p, p >= 1.
+template <int H, int SB>
+__device__ __forceinline__ void sweep_step(double* a, const int j, const int k, const bool odd, const bool store,
+                                           double* buf, bool& singular) {
+  double* b = buf + (odd ? SB : 0);
+  const int o = odd ? 1 : 0;
+  if (store) {
+    b[j + o] = a[0];
+    b[j + H + o] = a[0];
+  }
+  __syncwarp();
+  const double* v = b + k + o;
+  const double d = v[0];
+  if (d == 0.0) singular = true;  // a zero pivot: its row and column are left out
+  const double p = d == 0.0 ? 0.0 : rcp_newton(d);
+  const double c = a[0] * p;
+  const double cc = j == k ? 1.0 - p : c;
+  const double2* v2 = reinterpret_cast<const double2*>(v);
+  {
+    const double2 w = v2[0];
+    if (H > 1) a[0] = fma(-cc, w.y, a[1]);
+  }
+#pragma unroll
+  for (int i = 2; i < H; i += 2) {
+    const double2 w = v2[i / 2];
+    a[i - 1] = fma(-cc, w.x, a[i]);
+    if (i + 1 < H) a[i] = fma(-cc, w.y, a[i + 1]);
+  }
+  a[H - 1] = j == k ? -p : c;
+}
+
+template <int H, int SB, bool ROLL>
+__device__ __forceinline__ void sweep_inverse(double* a, const int j, const bool store, double* buf, bool& singular) {
+  if constexpr (ROLL) {
+    static_assert(!ROLL || H % 2 == 0, "steps in pairs");
+#pragma unroll 1
+    for (int k = 0; k < H; k += 2) {
+      sweep_step<H, SB>(a, j, k, false, store, buf, singular);
+      sweep_step<H, SB>(a, j, k + 1, true, store, buf, singular);
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < H; ++k) sweep_step<H, SB>(a, j, k, (k & 1) != 0, store, buf, singular);
+  }
+  __syncwarp();
+}
+
+// sum_i a[i] v[i], v broadcast from shared memory (HP long, padded with 0)
+template <int H>
+__device__ __forceinline__ double dot_reg(const double* a, const double* v) {
+  double s0 = 0.0, s1 = 0.0;
+  const double2* v2 = reinterpret_cast<const double2*>(v);
+#pragma unroll
+  for (int i = 0; i < H; i += 2) {
+    const double2 w = v2[i / 2];
+    s0 = fma(a[i], w.x, s0);
+    if (i + 1 < H) s1 = fma(a[i + 1], w.y, s1);
+  }
+  return s0 + s1;
+}
+// sum_i row[i] v[i], both in shared memory (row: this lane's own)
+template <int H>
+__device__ __forceinline__ double dot_row(const double* row, const double* v) {
+  double s0 = 0.0, s1 = 0.0;
+  const double2 *r2 = reinterpret_cast<const double2*>(row), *v2 = reinterpret_cast<const double2*>(v);
+#pragma unroll
+  for (int i = 0; i < H; i += 2) {
+    const double2 x = r2[i / 2], w = v2[i / 2];
+    s0 = fma(x.x, w.x, s0);
+    if (i + 1 < H) s1 = fma(x.y, w.y, s1);
+  }
+  return s0 + s1;
+}
+// sum_i col[i * ld] v[i]: column `col` across the lanes
+template <int H>
+__device__ __forceinline__ double dot_col(const double* col, const int ld, const double* v) {
+  double s0 = 0.0, s1 = 0.0;
+  const double2* v2 = reinterpret_cast<const double2*>(v);
+#pragma unroll
+  for (int i = 0; i < H; i += 2) {
+    const double2 w = v2[i / 2];
+    s0 = fma(col[i * ld], w.x, s0);
+    if (i + 1 < H) s1 = fma(col[(i + 1) * ld], w.y, s1);
+  }
+  return s0 + s1;
+}
+// acc[i] += M[k][i] f for one row k of a shared-memory matrix
+template <int H>
+__device__ __forceinline__ void axpy_row(double* acc, const double* row, const double f) {
+  const double2* r2 = reinterpret_cast<const double2*>(row);
+#pragma unroll
+  for (int i = 0; i < H; i += 2) {
+    const double2 m = r2[i / 2];
+    acc[i] = fma(m.x, f, acc[i]);
+    if (i + 1 < H) acc[i + 1] = fma(m.y, f, acc[i + 1]);
+  }
+}
+
+// The instances of one warp: team `team` solves chunk slot `slot` (-1: none).
+template <int N, bool GEN, bool SPH>
+__device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
+  using C = BCfg<N>;
+  constexpr int H = C::H, HP = C::HP, TEAM = C::TEAM, LDM = C::LDM, SB = C::SB;
+  constexpr bool ROLL = C::ROLL;
+  constexpr double PI = 3.14159265358979323846;
+  extern __shared__ double smem[];
+  const int t = threadIdx.x % TEAM;
+  const int j = t < H ? t : H - 1;  // lanes past the last column repeat it
+  const bool own = t < H;
+  double* const sm = smem + (threadIdx.x / TEAM) * C::STRIDE;
+  double* const Xs = sm + C::O_X;
+  double* const Ys = sm + C::O_Y;
+  double* const As = sm + C::O_A;
+  double* const Ws = sm + C::O_W;
+  double* const vec = sm + C::O_V;
+  double* const sbuf = sm + C::O_S;
+  double* const vg = sm + C::O_G;
+  double* const vw1 = vg + HP;
+  double* const vw2 = vw1 + HP;
+  double* const vgam = vw2 + HP;
+  double* const vsc = vgam + HP;
+  double* const ve = vsc + HP;  // E going down, phi going up
+  double* const vd = ve + HP;
+
+  const bool ifb = (p.flags & DSP_FLAG_INDEX_FROM_BOTTOM) != 0;
+  const int m = GEN ? p.g.m : 0;
+  // i: status / input / output index, L: layers, NT: output levels
+  const int sl = slot >= 0 ? slot : 0;
+  const int i = GEN ? p.g.ids[sl] : sl;
+  const int L = GEN ? p.g.Ls[i] : p.L;
+  const int NT = GEN ? (p.g.user_tau ? p.g.user_tau : L + 1) : L + 1;
+  const InstLayout il = GEN ? InstLayout::make(L, N) : p.il;
+  const double* const rec = p.inst_rec + (GEN ? p.g.inst_off[sl] : (long long)i * p.il.stride);
+  const long long lay0 = GEN ? p.g.lay_off[sl] : (long long)i * p.L;
+  const long long lstride = GEN ? p.g.lstride : (long long)lrec_stride(N);
+  const double* const lrec0 = p.layer_rec + lay0 * lstride;
+  double* const brec0 = p.bvp_rec + lay0 * brec_stride(N);
+  auto oidx = [&](int lev) {
+    if constexpr (GEN) return (long long)i * p.g.ntau_out + (ifb ? NT - 1 - lev : lev);
+    else return (long long)i * NT + (ifb ? L - lev : lev);
+  };
+  double* const* outp = GEN ? p.g.out_flux : p.out;
+  bool act = slot >= 0;
+  if (act) {
+    const int st0 = p.status ? p.status[i] : 0;
+    if (st0 == DSP_ERR_INVALID_INPUT || st0 == DSP_ERR_EIGEN) {
+      const double qnan = __longlong_as_double(0x7ff8000000000000ll);
+      if (m == 0)
+        for (int lev = t; lev < NT; lev += TEAM)
+          for (int f = 0; f < 8; ++f) outp[f][oidx(lev)] = qnan;
+      act = false;
+    }
+  }
+  if constexpr (GEN) {
+    if (act && (m > (int)rec[H_NAZ] || rec[H_DONE] != 0.0)) act = false;
+  }
+  const int ncut = act ? (int)rec[H_NCUT] : 0;
+  const int Lw = (int)__reduce_max_sync(0xffffffffu, (unsigned)ncut);
+  if (Lw == 0) return;
+  DSP_PHASE_BEGIN
+  const bool lyrcut = act && rec[H_LYRCUT] != 0.0;
+  // modes m > 0 carry the beam only (DisortSolver.cpp:1246-1250, 1693-1748)
+  const bool thermal = (p.flags & DSP_FLAG_THERMAL) != 0 && m == 0;
+  const bool dlbc = (p.flags & DSP_FLAG_DIFFUSION_LOWER_BC) != 0;
+  const double fbeam = act ? rec[H_FBEAM] : 0.0, umu0 = act ? rec[H_UMU0] : 1.0;
+  const bool beam = fbeam > 0.0;
+  const double* const taus = rec + il.tau_s;
+  const double* const btr = rec + il.btr;
+  const double* const dtau_s = rec + il.dtau_s;
+  const double dj = p.tables[tab_dsim(N) + j];
+  bool singular = false, sg = false;
+
+  // the layer record of layer l: X^T and the vectors, Y^T
+  auto load_x = [&](int l) {
+    if (l < ncut) {
+      const double* lr = lrec0 + (long long)l * lstride;
+      team_copy_rows_async<TEAM>(Xs, LDM, lr + mod_X(N), HP, H, HP, t);
+      team_copy_async<TEAM>(vec, lr + mod_k(N), C::NV, t);
+    }
+    cp_async_commit();
+  };
+  auto load_y = [&](int l) {
+    if (l < ncut) team_copy_rows_async<TEAM>(Ys, LDM, lrec0 + (long long)l * lstride + mod_Y(N), HP, H, HP, t);
+    cp_async_commit();
+  };
+  // per-layer scalars: dtau, scaled depths and beam factors of the two boundaries
+  struct Scal { double dt, t0, t1, b0, b1; };
+  auto load_s = [&](int l) {
+    Scal s{0.0, 0.0, 0.0, 0.0, 0.0};
+    if (l < ncut) {
+      s.dt = dtau_s[l];
+      s.t0 = taus[l];
+      s.t1 = taus[l + 1];
+      if (beam) {
+        s.b0 = btr[l];
+        s.b1 = btr[l + 1];
+      }
+    }
+    return s;
+  };
+  // pseudo-spherical beam: the record [c1 | d1 | xba | Chapman factor] of layer l
+  auto SR = [&](int l) { return p.sph + (lay0 + l) * sph_stride(N); };
+  // lane j's particular solution (c, d) at scaled depth tau of layer l; `bt` the
+  // beam factor there (computeBeamSourceSpherical's form when SPH)
+  auto particular = [&](int l, double tau, double bt, double& c, double& d) {
+    c = 0.0;
+    d = 0.0;
+    if (beam) {
+      if constexpr (SPH) {
+        const double* sr = SR(l < ncut ? l : 0);
+        const double e = exp(-sr[sph_xba(N)] * tau);
+        c = e * fma(sr[j], tau, vec[HP + j]);
+        d = e * fma(sr[H + j], tau, vec[2 * HP + j]);
+      } else {
+        c = vec[HP + j] * bt;
+        d = vec[2 * HP + j] * bt;
+      }
+    }
+    if (thermal) {
+      const double x0 = vec[5 * HP], x1 = vec[5 * HP + 1];
+      c = fma(vec[3 * HP + j], fma(x1, tau, x0), c);
+      d = fma(vec[4 * HP + j], x1, d);
+    }
+  };
+
+  // ------------------------------------------------------------------- down
+  load_x(0);
+  load_y(0);
+  Scal sc = load_s(0);
+  // odd h: the pad element of every gathered vector and row stays 0
+  if (own) {
+    for (int r = 0; r < HP; ++r) As[j * LDM + r] = r == j ? 1.0 : 0.0;
+    const double inc = m == 0 && act ? rec[H_FISOT] + rec[H_PTOP] : 0.0;
+    vg[j] = -2.0 * dj * inc;
+  }
+  if (HP != H && t == 0)
+    for (int v = 0; v < C::NG; ++v) vg[v * HP + H] = 0.0;
+  __syncwarp();
+
+  double a[H];
+  for (int l = 0; l < Lw; ++l) {
+    const bool on = l < ncut;
+    const Scal s = sc;
+    sc = load_s(l + 1);
+    cp_async_wait<1>();
+    __syncwarp();
+    const double k = vec[j];
+    const double ex = exp(-k * s.dt);
+    const double fx = -expm1(-2.0 * k * s.dt);
+    double ct, dt_, cb, db;
+    particular(l, s.t0, s.b0, ct, dt_);
+    particular(l, s.t1, s.b1, cb, db);
+    // I + M = I + X^T A X, column j
+    const double* xj = Xs + j * LDM;
+    double diag = 0.0;
+    {
+      double tv[H];
+#pragma unroll
+      for (int r = 0; r < H; ++r) tv[r] = 0.0;
+      if constexpr (ROLL) {
+#pragma unroll 2
+        for (int r = 0; r < H; ++r) axpy_row<H>(tv, As + r * LDM, xj[r]);
+      } else {
+#pragma unroll
+        for (int r = 0; r < H; ++r) axpy_row<H>(tv, As + r * LDM, xj[r]);
+      }
+      if constexpr (ROLL) {
+        __syncwarp();  // every lane is done with A
+#pragma unroll 2
+        for (int r = 0; r < H; ++r) As[r * LDM + j] = dot_reg<H>(tv, Xs + r * LDM);
+        diag = 1.0 + As[j * LDM + j];
+      } else {
+#pragma unroll
+        for (int r = 0; r < H; ++r) {
+          a[r] = dot_reg<H>(tv, Xs + r * LDM);
+          if (r == j) diag = 1.0 + a[r];
+        }
+      }
+    }
+    const double gam = dot_row<H>(xj, vg);
+    const double s1 = rsqrt(diag);
+    if (own) {
+      vw1[j] = gam - dt_ - ct;
+      vsc[j] = s1;
+      ve[j] = ex;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < H; ++r) {
+      const double v = ROLL ? As[r * LDM + j] : a[r];
+      a[r] = r == j ? 1.0 : v * (s1 * vsc[r]);
+    }
+    // X and the vectors are used up: the next layer's start loading
+    load_x(l + 1);
+    sweep_inverse<H, SB, ROLL>(a, j, own, sbuf, sg);
+    double* const br = brec0 + (long long)(on ? l : 0) * brec_stride(N);
+#pragma unroll
+    for (int r = 0; r < H; ++r) {
+      a[r] = -a[r] * (s1 * vsc[r]);
+      if (on && own) br[brec_H(N) + r * HP + j] = a[r];
+    }
+    const double rj = ct + dot_reg<H>(a, vw1);
+    if (on && own) br[brec_r(N) + j] = rj;
+    const double q = ex * rj;
+    // Z = (1 - E^2) + 2 E H E
+    const double ex2 = 2.0 * ex;
+#pragma unroll
+    for (int r = 0; r < H; ++r) {
+      a[r] *= ex2 * ve[r];
+      if (r == j) {
+        a[r] += fx;
+        diag = a[r];
+      }
+    }
+    const double s2 = rsqrt(diag);
+    __syncwarp();  // every lane has read the first scale
+    if (own) {
+      vsc[j] = s2;
+      vw2[j] = q - cb;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < H; ++r) a[r] = r == j ? 1.0 : a[r] * (s2 * vsc[r]);
+    sweep_inverse<H, SB, ROLL>(a, j, own, sbuf, sg);
+    if (on && sg) singular = true;
+    sg = false;
+#pragma unroll
+    for (int r = 0; r < H; ++r) {
+      a[r] = -a[r] * (s2 * vsc[r]);
+      if (on && own) br[brec_G(N) + r * HP + j] = a[r];
+    }
+    const double gb = cb + db + 2.0 * dot_reg<H>(a, vw2);
+    if (own) {
+      vgam[j] = gb;
+#pragma unroll
+      for (int r = 0; r < H; ++r) Ws[j * LDM + r] = r == j ? fma(2.0, a[r], -1.0) : 2.0 * a[r];
+    }
+    cp_async_wait<1>();  // Y of this layer
+    __syncwarp();
+    // A' = Y (2 G - I) Y^T, column j; g' = Y gamma'
+    {
+      double tv[H];
+#pragma unroll
+      for (int r = 0; r < H; ++r) tv[r] = 0.0;
+#pragma unroll(ROLL ? 2 : H)
+      for (int r = 0; r < H; ++r) axpy_row<H>(tv, Ws + r * LDM, Ys[r * LDM + j]);
+      const double gn = dot_col<H>(Ys + j, LDM, vgam);
+      double w[H];
+#pragma unroll
+      for (int r = 0; r < H; ++r) w[r] = 0.0;
+      if constexpr (ROLL) {
+        __syncwarp();  // every lane is done with the work matrix
+#pragma unroll
+        for (int r = 0; r < H; ++r) Ws[r * LDM + j] = tv[r];
+#pragma unroll 2
+        for (int r = 0; r < H; ++r) axpy_row<H>(w, Ys + r * LDM, Ws[r * LDM + j]);
+      } else {
+#pragma unroll
+        for (int r = 0; r < H; ++r) axpy_row<H>(w, Ys + r * LDM, tv[r]);
+      }
+      if (on && own) {
+#pragma unroll
+        for (int r = 0; r < H; ++r) As[j * LDM + r] = w[r];
+        vg[j] = gn;
+      }
+    }
+    __syncwarp();
+    load_y(l + 1);
+  }
+  cp_async_wait<0>();
+  __syncwarp();
+  DSP_PHASE(20)
+
+  // ----------------------------------------------------------------- surface
+  // up = R down + src at the bottom, psi = A phi + g:
+  // [(I - R) + (I + R) A] phi = 2 src - (I + R) g.
+  const double* sft = nullptr;
+  if constexpr (GEN)
+    if (p.g.brdf && !lyrcut && !dlbc) sft = p.g.brdf + (long long)sl * brdf_stride(N, p.g.numu);
+  const double alb = m == 0 && act && !lyrcut && !dlbc && !sft ? rec[H_ALB] : 0.0;
+  double* const bl = brec0 + (long long)(ncut > 0 ? ncut - 1 : 0) * brec_stride(N);  // the last layer's record
+  // pseudo-spherical beam: the reference reflects Z0 times the beam factor at the
+  // user angles (DisortSolver.cpp:3180-3218), not the solution at that depth; the
+  // difference, in the downward intensities at the bottom
+  double ddn = 0.0;
+  if constexpr (GEN && SPH) {
+    double dc = 0.0, dd = 0.0;
+    if (act && beam) {
+      const double* sr = SR(ncut - 1);
+      const double tau = taus[ncut], e = exp(-sr[sph_xba(N)] * tau), bt = btr[ncut];
+      dc = vec[HP + j] * bt - e * fma(sr[j], tau, vec[HP + j]);
+      dd = vec[2 * HP + j] * bt - e * fma(sr[H + j], tau, vec[2 * HP + j]);
+    }
+    if (own) {
+      vw1[j] = dc;
+      vw2[j] = dd;
+    }
+    __syncwarp();
+    ddn = 0.5 * (dot_col<H>(Xs + j, LDM, vw1) - dot_col<H>(Ys + j, LDM, vw2)) / dj;
+    __syncwarp();
+  }
+  {
+    // lane j's surface source (setMatrix :909-958, solve0 :993-1076)
+    double src = 0.0;
+    if (act) {
+      const double fisob = m == 0 ? rec[H_FISOB] : 0.0, pbot = m == 0 ? rec[H_PBOT] : 0.0;
+      if (dlbc) {
+        src = pbot + p.tables[tab_mu(N) + j] * (m == 0 ? rec[H_PBOTD] : 0.0);
+      } else {
+        const double* srow = sft ? sft + j * brdf_row(N) : nullptr;
+        if (!lyrcut && beam) src += (srow ? srow[0] : alb) * umu0 * fbeam * btr[ncut] / PI;
+        src += fisob;
+        if (thermal) src += (srow ? srow[H + 1] : 1.0 - alb) * pbot;
+      }
+    }
+    const double sh = dj * src;
+    if (own) {
+      vw1[j] = sh;
+      vw2[j] = dj;
+    }
+    __syncwarp();
+    double rhs;
+    if (!__any_sync(0xffffffffu, sft != nullptr)) {
+      // Lambertian: (I + R)^{-1} (I - R) = I - 4 alb/(1 + alb) d d^T, so the
+      // system is symmetric positive definite
+      const double f = alb / (1.0 + alb);
+      double dsrc = 0.0, diag = 0.0;
+#pragma unroll
+      for (int r = 0; r < H; ++r) {
+        dsrc = fma(vw2[r], vw1[r], dsrc);
+        a[r] = As[j * LDM + r] - 4.0 * f * dj * vw2[r];
+        if (r == j) {
+          a[r] += 1.0;
+          diag = a[r];
+        }
+      }
+      rhs = 2.0 * (sh - 2.0 * f * dj * dsrc) - vg[j];
+      const double s1 = rsqrt(diag);
+      __syncwarp();
+      if (own) {
+        vsc[j] = s1;
+        vw1[j] = rhs;
+      }
+      __syncwarp();
+#pragma unroll
+      for (int r = 0; r < H; ++r) a[r] = r == j ? 1.0 : a[r] * (s1 * vsc[r]);
+      sweep_inverse<H, SB, ROLL>(a, j, own, sbuf, singular);
+#pragma unroll
+      for (int r = 0; r < H; ++r) {
+        a[r] = -a[r] * (s1 * vsc[r]);
+        if (act && own) bl[brec_inv(N) + r * HP + j] = a[r];
+      }
+    } else {
+      // bidirectional surface: R_rc = (1 + delta_m0) d_r rho_rc d_c, not
+      // symmetric in general; Gauss-Jordan inverse with row pivoting, column j
+      // of [B | I] in the lane (B in shared memory for the pivot search)
+      const double cpl = m == 0 ? 2.0 : 1.0;
+      auto R = [&](int r, int c) { return sft ? cpl * vw2[r] * sft[r * brdf_row(N) + 1 + c] * vw2[c] : 0.0; };
+      rhs = 2.0 * sh - vg[j];
+      for (int c = 0; c < H; ++c) rhs -= R(j, c) * vg[c];
+      for (int r = 0; r < H; ++r) {
+        double v = As[r * LDM + j] + (r == j ? 1.0 : 0.0) - R(r, j);
+        for (int c = 0; c < H; ++c) v = fma(R(r, c), As[c * LDM + j], v);
+        if (own) Ws[r * LDM + j] = v;
+      }
+      __syncwarp();
+      if (own)
+        for (int r = 0; r < H; ++r) Xs[r * LDM + j] = r == j ? 1.0 : 0.0;
+      if (own) vw1[j] = rhs;
+      __syncwarp();
+      for (int k = 0; k < H; ++k) {
+        // the largest |B[r][k]|, r >= k (every lane runs the same search)
+        int pr = k;
+        double best = fabs(Ws[k * LDM + k]);
+        for (int r = k + 1; r < H; ++r) {
+          const double v = fabs(Ws[r * LDM + k]);
+          if (v > best) {
+            best = v;
+            pr = r;
+          }
+        }
+        __syncwarp();
+        if (own && pr != k) {
+          const double w0 = Ws[k * LDM + j], x0 = Xs[k * LDM + j];
+          Ws[k * LDM + j] = Ws[pr * LDM + j];
+          Ws[pr * LDM + j] = w0;
+          Xs[k * LDM + j] = Xs[pr * LDM + j];
+          Xs[pr * LDM + j] = x0;
+        }
+        __syncwarp();
+        const double d = Ws[k * LDM + k];
+        if (d == 0.0) singular = true;
+        const double pv = d == 0.0 ? 0.0 : 1.0 / d;
+        const double wk = Ws[k * LDM + j] * pv, xk = Xs[k * LDM + j] * pv;
+        // columns <= k of B are finished (unit columns); the others and the inverse update
+        for (int r = 0; r < H; ++r) {
+          if (r == k) continue;
+          const double f = Ws[r * LDM + k];
+          if (own) {
+            if (j > k) Ws[r * LDM + j] -= f * wk;
+            Xs[r * LDM + j] -= f * xk;
+          }
+        }
+        __syncwarp();
+        if (own) {
+          if (j > k) Ws[k * LDM + j] = wk;
+          Xs[k * LDM + j] = xk;
+        }
+        __syncwarp();
+      }
+      // lane j: row j of the inverse (phi_j = sum_c Binv[j][c] rhs_c)
+#pragma unroll
+      for (int c = 0; c < H; ++c) {
+        a[c] = Xs[j * LDM + c];
+        if (act && own) bl[brec_inv(N) + c * HP + j] = a[c];
+      }
+    }
+    __syncwarp();
+    const double phi = dot_reg<H>(a, vw1);
+    if (own) ve[j] = phi;
+    __syncwarp();
+    // downward intensities at the bottom, for the reflected field at the user angles
+    if constexpr (GEN) {
+      const double psi = dot_row<H>(As + j * LDM, ve) + vg[j];
+      if (act && own) bl[brec_dn(N) + j] = 0.5 * (phi - psi) / dj + ddn;
+    }
+    __syncwarp();
+  }
+  DSP_PHASE(21)
+
+  // --------------------------------------------------------------------- up
+  bool nonfinite = false;
+  auto ssa_of = [&](int l) {
+    const int lin = ifb ? L - 1 - l : l;
+    return GEN ? p.g.ssa[p.g.in_off[i] + lin] : p.ssa(i, lin);
+  };
+  // fluxes at output level lu of layer l from the modal amplitudes (c, d) of the
+  // homogeneous part there (computeFluxes, FluxSolver.cpp:1138-1287;
+  // DisortSolver.cpp:1980-2124); `put`: this team has the level
+  auto eval_level = [&](int l, int lu, double utaupr, double utau, double c, double d, bool put) {
+    const double ch = SPH && beam && put ? SR(l)[sph_ch(N)] : 1.0;
+    const double fact = beam ? exp(-utaupr / (SPH ? ch : umu0)) : 0.0;
+    double cp, dp;
+    particular(l, utaupr, fact, cp, dp);
+    __syncwarp();
+    if (own) {
+      vgam[j] = c + cp;
+      vd[j] = d + dp;
+    }
+    __syncwarp();
+    const double ph = dot_col<H>(Xs + j, LDM, vgam), ps = dot_col<H>(Ys + j, LDM, vd);
+    const double wd = own ? 0.5 * p.tables[tab_wt(N) + j] / dj : 0.0, md = own ? p.tables[tab_mu(N) + j] : 0.0;
+    double su = wd * (ph + ps), sd = wd * (ph - ps);
+    double fu = md * su, fd = md * sd;
+#pragma unroll
+    for (int off = TEAM / 2; off > 0; off >>= 1) {
+      su += __shfl_xor_sync(0xffffffffu, su, off);
+      sd += __shfl_xor_sync(0xffffffffu, sd, off);
+      fu += __shfl_xor_sync(0xffffffffu, fu, off);
+      fd += __shfl_xor_sync(0xffffffffu, fd, off);
+    }
+    if (put) {
+      double dirint = 0.0, fldir = 0.0, fdir = 0.0;
+      if (beam) {
+        dirint = fbeam * fact;
+        fldir = umu0 * fbeam * fact;
+        fdir = SPH ? fabs(umu0) * fbeam * exp(-utau / ch) : umu0 * fbeam * exp(-utau / umu0);
+      }
+      fu *= 2.0 * PI;
+      fd *= 2.0 * PI;
+      const double fdn = (fd + fldir) - fdir;
+      const double ua = (2.0 * PI * (su + sd) + dirint) / (4.0 * PI);
+      const double uaso = dirint / (4.0 * PI);
+      const double uad = 0.5 * sd, uau = 0.5 * su;
+      const double plsorc = thermal ? fma(vec[5 * HP + 1], utaupr, vec[5 * HP]) : 0.0;
+      const double dfdt = (1.0 - ssa_of(l)) * 4.0 * PI * (ua - plsorc);
+      const double o[8] = {fdir, fdn, fu, dfdt, ua, uad, uau, uaso};
+#pragma unroll
+      for (int f = 0; f < 8; ++f)
+        if ((f & (TEAM - 1)) == t) {
+          outp[f][oidx(lu)] = o[f];
+          if (!isfinite(o[f])) nonfinite = true;
+        }
+    }
+  };
+  const GenLayout gly = GenLayout::make(GEN ? L : 0, N, GEN ? NT : 0);
+  const double* const utau_l = rec + gly.utau;
+  const double* const utaus_l = rec + gly.utaus;
+  const double* const lyr_l = rec + gly.lyr;
+  // levels below the absorption cut carry zeros (computeFluxes :1151-1163;
+  // DisortSolver.cpp:1998-2009)
+  if constexpr (!GEN) {
+    for (int lev = ncut + 1 + t; act && lev <= L; lev += TEAM)
+      for (int f = 0; f < 8; ++f) outp[f][oidx(lev)] = 0.0;
+  } else {
+    if (m == 0)
+      for (int lu = t; act && lu < NT; lu += TEAM)
+        if ((int)lyr_l[lu] > ncut - 1)
+          for (int f = 0; f < 8; ++f) outp[f][oidx(lu)] = 0.0;
+  }
+  const int NTw = GEN && m == 0 ? (int)__reduce_max_sync(0xffffffffu, act ? (unsigned)NT : 0u) : 0;
+  auto load_up = [&](int l, int what) {
+    if (l >= 0 && l < ncut) {
+      const double* lr = lrec0 + (long long)l * lstride;
+      const double* br = brec0 + (long long)l * brec_stride(N);
+      if (what == 0) {
+        team_copy_rows_async<TEAM>(Ys, LDM, lr + mod_Y(N), HP, H, HP, t);
+        team_copy_rows_async<TEAM>(Xs, LDM, lr + mod_X(N), HP, H, HP, t);
+        team_copy_async<TEAM>(vec, lr + mod_k(N), C::NV, t);
+      } else {
+        team_copy_rows_async<TEAM>(Ws, LDM, br + brec_G(N), HP, H, HP, t);  // G
+        team_copy_rows_async<TEAM>(As, LDM, br + brec_H(N), HP, H, HP, t);  // H
+      }
+    }
+    cp_async_commit();
+  };
+  load_up(Lw - 1, 0);
+  load_up(Lw - 1, 1);
+  sc = load_s(Lw - 1);
+  double r_next = Lw - 1 < ncut && own ? brec0[(long long)(Lw - 1) * brec_stride(N) + brec_r(N) + j] : 0.0;
+  for (int l = Lw - 1; l >= 0; --l) {
+    const bool on = l < ncut;
+    const Scal s = sc;
+    const double rj = r_next;
+    if (l > 0) {
+      sc = load_s(l - 1);
+      r_next = l - 1 < ncut && own ? brec0[(long long)(l - 1) * brec_stride(N) + brec_r(N) + j] : 0.0;
+    }
+    cp_async_wait<0>();
+    __syncwarp();
+    const double k = vec[j];
+    const double ex = exp(-k * s.dt);
+    double ct, dt_, cb, db;
+    particular(l, s.t0, s.b0, ct, dt_);
+    particular(l, s.t1, s.b1, cb, db);
+    const double chom_b = dot_row<H>(Ys + j * LDM, ve) - cb;  // homogeneous C at the bottom
+    if (own) vw1[j] = fma(ex, rj, chom_b);
+    __syncwarp();
+    const double b = dot_col<H>(Ws + j, LDM, vw1);
+    if (own) vw2[j] = ex * b;
+    __syncwarp();
+    const double c = fma(2.0, dot_col<H>(As + j, LDM, vw2), -rj);  // homogeneous C at the top
+    const double av = c - ex * b;
+    if (own) vw1[j] = c + ct;
+    __syncwarp();
+    // G and H are used up
+    load_up(l - 1, 1);
+    const double phi = dot_col<H>(Xs + j, LDM, vw1);
+    if constexpr (GEN) {
+      if (on && own) {
+        double* cc = p.g.cc + (lay0 + l) * N;
+        cc[j] = b;
+        cc[H + j] = av;
+      }
+      if (m == 0) {
+        const double fx = -expm1(-2.0 * k * s.dt);
+        for (int lu = 0; lu < NTw; ++lu) {
+          const bool put = on && lu < NT && (int)lyr_l[lu] == l;
+          if (!__any_sync(0xffffffffu, put)) continue;
+          const double tu = put ? utaus_l[lu] : s.t0, x1 = tu - s.t0, x2 = s.t1 - tu;
+          const double e1 = exp(-k * x1), e2 = exp(-k * x2);
+          // C inside the layer from its values at the two boundaries (no cancellation)
+          double cu = c;
+          if (fx > 0.0) cu = (c * (e1 * -expm1(-2.0 * k * x2)) + chom_b * (e2 * -expm1(-2.0 * k * x1))) / fx;
+          eval_level(l, lu, tu, put ? utau_l[lu] : 0.0, cu, e2 * b - e1 * av, put);
+        }
+      }
+    } else {
+      eval_level(l, l + 1, s.t1, on ? rec[il.tauc + l + 1] : 0.0, chom_b, b - ex * av, on);
+      if (l == 0) eval_level(0, 0, s.t0, on ? rec[il.tauc] : 0.0, c, ex * b - av, on);
+    }
+    __syncwarp();
+    if (on && own) ve[j] = phi;
+    load_up(l - 1, 0);
+    __syncwarp();
+  }
+  cp_async_wait<0>();
+  DSP_PHASE(22)
+  DSP_PHASE_END
+  if (act) {
+    if (singular && t == 0) set_status(p.status, i, DSP_ERR_SINGULAR);
+    if (nonfinite) set_status(p.status, i, DSP_ERR_NONFINITE);
+  }
+}
+
+// One team per instance, in chunk-slot order.
+template <int N, bool GEN = false, bool SPH = false>
+__global__ void __launch_bounds__(32, BCfg<N>::MINB) flux_bvp_kernel(FluxParams p) {
+  using C = BCfg<N>;
+  const int slot = blockIdx.x * C::TPW + threadIdx.x / C::TEAM;
+  bvp_warp<N, GEN, SPH>(p, slot < p.n ? slot : -1);
+}
+
+// Persistent form (general solver): a resident grid whose warps take chunk slots
+// from a work queue -- `order`, the chunk's slots by descending layer count (the
+// size classes), consumed through the counter `head` -- so that the longest
+// instances start first, the instances of a warp have about the same depth and
+// the tail of the launch is short.
+template <int N, bool SPH = false>
+__global__ void __launch_bounds__(32, BCfg<N>::MINB) gen_bvp_persistent_kernel(FluxParams p, const int* order, int* head) {
+  using C = BCfg<N>;
+  for (;;) {
+    int k = 0;
+    if (threadIdx.x == 0) k = atomicAdd(head, C::TPW);
+    k = __shfl_sync(0xffffffffu, k, 0);
+    if (k >= p.n) break;
+    k += threadIdx.x / C::TEAM;
+    bvp_warp<N, true, SPH>(p, k < p.n ? order[k] : -1);
+    __syncwarp();  // the shared memory serves the next instances
+  }
+}
+
+}  // namespace dsp

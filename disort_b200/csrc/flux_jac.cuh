@@ -1,29 +1,22 @@
-// flux_jac.cuh — temperature Jacobians of the flux path (compute_temperature_jacobian).
+// flux_jac.cuh — temperature Jacobians (compute_temperature_jacobian), flux and
+// general path.
 //
-// Replaces computeThermalJacobian (FluxSolver.cpp:1294-1497) and the derivative
-// sources of computeIsotropicSource (:786-829).  The reference solves
-// A dC = dB_k with the band LU that solve0 left, for every level-Planck degree
-// of freedom k = 0..L and the surface, then propagates dC through the flux
-// formulas and chains with dB/dT.
+// Replaces computeThermalJacobian (FluxSolver.cpp:1294-1497, DisortSolver.cpp:
+// 2130-2358) and the derivative sources of computeIsotropicSource (:786-829).  The
+// reference solves A dC = dB_k with the band LU that solve0 left, for every
+// level-Planck degree of freedom k = 0..L and the surface, then propagates dC
+// through the flux formulas and chains with dB/dT.
 //
-// Here the boundary-value kernels, in their Jacobian form, record the
-// elimination itself: per layer and pivot column the multiplier applied to
-// every panel slot and the pivot slot (jrec_stride), next to the pivot rows
-// [U | V | c] they always keep.  flux_jac_kernel replays that elimination on
-// the L + 2 right-hand sides of the Jacobian, one CTA per instance and one
-// thread per degree of freedom:
-//  - going down, each thread keeps the right-hand side value of every panel
-//    slot of its column in shared memory; new rows enter the free slots in slot
-//    order exactly as in the elimination, pivot rows leave with their value
-//    (row c's right-hand side, stored per layer), and every pivot adds
-//    multiplier x pivot value to the other slots;
-//  - going up, U_l x_l = c_l - V_l x_{l+1} per column, and at each level the
-//    six outputs of the column (homogeneous part G (x o e) plus the derivative
-//    of the thermal particular solution), times dB/dT of its temperature.
-// The derivative sources come from the layer stage's P and Q (jpq_stride):
-// Z1 = xr1 P / 2 and Z0 = (xr0 P +/- xr1 Q) / 2, so a layer's source derivative
-// with respect to its top / bottom level Planck value is P, Q weighted by the
-// derivatives of its intercept xr0 and slope xr1 (FluxSolver.cpp:789-806).
+// Here the boundary-value kernel has left, per layer, the matrices X, Y (layer
+// record), H, G and the inverse of the surface system (flux_bvp.cuh): the
+// solution for further sources is its two vector recursions,
+//   down  r = c_t + H (X^T g - d - c_t),  q = E r,  g' = Y (c_b + d + 2 G (q - c_b)),
+//   up    b = G (Y^T phi_b - c_b + q),  c = 2 H E b - r,  phi_t = X (c + c_t),
+// one CTA per instance and one thread per degree of freedom, the matrices read
+// uniformly across the CTA.  The thermal source of a degree of freedom enters at
+// the two layers next to its level: the derivatives of the source's value at the
+// layer's top and of its slope (FluxSolver.cpp:789-806) times the record's thermal
+// (c, d).
 #pragma once
 
 #include "dsp_device.cuh"
@@ -57,18 +50,15 @@ static __device__ double planck_deriv2(double lo, double hi, double T, const Pla
 
 template <int N>
 struct JCfg {
-  static constexpr int NN = N / 2;
-  static constexpr int PR = 3 * NN;  // panel slots
+  static constexpr int H = N / 2, HP = mod_hp(N);
   static constexpr int KB = 64;      // degrees of freedom per pass (threads per CTA)
-  // shared memory (doubles): slot values [PR][KB] going down, x_l and x_{l+1}
-  // [2][N][KB] going up (the same area), exp factors of one level [N]
-  static constexpr int O_R = 0;
-  static constexpr int R_SIZE = (PR > 2 * N ? PR : 2 * N) * KB;
-  static constexpr int O_EX = O_R + R_SIZE;
-  static constexpr int O_TAB = O_EX + N;  // mu[N], wt[N]
-  static constexpr int SMEM = O_TAB + 2 * N;
+  // shared memory (doubles): two vectors of every thread [2][h][KB], then the
+  // quadrature vectors of the fluxes and E of the layer
+  static constexpr int O_V = 0;
+  static constexpr int O_Q = 2 * H * KB;  // dsim, w/(2d), w mu/(2d) [h] each
+  static constexpr int O_E = O_Q + 3 * H;
+  static constexpr int SMEM = O_E + 3 * H;  // E, e1, e2
   static constexpr size_t smem_bytes() { return sizeof(double) * (size_t)SMEM; }
-  static constexpr int NW = (PR + 31) / 32;
 };
 
 // GEN: the general path (mode 0 of a ragged chunk): outputs at the instance's
@@ -76,51 +66,37 @@ struct JCfg {
 template <int N, bool GEN = false>
 __global__ void __launch_bounds__(64) flux_jac_kernel(FluxParams p, JacView jv) {
   using C = JCfg<N>;
-  constexpr int NN = C::NN, PR = C::PR, KB = C::KB, NW = C::NW;
+  constexpr int H = C::H, HP = C::HP, KB = C::KB;
   constexpr double PI = 3.14159265358979323846;
   extern __shared__ double smem[];
-  double* Rv = smem + C::O_R;
-  double* ex = smem + C::O_EX;
-  double* mu = smem + C::O_TAB;
-  double* wt = smem + C::O_TAB + N;
   const int tid = threadIdx.x;
-  for (int k = tid; k < 2 * N; k += KB) smem[C::O_TAB + k] = p.tables[k];  // tab_mu, tab_wt
+  double* const dsv = smem + C::O_Q;
+  double* const wv = dsv + H;
+  double* const mv = wv + H;
+  double* const Ev = smem + C::O_E;
+  double* const e1v = Ev + H;
+  double* const e2v = e1v + H;
+  for (int r = tid; r < H; r += KB) {
+    const double d = p.tables[tab_dsim(N) + r];
+    dsv[r] = d;
+    wv[r] = 0.5 * p.tables[tab_wt(N) + r] / d;
+    mv[r] = 0.5 * d;  // w mu / (2 d), d^2 = w mu
+  }
   __syncthreads();
   const int slot = blockIdx.x;  // chunk-local instance
   if (slot >= p.n) return;
   // i: batch index; L: layers; NT: output depths; cvs: column stride of cv
-  int i, L, NT;
-  const double *rec, *lrec0, *brec0, *jrec0, *pq0;
-  double* cv0;
-  InstLayout il_gen;
-  long long lstride;
+  const int i = GEN ? p.g.ids[slot] : slot;
+  const int L = GEN ? p.g.Ls[i] : p.L;
+  const int NT = GEN ? (p.g.user_tau ? p.g.user_tau : L + 1) : L + 1;
+  const InstLayout il = GEN ? InstLayout::make(L, N) : p.il;
+  const double* const rec = p.inst_rec + (GEN ? p.g.inst_off[slot] : (long long)i * p.il.stride);
+  const long long l0 = GEN ? p.g.lay_off[slot] : (long long)i * p.L;
+  const long long lstride = GEN ? p.g.lstride : (long long)lrec_stride(N);
+  const double* const lrec0 = p.layer_rec + l0 * lstride;
+  const double* const brec0 = p.bvp_rec + l0 * brec_stride(N);
   const int cvs = jv.ndof;
-  if constexpr (GEN) {
-    i = p.g.ids[slot];
-    L = p.g.Ls[i];
-    NT = p.g.user_tau ? p.g.user_tau : L + 1;
-    il_gen = InstLayout::make(L, N);
-    rec = p.inst_rec + p.g.inst_off[slot];
-    const long long l0 = p.g.lay_off[slot];
-    lstride = p.g.lstride;
-    lrec0 = p.layer_rec + l0 * lstride;
-    brec0 = p.bvp_rec + l0 * brec_stride(N);
-    jrec0 = p.jac_rec + l0 * jrec_stride(N);
-    pq0 = p.jac_pq + l0 * jpq_stride(N);
-    cv0 = jv.cv + l0 * N * cvs;
-  } else {
-    i = slot;
-    L = p.L;
-    NT = L + 1;
-    rec = p.inst_rec + (long long)i * p.il.stride;
-    lstride = lrec_stride(N);
-    lrec0 = p.layer_rec + (long long)i * L * lstride;
-    brec0 = p.bvp_rec + (long long)i * L * brec_stride(N);
-    jrec0 = p.jac_rec + (long long)i * L * jrec_stride(N);
-    pq0 = p.jac_pq + (long long)i * L * jpq_stride(N);
-    cv0 = jv.cv + (long long)i * L * N * cvs;
-  }
-  const InstLayout& il = GEN ? il_gen : p.il;
+  double* const cv0 = jv.cv + l0 * H * cvs;
   const int ndof = L + 2;
   const bool ifb = (p.flags & DSP_FLAG_INDEX_FROM_BOTTOM) != 0;
   auto store = [&](int f, int lu, int k, double v) {
@@ -140,8 +116,8 @@ __global__ void __launch_bounds__(64) flux_jac_kernel(FluxParams p, JacView jv) 
     }
     return;
   }
-  const double* taus = rec + il.tau_s;
-  const double* dtau_s = rec + il.dtau_s;
+  const double* const taus = rec + il.tau_s;
+  const double* const dtau_s = rec + il.dtau_s;
   // output depth lu: its layer and scaled depth (general path: the user depths)
   const GenLayout gl_ = GenLayout::make(L, N, NT);
   auto out_layer = [&](int lu) { return GEN ? (int)rec[gl_.lyr + lu] : (lu == 0 ? 0 : lu - 1); };
@@ -154,219 +130,206 @@ __global__ void __launch_bounds__(64) flux_jac_kernel(FluxParams p, JacView jv) 
   if constexpr (GEN)
     if (p.g.brdf) sft = p.g.brdf + (long long)blockIdx.x * brdf_stride(N, p.g.numu);
   const double wlo = p.wlo(i), whi = p.whi(i);
-  const double* temp_in = GEN ? p.g.temp + p.g.in_off[i] + i : p.temp.row(i);
+  const double* const temp_in = GEN ? p.g.temp + p.g.in_off[i] + i : p.temp.row(i);
   const double dtau_last = dtau_s[L - 1];
-  // row width and 1/pivot position of the elimination record (flux_bvp_reg /
-  // flux_bvp_tile layouts)
-  constexpr int RL = N <= 16 ? 2 * N + 2 : 2 * N + 1;
-  auto rdiag = [&](const double* br, int c) { return N <= 16 ? br[c * RL + 2 * N + 1] : br[N * RL + c]; };
+  const double* const inv = brec0 + (long long)(L - 1) * brec_stride(N) + brec_inv(N);
 
   for (int k0 = 0; k0 < ndof; k0 += KB) {
     const int k = k0 + tid;
     const bool act = k < ndof;
-    // derivative coefficients of layer lc's intercept (a0) and slope (a1) with
-    // respect to degree of freedom k (FluxSolver.cpp:792-800)
+    // derivative of layer lc's thermal source with respect to degree of freedom
+    // k: its value at the layer's top (a0) and its slope (a1) (FluxSolver.cpp:792-800)
     auto coef = [&](int lc, double& a0, double& a1) {
-      a0 = 0.0;
+      a0 = k == lc ? 1.0 : 0.0;
       a1 = 0.0;
-      if (k != lc && k != lc + 1) return;
-      const double dts = dtau_s[lc], tc = taus[lc];
-      double d1t = 0.0, d1b = 0.0;
-      if (dts > 1e-4) {
-        d1t = -1.0 / dts;
-        d1b = 1.0 / dts;
-      }
-      if (k == lc) {
-        a0 += 1.0 - d1t * tc;
-        a1 += d1t;
-      }
-      if (k == lc + 1) {
-        a0 += -d1b * tc;
-        a1 += d1b;
-      }
+      const double dts = dtau_s[lc];
+      if ((k == lc || k == lc + 1) && dts > 1e-4) a1 = (k == lc ? -1.0 : 1.0) / dts;
     };
-    // derivative of the thermal source of layer lc at stream iq: z0 and z1 parts
-    auto dz = [&](int lc, int iq, double a0, double a1, double& d0, double& d1) {
-      if (a0 == 0.0 && a1 == 0.0) {
-        d0 = 0.0;
-        d1 = 0.0;
-        return;
-      }
-      const double* pq = pq0 + (long long)lc * jpq_stride(N);
-      const bool upper = iq >= NN;
-      const int r = upper ? iq - NN : NN - 1 - iq;
-      const double P = pq[r], Q = pq[NN + r];
-      d1 = 0.5 * (a1 * P);
-      d0 = upper ? 0.5 * (a0 * P + a1 * Q) : 0.5 * (a0 * P - a1 * Q);
-    };
+    double* const u = smem + C::O_V + tid;  // this thread's vectors, element r at u[r * KB]
+    double* const w = u + H * KB;
 
-    // ---- down: replay the elimination on this column's right-hand side ----
-    double* R = Rv + tid;  // slot s at R[s * KB]
-    for (int s = 0; s < PR; ++s) R[s * KB] = 0.0;
-    uint32_t carried[NW];
-#pragma unroll
-    for (int w = 0; w < NW; ++w) carried[w] = 0u;
-    for (int s = 0; s < NN; ++s) carried[s >> 5] |= 1u << (s & 31);
-    {
-      // top boundary rows, slot s = row NN-1-s of the source (solve0 :978-990)
-      double a0, a1;
-      coef(0, a0, a1);
-      for (int s = 0; s < NN; ++s) {
-        double d0, d1;
-        dz(0, NN - 1 - s, a0, a1, d0, d1);
-        R[s * KB] = -d0;
-      }
-    }
+    // ---- down: g in u --------------------------------------------------------
+    for (int r = 0; r < H; ++r) u[r * KB] = 0.0;
     for (int l = 0; l < L; ++l) {
-      const bool last = l == L - 1;
-      const int nnew = last ? NN : N;
-      double b0, b1, n0 = 0.0, n1 = 0.0;
-      coef(l, b0, b1);
-      if (!last) coef(l + 1, n0, n1);
-      uint32_t cand[NW];
-      int rank = 0;
-      for (int s = 0; s < PR; ++s) {
-        const bool isc = (carried[s >> 5] >> (s & 31)) & 1u;
-        if (isc || rank >= nnew) continue;
-        // new row `rank` in slot s
-        double v;
-        if (!last) {
-          // continuity row jq of interface (l, l+1) (solve0 :1080-1104)
-          const int jq = rank;
-          double dl0, dl1, dn0, dn1;
-          dz(l, jq, b0, b1, dl0, dl1);
-          dz(l + 1, jq, n0, n1, dn0, dn1);
-          v = dn0 - dl0 + (dn1 - dl1) * taus[l + 1];
-        } else {
-          // bottom boundary row rb (FluxSolver.cpp:1437-1461, 1477-1492)
-          const int rb = rank;
-          const double tb = taus[L];
-          if (k == L + 1) {  // the surface temperature
-            if (dlbc) {
-              v = 1.0;
-              if (dtau_last > 0.0) v += mu[rb] * (1.0 / dtau_last);
-            } else {
-              v = sft ? sft[rb * brdf_row(N) + NN + 1] : 1.0 - alb;
-            }
-          } else {
-            double d0, d1;
-            dz(l, NN + rb, b0, b1, d0, d1);
-            if (dlbc) {
-              v = -d0 - d1 * tb;
-              if (k == L - 1 && dtau_last > 0.0) v += mu[rb] * (-1.0 / dtau_last);
-            } else {
-              double refl = 0.0;
-              for (int jq = 0; jq < NN; ++jq) {
-                double e0, e1;
-                dz(l, NN - 1 - jq, b0, b1, e0, e1);
-                refl += wt[jq] * mu[jq] * (sft ? sft[rb * brdf_row(N) + 1 + jq] : alb) * (e0 + e1 * tb);
-              }
-              v = 2.0 * refl;
-              v -= d0 + d1 * tb;
-            }
-          }
-        }
-        R[s * KB] = v;
-        carried[s >> 5] |= 1u << (s & 31);  // now a candidate
-        ++rank;
-      }
+      const double* lr = lrec0 + (long long)l * lstride;
+      const double* br = brec0 + (long long)l * brec_stride(N);
+      double* cvl = cv0 + (long long)l * H * cvs;
+      __syncthreads();
+      for (int r = tid; r < H; r += KB) Ev[r] = exp(-lr[mod_k(N) + r] * dtau_s[l]);
+      __syncthreads();
+      double a0, a1;
+      coef(l, a0, a1);
+      const double f0 = a0, f1 = a0 + a1 * (taus[l + 1] - taus[l]);
+      for (int j = 0; j < H; ++j) {  // w = X^T g - d - c_t
+        double s = 0.0;
 #pragma unroll
-      for (int w = 0; w < NW; ++w) cand[w] = carried[w];
-      const double* jr = jrec0 + (long long)l * jrec_stride(N);
-      double* cvl = cv0 + (long long)l * N * cvs;
-      for (int c = 0; c < N; ++c) {
-        int ps = (int)jr[N * PR + c];
-        ps = ps < 0 ? 0 : (ps >= PR ? PR - 1 : ps);  // a record slot always, whatever was stored
-        const double rp = R[ps * KB];
-        if (act) cvl[c * cvs + k] = rp;
-        cand[ps >> 5] &= ~(1u << (ps & 31));
-        const double* m = jr + c * PR;
-        for (int s = 0; s < PR; ++s) R[s * KB] += m[s] * rp;
+        for (int r = 0; r < H; ++r) s = fma(lr[mod_X(N) + j * HP + r], u[r * KB], s);
+        w[j * KB] = s - a1 * lr[mod_dt(N) + j] - f0 * lr[mod_ct(N) + j];
       }
+      for (int j = 0; j < H; ++j) {  // u = q - c_b
+        double s = 0.0;
 #pragma unroll
-      for (int w = 0; w < NW; ++w) carried[w] = cand[w];
+        for (int r = 0; r < H; ++r) s = fma(br[brec_H(N) + r * HP + j], w[r * KB], s);
+        const double ct = lr[mod_ct(N) + j], rj = f0 * ct + s;
+        if (act) cvl[j * cvs + k] = rj;
+        u[j * KB] = Ev[j] * rj - f1 * ct;
+      }
+      for (int j = 0; j < H; ++j) {  // w = c_b + d + 2 G (q - c_b)
+        double s = 0.0;
+#pragma unroll
+        for (int r = 0; r < H; ++r) s = fma(br[brec_G(N) + r * HP + j], u[r * KB], s);
+        w[j * KB] = f1 * lr[mod_ct(N) + j] + a1 * lr[mod_dt(N) + j] + 2.0 * s;
+      }
+      for (int r = 0; r < H; ++r) {  // g = Y w
+        double s = 0.0;
+#pragma unroll
+        for (int j = 0; j < H; ++j) s = fma(lr[mod_Y(N) + j * HP + r], w[j * KB], s);
+        u[r * KB] = s;
+      }
     }
-    __syncthreads();  // R's area becomes X
-
-    // ---- up: U_l x_l = c_l - V_l x_{l+1}, outputs level by level ----------
-    double* X = Rv + tid;  // x of parity b at X[(b * N + j) * KB]
-    for (int j = 0; j < N; ++j) X[(N + j) * KB] = 0.0;
+    // ---- surface: phi in u (flux_bvp.cuh) --------------------------------------
+    {
+      const double fl = !dlbc && !sft ? alb / (1.0 + alb) : 0.0;
+      double dsrc = 0.0;
+      for (int r = 0; r < H; ++r) {
+        // D times the derivative of the surface source (FluxSolver.cpp:1437-1461, 1477-1492)
+        double v = 0.0;
+        const double mur = p.tables[tab_mu(N) + r];
+        if (k == L + 1) {  // the surface temperature
+          if (dlbc) {
+            v = 1.0;
+            if (dtau_last > 0.0) v += mur * (1.0 / dtau_last);
+          } else {
+            v = sft ? sft[r * brdf_row(N) + H + 1] : 1.0 - alb;
+          }
+        } else if (dlbc && k == L - 1 && dtau_last > 0.0) {
+          v = mur * (-1.0 / dtau_last);
+        }
+        v *= dsv[r];
+        dsrc = fma(dsv[r], v, dsrc);
+        w[r * KB] = v;
+      }
+      for (int r = 0; r < H; ++r) {
+        double v = 2.0 * (w[r * KB] - 2.0 * fl * dsv[r] * dsrc) - u[r * KB];
+        if (sft && !dlbc)
+          for (int c = 0; c < H; ++c) v -= 2.0 * dsv[r] * sft[r * brdf_row(N) + 1 + c] * dsv[c] * u[c * KB];
+        w[r * KB] = v;
+      }
+      for (int r = 0; r < H; ++r) {
+        double s = 0.0;
+#pragma unroll
+        for (int c = 0; c < H; ++c) s = fma(inv[c * HP + r], w[c * KB], s);
+        u[r * KB] = s;
+      }
+    }
     double chain_lev = 0.0;
     if (act) {
       if (k <= L) chain_lev = planck_deriv2(wlo, whi, temp_in[ifb ? L - k : k], p.pk);
       else chain_lev = planck_deriv2(wlo, whi, p.tbot(i), p.pk);
     }
+    // ---- up, outputs level by level -------------------------------------------
     for (int l = L - 1; l >= 0; --l) {
-      const int b = l & 1;
-      double* x = X + b * N * KB;
-      const double* xn = X + (b ^ 1) * N * KB;
+      const double* lr = lrec0 + (long long)l * lstride;
       const double* br = brec0 + (long long)l * brec_stride(N);
-      const double* cvl = cv0 + (long long)l * N * cvs;
-      for (int c = N - 1; c >= 0; --c) {
-        double s = act ? cvl[c * cvs + k] : 0.0;
-        const double* row = br + c * RL;
-        for (int j = c + 1; j < N; ++j) s -= row[j] * x[j * KB];
-        if (l < L - 1)
-          for (int j = 0; j < N; ++j) s -= row[N + j] * xn[j * KB];
-        x[c * KB] = s * rdiag(br, c);
+      const double* cvl = cv0 + (long long)l * H * cvs;
+      __syncthreads();
+      for (int r = tid; r < H; r += KB) Ev[r] = exp(-lr[mod_k(N) + r] * dtau_s[l]);
+      __syncthreads();
+      double a0, a1;
+      coef(l, a0, a1);
+      const double f0 = a0, f1 = a0 + a1 * (taus[l + 1] - taus[l]);
+      double rv[H], cb[H], b[H], av[H], c[H];
+#pragma unroll
+      for (int j = 0; j < H; ++j) rv[j] = act ? cvl[j * cvs + k] : 0.0;
+#pragma unroll
+      for (int j = 0; j < H; ++j) {  // homogeneous C at the bottom
+        double s = 0.0;
+#pragma unroll
+        for (int r = 0; r < H; ++r) s = fma(lr[mod_Y(N) + j * HP + r], u[r * KB], s);
+        cb[j] = s - f1 * lr[mod_ct(N) + j];
+        w[j * KB] = fma(Ev[j], rv[j], cb[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < H; ++j) {
+        double s = 0.0;
+#pragma unroll
+        for (int r = 0; r < H; ++r) s = fma(br[brec_G(N) + r * HP + j], w[r * KB], s);
+        b[j] = s;
+      }
+#pragma unroll
+      for (int j = 0; j < H; ++j) u[j * KB] = Ev[j] * b[j];
+#pragma unroll
+      for (int j = 0; j < H; ++j) {
+        double s = 0.0;
+#pragma unroll
+        for (int r = 0; r < H; ++r) s = fma(br[brec_H(N) + r * HP + j], u[r * KB], s);
+        c[j] = 2.0 * s - rv[j];  // homogeneous C at the top
+        av[j] = c[j] - Ev[j] * b[j];
       }
       // outputs at the depths of layer l (flux path: its bottom level, and the
       // top for l = 0)
-      const double* lr = lrec0 + (long long)l * lstride;
-      const double* eig = lr + lrec_eig(N);
-      const double* G = lr + lrec_G(N);
-      double a0, a1;
-      coef(l, a0, a1);
       const int lin = ifb ? L - 1 - l : l;
       const double w0 = GEN ? p.g.ssa[p.g.in_off[i] + lin] : p.ssa(i, lin);
       const int npass = GEN ? NT : (l == 0 ? 2 : 1);
       for (int pass = 0; pass < npass; ++pass) {
         const int lu = GEN ? pass : (pass == 0 ? l + 1 : 0);
         if (GEN && out_layer(lu) != l) continue;  // uniform over the CTA
-        const double utaupr = out_taus(lu);
+        const double tu = out_taus(lu), x1 = tu - taus[l], x2 = taus[l + 1] - tu;
         __syncthreads();
-        for (int j = tid; j < N; j += KB) {
-          const double d = (j < NN) ? (utaupr - taus[l + 1]) : (utaupr - taus[l]);
-          ex[j] = exp(-eig[j] * d);
+        for (int r = tid; r < H; r += KB) {
+          e1v[r] = exp(-lr[mod_k(N) + r] * x1);
+          e2v[r] = exp(-lr[mod_k(N) + r] * x2);
         }
         __syncthreads();
-        double dmi = 0.0, dmidn = 0.0, dmiup = 0.0, dfdn = 0.0, dfup = 0.0;
-        for (int iq = 0; iq < N; ++iq) {
-          double v = 0.0;
-          for (int j = 0; j < N; ++j) v += G[iq * N + j] * (x[j * KB] * ex[j]);
-          double d0, d1;
-          dz(l, iq, a0, a1, d0, d1);
-          v += d0 + d1 * utaupr;
-          if (iq < NN) {
-            const int c = NN - iq - 1;
-            dmi += wt[c] * v;
-            dmidn += wt[c] * v;
-            dfdn += wt[c] * v * mu[c];
-          } else {
-            const int c = iq - NN;
-            dmi += wt[c] * v;
-            dmiup += wt[c] * v;
-            dfup += wt[c] * v * mu[c];
+        // C from its values at the boundaries (no cancellation), D_ = E2 b - E1 a
+        const double ft = a0 + a1 * x1;
+#pragma unroll
+        for (int j = 0; j < H; ++j) {
+          const double kj = lr[mod_k(N) + j];
+          double cu = x1 > x2 ? cb[j] : c[j];
+          if (x1 != 0.0 && x2 != 0.0) {
+            const double fx = -expm1(-2.0 * kj * (taus[l + 1] - taus[l]));
+            if (fx > 0.0)
+              cu = (c[j] * (e1v[j] * -expm1(-2.0 * kj * x2)) + cb[j] * (e2v[j] * -expm1(-2.0 * kj * x1))) / fx;
           }
+          u[j * KB] = cu + ft * lr[mod_ct(N) + j];
+          w[j * KB] = e2v[j] * b[j] - e1v[j] * av[j] + a1 * lr[mod_dt(N) + j];
+        }
+        double su = 0.0, sd = 0.0, fu = 0.0, fd = 0.0;
+        for (int r = 0; r < H; ++r) {
+          double ph = 0.0, ps = 0.0;
+#pragma unroll
+          for (int j = 0; j < H; ++j) {
+            ph = fma(lr[mod_X(N) + j * HP + r], u[j * KB], ph);
+            ps = fma(lr[mod_Y(N) + j * HP + r], w[j * KB], ps);
+          }
+          su = fma(wv[r], ph + ps, su);
+          sd = fma(wv[r], ph - ps, sd);
+          fu = fma(mv[r], ph + ps, fu);
+          fd = fma(mv[r], ph - ps, fd);
         }
         if (act) {
-          dfup *= 2.0 * PI;
-          dfdn *= 2.0 * PI;
-          const double dmi_t = (2.0 * PI * dmi) / (4.0 * PI);
-          const double dmi_d = (2.0 * PI * dmidn) / (4.0 * PI);
-          const double dmi_u = (2.0 * PI * dmiup) / (4.0 * PI);
-          const double dpls = a0 + a1 * utaupr;
-          const double dfdiv = (1.0 - w0) * 4.0 * PI * (dmi_t - dpls);
-          store(0, lu, k, chain_lev * dfup);
-          store(1, lu, k, chain_lev * dfdn);
-          store(2, lu, k, chain_lev * dmi_t);
-          store(3, lu, k, chain_lev * dmi_d);
-          store(4, lu, k, chain_lev * dmi_u);
-          store(5, lu, k, chain_lev * dfdiv);
+          const double dpls = a0 + a1 * x1;
+          const double dmi = 0.5 * (su + sd);
+          store(0, lu, k, chain_lev * (2.0 * PI * fu));
+          store(1, lu, k, chain_lev * (2.0 * PI * fd));
+          store(2, lu, k, chain_lev * dmi);
+          store(3, lu, k, chain_lev * (0.5 * sd));
+          store(4, lu, k, chain_lev * (0.5 * su));
+          store(5, lu, k, chain_lev * ((1.0 - w0) * 4.0 * PI * (dmi - dpls)));
         }
       }
+      // phi at the top of the layer
+#pragma unroll
+      for (int j = 0; j < H; ++j) w[j * KB] = c[j] + f0 * lr[mod_ct(N) + j];
+      for (int r = 0; r < H; ++r) {
+        double s = 0.0;
+#pragma unroll
+        for (int j = 0; j < H; ++j) s = fma(lr[mod_X(N) + j * HP + r], w[j * KB], s);
+        u[r * KB] = s;
+      }
     }
-    __syncthreads();  // X's area is the next pass's R
+    __syncthreads();  // the next pass reuses the shared vectors
   }
 }
 

@@ -1,30 +1,39 @@
-// flux_layer.cuh — per-(instance, layer) eigensystem and particular solutions.
+// flux_layer.cuh — per-(instance, layer) eigensystems and particular solutions.
 //
-// Replaces solveEigen (FluxSolver.cpp:459-588), computeBeamSource (:595-643)
-// and computeIsotropicSource (:745-831).  One team of TEAM = pow2ceil(N)
-// threads per layer task; every matrix lives in the team's shared memory.
+// Replaces solveEigen (FluxSolver.cpp:459-588), computeBeamSource (:595-643) and
+// computeIsotropicSource (:745-831), and interpEigenvec / interpSource of the
+// general solver (DisortSolver.cpp:2468-2580).
 //
 // Eigenproblem: the reference symmetrises (a+b)(a-b) with D = diag(sqrt(w mu)),
-// factors -B_s = L L^T and diagonalises S = L^T (-A_s) L (SelfAdjointEigenSolver).
-// Here S is diagonalised with a parallel cyclic Jacobi method (round-robin pair
-// ordering, NN/2 disjoint rotations per round, one 2x2 block per thread), which
-// yields the same eigenpairs to rounding; eigenvalues are sorted ascending like
-// the reference's.  When -B_s is not SPD (the reference's general-eigensolver
-// branch, omega' >= 1-1e-12), -A_s = L'L'^T and S' = L'^T(-B_s)L' give the same
-// eigenpairs of (a+b)(a-b) with u = D^{-1} L' w.
+// factors -B_s = L L^T and diagonalises S = L^T (-A_s) L (SelfAdjointEigenSolver),
+// A_s = D (a+b) D^{-1}, B_s = D (a-b) D^{-1}.  With S = U K^2 U^T the modes of
+// phi = D (up + down), psi = D (up - down) are
+//   X = L U K^{-1/2},  Y = L^{-T} U K^{1/2},  X^T Y = I,
+//   -A_s = Y K Y^T, -B_s = X K X^T, and their inverses X K^{-1} X^T, Y K^{-1} Y^T,
+// so the particular solutions are diagonal in them: for thermal emission
+// (xr0 + xr1 tau), with v = X^T (D M^{-1} 1), M = diag(mu),
+//   c = 2 (1 - w') v / k,  d = c / k;
+// for the beam exp(-tau/mu0) with alpha = X^T D M^{-1} (q+ + q-) and
+// beta = Y^T D M^{-1} (q+ - q-), q+- the source at the up/down quadrature angles,
+//   c = (k alpha - beta/mu0) / (k^2 - mu0^{-2}),
+//   d = (k beta - alpha/mu0) / (k^2 - mu0^{-2}).
+// When -B_s is not positive definite, -A_s = L L^T and S = L^T (-B_s) L give
+// the same modes with the two forms exchanged (X = L^{-T} U K^{1/2}, Y = L U K^{-1/2}).
+// The quadrature is symmetric (mu_{h+j} = -mu_j, P_l^m(-mu) = (-1)^{l+m} P_l^m(mu)),
+// so -B_s holds the phase sums of odd l + m only and -A_s those of even l + m:
+//   alpha -/+ beta = M^{-1} (O W - I), M^{-1} (E W - I),
+//   O_ij, E_ij = sum_{l + m odd, even} g'_l P_l^m(mu_i) P_l^m(mu_j).
 //
-// Shared-memory layout per team: the phase matrix is kept as its unique half
-// cc_top (NN x N; C = [[P, Q], [Q, P]] with P = cc_top[:, :NN], Q = cc_top[:, NN:]),
-// NN x NN matrices use a padded row stride NS = NN + 1 (conflict-free columns),
-// and the N x N LU matrix of the particular solutions overlays the eigen work
-// area once the eigenvectors have been written out.
+// N <= 16: one thread per layer task, every matrix in registers (front kernel,
+// then the eigensolver with the record's output).  Larger N (and, on the flux
+// path, when a schedule asks for it): a team of threads per task in shared memory.
 #pragma once
 
 #include "dsp_device.cuh"
 
 namespace dsp {
 
-template <int N, bool GEN = false>
+template <int N>
 struct LCfg {
   static constexpr int NN = N / 2;
   // 64 streams: a 128-thread team per layer (two threads per stream)
@@ -36,32 +45,19 @@ struct LCfg {
   static constexpr int BPT = (NPAIR * NPAIR + TEAM - 1) / TEAM;  // Jacobi 2x2 blocks per thread
   static constexpr int NS = NN + 1;  // padded row stride of NN x NN matrices
   static constexpr int MAT = NN * NS;
-  // team shared-memory layout (doubles).  The phase matrix is dead once
-  // alpha -/+ beta are formed; where it is large enough (N >= 10) the
-  // eigenvector matrix V and the vectors b, z are placed over it.
-  static constexpr bool OVL = MAT + 2 * N <= NN * N;
-  static constexpr int O_CC = 0;                     // cc_top[NN][N]
-  static constexpr int O_GL = O_CC + NN * N;         // gl[N]
-  static constexpr int O_W = O_GL + N;               // work area: AMB, APB, S0, S1, LC (, V)
-  static constexpr int W_SIZE = (OVL ? 5 : 6) * MAT;
-  static constexpr int O_V = OVL ? O_CC : O_W + 5 * MAT;
-  static constexpr int O_LAM = O_W + W_SIZE;         // NN: k = sqrt|lambda|
-  static constexpr int O_LAMR = O_LAM + NN;          // NN: lambda
-  static constexpr int O_ROT = O_LAMR + NN;          // c, s, t per pair
-  static constexpr int O_B = OVL ? O_CC + MAT : O_ROT + 3 * NPAIR;  // b[N]
-  static constexpr int O_Z = O_B + N;                // z[N]
-  static constexpr int O_MISC = OVL ? O_ROT + 3 * NPAIR : O_Z + N;  // flags, reduction scratch
-  static constexpr int O_PIV = O_MISC + 8;           // N ints
-  // general solver: P_l^m(-mu0), then psi0 / p0 / p1 source moments [N] each
-  static constexpr int O_GX = O_PIV + N / 2 + 1;
-  static constexpr int TEAM_SMEM = round4(O_GX + (GEN ? 4 * N : 0));
-  // user angles whose P_l^m columns fit next to W[N][N] in the work area
-  static constexpr int UCH = (W_SIZE - N * N) / N;
-  static_assert(!GEN || UCH >= 1, "work area too small for the user-angle tables");
-  // the Legendre table stays in global memory (L1) for N >= 16, where it would
-  // take about as much shared memory as a team
-  static constexpr bool Y_GLOBAL = N >= 16;
-  static constexpr int TAB = Y_GLOBAL ? tab_ylm(N) : tab_size(N);
+  // team shared-memory layout (doubles)
+  static constexpr int O_A = 0;            // -A_s, then X
+  static constexpr int O_B = O_A + MAT;    // -B_s, then S
+  static constexpr int O_L = O_B + MAT;    // Cholesky factor
+  static constexpr int O_V = O_L + MAT;    // scratch, then the eigenvectors
+  static constexpr int O_T = O_V + MAT;    // scratch, then Y
+  static constexpr int O_GL = O_T + MAT;   // g'_l [N]
+  static constexpr int O_B1 = O_GL + N;    // beam source sums, D M^{-1} (q+ +/- q-) [NN] each
+  static constexpr int O_B2 = O_B1 + NN;
+  static constexpr int O_ROT = O_B2 + NN;  // c, s, t per pair
+  static constexpr int O_MISC = O_ROT + 3 * NPAIR;  // flags
+  static constexpr int TEAM_SMEM = round4(O_MISC + 8);
+  static constexpr int TAB = tab_ylm(N);   // mu, wt, dsim, dinv; the Legendre table is read through L1
   static constexpr size_t smem_bytes() { return sizeof(double) * (size_t)(TAB + TPC * TEAM_SMEM); }
   // resident CTAs per SM the register budget is sized for: as many as shared
   // memory admits (228 KB, 1 KB reserved per CTA), never below 80 registers
@@ -70,13 +66,9 @@ struct LCfg {
   static constexpr int MINB = MINB_SMEM < 1 ? 1 : (MINB_SMEM < MINB_REGS ? MINB_SMEM : MINB_REGS);
 };
 
-// Whether the layer stage of an N-stream flux solve is split in three launches:
-// the front of the layer kernel (phase matrix, alpha -/+ beta, Cholesky,
-// S = L^T M L), the eigensolver with one thread per layer task
-// (flux_jacobi_kernel), and the back of the layer kernel (eigenvectors, G,
-// particular solutions).  A thread that owns a whole 8 x 8 S and its eigenvector
-// matrix in registers runs the rotations of a sweep with no shuffles or
-// barriers; the team form spends most of its time waiting on them.
+// Whether the layer stage of N streams runs as one thread per task: a thread
+// that owns a whole h x h S and its eigenvector matrix in registers runs the
+// rotations of a sweep with no shuffles or barriers.
 template <int N>
 __host__ __device__ constexpr bool layer_split() { return N <= 16; }
 
@@ -85,27 +77,19 @@ __host__ __device__ constexpr int tri_idx(int r, int c) {
   return r >= c ? r * (r + 1) / 2 + c : c * (c + 1) / 2 + r;
 }
 
-// Hand-off between the three launches of a split layer stage, kept in the
+// Hand-off between the two launches of a split layer stage, kept in the
 // boundary-value records' area (dead until the boundary-value kernel runs):
 // blocks of 32 layer tasks, element e of the block's lane k at
 // 32 HS b + e w + k (w = tasks in the block), so that a warp of the
 // one-thread-per-task kernels reads or writes an element of 32 tasks in one
 // coalesced access.  Per task: flag (0 skipped, 1 primary factorisation,
-// 2 fallback), S, the Cholesky factor L, and the odd- and even-order halves
-// O, E of the phase sums (all symmetric NN x NN, packed lower; E only with a
-// beam), then the eigensolver's diagonal and eigenvector matrix (row-major,
-// column j the eigenvector of diagonal entry j).
-//   O_ij = sum_{l odd} g'_l P_l(mu_i) P_l(mu_j),  E_ij = sum_{l even} (...),
-//   alpha - beta = M^{-1} (O W - I),  alpha + beta = M^{-1} (E W - I)
-// with M = diag(mu_1..mu_NN), W = diag(w_1..w_NN): the quadrature is
-// symmetric (mu_{NN+j} = -mu_j, P_l(-mu) = (-1)^l P_l(mu)), so the sums over
-// the other hemisphere only flip the sign of the odd orders.
+// 2 fallback), S and the Cholesky factor L (packed lower), and with a beam the
+// source vectors D M^{-1} (q+ + q-), D M^{-1} (q+ - q-).
 template <int NN>
 struct Handoff {
   static constexpr int TRI = NN * (NN + 1) / 2;
-  static constexpr int S_FLAG = 0, S_S = 1, S_L = 1 + TRI, S_O = 1 + 2 * TRI, S_E = 1 + 3 * TRI;
-  static constexpr int S_D = 1 + 4 * TRI, S_V = S_D + NN;
-  static constexpr int HS = S_V + NN * NN;
+  static constexpr int S_FLAG = 0, S_S = 1, S_L = 1 + TRI, S_B1 = 1 + 2 * TRI, S_B2 = S_B1 + NN;
+  static constexpr int HS = S_B2 + NN;
 };
 
 // Quadrature tables of an N-stream solve passed by value: kernel parameters
@@ -114,7 +98,7 @@ struct Handoff {
 template <int N>
 struct ConstTab {
   double mu[N / 2], rmu[N / 2], wt[N / 2], dsim[N / 2], dinv[N / 2];
-  double y[N * N];  // P_l(mu_i) at [l * N + i]
+  double y[N * (N / 2)];  // P_l^m(mu_i), mu_i > 0, at [l * N/2 + i]
 };
 
 // ConstTab from a host copy of the tab_* table layout
@@ -128,7 +112,8 @@ inline ConstTab<N> make_const_tab(const double* tab) {
     c.dsim[k] = tab[tab_dsim(N) + k];
     c.dinv[k] = tab[tab_dinv(N) + k];
   }
-  for (int k = 0; k < N * N; ++k) c.y[k] = tab[tab_ylm(N) + k];
+  for (int l = 0; l < N; ++l)
+    for (int k = 0; k < N / 2; ++k) c.y[l * (N / 2) + k] = tab[tab_ylm(N) + l * N + k];
   return c;
 }
 
@@ -257,172 +242,99 @@ __device__ __forceinline__ void jacobi_rot(double apq, double app, double aqq, d
   }
 }
 
+// One layer task: its instance, layer and addresses.
+template <int N, bool GEN>
+struct LayerTask {
+  int i, lc;          // input / status index, layer (top down)
+  long long slot;     // instance slot of the launch
+  const double* rec;  // instance record
+  InstLayout il;
+  const double* pml;  // phase-function moments
+  double* lrec;       // layer record
+  bool live;          // solved in this launch
+};
+template <int N, bool GEN>
+__device__ __forceinline__ LayerTask<N, GEN> layer_task(const FluxParams& p, long long task) {
+  LayerTask<N, GEN> q;
+  int Lin;
+  if constexpr (GEN) {  // ragged layers; task = chunk-local layer
+    q.slot = p.g.layer_inst[task];
+    q.i = p.g.ids[q.slot];
+    q.lc = (int)(task - p.g.lay_off[q.slot]);
+    Lin = p.g.Ls[q.i];
+    q.il = InstLayout::make(Lin, N);
+    q.rec = p.inst_rec + p.g.inst_off[q.slot];
+    q.lrec = p.layer_rec + task * p.g.lstride;
+    const int lin = (p.flags & DSP_FLAG_INDEX_FROM_BOTTOM) ? Lin - 1 - q.lc : q.lc;
+    q.pml = p.g.pmom + (p.g.in_off[q.i] + lin) * (long long)p.pc;
+  } else {
+    q.i = (int)(task / p.L);
+    q.slot = q.i;
+    q.lc = (int)(task % p.L);
+    q.il = p.il;
+    q.rec = p.inst_rec + (long long)q.i * p.il.stride;
+    q.lrec = p.layer_rec + task * lrec_stride(N);
+    const int lin = (p.flags & DSP_FLAG_INDEX_FROM_BOTTOM) ? p.L - 1 - q.lc : q.lc;
+    q.pml = p.pmom.row(q.i) + (long long)lin * p.pc;
+  }
+  // invalid instances and layers below the absorption cut are not solved; the
+  // general solver also skips modes past the instance's last one or after its
+  // azimuthal series converged
+  q.live = !(p.status && p.status[q.i] == DSP_ERR_INVALID_INPUT) && q.lc < (int)q.rec[H_NCUT];
+  if constexpr (GEN) q.live = q.live && p.g.m <= (int)q.rec[H_NAZ] && q.rec[H_DONE] == 0.0;
+  return q;
+}
+template <bool GEN>
+__device__ __forceinline__ long long layer_tasks(const FluxParams& p) {
+  if constexpr (GEN) return p.g.lay_off[p.n];
+  else return (long long)p.n * p.L;
+}
+// P_l^m(-mu0) of an instance
+template <int N, bool GEN>
+__device__ __forceinline__ const double* beam_legendre(const FluxParams& p, const LayerTask<N, GEN>& q) {
+  if constexpr (GEN) return p.g.ptab + q.slot * (long long)(N * (1 + p.g.numu));
+  else return q.rec + q.il.yb;
+}
+
+// scaled phase coefficient g'_k (disortSet, FluxSolver.cpp:336-386; the general
+// solver normalises P_0 to 1, DisortSolver.cpp:669)
+template <bool GEN>
+__device__ __forceinline__ double phase_coeff(int k, double pk, int mode, double ws, double f, double sig) {
+  if (GEN && k == 0) pk = 1.0;
+  if (mode == 0) return (2.0 * k + 1.0) * ws * pk;
+  if (mode == 1) return (2.0 * k + 1.0) * ws * (pk - f) / (1.0 - f);
+  const double kd = (double)k;
+  return (2.0 * k + 1.0) * ws * (pk - f * exp(-kd * kd / (2.0 * sig))) / (1.0 - f);
+}
+
+// k = sqrt|lambda|, kept off zero: at omega' = 1 one eigenvalue is zero to
+// rounding (k ~ 1e-8 either way), and a k below 1e-9 changes no result (the
+// solution depends on k^2)
+__device__ __forceinline__ double mode_k(double lambda) { return fmax(sqrt(fabs(lambda)), 1e-9); }
+
+// the beam's cosine, moved off a resonance mu0 k = 1 (FluxSolver.cpp:610-618)
+__device__ __forceinline__ bool beam_resonant(double k, double umu0) {
+  return fabs(1.0 - umu0 * umu0 * k * k) < 1000.0 * 2.220446049250313e-16;
+}
+
+// thermal source of a layer: intercept and slope in scaled depth (FluxSolver.cpp:745-787)
+template <class Q>
+__device__ __forceinline__ void thermal_source(const Q& q, double& xr0, double& xr1) {
+  const double dts = q.rec[q.il.dtau_s + q.lc], taus_top = q.rec[q.il.tau_s + q.lc];
+  const double pk0 = q.rec[q.il.pkag + q.lc], pk1 = q.rec[q.il.pkag + q.lc + 1];
+  xr1 = 0.0;
+  if (dts > 1e-4) xr1 = (pk1 - pk0) / dts;
+  xr0 = pk0 - xr1 * taus_top;
+}
+
 // ---------------------------------------------------------------------------
-// Length-NN vectors distributed one element per team thread (thread t < NN
-// holds element t).  Sub-warp teams broadcast with shuffles; larger teams go
-// through a shared scratch word.  Matrices are NN x NN, row stride NS.
+// Layer stage with a team of threads per task, matrices in shared memory.
 // ---------------------------------------------------------------------------
-template <int TEAM>
-__device__ __forceinline__ double team_bcast(double v, int k, int t, double* scratch) {
-  if constexpr (TEAM <= 32) {
-    return __shfl_sync(team_mask<TEAM>(), v, k, TEAM);
-  } else {
-    if (t == k) scratch[0] = v;
-    __syncthreads();
-    const double r = scratch[0];
-    __syncthreads();
-    return r;
-  }
-}
-
-// y = A x (trans = false) or A^T x (trans = true); part: 0 full, 1 lower, 2 upper
-template <int NN, int NS, int TEAM>
-__device__ __forceinline__ double team_matvec(const double* A, double x, bool trans, int part, int t,
-                                              double* scratch) {
-  double acc = 0.0;
-  if constexpr (TEAM <= 32) {
-#pragma unroll
-    for (int k = 0; k < NN; ++k) {
-      const double xk = __shfl_sync(team_mask<TEAM>(), x, k, TEAM);
-      if (t < NN) {
-        const int r = trans ? k : t, c = trans ? t : k;  // element A[r][c]
-        const bool in = part == 0 || (part == 1 ? c <= r : c >= r);
-        if (in) acc += A[r * NS + c] * xk;
-      }
-    }
-  } else {
-    if (t < NN) scratch[t] = x;
-    __syncthreads();
-    if (t < NN)
-      for (int k = 0; k < NN; ++k) {
-        const int r = trans ? k : t, c = trans ? t : k;
-        const bool in = part == 0 || (part == 1 ? c <= r : c >= r);
-        if (in) acc += A[r * NS + c] * scratch[k];
-      }
-    __syncthreads();
-  }
-  return acc;
-}
-
-// x <- L^{-1} x (forward) or L^{-T} x (backward), L lower triangular
-template <int NN, int NS, int TEAM>
-__device__ __forceinline__ double team_trsv(const double* Lm, double x, bool transposed, int t,
-                                            double* scratch) {
-  if (!transposed) {
-    for (int k = 0; k < NN; ++k) {
-      if (t == k) x = x / Lm[k * NS + k];
-      const double xk = team_bcast<TEAM>(x, k, t, scratch);
-      if (t > k && t < NN) x -= Lm[t * NS + k] * xk;
-    }
-  } else {
-    for (int k = NN - 1; k >= 0; --k) {
-      if (t == k) x = x / Lm[k * NS + k];
-      const double xk = team_bcast<TEAM>(x, k, t, scratch);
-      if (t < k) x -= Lm[k * NS + t] * xk;
-    }
-  }
-  return x;
-}
-
-// Eigenvectors and sources of one layer at the user polar angles for mode m
-// (interpEigenvec, DisortSolver.cpp:2468-2504; interpSource, :2506-2580):
-//   W(l, c)   = 0.5 g'_l sum_jq P_l^m(mu_jq) w_jq G(row(jq), c)
-//   GU(iu, c) = sum_l P_l^m(mu_u) W(l, c)
-// with row(jq) = NN + jq for jq < NN, N - 1 - jq otherwise (the reference's
-// reduced-eigenvector ordering); the beam and thermal sources likewise.
-// Team thread c owns column c; the P_l^m columns of up to UCH user angles at a
-// time sit beside W in the (now free) eigen work area.
-template <int N>
-__device__ void gen_user_angles(const FluxParams& p, int i, double* sm, const double* Y, const double* wt,
-                                const double* gl, double* lrec, double fbeam, double ws, bool thermal,
-                                int t) {
-  using C = LCfg<N, true>;
-  constexpr int NN = N / 2, TEAM = C::TEAM, UCH = C::UCH;
-  const int m = p.g.m, numu = p.g.numu;
-  double* W = sm + C::O_W;           // [N][N]
-  double* U = W + N * N;             // [N][UCH]
-  const double* ybm = sm + C::O_GX;  // P_l^m(-mu0) (written by the beam source)
-  double* psi0 = sm + C::O_GX + N;
-  double* p0 = psi0 + N;
-  double* p1 = p0 + N;
-  const double* G = lrec + lrec_G(N);
-  const bool beam = fbeam > 0.0;
-  team_sync<TEAM>();  // G and the particular solutions of this team are written
-  if (t < N) {
-    const int c = t;
-    double gcol[N];
-#pragma unroll
-    for (int jq = 0; jq < N; ++jq) gcol[jq] = G[(jq < NN ? NN + jq : N - 1 - jq) * N + c];
-    for (int l = 0; l < N; ++l) {
-      double s = 0.0;
-      if (l >= m) {
-#pragma unroll
-        for (int jq = 0; jq < N; ++jq) s += (Y[l * N + jq] * wt[jq]) * gcol[jq];
-        s *= 0.5 * gl[l];
-      }
-      W[l * N + c] = s;
-    }
-    // source moments: psi0(l) = 0.5 g'_l sum_jq w_jq P_l^m(mu_jq) z(jq) with the
-    // unordered beam solution z(jq) = zb[row(jq)], and the thermal z0 / z1 alike
-    const int l = t;
-    double sb = 0.0, s0 = 0.0, s1 = 0.0;
-    if (l >= m) {
-      for (int jq = 0; jq < N; ++jq) {
-        const int r = jq < NN ? NN + jq : N - 1 - jq;
-        const double yw = wt[jq] * Y[l * N + jq];
-        if (beam) sb += yw * lrec[lrec_zb(N) + r];
-        if (thermal) {
-          s0 += yw * lrec[lrec_z0(N) + r];
-          s1 += yw * lrec[lrec_z1(N) + r];
-        }
-      }
-    }
-    psi0[l] = 0.5 * gl[l] * sb;
-    p0[l] = 0.5 * gl[l] * s0;
-    p1[l] = 0.5 * gl[l] * s1;
-  }
-  team_sync<TEAM>();
-  const double xr0 = lrec[lrec_xr(N)], xr1 = lrec[lrec_xr(N) + 1];
-  const double fact = (m == 0 ? 1.0 : 2.0) * fbeam / (4.0 * 3.14159265358979323846);
-  double* GU = lrec + glrec_gu(N);
-  double* zbu = GU + numu * N;
-  double* z0u = zbu + numu;
-  double* z1u = z0u + numu;
-  const double* umu = p.g.umu.row(i);
-  for (int u0 = 0; u0 < numu; u0 += UCH) {
-    const int nu = numu - u0 < UCH ? numu - u0 : UCH;
-    for (int k = t; k < nu; k += TEAM) legendre_column(m, umu[u0 + k], N - 1, U + k, UCH);
-    team_sync<TEAM>();
-    if (t < N)
-      for (int k = 0; k < nu; ++k) {
-        double s = 0.0;
-        for (int l = m; l < N; ++l) s += U[l * UCH + k] * W[l * N + t];
-        GU[(u0 + k) * N + t] = s;
-      }
-    for (int k = t; k < nu; k += TEAM) {
-      if (beam) {
-        double s = 0.0;
-        for (int l = m; l < N; ++l) s += U[l * UCH + k] * (psi0[l] + fact * gl[l] * ybm[l]);
-        zbu[u0 + k] = s;
-      }
-      if (thermal) {
-        double s0 = 0.0, s1 = 0.0;
-        for (int l = m; l < N; ++l) {
-          s0 += U[l * UCH + k] * p0[l];
-          s1 += U[l * UCH + k] * p1[l];
-        }
-        z0u[u0 + k] = s0 + (1.0 - ws) * xr0;
-        z1u[u0 + k] = s1 + (1.0 - ws) * xr1;
-      }
-    }
-    team_sync<TEAM>();
-  }
-}
-
-template <int N, bool GEN = false, bool JAC = false>
-__global__ void __launch_bounds__(LCfg<N, GEN>::CTA, LCfg<N, GEN>::MINB) flux_layer_kernel(FluxParams p) {
-  using C = LCfg<N, GEN>;
+template <int N, bool GEN = false>
+__global__ void __launch_bounds__(LCfg<N>::CTA, LCfg<N>::MINB) flux_layer_kernel(FluxParams p) {
+  using C = LCfg<N>;
   constexpr int NN = C::NN, TEAM = C::TEAM, NNP = C::NNP, NPAIR = C::NPAIR, NS = C::NS, BPT = C::BPT;
+  constexpr int HP = mod_hp(N);
   constexpr int BPA = NPAIR;  // blocks (a, b) per column pair b
   extern __shared__ double smem[];
   // CTA-level constant tables
@@ -432,165 +344,99 @@ __global__ void __launch_bounds__(LCfg<N, GEN>::CTA, LCfg<N, GEN>::MINB) flux_la
   const double* wt = smem + tab_wt(N);
   const double* dsim = smem + tab_dsim(N);
   const double* dinv = smem + tab_dinv(N);
-  const double* Y = C::Y_GLOBAL ? p.tables + tab_ylm(N) : smem + tab_ylm(N);
+  const double* Y = p.tables + tab_ylm(N);
 
   const int team = threadIdx.x / TEAM, t = threadIdx.x % TEAM;
   const long long task = (long long)blockIdx.x * C::TPC + team;
-  // i: status / input index; lc: layer; Lin: layers of the instance
-  int i, lc, Lin;
-  const double* rec;
-  InstLayout il_gen;  // general solver: the layout of this instance
-  const double* pml;
-  if constexpr (GEN) {
-    // general solver: ragged layers; task = chunk-local layer
-    if (task >= p.g.lay_off[p.n]) return;
-    const int ci = p.g.layer_inst[task];
-    i = p.g.ids[ci];
-    lc = (int)(task - p.g.lay_off[ci]);
-    Lin = p.g.Ls[i];
-    il_gen = InstLayout::make(Lin, N);
-    rec = p.inst_rec + p.g.inst_off[ci];
-    const int lin = (p.flags & DSP_FLAG_INDEX_FROM_BOTTOM) ? Lin - 1 - lc : lc;
-    pml = p.g.pmom + (p.g.in_off[i] + lin) * (long long)p.pc;
-  } else {
-    if (task >= (long long)p.n * p.L) return;
-    i = (int)(task / p.L);
-    lc = (int)(task % p.L);
-    Lin = p.L;
-    rec = p.inst_rec + (long long)i * p.il.stride;
-    const int lin = (p.flags & DSP_FLAG_INDEX_FROM_BOTTOM) ? p.L - 1 - lc : lc;
-    pml = p.pmom.row(i) + (long long)lin * p.pc;
-  }
-  const InstLayout& il = GEN ? il_gen : p.il;
-  if (p.status && p.status[i] == DSP_ERR_INVALID_INPUT) return;
-  const int ncut = (int)rec[H_NCUT];
-  if (lc >= ncut) return;  // layers below the absorption cut are never used
-  if constexpr (GEN) {
-    // modes past the instance's last one, or after its azimuthal series converged
-    if (p.g.m > (int)rec[H_NAZ] || rec[H_DONE] != 0.0) return;
-  }
-
+  if (task >= layer_tasks<GEN>(p)) return;
+  const LayerTask<N, GEN> q = layer_task<N, GEN>(p, task);
+  if (!q.live) return;
   double* sm = smem + C::TAB + team * C::TEAM_SMEM;
-  double* CC = sm + C::O_CC;
+  double* MA = sm + C::O_A;
+  double* MB = sm + C::O_B;
+  double* LC = sm + C::O_L;
+  double* V = sm + C::O_V;
+  double* T = sm + C::O_T;
   double* gl = sm + C::O_GL;
-  double* W = sm + C::O_W;
-  double* AMB = W + 0 * C::MAT;
-  double* APB = W + 1 * C::MAT;
-  double* S0 = W + 2 * C::MAT;
-  double* S1 = W + 3 * C::MAT;
-  double* LC = W + 4 * C::MAT;
-  double* V = sm + C::O_V;  // over the phase matrix when C::OVL (first written after alpha -/+ beta)
-  double* EV = S0;  // eigenvectors of (a+b)(a-b); S0 is dead by then
-  double* lam = sm + C::O_LAM;
-  double* lamraw = sm + C::O_LAMR;
+  double* b1 = sm + C::O_B1;
+  double* b2 = sm + C::O_B2;
   double* rot = sm + C::O_ROT;
-  double* bv = sm + C::O_B;
-  double* zv = sm + C::O_Z;
   double* misc = sm + C::O_MISC;
-  int* piv = reinterpret_cast<int*>(sm + C::O_PIV);
-
-  DSP_PHASE_BEGIN
-  const double ws = rec[il.ssa_s + lc];
-  const double dts = rec[il.dtau_s + lc];
-  // ---- scaled phase coefficients (disortSet, FluxSolver.cpp:336-386) ----
+  const double ws = q.rec[q.il.ssa_s + q.lc];
   {
-    const int mode = (int)rec[il.mode + lc];
-    const double f = rec[il.fsc + lc], sig = rec[il.sig + lc];
-    for (int k = t; k < N; k += TEAM) {
-      // the general solver normalises P_0 to 1 (DisortSolver.cpp:669)
-      const double pk = (GEN && k == 0) ? 1.0 : pml[k];
-      double g;
-      if (mode == 0) g = (2.0 * k + 1.0) * ws * pk;
-      else if (mode == 1) g = (2.0 * k + 1.0) * ws * (pk - f) / (1.0 - f);
-      else {
-        const double kd = (double)k;
-        g = (2.0 * k + 1.0) * ws * (pk - f * exp(-kd * kd / (2.0 * sig))) / (1.0 - f);
-      }
-      gl[k] = g;
-    }
+    const int mode = (int)q.rec[q.il.mode + q.lc];
+    const double f = q.rec[q.il.fsc + q.lc], sig = q.rec[q.il.sig + q.lc];
+    for (int k = t; k < N; k += TEAM) gl[k] = phase_coeff<GEN>(k, q.pml[k], mode, ws, f, sig);
   }
   team_sync<TEAM>();
-  DSP_PHASE(0)
-  // ---- phase matrix, unique half (FluxSolver.cpp:466-482) ---------------
-  // thread t owns column jq = t; its Legendre column is held in registers
-  if (t < N) {
-    const int jq = t;
-    double yj[N];
-#pragma unroll
-    for (int l = 0; l < N; ++l) yj[l] = Y[l * N + jq];
-    const double wj = wt[jq];
-    for (int iq = 0; iq < NN; ++iq) {
-      double s = 0.0;
-#pragma unroll
-      for (int l = 0; l < N; ++l) s += (gl[l] * Y[l * N + iq]) * yj[l];
-      CC[iq * N + jq] = (s * 0.5) * wj;
-    }
-  }
-  team_sync<TEAM>();
-  DSP_PHASE(1)
-  // ---- alpha -/+ beta and the similarity transform (:485-514) ------------
+  const int odd0 = GEN ? 1 - (p.g.m & 1) : 1;  // first l of odd l + m
+  // ---- -A_s and -B_s from the even and odd phase sums ----------------------
   for (int it = t; it < NN * NN; it += TEAM) {
-    const int iq = it / NN, jq = it % NN;
-    const double inv_cmu = 1.0 / mu[iq];
-    const double a = CC[iq * N + jq], b = CC[iq * N + NN + jq];
-    double amb = inv_cmu * (a - b), apb = inv_cmu * (a + b);
-    if (iq == jq) { amb -= inv_cmu; apb -= inv_cmu; }
-    AMB[iq * NS + jq] = amb;
-    APB[iq * NS + jq] = apb;
-    S0[iq * NS + jq] = dsim[iq] * apb * dinv[jq];     // A_s
-    S1[iq * NS + jq] = -dsim[iq] * amb * dinv[jq];    // -B_s
+    const int r = it / NN, c = it % NN;
+    if (c > r) continue;
+    double so = 0.0, se = 0.0;
+    for (int l = 0; l < N; l += 2) {
+      so += (gl[l + odd0] * Y[(l + odd0) * N + r]) * Y[(l + odd0) * N + c];
+      se += (gl[l + 1 - odd0] * Y[(l + 1 - odd0) * N + r]) * Y[(l + 1 - odd0) * N + c];
+    }
+    const double rm = 1.0 / mu[r], dl = r == c ? rm : 0.0;
+    const double vb = -dsim[r] * ((wt[c] * so) * rm - dl) * dinv[c];
+    const double va = -dsim[r] * ((wt[c] * se) * rm - dl) * dinv[c];
+    MB[r * NS + c] = vb;
+    MB[c * NS + r] = vb;
+    MA[r * NS + c] = va;
+    MA[c * NS + r] = va;
+  }
+  const double fbeam = q.rec[H_FBEAM];
+  const bool beam = fbeam > 0.0;
+  if (beam) {
+    // (2 - delta_m0) F0 / 4pi sum_k g'_k P_k^m(mu_r) P_k^m(-mu0) by parity (DisortSolver.cpp:1361-1368)
+    const double* yb = beam_legendre<N, GEN>(p, q);
+    const double fac = ((GEN && p.g.m > 0) ? 2.0 * fbeam : fbeam) / (4.0 * 3.14159265358979323846);
+    for (int r = t; r < NN; r += TEAM) {
+      double so = 0.0, se = 0.0;
+      for (int l = 0; l < N; l += 2) {
+        so += gl[l + odd0] * Y[(l + odd0) * N + r] * yb[l + odd0];
+        se += gl[l + 1 - odd0] * Y[(l + 1 - odd0) * N + r] * yb[l + 1 - odd0];
+      }
+      const double dm = dsim[r] / mu[r];
+      b1[r] = dm * (2.0 * fac * se);
+      b2[r] = dm * (2.0 * fac * so);
+    }
   }
   team_sync<TEAM>();
-  // ---- Cholesky of -B_s, else of -A_s (:521-558) -------------------------
-  bool primary = ws < 1.0 - 1e-12;
-  if (primary) primary = team_chol<NN, NS, TEAM>(S1, LC, misc, t);
-  if (!primary) {
+  // ---- Cholesky of -B_s, else of -A_s (:521-558) ---------------------------
+  bool primary = team_chol<NN, NS, TEAM>(MB, LC, misc, t);
+  if (!primary && !team_chol<NN, NS, TEAM>(MA, LC, misc, t)) {
+    if (t == 0) set_status(p.status, q.i, DSP_ERR_EIGEN);
+    return;
+  }
+  // S = L^T M L, M = -A_s (primary) or -B_s (fallback)
+  {
+    const double* M = primary ? MA : MB;
     for (int it = t; it < NN * NN; it += TEAM) {
       const int r = it / NN, c = it % NN;
-      V[r * NS + c] = -S0[r * NS + c];
+      double s = 0.0;
+      for (int k = c; k < NN; ++k) s += M[r * NS + k] * LC[k * NS + c];
+      T[r * NS + c] = s;
     }
-    team_sync<TEAM>();
-    if (!team_chol<NN, NS, TEAM>(V, LC, misc, t)) {
-      // -A_s not SPD either: try the primary factorisation regardless of omega'
-      primary = team_chol<NN, NS, TEAM>(S1, LC, misc, t);
-      if (!primary) {
-        if (t == 0) set_status(p.status, i, DSP_ERR_EIGEN);
-        return;
-      }
-    }
-  }
-  DSP_PHASE(2)
-  // S = L^T M L with M = -A_s (primary) or -B_s (fallback); V used as scratch
-  for (int it = t; it < NN * NN; it += TEAM) {
-    const int r = it / NN, c = it % NN;
-    double s = 0.0;
-    if (primary)
-      for (int k = 0; k < NN; ++k) s += -S0[r * NS + k] * LC[k * NS + c];
-    else
-      for (int k = 0; k < NN; ++k) s += S1[r * NS + k] * LC[k * NS + c];
-    V[r * NS + c] = s;
   }
   team_sync<TEAM>();
   for (int it = t; it < NN * NN; it += TEAM) {
     const int r = it / NN, c = it % NN;
-    double s = 0.0;
-    for (int k = 0; k < NN; ++k) s += LC[k * NS + r] * V[k * NS + c];
-    S0[r * NS + c] = s;
-  }
-  team_sync<TEAM>();
-  // ---- cyclic Jacobi on S (symmetrised from its lower triangle) -----------
-  for (int it = t; it < NN * NN; it += TEAM) {
-    const int r = it / NN, c = it % NN;
-    S1[r * NS + c] = (c > r) ? S0[c * NS + r] : S0[r * NS + c];
     V[r * NS + c] = (r == c) ? 1.0 : 0.0;
+    if (c > r) continue;
+    double s = 0.0;
+    for (int k = r; k < NN; ++k) s += LC[k * NS + r] * T[k * NS + c];
+    MB[r * NS + c] = s;
+    MB[c * NS + r] = s;
   }
   team_sync<TEAM>();
-  DSP_PHASE(3)
+  double* const Sc = MB;
+  double* const Sn = MB;
   // In place: in a round every 2x2 block of S is read and written by its owner
   // only, and the diagonal blocks a rotation is computed from are written by
   // their owner after it has received that rotation.
-  double* const Sc = S1;
-  double* const Sn = S1;
   for (int sweep = 0; sweep < 20; ++sweep) {
     for (int r = 0; r < NNP - 1; ++r) {
       // rotation of pair a is computed by thread a; each thread then needs the
@@ -710,237 +556,74 @@ __global__ void __launch_bounds__(LCfg<N, GEN>::CTA, LCfg<N, GEN>::MINB) flux_la
     team_sync<TEAM>();
     const bool more = misc[1] != 0.0;
     team_sync<TEAM>();
-    DSP_PHASE(6)
     if (!more) break;
   }
-  DSP_PHASE(4)
-  // ---- sort ascending; eigenvectors of (a+b)(a-b) ------------------------
-  for (int k = t; k < NN; k += TEAM) {
-    const double lk = Sc[k * NS + k];
-    int rank = 0;
-    for (int j = 0; j < NN; ++j) {
-      const double lj = Sc[j * NS + j];
-      if (lj < lk || (lj == lk && j < k)) ++rank;
-    }
-    lam[rank] = lk;
-    piv[rank] = k;
-  }
-  team_sync<TEAM>();
-  double* Wm = S1;  // sorted eigenvectors of S (columns), over the diagonalised S
-  for (int it = t; it < NN * NN; it += TEAM) {
-    const int row = it / NN, rank = it % NN;
-    Wm[row * NS + rank] = V[row * NS + piv[rank]];
-  }
-  team_sync<TEAM>();
-  // primary: evec = D^{-1} L^{-T} w ; fallback: evec = D^{-1} L' w
+  // ---- modes and particular solutions, one thread per mode ------------------
   for (int c = t; c < NN; c += TEAM) {
-    if (primary) {
-      for (int r = NN - 1; r >= 0; --r) {
-        double s = Wm[r * NS + c];
-        for (int k = r + 1; k < NN; ++k) s -= LC[k * NS + r] * EV[k * NS + c];
-        EV[r * NS + c] = s / LC[r * NS + r];
+    const double k = mode_k(Sc[c * NS + c]);
+    const double sk = sqrt(k), rsk = 1.0 / sk;
+    // T: L^{-T} u, MA: L u (MA is dead once S is formed)
+    for (int r = NN - 1; r >= 0; --r) {
+      double s = V[r * NS + c];
+      for (int e = r + 1; e < NN; ++e) s -= LC[e * NS + r] * T[e * NS + c];
+      T[r * NS + c] = s / LC[r * NS + r];
+    }
+    for (int r = NN - 1; r >= 0; --r) {
+      double s = 0.0;
+      for (int e = 0; e <= r; ++e) s += LC[r * NS + e] * V[e * NS + c];
+      MA[r * NS + c] = s;
+    }
+    for (int r = 0; r < NN; ++r) {
+      T[r * NS + c] *= sk;
+      MA[r * NS + c] *= rsk;
+    }
+    const double* x = (primary ? MA : T) + c;
+    const double* y = (primary ? T : MA) + c;
+    double* vec = q.lrec + mod_k(N);
+    vec[c] = k;
+    if (beam) {
+      double umu0 = q.rec[H_UMU0];
+      bool res = false;
+      for (int e = 0; e < NN; ++e) res = res || beam_resonant(mode_k(Sc[e * NS + e]), umu0);
+      if (res) umu0 = 0.999 * umu0;
+      if (GEN && (p.flags & DSP_FLAG_SPHERICAL_BEAM)) {
+        // pseudo-spherical beam (general solver): the raw source at the quadrature
+        // angles, up and down, for the user-angle interpolation and
+        // flux_sph_source_kernel (DisortSolver.cpp:1524-1527)
+        const double dm = 0.5 * mu[c] / dsim[c];
+        vec[HP + c] = dm * (b1[c] + b2[c]);
+        vec[2 * HP + c] = dm * (b1[c] - b2[c]);
+      } else {
+        double al = 0.0, be = 0.0;
+        for (int r = 0; r < NN; ++r) {
+          al += x[r * NS] * b1[r];
+          be += y[r * NS] * b2[r];
+        }
+        const double r0 = 1.0 / umu0, den = k * k - r0 * r0;
+        vec[HP + c] = (k * al - be * r0) / den;
+        vec[2 * HP + c] = (k * be - al * r0) / den;
       }
-      for (int r = 0; r < NN; ++r) EV[r * NS + c] *= dinv[r];
-    } else {
-      for (int r = NN - 1; r >= 0; --r) {
-        double s = 0.0;
-        for (int k = 0; k <= r; ++k) s += LC[r * NS + k] * Wm[k * NS + c];
-        EV[r * NS + c] = dinv[r] * s;
-      }
+    }
+    if ((p.flags & DSP_FLAG_THERMAL) && (!GEN || p.g.m == 0)) {
+      double v = 0.0;
+      for (int r = 0; r < NN; ++r) v += x[r * NS] * (dsim[r] / mu[r]);
+      v = 2.0 * (1.0 - ws) * v / k;
+      vec[3 * HP + c] = v;
+      vec[4 * HP + c] = v / k;
+      if (c == 0) thermal_source(q, vec[5 * HP], vec[5 * HP + 1]);
     }
   }
   team_sync<TEAM>();
-  // ---- k, G+/-  (FluxSolver.cpp:561-587) ---------------------------------
-  double* lrec;
-  if constexpr (GEN) lrec = p.layer_rec + task * p.g.lstride;
-  else lrec = p.layer_rec + ((long long)i * p.L + lc) * lrec_stride(N);
-  for (int k = t; k < NN; k += TEAM) {
-    const double kr = sqrt(fabs(lam[k]));
-    lamraw[k] = lam[k];
-    lam[k] = kr;
-    lrec[lrec_eig(N) + k + NN] = kr;
-    lrec[lrec_eig(N) + NN - 1 - k] = -kr;
-  }
-  team_sync<TEAM>();
-  for (int it = t; it < NN * NN; it += TEAM) {
-    const int iq = it / NN, jq = it % NN;
-    double s = 0.0;
-    for (int k = 0; k < NN; ++k) s += AMB[iq * NS + k] * EV[k * NS + jq];
-    const double gpplgm = s / lam[jq];
-    const double gpmigm = EV[iq * NS + jq];
-    double* G = lrec + lrec_G(N);
-    G[(NN + iq) * N + NN + jq] = 0.5 * (gpplgm + gpmigm);
-    G[(NN - iq - 1) * N + NN + jq] = 0.5 * (gpplgm - gpmigm);
-    G[(NN + iq) * N + NN - jq - 1] = 0.5 * (-gpplgm + gpmigm);
-    G[(NN - iq - 1) * N + NN - jq - 1] = 0.5 * (-gpplgm - gpmigm);
-  }
-  team_sync<TEAM>();
-  DSP_PHASE(5)
-
-  // ---- particular solutions in the eigen basis ------------------------------
-  // The reference factors the N x N matrices I - C and I + diag(mu)/mu0 - C with
-  // a partial-pivot LU (FluxSolver.cpp:634, :758).  With s = z+ + z-, d = z+ - z-
-  // and M = diag(mu_1..mu_NN) these split into the NN x NN blocks
-  //   I - P - Q = -M (a+b),   I - P + Q = -M (a-b),
-  // whose inverses the eigensystem already provides:
-  //   (a+b)^{-1} = D^{-1} A_s^{-1} D,  (a-b)^{-1} = D^{-1} B_s^{-1} D,
-  //   primary  (-B_s = L L^T, L^T(-A_s)L = W Lam W^T):
-  //     B_s^{-1} = -L^{-T} L^{-1},   A_s^{-1} = -L W Lam^{-1} W^T L^T;
-  //   fallback (-A_s = L L^T, L^T(-B_s)L = W Lam W^T): the two roles swap.
-  // The beam matrix reduces to (a-b)(a+b) - mu0^{-2} = D^{-1}(B_s A_s - mu0^{-2})D,
-  // diagonal in the same basis: B_s A_s = L W Lam W^T L^{-1} (primary) or
-  // L^{-T} W Lam W^T L^T (fallback); its singular points are the reference's
-  // dithering condition |1 - mu0^2 k^2| ~ 0 (FluxSolver.cpp:610-618).
-  double* scratch = zv;
-  const double dt_ = (t < NN) ? dsim[t] : 1.0;
-  const double di_ = (t < NN) ? dinv[t] : 1.0;
-  const double mui = (t < NN) ? mu[t] : 1.0;
-  const double lami = (t < NN) ? lamraw[t] : 1.0;
-  // X1 x = -L^{-T} L^{-1} x ;  X2 x = -L W Lam^{-1} W^T L^T x   (shift: Lam -> Lam - shift)
-  auto applyX1 = [&](double x) {
-    x = team_trsv<NN, NS, TEAM>(LC, x, false, t, scratch);
-    x = team_trsv<NN, NS, TEAM>(LC, x, true, t, scratch);
-    return -x;
-  };
-  auto applyX2 = [&](double x) {
-    x = team_matvec<NN, NS, TEAM>(LC, x, true, 1, t, scratch);   // L^T x
-    x = team_matvec<NN, NS, TEAM>(Wm, x, true, 0, t, scratch);   // W^T
-    x = x / lami;
-    x = team_matvec<NN, NS, TEAM>(Wm, x, false, 0, t, scratch);  // W
-    x = team_matvec<NN, NS, TEAM>(LC, x, false, 1, t, scratch);  // L
-    return -x;
-  };
-  // (a+b)^{-1} y and (a-b)^{-1} y
-  auto inv_apb = [&](double y) {
-    const double x = dt_ * y;
-    return di_ * (primary ? applyX2(x) : applyX1(x));
-  };
-  auto inv_amb = [&](double y) {
-    const double x = dt_ * y;
-    return di_ * (primary ? applyX1(x) : applyX2(x));
-  };
-
-  const double fbeam = rec[H_FBEAM];
-  if (fbeam > 0.0) {
-    // ---- beam (computeBeamSource, FluxSolver.cpp:595-643) -----------------
-    // source coefficients zj in bv
-    const double umu0 = rec[H_UMU0];
-    const double* yb;
-    if constexpr (GEN) {
-      // P_l^m(-mu0) of this mode (DisortSolver.cpp:1334-1335); Y rows l < m are zero
-      double* ybm = sm + C::O_GX;
-      if (t == 0) legendre_column(p.g.m, -umu0, N - 1, ybm, 1);
-      team_sync<TEAM>();
-      yb = ybm;
-    } else {
-      yb = rec + il.yb;
-    }
-    // (2 - delta_m0) F0 sum_k g'_k P_k^m(mu_r) P_k^m(-mu0) / 4pi (DisortSolver.cpp:1361-1368)
-    const double bfac = (GEN && p.g.m > 0) ? 2.0 * fbeam : fbeam;
-    for (int r = t; r < N; r += TEAM) {
-      double sacc = 0.0;
-      for (int k = 0; k < N; ++k) sacc += gl[k] * Y[k * N + r] * yb[k];
-      bv[r] = bfac * sacc / (4.0 * 3.14159265358979323846);
-    }
-    team_sync<TEAM>();
-  }
-  if (fbeam > 0.0 && GEN && (p.flags & DSP_FLAG_SPHERICAL_BEAM)) {
-    // pseudo-spherical beam (general solver): the source coefficients zj go to
-    // the particular-solution slot in its row order, where the user-angle
-    // interpolation reads them (computeBeamSourceSpherical keeps the raw zj
-    // for interpSource, DisortSolver.cpp:1524-1527); gen_sph_source_kernel
-    // then replaces them with Z0
-    if (t < NN) {
-      lrec[lrec_zb(N) + NN + t] = bv[t];
-      lrec[lrec_zb(N) + NN - t - 1] = bv[NN + t];
-    }
-    team_sync<TEAM>();
-  } else if (fbeam > 0.0) {
-    const double umu0 = rec[H_UMU0];
-    double beam_mu = umu0;
-    const double mu0sq = umu0 * umu0;
-    const double dither = 1000.0 * 2.220446049250313e-16;
-    bool dith = false;
-    for (int k = 0; k < NN; ++k) {
-      const double kk = lam[k];
-      if (fabs(1.0 - mu0sq * kk * kk) < dither) dith = true;
-    }
-    if (dith) beam_mu = 0.999 * umu0;
-    const double bp = (t < NN) ? bv[t] : 0.0, bm = (t < NN) ? bv[NN + t] : 0.0;
-    const double m1 = (bp + bm) / mui;  // M^{-1} r1
-    const double m2 = (bp - bm) / mui;  // M^{-1} r2
-    // rhs = mu0^{-1} M^{-1} r2 + (a-b) M^{-1} r1
-    double y = m2 / beam_mu + team_matvec<NN, NS, TEAM>(AMB, m1, false, 0, t, scratch);
-    // s = -(D^{-1} (B_s A_s - mu0^{-2})^{-1} D) y
-    const double shift = 1.0 / (beam_mu * beam_mu);
-    double x = dt_ * y;
-    if (primary) {
-      x = team_trsv<NN, NS, TEAM>(LC, x, false, t, scratch);          // L^{-1}
-      x = team_matvec<NN, NS, TEAM>(Wm, x, true, 0, t, scratch);       // W^T
-      x = x / (lami - shift);
-      x = team_matvec<NN, NS, TEAM>(Wm, x, false, 0, t, scratch);      // W
-      x = team_matvec<NN, NS, TEAM>(LC, x, false, 1, t, scratch);      // L
-    } else {
-      x = team_matvec<NN, NS, TEAM>(LC, x, true, 1, t, scratch);       // L^T
-      x = team_matvec<NN, NS, TEAM>(Wm, x, true, 0, t, scratch);       // W^T
-      x = x / (lami - shift);
-      x = team_matvec<NN, NS, TEAM>(Wm, x, false, 0, t, scratch);      // W
-      x = team_trsv<NN, NS, TEAM>(LC, x, true, t, scratch);            // L^{-T}
-    }
-    const double sv = -di_ * x;
-    // d = mu0 ((a+b) s + M^{-1} r1)
-    const double dv = beam_mu * (team_matvec<NN, NS, TEAM>(APB, sv, false, 0, t, scratch) + m1);
-    if (t < NN) {
-      lrec[lrec_zb(N) + NN + t] = 0.5 * (sv + dv);      // z+ (quadrature index t)
-      lrec[lrec_zb(N) + NN - t - 1] = 0.5 * (sv - dv);  // z- (quadrature index NN+t)
-    }
-    team_sync<TEAM>();
-  }
-  const bool thermal_src = (p.flags & DSP_FLAG_THERMAL) && (!GEN || p.g.m == 0);
-  if (thermal_src) {
-    // ---- thermal (computeIsotropicSource, FluxSolver.cpp:745-787) ---------
-    // Z1 solves (I-C) z = (1-w') xr1 (isotropic: d1 = 0); Z0 solves
-    // (I-C) z = (1-w') xr0 + mu Z1, i.e. r1 = 2(1-w') xr0, r2 = M s1.
-    const double taus_top = rec[il.tau_s + lc];
-    const double pk0 = rec[il.pkag + lc], pk1 = rec[il.pkag + lc + 1];
-    double xr1 = 0.0;
-    if (dts > 1e-4) xr1 = (pk1 - pk0) / dts;
-    const double xr0 = pk0 - xr1 * taus_top;
-    // omega' = 1: no thermal source; (a+b) is singular there, so skip it (uniform per team)
-    const bool src = (1.0 - ws) != 0.0;
-    const double u = src ? -inv_apb(1.0 / mui) : 0.0;  // -(a+b)^{-1} M^{-1} 1
-    const double s1 = 2.0 * (1.0 - ws) * xr1 * u;
-    const double s0 = 2.0 * (1.0 - ws) * xr0 * u;
-    const double d0 = src ? -inv_amb(s1) : 0.0;        // -(a-b)^{-1} M^{-1} (M s1)
-    if (t < NN) {
-      lrec[lrec_z1(N) + NN + t] = 0.5 * s1;
-      lrec[lrec_z1(N) + NN - t - 1] = 0.5 * s1;
-      lrec[lrec_z0(N) + NN + t] = 0.5 * (s0 + d0);
-      lrec[lrec_z0(N) + NN - t - 1] = 0.5 * (s0 - d0);
-    }
-    if (t == 0) {
-      lrec[lrec_xr(N)] = xr0;
-      lrec[lrec_xr(N) + 1] = xr1;
-    }
-    if constexpr (JAC) {
-      // the source per unit intercept (P) and slope (Q) for the temperature
-      // Jacobian: s0 = xr0 P, d0 = xr1 Q
-      const double P = 2.0 * (1.0 - ws) * u;
-      const double Q = src ? -inv_amb(P) : 0.0;
-      if (t < NN) {
-        p.jac_pq[task * jpq_stride(N) + t] = P;
-        p.jac_pq[task * jpq_stride(N) + NN + t] = Q;
-      }
+  {
+    const double* X = primary ? MA : T;
+    const double* Yv = primary ? T : MA;
+    for (int it = t; it < NN * HP; it += TEAM) {
+      const int c = it / HP, r = it % HP;
+      q.lrec[mod_X(N) + it] = r < NN ? X[r * NS + c] : 0.0;
+      q.lrec[mod_Y(N) + it] = r < NN ? Yv[r * NS + c] : 0.0;
     }
   }
-  DSP_PHASE(7)
-  if constexpr (GEN) {
-    if (p.g.numu > 0) gen_user_angles<N>(p, i, sm, Y, wt, gl, lrec, rec[H_FBEAM], ws, thermal_src, t);
-  }
-  DSP_PHASE(8)
-  DSP_PHASE_END
 }
-
 
 // The rotation of jacobi_rot from two reciprocal square roots, without branches
 // or divisions (a sweep is then one scheduling region): with
@@ -965,14 +648,6 @@ __device__ __forceinline__ void jacobi_rot_rsq(double apq, double app, double aq
   tt = rot ? sv * g : 0.0;
 }
 
-// ---------------------------------------------------------------------------
-// Front of a split layer stage, one thread per layer task (the STAGE before the
-// eigensolver): scaled phase coefficients (disortSet, FluxSolver.cpp:336-386),
-// the phase sums, alpha -/+ beta in the symmetric form of the reference
-// (FluxSolver.cpp:466-514), the Cholesky factorisation of -B_s, else of -A_s
-// (:521-558), and S = L^T M L, written to the hand-off.  Every matrix is a
-// packed symmetric NN x NN in registers; the tables are constant-bank operands.
-// ---------------------------------------------------------------------------
 // Cholesky of a packed lower triangle in place; false when a pivot is not
 // positive (the factor is then not used).  The updates are subtracted in the
 // order of the right-looking form and the column is divided by its pivot, as
@@ -1000,70 +675,81 @@ __device__ __forceinline__ bool chol_packed(double* A) {
   return ok;
 }
 
-template <int N>
+// ---------------------------------------------------------------------------
+// Front of a split layer stage, one thread per layer task: scaled phase
+// coefficients (disortSet, FluxSolver.cpp:336-386), the phase sums, alpha -/+ beta
+// in the symmetric form of the reference (FluxSolver.cpp:466-514), the Cholesky
+// factorisation of -B_s, else of -A_s (:521-558), S = L^T M L and the beam's
+// source vectors, written to the hand-off.  Every matrix is a packed symmetric
+// h x h in registers; the tables are constant-bank operands.
+// ---------------------------------------------------------------------------
+template <int N, bool GEN>
 __global__ void __launch_bounds__(128) flux_layer_front_kernel(FluxParams p, ConstTab<N> tc) {
   constexpr int NN = N / 2;
-  using H = Handoff<NN>;
-  constexpr int TRI = H::TRI;
-  const long long nt = (long long)p.n * p.L;
+  using HO = Handoff<NN>;
+  constexpr int TRI = HO::TRI;
+  const long long nt = layer_tasks<GEN>(p);
   const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= nt) return;
   auto hp = [&](int e) { return handoff_lane<NN>(p.bvp_rec, nt, j, e); };
-  const int i = (int)(j / p.L), lc = (int)(j % p.L);
-  const double* rec = p.inst_rec + (long long)i * p.il.stride;
-  const InstLayout& il = p.il;
-  // the layer's inputs are requested before the test that may skip it
-  const int lin = (p.flags & DSP_FLAG_INDEX_FROM_BOTTOM) ? p.L - 1 - lc : lc;
-  const double* pml = p.pmom.row(i) + (long long)lin * p.pc;
-  double pmk[N];
-#pragma unroll
-  for (int k = 0; k < N; ++k) pmk[k] = pml[k];
-  const double ws = rec[il.ssa_s + lc];
-  const bool beam = rec[H_FBEAM] > 0.0;
-  const int mode = (int)rec[il.mode + lc];
-  const double f = rec[il.fsc + lc], sig = rec[il.sig + lc];
-  // invalid instances and layers below the absorption cut are not solved
-  if ((p.status && p.status[i] == DSP_ERR_INVALID_INPUT) || lc >= (int)rec[H_NCUT]) {
-    *hp(H::S_FLAG) = 0.0;
+  const LayerTask<N, GEN> q = layer_task<N, GEN>(p, j);
+  if (!q.live) {
+    *hp(HO::S_FLAG) = 0.0;
     return;
   }
-  // ---- phase sums O (odd orders) and E (even orders) ----------------------
+  const double ws = q.rec[q.il.ssa_s + q.lc];
+  // ---- phase sums of odd (O) and even (E) l + m ----------------------------
   double O[TRI], E[TRI];
   {
     double gl[N];
+    const int mode = (int)q.rec[q.il.mode + q.lc];
+    const double f = q.rec[q.il.fsc + q.lc], sig = q.rec[q.il.sig + q.lc];
 #pragma unroll
-    for (int k = 0; k < N; ++k) {
-      const double pk = pmk[k];
-      double g;
-      if (mode == 0) g = (2.0 * k + 1.0) * ws * pk;
-      else if (mode == 1) g = (2.0 * k + 1.0) * ws * (pk - f) / (1.0 - f);
-      else {
-        const double kd = (double)k;
-        g = (2.0 * k + 1.0) * ws * (pk - f * exp(-kd * kd / (2.0 * sig))) / (1.0 - f);
-      }
-      gl[k] = g;
-    }
+    for (int k = 0; k < N; ++k) gl[k] = phase_coeff<GEN>(k, q.pml[k], mode, ws, f, sig);
 #pragma unroll
     for (int a = 0; a < NN; ++a) {
       double z[N];
 #pragma unroll
-      for (int l = 0; l < N; ++l) z[l] = gl[l] * tc.y[l * N + a];
+      for (int l = 0; l < N; ++l) z[l] = gl[l] * tc.y[l * NN + a];
 #pragma unroll
       for (int b = 0; b <= a; ++b) {
         double se = 0.0, so = 0.0;
 #pragma unroll
-        for (int l = 0; l < N; l += 2) se += z[l] * tc.y[l * N + b];
+        for (int l = 0; l < N; l += 2) se += z[l] * tc.y[l * NN + b];
 #pragma unroll
-        for (int l = 1; l < N; l += 2) so += z[l] * tc.y[l * N + b];
+        for (int l = 1; l < N; l += 2) so += z[l] * tc.y[l * NN + b];
         E[tri_idx(a, b)] = se;
         O[tri_idx(a, b)] = so;
       }
     }
-  }
+    const double fbeam = q.rec[H_FBEAM];
+    const bool swap = GEN && (p.g.m & 1);
+    if (fbeam > 0.0) {
+      // (2 - delta_m0) F0 / 4pi sum_k g'_k P_k^m(mu_r) P_k^m(-mu0) by parity (DisortSolver.cpp:1361-1368)
+      const double* yb = beam_legendre<N, GEN>(p, q);
 #pragma unroll
-  for (int e = 0; e < TRI; ++e) {
-    *hp(H::S_O + e) = O[e];
-    if (beam) *hp(H::S_E + e) = E[e];
+      for (int k = 0; k < N; ++k) gl[k] *= yb[k];
+      const double fac = ((GEN && p.g.m > 0) ? 4.0 : 2.0) * fbeam / (4.0 * 3.14159265358979323846);
+#pragma unroll
+      for (int r = 0; r < NN; ++r) {
+        double se = 0.0, so = 0.0;
+#pragma unroll
+        for (int l = 0; l < N; l += 2) se += gl[l] * tc.y[l * NN + r];
+#pragma unroll
+        for (int l = 1; l < N; l += 2) so += gl[l] * tc.y[l * NN + r];
+        const double dm = tc.dsim[r] * tc.rmu[r] * fac;
+        *hp(HO::S_B1 + r) = dm * (swap ? so : se);
+        *hp(HO::S_B2 + r) = dm * (swap ? se : so);
+      }
+    }
+    if (swap) {
+#pragma unroll
+      for (int e = 0; e < TRI; ++e) {
+        const double x = O[e];
+        O[e] = E[e];
+        E[e] = x;
+      }
+    }
   }
   // -B_s = -D (a-b) D^{-1} and -A_s = -D (a+b) D^{-1} (packed lower; both symmetric)
   auto minus_s = [&](const double* P, double* X) {
@@ -1075,28 +761,23 @@ __global__ void __launch_bounds__(128) flux_layer_front_kernel(FluxParams p, Con
         X[tri_idx(r, c)] = -tc.dsim[r] * a * tc.dinv[c];
       }
   };
-  // ---- Cholesky of -B_s, else of -A_s, else of -B_s regardless of omega' --
+  // ---- Cholesky of -B_s, else of -A_s --------------------------------------
   double Lf[TRI];
-  bool primary = ws < 1.0 - 1e-12;
-  if (primary) {
-    minus_s(O, Lf);
-    primary = chol_packed<NN>(Lf);
-  }
+  minus_s(O, Lf);
+  const bool primary = chol_packed<NN>(Lf);
   if (!primary) {
     minus_s(E, Lf);
     if (!chol_packed<NN>(Lf)) {
-      minus_s(O, Lf);
-      primary = chol_packed<NN>(Lf);
-      if (!primary) {
-        set_status(p.status, i, DSP_ERR_EIGEN);
-        *hp(H::S_FLAG) = 0.0;
-        return;
-      }
+      set_status(p.status, q.i, DSP_ERR_EIGEN);
+      *hp(HO::S_FLAG) = 0.0;
+      return;
     }
   }
   // ---- S = L^T M L, M = -A_s (primary) or -B_s (fallback), by columns ----
   double M[TRI];
-  minus_s(primary ? E : O, M);
+#pragma unroll
+  for (int e = 0; e < TRI; ++e) E[e] = primary ? E[e] : O[e];
+  minus_s(E, M);
 #pragma unroll
   for (int c = 0; c < NN; ++c) {
     double t[NN];  // (M L)[:, c]; L[k][c] = 0 for k < c
@@ -1112,12 +793,12 @@ __global__ void __launch_bounds__(128) flux_layer_front_kernel(FluxParams p, Con
       double s = 0.0;
 #pragma unroll
       for (int k = r; k < NN; ++k) s += Lf[tri_idx(k, r)] * t[k];
-      *hp(H::S_S + tri_idx(r, c)) = s;
+      *hp(HO::S_S + tri_idx(r, c)) = s;
     }
   }
 #pragma unroll
-  for (int e = 0; e < TRI; ++e) *hp(H::S_L + e) = Lf[e];
-  *hp(H::S_FLAG) = primary ? 1.0 : 2.0;
+  for (int e = 0; e < TRI; ++e) *hp(HO::S_L + e) = Lf[e];
+  *hp(HO::S_FLAG) = primary ? 1.0 : 2.0;
 }
 
 // Rotation of the pair (p, q) applied to S (packed lower, both sides) and to the
@@ -1185,120 +866,35 @@ __device__ __forceinline__ void jacobi_sweeps(double* S, double* V, bool act) {
   }
 }
 
-// Eigensolver of the split layer stage: one thread per layer task, S from the
-// hand-off into registers, jacobi_sweeps, the diagonal and the eigenvectors
-// back to the hand-off.  (Fusing it into the front kernel, S staying in
-// registers, was slower: 4.30 against 4.03 ms for the layer stage of a
-// 20,000-band thermal step.)
-template <int NN>
-__global__ void __launch_bounds__(128) flux_jacobi_kernel(FluxParams p) {
-  using H = Handoff<NN>;
-  constexpr int NNP = NN + (NN & 1), NPAIR = NNP / 2;
-  const long long nt = (long long)p.n * p.L;
-  const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j - (threadIdx.x & 31) >= nt) return;  // whole warp past the end (warp-uniform)
-  const bool in = j < nt;
-  double* const flag = handoff_lane<NN>(p.bvp_rec, nt, in ? j : nt - 1, H::S_FLAG);
-  const bool act = in && *flag != 0.0;
-  double S[H::TRI], V[NN * NN];
-#pragma unroll
-  for (int e = 0; e < H::TRI; ++e) S[e] = act ? *handoff_lane<NN>(p.bvp_rec, nt, j, H::S_S + e) : 0.0;
-#pragma unroll
-  for (int e = 0; e < NN * NN; ++e) V[e] = (e / NN == e % NN) ? 1.0 : 0.0;
-  jacobi_sweeps<NN>(S, V, act);
-  if (!act) return;
-#pragma unroll
-  for (int k = 0; k < NN; ++k) *handoff_lane<NN>(p.bvp_rec, nt, j, H::S_D + k) = S[tri_idx(k, k)];
-#pragma unroll
-  for (int e = 0; e < NN * NN; ++e) *handoff_lane<NN>(p.bvp_rec, nt, j, H::S_V + e) = V[e];
-}
-
-// ---------------------------------------------------------------------------
-// Back of a split layer stage, one thread per layer task: from the eigenpairs
-// of S to the layer record (the STAGE 0 kernel's steps after its Jacobi loop:
-// FluxSolver.cpp:561-587 for k and G+/-, :595-643 and :745-787 for the
-// particular solutions, in the eigen basis described there).  NN x NN operands
-// are held in registers with compile-time indices or read from the
-// lane-interleaved hand-off, whose loads are coalesced across the warp; the
-// Cholesky factor is read again by each phase that needs it (registers, not
-// bandwidth, bound a one-thread task).  Eigenpairs stay in the eigensolver's
-// order: the rank of each eigenvalue in the ascending order places its column
-// of G and its k, and the sums over eigenpairs (W Lam^{-1} W^T) do not depend
-// on the order.
-// ---------------------------------------------------------------------------
-template <int NN>
-struct BackOps {
-  const double* L;    // packed lower
-  const double* rdg;  // 1 / L_kk
-  // x <- L^{-1} x
-  __device__ __forceinline__ void fwd(double* x) const {
-#pragma unroll
-    for (int k = 0; k < NN; ++k) {
-      x[k] *= rdg[k];
-#pragma unroll
-      for (int r = k + 1; r < NN; ++r) x[r] -= L[tri_idx(r, k)] * x[k];
-    }
-  }
-  // x <- L^{-T} x
-  __device__ __forceinline__ void bwd(double* x) const {
-#pragma unroll
-    for (int k = NN - 1; k >= 0; --k) {
-      x[k] *= rdg[k];
-#pragma unroll
-      for (int r = 0; r < k; ++r) x[r] -= L[tri_idx(k, r)] * x[k];
-    }
-  }
-  // x <- L x
-  __device__ __forceinline__ void lmul(double* x) const {
-#pragma unroll
-    for (int r = NN - 1; r >= 0; --r) {
-      double s = 0.0;
-#pragma unroll
-      for (int c = 0; c <= r; ++c) s += L[tri_idx(r, c)] * x[c];
-      x[r] = s;
-    }
-  }
-  // x <- L^T x
-  __device__ __forceinline__ void ltmul(double* x) const {
-#pragma unroll
-    for (int r = 0; r < NN; ++r) {
-      double s = 0.0;
-#pragma unroll
-      for (int k = r; k < NN; ++k) s += L[tri_idx(k, r)] * x[k];
-      x[r] = s;
-    }
-  }
+// Eigensolver and output of the split layer stage, one thread per layer task: S
+// from the hand-off into registers, jacobi_sweeps, then mode by mode X and Y
+// (from the eigenvector and the Cholesky factor), k and the particular solutions
+// in the modes.  The layer record is staged per warp in shared memory and written
+// with consecutive lanes on consecutive doubles.  (An eigensolver that writes its
+// vectors to the hand-off for a third launch to read again spent a third of the
+// layer stage on those reads.)
+template <int N>
+struct ECfg {
+  static constexpr int HP = mod_hp(N);
+  static constexpr int RS = 2 * HP + 1;   // staging row: one mode's X and Y
+  static constexpr int VS = 5 * HP + 3;   // staging row: the vectors
+  static constexpr int WARP = 32 * (RS + VS);
+  static constexpr size_t smem_bytes(int cta) { return sizeof(double) * (size_t)(cta / 32) * WARP; }
 };
 
-// The warp's 32 tasks have consecutive layer records; a row of W doubles that
-// each lane has put at stg[lane * RS + k] is written for every task of `ok`
-// with consecutive lanes on consecutive doubles (32 / W tasks per store).
-template <int RS>
-__device__ __forceinline__ void warp_flush_rows(const double* stg, double* rec0, int rstride, int W, int off,
-                                                unsigned ok, int lane) {
-  __syncwarp();
-  const int tpi = 32 / W;
-  const int tl = lane / W, k = lane - tl * W;
-  if (tl < tpi)
-    for (int b = tl; b < 32; b += tpi)
-      if ((ok >> b) & 1u) rec0[(long long)b * rstride + off + k] = stg[b * RS + k];
-  __syncwarp();
-}
-
-template <int N, bool JAC = false>
-__global__ void __launch_bounds__(128) flux_layer_back_kernel(FluxParams p, ConstTab<N> tc) {
+template <int N, bool GEN>
+__global__ void __launch_bounds__(128) flux_eigen_kernel(FluxParams p, ConstTab<N> tc) {
   constexpr int NN = N / 2;
-  constexpr int RS = N + 3;  // staging row stride: a row of N (+2 for xr after z1)
-  constexpr int LS = lrec_stride(N);
-  using H = Handoff<NN>;
-  constexpr double PI = 3.14159265358979323846;
-  __shared__ double stage[4][2][32 * RS];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const double* const stA = stage[wid][0];
-  const double* const stB = stage[wid][1];
-  double* const sA = stage[wid][0] + lane * RS;
-  double* const sB = stage[wid][1] + lane * RS;
-  const long long nt = (long long)p.n * p.L;
+  using HO = Handoff<NN>;
+  using C = ECfg<N>;
+  constexpr int HP = C::HP, RS = C::RS, VS = C::VS;
+  extern __shared__ double smem[];
+  const int lane = threadIdx.x & 31;
+  double* const stg = smem + (threadIdx.x >> 5) * C::WARP;
+  double* const vst = stg + 32 * RS;
+  double* const row = stg + lane * RS;
+  double* const vrow = vst + lane * VS;
+  const long long nt = layer_tasks<GEN>(p);
   const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long j0 = j - lane;
   if (j0 >= nt) return;  // whole warp past the end (warp-uniform)
@@ -1306,318 +902,155 @@ __global__ void __launch_bounds__(128) flux_layer_back_kernel(FluxParams p, Cons
   // addresses and write nothing (no early exit: the warp writes rows together)
   const long long jj = j < nt ? j : nt - 1;
   auto hv = [&](int e) { return *handoff_lane<NN>(p.bvp_rec, nt, jj, e); };
-  // the hand-off operands of the eigenvector phase are all requested up front,
-  // so that their latency overlaps the ordering of the eigenvalues
-  double d[NN], L[H::TRI], rdg[NN], EV[NN][NN];  // EV[c][r]: column c
-  const double flag = hv(H::S_FLAG);
-#pragma unroll
-  for (int k = 0; k < NN; ++k) d[k] = hv(H::S_D + k);
-#pragma unroll
-  for (int e = 0; e < H::TRI; ++e) L[e] = hv(H::S_L + e);
-#pragma unroll
-  for (int c = 0; c < NN; ++c)
-#pragma unroll
-    for (int r = 0; r < NN; ++r) EV[c][r] = hv(H::S_V + r * NN + c);
+  const double flag = hv(HO::S_FLAG);
   const bool act = j < nt && flag != 0.0;  // skipped: cut layer, invalid input, no factorisation
   const unsigned okm = __ballot_sync(0xffffffffu, act);
   if (okm == 0u) return;  // warp-uniform
+  double S[HO::TRI], V[NN * NN];
+#pragma unroll
+  for (int e = 0; e < HO::TRI; ++e) S[e] = act ? hv(HO::S_S + e) : 0.0;
+#pragma unroll
+  for (int e = 0; e < NN * NN; ++e) V[e] = (e / NN == e % NN) ? 1.0 : 0.0;
+  jacobi_sweeps<NN>(S, V, act);
+
   const bool primary = flag == 1.0;
-  const int i = (int)(jj / p.L), lc = (int)(jj % p.L);
-  const double* rec = p.inst_rec + (long long)i * p.il.stride;
-  const InstLayout& il = p.il;
-  double* const rec0 = p.layer_rec + j0 * LS;
-
-  // ---- ascending order of the eigenvalues; k = sqrt|lambda| ----------------
-  double kr[NN], rk[NN];
-  int rank[NN];
-  {
+  const LayerTask<N, GEN> q = layer_task<N, GEN>(p, jj);
+  const double fbeam = act ? q.rec[H_FBEAM] : 0.0;
+  const bool beam = fbeam > 0.0;
+  const bool raw = GEN && (p.flags & DSP_FLAG_SPHERICAL_BEAM);
+  const bool thermal = (p.flags & DSP_FLAG_THERMAL) && (!GEN || p.g.m == 0);
+  double r0 = 0.0;
+  if (beam) {
+    double umu0 = q.rec[H_UMU0];
+    bool res = false;
 #pragma unroll
-    for (int k = 0; k < NN; ++k) {
-      int r = 0;
-#pragma unroll
-      for (int q = 0; q < NN; ++q)
-        if (d[q] < d[k] || (d[q] == d[k] && q < k)) ++r;
-      rank[k] = r;
-      kr[k] = sqrt(fabs(d[k]));
-      rk[k] = 1.0 / kr[k];
-      sA[NN + r] = kr[k];
-      sA[NN - 1 - r] = -kr[k];
-    }
+    for (int c = 0; c < NN; ++c) res = res || beam_resonant(mode_k(S[tri_idx(c, c)]), umu0);
+    if (res) umu0 = 0.999 * umu0;
+    r0 = 1.0 / umu0;
   }
-  warp_flush_rows<RS>(stA, rec0, LS, N, lrec_eig(N), okm, lane);
-  auto load_L = [&]() {
+  const double ws2 = act ? 2.0 * (1.0 - q.rec[q.il.ssa_s + q.lc]) : 0.0;
+  double L[HO::TRI];
 #pragma unroll
-    for (int e = 0; e < H::TRI; ++e) L[e] = hv(H::S_L + e);
+  for (int e = 0; e < HO::TRI; ++e) L[e] = act ? hv(HO::S_L + e) : 1.0;
+  double rdg[NN];
 #pragma unroll
-    for (int k = 0; k < NN; ++k) rdg[k] = 1.0 / L[tri_idx(k, k)];
-  };
-  const BackOps<NN> ops{L, rdg};
-  {
-    // ---- eigenvectors of (a+b)(a-b): D^{-1} L^{-T} w (primary), D^{-1} L w --
+  for (int k = 0; k < NN; ++k) rdg[k] = 1.0 / L[tri_idx(k, k)];
+  const long long ls = GEN ? p.g.lstride : (long long)lrec_stride(N);
+  double* const rec0 = p.layer_rec + j0 * ls;
 #pragma unroll
-    for (int k = 0; k < NN; ++k) rdg[k] = 1.0 / L[tri_idx(k, k)];
+  for (int c = 0; c < NN; ++c) {
+    const double k = mode_k(S[tri_idx(c, c)]);
+    const double sk = sqrt(k), rsk = 1.0 / sk;
+    double x[NN], y[NN];
+    // y = L^{-T} u, x = L u
 #pragma unroll
-    for (int c = 0; c < NN; ++c) {
-      if (primary) ops.bwd(EV[c]);
-      else ops.lmul(EV[c]);
+    for (int r = 0; r < NN; ++r) y[r] = V[r * NN + c];
 #pragma unroll
-      for (int r = 0; r < NN; ++r) EV[c][r] *= tc.dinv[r];
+    for (int e = NN - 1; e >= 0; --e) {
+      y[e] *= rdg[e];
+#pragma unroll
+      for (int r = 0; r < e; ++r) y[r] -= L[tri_idx(e, r)] * y[e];
     }
-    // ---- G+/- (FluxSolver.cpp:575-587), two rows per step -------------------
-    // row iq of O is loaded one step ahead
-    double orow[NN];
-#pragma unroll
-    for (int k = 0; k < NN; ++k) orow[k] = hv(H::S_O + tri_idx(0, k));
-#pragma unroll 1
-    for (int iq = 0; iq < NN; ++iq) {
-      // row iq of alpha - beta = M^{-1} (O W - I)
-      double rm = 0.0, arow[NN];
-#pragma unroll
-      for (int k = 0; k < NN; ++k) rm = (k == iq) ? tc.rmu[k] : rm;
-#pragma unroll
-      for (int k = 0; k < NN; ++k) arow[k] = (tc.wt[k] * orow[k]) * rm - (k == iq ? rm : 0.0);
-      const int iqn = iq + 1 < NN ? iq + 1 : iq;
-#pragma unroll
-      for (int k = 0; k < NN; ++k) orow[k] = hv(H::S_O + tri_idx(iqn, k));
-      double* g0 = sA;  // row NN + iq
-      double* g1 = sB;  // row NN - iq - 1
-#pragma unroll
-      for (int c = 0; c < NN; ++c) {
-        double s = 0.0, gpmigm = 0.0;
-#pragma unroll
-        for (int k = 0; k < NN; ++k) {
-          s += arow[k] * EV[c][k];
-          gpmigm = (k == iq) ? EV[c][k] : gpmigm;
-        }
-        const double gpplgm = s * rk[c];
-        const int jq = rank[c];
-        g0[NN + jq] = 0.5 * (gpplgm + gpmigm);
-        g1[NN + jq] = 0.5 * (gpplgm - gpmigm);
-        g0[NN - jq - 1] = 0.5 * (-gpplgm + gpmigm);
-        g1[NN - jq - 1] = 0.5 * (-gpplgm - gpmigm);
-      }
-      warp_flush_rows<RS>(stA, rec0, LS, N, lrec_G(N) + (NN + iq) * N, okm, lane);
-      warp_flush_rows<RS>(stB, rec0, LS, N, lrec_G(N) + (NN - iq - 1) * N, okm, lane);
-    }
-  }
-  // x <- V diag(1 / (d - shift)) V^T x, one eigenpair at a time
-  auto vsolve = [&](double* x, double shift) {
-    double acc[NN];
-#pragma unroll
-    for (int r = 0; r < NN; ++r) acc[r] = 0.0;
-#pragma unroll 2
-    for (int c = 0; c < NN; ++c) {
-      double v[NN], s = 0.0;
-#pragma unroll
-      for (int r = 0; r < NN; ++r) {
-        v[r] = hv(H::S_V + r * NN + c);
-        s += v[r] * x[r];
-      }
-      const double coef = s / (hv(H::S_D + c) - shift);
-#pragma unroll
-      for (int r = 0; r < NN; ++r) acc[r] += coef * v[r];
-    }
-#pragma unroll
-    for (int r = 0; r < NN; ++r) x[r] = acc[r];
-  };
-  // X1 x = -L^{-T} L^{-1} x ;  X2 x = -L W Lam^{-1} W^T L^T x
-  auto applyX1 = [&](double* x) {
-    ops.fwd(x);
-    ops.bwd(x);
-#pragma unroll
-    for (int r = 0; r < NN; ++r) x[r] = -x[r];
-  };
-  auto applyX2 = [&](double* x) {
-    ops.ltmul(x);
-    vsolve(x, 0.0);
-    ops.lmul(x);
-#pragma unroll
-    for (int r = 0; r < NN; ++r) x[r] = -x[r];
-  };
-
-  const double ws = rec[il.ssa_s + lc];
-  const double dts = rec[il.dtau_s + lc];
-  const double fbeam = rec[H_FBEAM];
-  const unsigned beamm = __ballot_sync(0xffffffffu, act && fbeam > 0.0);
-  if (beamm != 0u && fbeam > 0.0) {
-    // ---- beam (computeBeamSource, FluxSolver.cpp:595-643) -------------------
-    load_L();
-    const double umu0 = rec[H_UMU0];
-    double beam_mu = umu0;
-    const double mu0sq = umu0 * umu0;
-    const double dither = 1000.0 * 2.220446049250313e-16;
-    bool dith = false;
-#pragma unroll
-    for (int k = 0; k < NN; ++k)
-      if (fabs(1.0 - mu0sq * kr[k] * kr[k]) < dither) dith = true;
-    if (dith) beam_mu = 0.999 * umu0;
-    // scaled phase coefficients g'_k (disortSet, FluxSolver.cpp:336-386) times
-    // P_k(-mu0), summed against P_k(+/-mu_r)
-    const int lin = (p.flags & DSP_FLAG_INDEX_FROM_BOTTOM) ? p.L - 1 - lc : lc;
-    const double* pml = p.pmom.row(i) + (long long)lin * p.pc;
-    const int mode = (int)rec[il.mode + lc];
-    const double f = rec[il.fsc + lc], sig = rec[il.sig + lc];
-    const double* yb = rec + il.yb;
-    double sp[NN], sm[NN];
-#pragma unroll
-    for (int r = 0; r < NN; ++r) sp[r] = sm[r] = 0.0;
-#pragma unroll 1
-    for (int k = 0; k < N; ++k) {
-      const double pk = pml[k];
-      double g;
-      if (mode == 0) g = (2.0 * k + 1.0) * ws * pk;
-      else if (mode == 1) g = (2.0 * k + 1.0) * ws * (pk - f) / (1.0 - f);
-      else {
-        const double kd = (double)k;
-        g = (2.0 * k + 1.0) * ws * (pk - f * exp(-kd * kd / (2.0 * sig))) / (1.0 - f);
-      }
-      const double gy = g * yb[k];
-#pragma unroll
-      for (int r = 0; r < NN; ++r) {
-        sp[r] += gy * tc.y[k * N + r];
-        sm[r] += gy * tc.y[k * N + NN + r];
-      }
-    }
-    double m1[NN], y[NN];
-#pragma unroll
-    for (int r = 0; r < NN; ++r) {
-      const double bp = fbeam * sp[r] / (4.0 * PI), bm = fbeam * sm[r] / (4.0 * PI);
-      m1[r] = (bp + bm) * tc.rmu[r];
-      y[r] = (bp - bm) * tc.rmu[r];  // M^{-1} r2
-    }
-    // rhs = mu0^{-1} M^{-1} r2 + (a-b) M^{-1} r1, then D rhs
 #pragma unroll
     for (int r = 0; r < NN; ++r) {
       double s = 0.0;
 #pragma unroll
-      for (int k = 0; k < NN; ++k)
-        s += ((tc.wt[k] * hv(H::S_O + tri_idx(r, k))) * tc.rmu[r] - (k == r ? tc.rmu[r] : 0.0)) * m1[k];
-      y[r] = tc.dsim[r] * (y[r] / beam_mu + s);
+      for (int e = 0; e <= r; ++e) s += L[tri_idx(r, e)] * V[e * NN + c];
+      x[r] = s;
     }
-    // s = -(D^{-1} (B_s A_s - mu0^{-2})^{-1} D) rhs
-    const double shift = 1.0 / (beam_mu * beam_mu);
-    if (primary) {
-      ops.fwd(y);
-      vsolve(y, shift);
-      ops.lmul(y);
-    } else {
-      ops.ltmul(y);
-      vsolve(y, shift);
-      ops.bwd(y);
-    }
-#pragma unroll
-    for (int r = 0; r < NN; ++r) y[r] = -tc.dinv[r] * y[r];
-    // d = mu0 ((a+b) s + M^{-1} r1)
+    double ve = 0.0, al = 0.0, be = 0.0;
 #pragma unroll
     for (int r = 0; r < NN; ++r) {
-      double s = 0.0;
-#pragma unroll
-      for (int k = 0; k < NN; ++k)
-        s += ((tc.wt[k] * hv(H::S_E + tri_idx(r, k))) * tc.rmu[r] - (k == r ? tc.rmu[r] : 0.0)) * y[k];
-      const double dv = beam_mu * (s + m1[r]);
-      sA[NN + r] = 0.5 * (y[r] + dv);
-      sA[NN - r - 1] = 0.5 * (y[r] - dv);
+      const double lu = x[r] * rsk, li = y[r] * sk;
+      x[r] = primary ? lu : li;
+      y[r] = primary ? li : lu;
+      row[r] = x[r];
+      row[HP + r] = y[r];
+      ve += x[r] * (tc.dsim[r] * tc.rmu[r]);
     }
-  }
-  if (beamm != 0u) warp_flush_rows<RS>(stA, rec0, LS, N, lrec_zb(N), beamm, lane);
-  if (p.flags & DSP_FLAG_THERMAL) {
-    // ---- thermal (computeIsotropicSource, FluxSolver.cpp:745-787) -----------
-    load_L();
-    const double taus_top = rec[il.tau_s + lc];
-    const double pk0 = rec[il.pkag + lc], pk1 = rec[il.pkag + lc + 1];
-    double xr1 = 0.0;
-    if (dts > 1e-4) xr1 = (pk1 - pk0) / dts;
-    const double xr0 = pk0 - xr1 * taus_top;
-    // omega' = 1: no thermal source ((a+b) is singular there)
-    const bool src = (1.0 - ws) != 0.0;
-    double u[NN], dd[NN];
-    // u = -(a+b)^{-1} M^{-1} 1 with (a+b)^{-1} y = D^{-1} X D y (X2 primary, X1 fallback)
-#pragma unroll
-    for (int r = 0; r < NN; ++r) u[r] = tc.dsim[r] * tc.rmu[r];
-    if (src) {
-      if (primary) applyX2(u);
-      else applyX1(u);
+    if (HP != NN) {
+      row[NN] = 0.0;
+      row[HP + NN] = 0.0;
     }
-#pragma unroll
-    for (int r = 0; r < NN; ++r) u[r] = src ? -tc.dinv[r] * u[r] : 0.0;
-    const double c1 = 2.0 * (1.0 - ws) * xr1, c0 = 2.0 * (1.0 - ws) * xr0;
-    // d0 = -(a-b)^{-1} s1 with (a-b)^{-1} y = D^{-1} X D y (X1 primary, X2 fallback)
-#pragma unroll
-    for (int r = 0; r < NN; ++r) dd[r] = tc.dsim[r] * (c1 * u[r]);
-    if (src) {
-      if (primary) applyX1(dd);
-      else applyX2(dd);
-    }
-#pragma unroll
-    for (int r = 0; r < NN; ++r) {
-      const double s1 = c1 * u[r], s0 = c0 * u[r];
-      const double d0 = src ? -tc.dinv[r] * dd[r] : 0.0;
-      sB[NN + r] = 0.5 * s1;
-      sB[NN - r - 1] = 0.5 * s1;
-      sA[NN + r] = 0.5 * (s0 + d0);
-      sA[NN - r - 1] = 0.5 * (s0 - d0);
-    }
-    sB[N] = xr0;  // xr0, xr1 follow z1 in the record
-    sB[N + 1] = xr1;
-    warp_flush_rows<RS>(stA, rec0, LS, N, lrec_z0(N), okm, lane);
-    warp_flush_rows<RS>(stB, rec0, LS, N + 2, lrec_z1(N), okm, lane);
-    if constexpr (JAC) {
-      // the source per unit intercept (P) and slope (Q) for the temperature
-      // Jacobian: s0 = xr0 P, d0 = xr1 Q
-      const double cu = 2.0 * (1.0 - ws);
-      double qq[NN];
-#pragma unroll
-      for (int r = 0; r < NN; ++r) qq[r] = tc.dsim[r] * (cu * u[r]);
-      if (src) {
-        if (primary) applyX1(qq);
-        else applyX2(qq);
-      }
-      if (act) {
-        double* pq = p.jac_pq + jj * jpq_stride(N);
+    vrow[c] = k;
+    if (beam) {
+      if (raw) {
+        // pseudo-spherical beam (general solver): the raw source at the quadrature
+        // angles, up and down, for the user-angle interpolation and
+        // flux_sph_source_kernel (DisortSolver.cpp:1524-1527)
+        const double dm = 0.5 * tc.mu[c] * tc.dinv[c], u1 = hv(HO::S_B1 + c), u2 = hv(HO::S_B2 + c);
+        vrow[HP + c] = dm * (u1 + u2);
+        vrow[2 * HP + c] = dm * (u1 - u2);
+      } else {
 #pragma unroll
         for (int r = 0; r < NN; ++r) {
-          pq[r] = cu * u[r];
-          pq[NN + r] = src ? -tc.dinv[r] * qq[r] : 0.0;
+          al += x[r] * hv(HO::S_B1 + r);
+          be += y[r] * hv(HO::S_B2 + r);
         }
+        const double den = 1.0 / (k * k - r0 * r0);
+        vrow[HP + c] = (k * al - be * r0) * den;
+        vrow[2 * HP + c] = (k * be - al * r0) * den;
       }
     }
+    if (thermal) {
+      ve = ws2 * ve / k;
+      vrow[3 * HP + c] = ve;
+      vrow[4 * HP + c] = ve / k;
+    }
+    // X^T row c and Y^T row c of every task: lane group (task, X or Y) x HP
+    __syncwarp();
+    constexpr int TPI = 32 / (2 * HP) < 1 ? 1 : 32 / (2 * HP);  // tasks per store
+    const int tl = lane / (2 * HP), e = lane % (2 * HP);
+    if (tl < TPI)
+#pragma unroll 4
+      for (int b = tl; b < 32; b += TPI)
+        if ((okm >> b) & 1u)
+          rec0[b * ls + (e < HP ? mod_X(N) + c * HP + e : mod_Y(N) + c * HP + e - HP)] = stg[b * RS + e];
+    __syncwarp();
   }
+  if (thermal && act) thermal_source(q, vrow[5 * HP], vrow[5 * HP + 1]);
+  __syncwarp();
+  for (int b = 0; b < 32; ++b)
+    if ((okm >> b) & 1u)
+      for (int e = lane; e < 5 * HP + 2; e += 32) rec0[b * ls + mod_k(N) + e] = vst[b * VS + e];
 }
 
-// Host side of the layer stage: launches (through `wrap(name, launch)`, which
-// may time them) one layer kernel, or the three launches of a split stage;
-// `host_tab` is a host copy of the tab_* tables of N.
-template <int N, bool JAC = false>
+// Host side of the layer stage: launches (through `wrap(kind, launch)`, which may
+// time them; kind 0: front, 1: eigensolver, 2: team kernel) the two launches of a split stage or the team kernel; `host_tab` is a
+// host copy of the (mode's) tab_* tables of N.
+template <int N, bool GEN = false>
 inline void flux_layer_set_attrs() {
   using C = LCfg<N>;
-  if constexpr (layer_split<N>())
+  if constexpr (layer_split<N>()) {
     static_assert(Handoff<N / 2>::HS <= brec_stride(N), "the hand-off must fit in the boundary-value records");
-  // the team kernel serves every N (N <= 16: when a schedule asks for it)
-  cudaFuncSetAttribute(flux_layer_kernel<N, false, JAC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)C::smem_bytes());
+    cudaFuncSetAttribute(flux_eigen_kernel<N, GEN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)ECfg<N>::smem_bytes(128));
+  }
+  // the team kernel serves every N of the flux path (N <= 16: when a schedule asks for it)
+  if constexpr (!GEN || !layer_split<N>())
+    cudaFuncSetAttribute(flux_layer_kernel<N, GEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem_bytes());
 }
 
-// The layer stage of a flux chunk.  split: the three one-thread-per-task
-// launches (N <= 16 only), with `cta` threads per CTA (64 or 128); otherwise
-// the team kernel (shared-memory eigensolver, one team per layer task).
-template <int N, bool JAC = false, class Wrap>
-inline void flux_layer_launch(const FluxParams& p, const double* host_tab, cudaStream_t s, Wrap&& wrap,
-                              bool split = layer_split<N>(), int cta = 128) {
+// The layer stage of `tasks` layer tasks.  split: one thread per task (N <= 16
+// only), with `cta` threads per CTA (64 or 128); otherwise the team kernel.
+template <int N, bool GEN = false, class Wrap>
+inline void flux_layer_launch(const FluxParams& p, long long tasks, const double* host_tab, cudaStream_t s,
+                              Wrap&& wrap, bool split = layer_split<N>(), int cta = 128) {
   using C = LCfg<N>;
-  const long long tasks = (long long)p.n * p.L;
   if constexpr (layer_split<N>()) {
-    if (split) {
+    if (split || GEN) {
       const int b = cta == 64 ? 64 : 128;
       const ConstTab<N> tc = make_const_tab<N>(host_tab);
       const unsigned g = (unsigned)((tasks + b - 1) / b);
-      wrap("flux_layer_kernel", [&] { flux_layer_front_kernel<N><<<g, b, 0, s>>>(p, tc); });
-      wrap("flux_jacobi_kernel", [&] { flux_jacobi_kernel<N / 2><<<g, b, 0, s>>>(p); });
-      wrap("flux_layer_kernel", [&] { flux_layer_back_kernel<N, JAC><<<g, b, 0, s>>>(p, tc); });
+      wrap(0, [&] { flux_layer_front_kernel<N, GEN><<<g, b, 0, s>>>(p, tc); });
+      wrap(1, [&] { flux_eigen_kernel<N, GEN><<<g, b, ECfg<N>::smem_bytes(b), s>>>(p, tc); });
       return;
     }
   }
-  const unsigned grid = (unsigned)((tasks + C::TPC - 1) / C::TPC);
-  wrap("flux_layer_kernel", [&] { flux_layer_kernel<N, false, JAC><<<grid, C::CTA, C::smem_bytes(), s>>>(p); });
+  if constexpr (!GEN || !layer_split<N>()) {
+    const unsigned grid = (unsigned)((tasks + C::TPC - 1) / C::TPC);
+    wrap(2, [&] { flux_layer_kernel<N, GEN><<<grid, C::CTA, C::smem_bytes(), s>>>(p); });
+  }
 }
 
 }  // namespace dsp

@@ -220,8 +220,8 @@ __global__ void __launch_bounds__(128) flux_sph_source_kernel(FluxParams p) {
   // rows iq < NN from the quadrature sums, the other half by symmetry
   if constexpr (GEN) {
     for (int iq = lane; iq < NN; iq += 32) {
-      zj[iq] = lrec[lrec_zb(N) + NN + iq];
-      zj[NN + iq] = lrec[lrec_zb(N) + NN - 1 - iq];
+      zj[iq] = lrec[mod_cb(N) + iq];
+      zj[NN + iq] = lrec[mod_db(N) + iq];
     }
   } else {
     const double* yb = rec + il.yb;
@@ -338,11 +338,23 @@ __global__ void __launch_bounds__(128) flux_sph_source_kernel(FluxParams p) {
     solve(bv);
   }
   __syncwarp();
-  for (int iq = lane; iq < NN; iq += 32) {
-    lrec[lrec_zb(N) + NN + iq] = bv[iq];
-    lrec[lrec_zb(N) + NN - 1 - iq] = bv[iq + NN];
-    sr[NN + iq] = z1[iq];
-    sr[NN - 1 - iq] = z1[iq + NN];
+  // Z0 and Z1 in the layer's modes: c = Y^T D (z+ + z-), d = X^T D (z+ - z-)
+  const double* dsim = p.tables + tab_dsim(N);
+  for (int c = lane; c < NN; c += 32) {
+    const double* x = lrec + mod_X(N) + c * mod_hp(N);
+    const double* y = lrec + mod_Y(N) + c * mod_hp(N);
+    double c0 = 0.0, d0 = 0.0, c1 = 0.0, d1 = 0.0;
+    for (int r = 0; r < NN; ++r) {
+      const double dy = dsim[r] * y[r], dx = dsim[r] * x[r];
+      c0 = fma(dy, bv[r] + bv[NN + r], c0);
+      d0 = fma(dx, bv[r] - bv[NN + r], d0);
+      c1 = fma(dy, z1[r] + z1[NN + r], c1);
+      d1 = fma(dx, z1[r] - z1[NN + r], d1);
+    }
+    lrec[mod_cb(N) + c] = c0;
+    lrec[mod_db(N) + c] = d0;
+    sr[c] = c1;
+    sr[NN + c] = d1;
   }
   if (lane == 0) sr[sph_xba(N)] = xba;
 }

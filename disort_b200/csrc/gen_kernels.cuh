@@ -1,14 +1,14 @@
 // gen_kernels.cuh — the general solver's own kernels (DisortSolver::solve):
 // per-instance setup and the user-angle intensities of one azimuth mode.
 //
-// The per-layer eigensystems and particular solutions (flux_layer_kernel<N,
-// true>) and the boundary-value problem (flux_bvp*_kernel<N, true>) are shared
-// with the flux solver; these kernels add what only the general solver has:
+// The per-layer eigensystems and particular solutions (flux_layer.cuh) and the
+// boundary-value problem (flux_bvp.cuh) are shared with the flux solver; these kernels add what only the general solver has:
 // ragged layer counts, user optical depths, the azimuth-mode schedule and
 // intensities at user polar angles and azimuths.
 #pragma once
 
 #include "dsp_device.cuh"
+#include "flux_layer.cuh"
 #include "flux_setup.cuh"
 
 namespace dsp {
@@ -218,6 +218,144 @@ static __global__ void __launch_bounds__(128) gen_setup_kernel(FluxParams p) {
   }
 }
 
+// P_l^m(-mu0) and P_l^m(mu_u) of mode m for every chunk slot (ptab): one thread
+// per (slot, angle).
+static __global__ void __launch_bounds__(128) gen_ptab_kernel(FluxParams p) {
+  const GenView& g = p.g;
+  const int na = 1 + g.numu;
+  const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= (long long)p.n * na) return;
+  const int slot = (int)(k / na), v = (int)(k % na);
+  const int i = g.ids[slot];
+  const double x = v == 0 ? -p.umu0(i) : g.umu.row(i)[v - 1];
+  legendre_column(g.m, x, p.N - 1, g.ptab + k * p.N, 1);
+}
+
+// Eigenvectors and sources of every layer at the user polar angles for mode m
+// (interpEigenvec, DisortSolver.cpp:2468-2504; interpSource, :2506-2580).  With
+//   S_i, A_i = w_i / d_i sum_{l + m even, odd} g'_l / 2 P_l^m(mu_u) P_l^m(mu_i)
+// (the two hemispheres differ in the sign of the odd terms) the intensity at mu_u
+// scattered from the modes is (S X) C + (A Y) D, so that its coefficients of a
+// and b are S X -/+ A Y.  A team of pow2ceil(h) lanes per layer task: lane i
+// forms S_i, A_i, then lane j the products with row j of X^T and Y^T, which it
+// keeps in registers over the angles.
+template <int N>
+struct ACfg {
+  static constexpr int H = N / 2, HP = mod_hp(N), TEAM = pow2ceil(H), TPC = 128 / TEAM;
+  static constexpr int TEAM_SMEM = N + 2 * HP;
+};
+template <int N>
+__global__ void __launch_bounds__(128) gen_angle_kernel(FluxParams p) {
+  using C = ACfg<N>;
+  constexpr int H = C::H, HP = C::HP, TEAM = C::TEAM;
+  __shared__ double smem[C::TPC * C::TEAM_SMEM];
+  const int t = threadIdx.x % TEAM, j = t < H ? t : H - 1;
+  const bool own = t < H;
+  double* const gl = smem + (threadIdx.x / TEAM) * C::TEAM_SMEM;
+  double* const sv = gl + N;
+  double* const av = sv + HP;
+  const unsigned msk = team_mask<TEAM>();
+  const long long task = (long long)blockIdx.x * C::TPC + threadIdx.x / TEAM;
+  if (task >= p.g.lay_off[p.n]) return;
+  const LayerTask<N, true> q = layer_task<N, true>(p, task);
+  if (!q.live) return;
+  const int st0 = p.status ? p.status[q.i] : 0;
+  if (st0 == DSP_ERR_EIGEN) return;
+  const int m = p.g.m, numu = p.g.numu;
+  const double ws = q.rec[q.il.ssa_s + q.lc];
+  {
+    const int mode = (int)q.rec[q.il.mode + q.lc];
+    const double f = q.rec[q.il.fsc + q.lc], sig = q.rec[q.il.sig + q.lc];
+    for (int k = t; k < N; k += TEAM) gl[k] = 0.5 * phase_coeff<true>(k, q.pml[k], mode, ws, f, sig);
+  }
+  if (HP != H && t == 0) {
+    sv[H] = 0.0;
+    av[H] = 0.0;
+  }
+  const double fbeam = q.rec[H_FBEAM];
+  const bool beam = fbeam > 0.0, sph = (p.flags & DSP_FLAG_SPHERICAL_BEAM) != 0;
+  const bool thermal = (p.flags & DSP_FLAG_THERMAL) && m == 0;
+  double x[H], y[H];
+#pragma unroll
+  for (int r = 0; r < H; ++r) {
+    x[r] = q.lrec[mod_X(N) + j * HP + r];
+    y[r] = q.lrec[mod_Y(N) + j * HP + r];
+  }
+  // lane j's beam and thermal amplitudes (pseudo-spherical: the raw source at the
+  // quadrature angles j, as the reference's interpSource reads it)
+  double cb = 0.0, db = 0.0, ctv = 0.0, dtv = 0.0, xr0 = 0.0, xr1 = 0.0;
+  if (beam) {
+    cb = q.lrec[mod_cb(N) + j];
+    db = q.lrec[mod_db(N) + j];
+  }
+  if (thermal) {
+    ctv = q.lrec[mod_ct(N) + j];
+    dtv = q.lrec[mod_dt(N) + j];
+    xr0 = q.lrec[mod_xr(N)];
+    xr1 = q.lrec[mod_xr(N) + 1];
+  }
+  const double dj = p.tables[tab_dsim(N) + j], wd = p.tables[tab_wt(N) + j] / dj;
+  const double* const Y = p.tables + tab_ylm(N);
+  const double* const yb = beam_legendre<N, true>(p, q);
+  const double fact = 2.0 * (m == 0 ? 1.0 : 2.0) * fbeam / (4.0 * 3.14159265358979323846);
+  const int odd0 = 1 - (m & 1);  // first l of odd l + m
+  double* const GU = q.lrec + glrec_gu(N);
+  double* const zbu = GU + (long long)numu * N;
+  __syncwarp(msk);
+  for (int iu = 0; iu < numu; ++iu) {
+    const double* pu = yb + (long long)N * (1 + iu);
+    double se = 0.0, so = 0.0;
+#pragma unroll 4
+    for (int l = 0; l < N; l += 2) {
+      se = fma(gl[l + 1 - odd0] * pu[l + 1 - odd0], Y[(l + 1 - odd0) * N + j], se);
+      so = fma(gl[l + odd0] * pu[l + odd0], Y[(l + odd0) * N + j], so);
+    }
+    se *= wd;
+    so *= wd;
+    if (own) {
+      sv[j] = se;
+      av[j] = so;
+    }
+    __syncwarp(msk);
+    double sx = 0.0, sy = 0.0;
+#pragma unroll
+    for (int r = 0; r < H; ++r) {
+      sx = fma(x[r], sv[r], sx);
+      sy = fma(y[r], av[r], sy);
+    }
+    if (own) {
+      GU[(long long)iu * N + j] = sx + sy;
+      GU[(long long)iu * N + H + j] = sx - sy;
+    }
+    // source terms: sums over the lanes
+    double zb = 0.0, z0 = 0.0, z1 = 0.0;
+    if (own) {
+      if (beam) {
+        zb = sph ? dj * (se * (cb + db) + so * (cb - db)) : sx * cb + sy * db;
+        for (int l = j; l < N; l += H) zb = fma(gl[l] * pu[l], fact * yb[l], zb);
+      }
+      z0 = sx * ctv;
+      z1 = sy * dtv;
+    }
+    if (beam || thermal) {
+#pragma unroll
+      for (int off = TEAM / 2; off > 0; off >>= 1) {
+        zb += __shfl_xor_sync(msk, zb, off, TEAM);
+        z0 += __shfl_xor_sync(msk, z0, off, TEAM);
+        z1 += __shfl_xor_sync(msk, z1, off, TEAM);
+      }
+      if (t == 0) {
+        if (beam) zbu[iu] = zb;
+        if (thermal) {
+          zbu[numu + iu] = fma(xr0, z0 + (1.0 - ws), xr1 * z1);
+          zbu[2 * numu + iu] = xr1 * (z0 + (1.0 - ws));
+        }
+      }
+    }
+    __syncwarp(msk);
+  }
+}
+
 // Intensities at the user angles for mode m (computeUserIntensities,
 // DisortSolver.cpp:2938-3268): one warp per instance, a lane per (level, angle)
 // pair, looping over the layers between the level and the boundary.
@@ -269,52 +407,33 @@ __global__ void __launch_bounds__(128) gen_intensity_kernel(FluxParams p) {
   auto LR = [&](int l) { return lrec0 + (long long)l * g.lstride; };
   const double* um = g.umu.row(i);
 
-  // bottom-boundary reflection of the mode-0 downward field (DisortSolver.cpp:3180-3218):
-  // S = sum_iq mu w dfuint(iq), in the reference's order iq = NN-1 .. 0
+  // reflected field: the downward intensities at the bottom come with the
+  // boundary-value solution
   double bsum = 0.0;
   // bidirectional surface: this mode's table; its user rows receive the
   // reflected sum of each user angle in their last slot
   double* sft = g.brdf ? g.brdf + (long long)slot * brdf_stride(N, g.numu) : nullptr;
   const bool lambert_bnd = (m == 0) && !lyrcut && !dlbc && !sft;
-  if (sft && !lyrcut) {
-    // sum_iq (1 + delta_m0) R_m(mu_u, mu_iq) mu_iq w_iq dfuint(iq) per user angle
-    // (DisortSolver.cpp:3180-3218), dfuint as below, summed across the warp
-    const double* lr = LR(L - 1);
-    const double* G = lr + lrec_G(N);
-    const double* x = cc0 + (long long)(L - 1) * N;
-    double dfu = 0.0;
-    const int iq = lane;
-    if (iq < NN) {
-      for (int jq = 0; jq < NN; ++jq) dfu += G[iq * N + jq] * x[jq];
-      for (int jq = NN; jq < N; ++jq) dfu += G[iq * N + jq] * x[jq] * exp(-lr[lrec_eig(N) + jq] * dts[L - 1]);
-      if (beam) dfu += lr[lrec_zb(N) + iq] * btr[L];
-      if (thermal) dfu += lr[lrec_z0(N) + iq] + lr[lrec_z1(N) + iq] * taus[L];
-    }
+  if ((sft && !lyrcut) || lambert_bnd) {
+    const double dfu = lane < NN ? p.bvp_rec[(g.lay_off[slot] + ncut - 1) * brec_stride(N) + brec_dn(N) + lane] : 0.0;
+    const double muw = lane < NN ? mu[lane] * wt[lane] : 0.0;
     const double cpl = m == 0 ? 2.0 : 1.0;
-    for (int iu = 0; iu < numu; ++iu) {
-      double* ur = sft + (NN + iu) * brdf_row(N);
-      double v = iq < NN ? cpl * ur[NN - iq] * mu[NN - iq - 1] * wt[NN - iq - 1] * dfu : 0.0;
+    auto total = [](double v) {
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-      if (lane == 0) ur[NN + 2] = v;
-    }
-    __syncwarp();
-  }
-  if (lambert_bnd) {
-    const double* lr = LR(L - 1);
-    const double* G = lr + lrec_G(N);
-    const double* x = cc0 + (long long)(L - 1) * N;
-    double dfu = 0.0;
-    const int iq = lane;
-    if (iq < NN) {
-      for (int jq = 0; jq < NN; ++jq) dfu += G[iq * N + jq] * x[jq];
-      for (int jq = NN; jq < N; ++jq) dfu += G[iq * N + jq] * x[jq] * exp(-lr[lrec_eig(N) + jq] * dts[L - 1]);
-      if (beam) dfu += lr[lrec_zb(N) + iq] * btr[L];
-      if (p.flags & DSP_FLAG_THERMAL) dfu += lr[lrec_z0(N) + iq] + lr[lrec_z1(N) + iq] * taus[L];
-    }
-    for (int k = NN - 1; k >= 0; --k) {
-      const double v = __shfl_sync(0xffffffffu, dfu, k);
-      bsum += 2.0 * mu[NN - k - 1] * wt[NN - k - 1] * v;
+      return v;
+    };
+    if (lambert_bnd) {
+      // sum_iq 2 mu w dfuint (DisortSolver.cpp:3180-3218)
+      bsum = total(2.0 * muw * dfu);
+    } else {
+      // sum_iq (1 + delta_m0) R_m(mu_u, mu_iq) mu_iq w_iq dfuint(iq) per user angle
+      for (int iu = 0; iu < numu; ++iu) {
+        double* ur = sft + (NN + iu) * brdf_row(N);
+        const double v = total(lane < NN ? cpl * ur[1 + lane] * muw * dfu : 0.0);
+        if (lane == 0) ur[NN + 2] = v;
+      }
+      __syncwarp();
     }
   }
 
@@ -336,7 +455,7 @@ __global__ void __launch_bounds__(128) gen_intensity_kernel(FluxParams p) {
         const double* lr = LR(lc);
         const double* gu = lr + glrec_gu(N) + iu * N;
         const double* x = cc0 + (long long)lc * N;
-        const double* kk = lr + lrec_eig(N);
+        const double* kk = lr + mod_k(N);
         const double dt = dts[lc];
         const double e1 = exp((ut - taus[lc]) / umv);
         const double e2 = exp((ut - taus[lc + 1]) / umv);
@@ -353,23 +472,18 @@ __global__ void __launch_bounds__(128) gen_intensity_kernel(FluxParams p) {
           else expn = (e1 * btr[lc] - e2 * btr[lc + 1]) * sgn / den;
           palint += lr[glrec_gu(N) + numu * N + iu] * expn;
         }
-        double wk[NN];
-#pragma unroll
+#pragma unroll 4
         for (int iq = 0; iq < NN; ++iq) {
-          wk[iq] = exp(kk[iq] * dt);
-          const double den = 1.0 + umv * kk[iq];
-          double expn;
+          const double k = kk[iq], wk = exp(-k * dt);
+          // b: exp(-k (tau_bot - tau)), a: exp(-k (tau - tau_top))
+          double den = 1.0 - umv * k, expn;
           if (fabs(den) < 0.0001) expn = (dt / umv) * e2;
-          else expn = sgn * (e1 * wk[iq] - e2) / den;
+          else expn = sgn * (e1 * wk - e2) / den;
           palint += (gu[iq] * x[iq]) * expn;
-        }
-#pragma unroll
-        for (int iq = NN; iq < N; ++iq) {
-          const double den = 1.0 + umv * kk[iq];
-          double expn;
+          den = 1.0 + umv * k;
           if (fabs(den) < 0.0001) expn = -(dt / umv) * e1;
-          else expn = sgn * (e1 - e2 * wk[N - 1 - iq]) / den;
-          palint += (gu[iq] * x[iq]) * expn;
+          else expn = sgn * (e1 - e2 * wk) / den;
+          palint += (gu[NN + iq] * x[NN + iq]) * expn;
         }
       }
       // the part of the level's own layer on the boundary side
@@ -378,7 +492,7 @@ __global__ void __launch_bounds__(128) gen_intensity_kernel(FluxParams p) {
         const double* lr = LR(y);
         const double* gu = lr + glrec_gu(N) + iu * N;
         const double* x = cc0 + (long long)y * N;
-        const double* kk = lr + lrec_eig(N);
+        const double* kk = lr + mod_k(N);
         const double e1c = neg ? exp(dt1 / umv) : 0.0;
         const double e2c = neg ? 0.0 : exp(dt2 / umv);
         if (beam) {
@@ -392,21 +506,17 @@ __global__ void __launch_bounds__(128) gen_intensity_kernel(FluxParams p) {
         const double dty = dts[y];
 #pragma unroll 4
         for (int iq = 0; iq < NN; ++iq) {
-          const double den = 1.0 + umv * kk[iq];
-          double expn;
+          const double k = kk[iq], wk = exp(-k * dty);
+          double den = 1.0 - umv * k, expn;
           if (fabs(den) < 0.0001) expn = -dt2 / umv * e2c;
-          else if (neg) expn = (exp(-kk[iq] * dt2) - exp(kk[iq] * dty) * e1c) / den;
-          else expn = (exp(-kk[iq] * dt2) - e2c) / den;
+          else if (neg) expn = (exp(k * dt2) - wk * e1c) / den;
+          else expn = (exp(k * dt2) - e2c) / den;
           palint += (gu[iq] * x[iq]) * expn;
-        }
-#pragma unroll 4
-        for (int iq = NN; iq < N; ++iq) {
-          const double den = 1.0 + umv * kk[iq];
-          double expn;
+          den = 1.0 + umv * k;
           if (fabs(den) < 0.0001) expn = -(dt1 / umv) * e1c;
-          else if (neg) expn = (exp(-kk[iq] * dt1) - e1c) / den;
-          else expn = (exp(-kk[iq] * dt1) - exp(-kk[iq] * dty) * e2c) / den;
-          palint += (gu[iq] * x[iq]) * expn;
+          else if (neg) expn = (exp(-k * dt1) - e1c) / den;
+          else expn = (exp(-k * dt1) - wk * e2c) / den;
+          palint += (gu[NN + iq] * x[NN + iq]) * expn;
         }
         if (thermal) {
           const double expn = neg ? e1c : e2c;

@@ -1,0 +1,61 @@
+"""GPU tests of the modal boundary-value kernel (csrc/flux_bvp.cuh) and the layer
+records it reads, where their shapes have edges: instance counts that leave
+teams of a warp empty, one to a few layers, every stream count (odd half counts
+are padded), layers of zero and of very large optical depth, no scattering and
+conservative scattering.
+
+Tolerances: the flux parity of tests/parity.py (1e-9 relative, 1e-12 absolute)
+against the extended-precision oracle.  At omega = 1 the oracle's own noise is
+1e-8 (one eigenvalue is zero to rounding), so there the physics is the checker:
+without absorption or emission the net flux is the same at every level, to a few
+hundred rounding units of the flux scale (1e-13 x the incoming flux).
+"""
+import numpy as np
+import pytest
+
+import gpu_lib
+import oracle_lib
+from disort_b200 import capi, workloads
+from parity import assert_parity
+
+pytestmark = pytest.mark.gpu
+
+
+def columns(N, n, L, seed, thermal, ssa=None):
+    rng = np.random.default_rng(seed)
+    dtau = np.clip(rng.lognormal(-2.0, 2.0, (n, L)), 1e-6, 20.0)
+    om = rng.uniform(0.0, 0.99, (n, L)) if ssa is None else np.full((n, L), ssa)
+    if ssa is None:
+        dtau[:, L // 2] = 0.0        # an empty layer
+        om[:, 0] = 0.0               # no scattering
+        dtau[n // 2, L - 1] = 200.0  # opaque
+    pc = N + 1
+    arrays = dict(wavenumber_low=rng.uniform(300.0, 900.0, n), delta_tau=dtau, single_scat_albedo=om,
+                  phase_function_moments=workloads.hg_moments(rng.uniform(-0.3, 0.85, (n, L)), pc),
+                  temperature=200.0 + 90.0 * rng.random(L + 1), surface_albedo=rng.uniform(0.0, 1.0, n),
+                  emissivity_top=0.7, direct_beam_flux=2.0, direct_beam_mu=rng.uniform(0.15, 0.95, n),
+                  isotropic_flux_top=0.3, isotropic_flux_bottom=0.1, temperature_top=150.0, temperature_bottom=290.0)
+    arrays["wavenumber_high"] = arrays["wavenumber_low"] + 5.0
+    return dict(n_inst=n, num_streams=N, num_layers=L, num_phase_func_moments=0, pmom_count=pc,
+                flags=capi.FLAG_THERMAL if thermal else 0, arrays=arrays)
+
+
+@pytest.mark.parametrize("N", capi.SUPPORTED_NSTR)
+@pytest.mark.parametrize("n,L", [(1, 1), (3, 2), (5, 7), (33, 3)])
+def test_partial_warps_and_extreme_layers(N, n, L):
+    for thermal in (True, False):
+        w = columns(N, n, L, 100 * N + 10 * n + L, thermal)
+        got, gst, rc = gpu_lib.flux_solve(w)
+        ref, rst = oracle_lib.flux_solve(w, ext=True)
+        assert rc == 0 and not gst.any() and not rst.any()
+        assert_parity(got, ref, f"N={N} n={n} L={L} thermal={thermal}")
+
+
+@pytest.mark.parametrize("N", capi.SUPPORTED_NSTR)
+def test_conservative_columns_conserve_the_net_flux(N):
+    w = columns(N, 9, 12, 7 * N, False, ssa=1.0)
+    got, gst, rc = gpu_lib.flux_solve(w)
+    assert rc == 0 and not gst.any()
+    net = got["flux_up"] - got["flux_down"] - got["flux_direct_beam"]
+    incoming = np.pi * 0.3 + got["flux_direct_beam"][:, :1]
+    assert np.max(np.abs(net - net[:, :1]) / incoming) <= 1e-13 * 300
