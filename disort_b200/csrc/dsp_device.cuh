@@ -93,8 +93,9 @@ struct GenLayout {
 
 // Layer record (doubles) written by the layer stage, h = N/2 (rows of HP, h rounded
 // up to even, pads zero):
-//   X^T [h][HP] | Y^T [h][HP] | k [HP] | beam c, d [HP] each | thermal c, d [HP]
-//   each | xr0 | xr1
+//   X^T [h][HP] | Y^T [h][HP] | k [HP] | E [HP] | F [HP] | beam c, d [HP] each |
+//   thermal c, d [HP] each | xr0 | xr1
+// (E = exp(-k dtau'), F = 1 - E^2).
 // With D = diag(sqrt(w_i mu_i)) and up/down the intensities at the h quadrature
 // angles, the layer's modes are phi = D (up + down) = X C, psi = D (up - down) =
 // Y D_, where C = E1 a + E2 b + c_p, D_ = E2 b - E1 a + d_p with
@@ -106,11 +107,13 @@ __host__ __device__ constexpr int mod_hp(int N) { return N / 2 + ((N / 2) & 1); 
 __host__ __device__ constexpr int mod_X(int) { return 0; }
 __host__ __device__ constexpr int mod_Y(int N) { return (N / 2) * mod_hp(N); }
 __host__ __device__ constexpr int mod_k(int N) { return 2 * (N / 2) * mod_hp(N); }
-__host__ __device__ constexpr int mod_cb(int N) { return mod_k(N) + mod_hp(N); }
-__host__ __device__ constexpr int mod_db(int N) { return mod_k(N) + 2 * mod_hp(N); }
-__host__ __device__ constexpr int mod_ct(int N) { return mod_k(N) + 3 * mod_hp(N); }
-__host__ __device__ constexpr int mod_dt(int N) { return mod_k(N) + 4 * mod_hp(N); }
-__host__ __device__ constexpr int mod_xr(int N) { return mod_k(N) + 5 * mod_hp(N); }
+__host__ __device__ constexpr int mod_E(int N) { return mod_k(N) + mod_hp(N); }
+__host__ __device__ constexpr int mod_F(int N) { return mod_k(N) + 2 * mod_hp(N); }
+__host__ __device__ constexpr int mod_cb(int N) { return mod_k(N) + 3 * mod_hp(N); }
+__host__ __device__ constexpr int mod_db(int N) { return mod_k(N) + 4 * mod_hp(N); }
+__host__ __device__ constexpr int mod_ct(int N) { return mod_k(N) + 5 * mod_hp(N); }
+__host__ __device__ constexpr int mod_dt(int N) { return mod_k(N) + 6 * mod_hp(N); }
+__host__ __device__ constexpr int mod_xr(int N) { return mod_k(N) + 7 * mod_hp(N); }
 __host__ __device__ constexpr int mod_size(int N) { return mod_xr(N) + 2; }
 __host__ __device__ constexpr int lrec_stride(int N) { return round4(N * N + 4 * N + 2); }
 // Boundary-value record (doubles) per layer: H [h][HP] | G [h][HP] | r [HP], and
@@ -147,8 +150,13 @@ __host__ __device__ constexpr int glrec_stride(int N, int numu) { return round4(
 
 // Per-launch view of a general (DisortSolver) chunk.  Instances are addressed by
 // chunk slot ci; ids[ci] is the batch index (inputs, outputs, status).
+// A launch covers the modes m .. m + gridDim.y - 1; block row y works on mode m + y,
+// with its own copy of the per-mode areas, ms_* doubles apart.
 struct GenView {
-  int m;                       // azimuth mode of this launch
+  int m;                       // first azimuth mode of this launch
+  long long ms_layer, ms_bvp, ms_cc, ms_ptab, ms_sph, ms_int;  // per-mode strides
+  double* imode;               // per mode and slot: I_m [nt_max][numu]
+  int nt_max;                  // output depths per slot in imode
   int numu;                    // user polar angles (0: no intensities)
   int numu_in;                 // num_user_mu of the batch (validated when use_user_mu)
   int nphi, ntau_out, numu_out;
@@ -307,46 +315,29 @@ __device__ __forceinline__ double rcp_newton(double x) {
   return fma(y, e, y);
 }
 
-// Team copy of nd doubles from global to shared memory: 16-byte cp.async
-// (LDGSTS) chunks when both ends are 16-byte aligned and nd is even, plain
-// loads and stores otherwise.  The copies are waited for with cp_async_wait
-// and made visible to the team by the next team barrier.  Plain (coherent)
-// loads: the source may have been written by this kernel.
-template <int TEAM>
-__device__ __forceinline__ void team_copy_async(double* dst, const double* src, int nd, int t) {
-  const bool al = ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15u) == 0 && (nd & 1) == 0;
-  if (al) {
-    const unsigned s0 = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-    for (int k = t; k < nd / 2; k += TEAM)
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s0 + 16u * k), "l"(src + 2 * k) : "memory");
-  } else {
-    for (int k = t; k < nd; k += TEAM) dst[k] = src[k];
+// Team copies from global to shared memory with 16-byte cp.async (LDGSTS): ROWS
+// rows of COLS doubles, contiguous in global memory, LD doubles apart in shared
+// memory; and a vector of ND doubles.  COLS, LD and ND even, both ends 16-byte
+// aligned (records start on 32 bytes, their parts at even offsets).  Waited for
+// with cp_async_wait and made visible to the team by its next barrier.
+template <int TEAM, int COLS, int ROWS, int LD>
+__device__ __forceinline__ void team_copy_mat(double* dst, const double* src, int t) {
+  constexpr int CPR = COLS / 2, CH = ROWS * CPR;
+  const unsigned s0 = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+#pragma unroll(CH / TEAM <= 8 ? (CH + TEAM - 1) / TEAM : 4)
+  for (int k = t; k < CH; k += TEAM) {
+    const int r = k / CPR, c2 = k - r * CPR;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s0 + 8u * (unsigned)(r * LD + 2 * c2)),
+                 "l"(src + 2 * k)
+                 : "memory");
   }
 }
-// Team copy of `rows` rows of `cols` doubles (cols even) from global memory
-// (row stride sstride) into shared memory (row stride dstride), 16-byte cp.async
-// chunks when both layouts keep every chunk 16-byte aligned, plain loads and
-// stores otherwise; waited for like team_copy_async.
-template <int TEAM>
-__device__ __forceinline__ void team_copy_rows_async(double* dst, int dstride, const double* src, int sstride,
-                                                     int rows, int cols, int t) {
-  const bool al = ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15u) == 0 &&
-                  ((dstride | sstride | cols) & 1) == 0;
-  const int cpr = cols / 2;
-  if (al) {
-    const unsigned s0 = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-    for (int k = t; k < rows * cpr; k += TEAM) {
-      const int r = k / cpr, c2 = k - r * cpr;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s0 + 8u * (unsigned)(r * dstride + 2 * c2)),
-                   "l"(src + (long long)r * sstride + 2 * c2)
-                   : "memory");
-    }
-  } else {
-    for (int k = t; k < rows * cols; k += TEAM) {
-      const int r = k / cols, c = k - r * cols;
-      dst[r * dstride + c] = src[(long long)r * sstride + c];
-    }
-  }
+template <int TEAM, int ND>
+__device__ __forceinline__ void team_copy_vec(double* dst, const double* src, int t) {
+  const unsigned s0 = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+#pragma unroll(ND / 2 / TEAM <= 8 ? (ND / 2 + TEAM - 1) / TEAM : 4)
+  for (int k = t; k < ND / 2; k += TEAM)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s0 + 16u * k), "l"(src + 2 * k) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 // wait until at most N of this thread's most recent groups are pending

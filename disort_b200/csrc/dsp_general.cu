@@ -132,15 +132,15 @@ int resident_ctas(dsp_context ctx, K kernel, int threads, size_t smem) {
   return per_sm * ctx->sm_count;
 }
 
-// The mode-m layer, user-angle and boundary-value launches of a chunk; SPH: with
-// the pseudo-spherical beam, whose particular solution of the mode is formed
-// between them (after the user angles, which read its raw source).
-// `order`/`head` (persistent boundary-value launch): the chunk's slots by
-// descending layer count and this mode's queue counter; null: one team per slot.
-// `host_tab`: host copy of the mode's tables.
+// The layer, user-angle and boundary-value launches of `modes` azimuth modes of a
+// chunk, from p.g.m on; SPH: with the pseudo-spherical beam, whose particular
+// solution of the mode is formed between them (after the user angles, which read
+// its raw source).  `order`/`heads` (persistent boundary-value launch): the chunk's
+// slots by descending layer count and the modes' queue counters; null: one team
+// per slot.  `host_tab`: host copy of the first mode's tables.
 template <int N, bool SPH>
-void launch_general_mode(dsp_context ctx, const FluxParams& p, long long layers, cudaStream_t s, const int* order,
-                         int* head, const double* host_tab) {
+void launch_general_modes(dsp_context ctx, const FluxParams& p, long long layers, cudaStream_t s, const int* order,
+                          int* heads, const double* host_tab, int modes) {
   static bool attr = false;
   if (!attr) {
     flux_layer_set_attrs<N, true>();
@@ -157,24 +157,25 @@ void launch_general_mode(dsp_context ctx, const FluxParams& p, long long layers,
     // P_l^m at -mu0 and at the user angles
     const long long items = (long long)p.n * (1 + p.g.numu);
     KernelTimer kt(ctx, "gen_setup_kernel");
-    gen_ptab_kernel<<<(unsigned)((items + 127) / 128), 128, 0, s>>>(p);
+    gen_ptab_kernel<<<dim3((unsigned)((items + 127) / 128), (unsigned)modes), 128, 0, s>>>(p);
   }
   if (layers > 0) {
     flux_layer_launch<N, true>(p, layers, host_tab, s, [&](int, auto&& launch) {
       KernelTimer kt(ctx, "gen_layer_kernel");
       launch();
-    });
+    }, layer_split<N>(), 128, modes);
     if (p.g.numu > 0) {
       using C = ACfg<N>;
       KernelTimer kt(ctx, "gen_angle_kernel");
-      gen_angle_kernel<N><<<(unsigned)((layers + C::TPC - 1) / C::TPC), 128, 0, s>>>(p);
+      gen_angle_kernel<N><<<dim3((unsigned)((layers + C::TPC - 1) / C::TPC), (unsigned)modes), 128, 0, s>>>(p);
     }
   }
   if constexpr (SPH) {
     if (layers > 0) {
       using C = SCfg<N>;
       KernelTimer kt(ctx, "gen_sph_source_kernel");
-      flux_sph_source_kernel<N, true><<<(unsigned)((layers + C::WPC - 1) / C::WPC), 32 * C::WPC, C::smem_bytes(), s>>>(p);
+      flux_sph_source_kernel<N, true><<<dim3((unsigned)((layers + C::WPC - 1) / C::WPC), (unsigned)modes), 32 * C::WPC,
+                                        C::smem_bytes(), s>>>(p);
     }
   }
   using C = BCfg<N>;
@@ -182,14 +183,16 @@ void launch_general_mode(dsp_context ctx, const FluxParams& p, long long layers,
   const int warps = (p.n + C::TPW - 1) / C::TPW;
   if (order) {
     static const int cap = resident_ctas(ctx, gen_bvp_persistent_kernel<N, SPH>, 32, C::smem_bytes());
-    gen_bvp_persistent_kernel<N, SPH><<<warps < cap ? warps : cap, 32, C::smem_bytes(), s>>>(p, order, head);
+    const int per = (cap + modes - 1) / modes;  // resident warps of each mode's queue
+    gen_bvp_persistent_kernel<N, SPH><<<dim3((unsigned)(warps < per ? warps : per), (unsigned)modes), 32,
+                                        C::smem_bytes(), s>>>(p, order, heads);
   } else {
-    flux_bvp_kernel<N, true, SPH><<<warps, 32, C::smem_bytes(), s>>>(p);
+    flux_bvp_kernel<N, true, SPH><<<dim3((unsigned)warps, (unsigned)modes), 32, C::smem_bytes(), s>>>(p);
   }
 }
 
 template <int N, bool SPH>
-dsp_status launch_general_chunk(dsp_context ctx, FluxParams p, long long layers, int maxm, const double* tabs,
+dsp_status launch_general_chunk(dsp_context ctx, FluxParams p, long long layers, int maxm, int batch, const double* tabs,
                                 const JacView* jv, const int* order, int* heads) {
   cudaStream_t s = ctx->stream;
   const double* const host_tabs = ctx->host_mode_tables.at(N).data();
@@ -203,18 +206,20 @@ dsp_status launch_general_chunk(dsp_context ctx, FluxParams p, long long layers,
     KernelTimer kt(ctx, "gen_sph_chapman_kernel");
     flux_sph_chapman_kernel<true><<<(p.n + 3) / 4, 128, 0, s>>>(p);
   }
-  for (int m = 0; m <= maxm; ++m) {
+  for (int m = 0; m <= maxm; m += batch) {
+    const int modes = std::min(batch, maxm + 1 - m);
     p.g.m = m;
     p.tables = tabs + (size_t)m * tab_size(N);
-    int* head = order ? heads + m : nullptr;
     if (p.g.brdf) {
-      // the surface's Fourier coefficients of this mode, before the boundary-value problem
+      // the surface's Fourier coefficients of this mode, before the boundary-value
+      // problem (one mode per launch: the table is the instance's)
       KernelTimer kt(ctx, "gen_brdf_kernel");
       gen_brdf_kernel<N><<<p.n, 128, 0, s>>>(p);
     }
-    launch_general_mode<N, SPH>(ctx, p, layers, s, order, head, host_tabs + (size_t)m * tab_size(N));
+    launch_general_modes<N, SPH>(ctx, p, layers, s, order, order ? heads + m : nullptr,
+                                 host_tabs + (size_t)m * tab_size(N), modes);
     if (m == 0 && jv) {
-      // the Jacobians use the mode-0 matrices before the next mode replaces them
+      // the Jacobians use the mode-0 matrices before a later mode replaces them
       using C = JCfg<N>;
       static bool attr = false;
       if (!attr) {
@@ -226,8 +231,11 @@ dsp_status launch_general_chunk(dsp_context ctx, FluxParams p, long long layers,
       flux_jac_kernel<N, true><<<p.n, C::KB, C::smem_bytes(), s>>>(p, *jv);
     }
     if (p.g.numu > 0) {
+      using C = ICfg<N>;
+      const long long items = (long long)p.n * p.g.numu;
       KernelTimer kt(ctx, "gen_intensity_kernel");
-      gen_intensity_kernel<N><<<(p.n + 3) / 4, 128, 0, s>>>(p);
+      gen_intensity_kernel<N><<<dim3((unsigned)((items + C::TPC - 1) / C::TPC), (unsigned)modes), 128, 0, s>>>(p);
+      gen_fourier_kernel<<<(p.n + 3) / 4, 128, 0, s>>>(p, modes);
     }
   }
   if ((p.flags & DSP_GFLAG_INTENSITY_CORR) && p.g.numu > 0) {
@@ -241,25 +249,25 @@ dsp_status launch_general_chunk(dsp_context ctx, FluxParams p, long long layers,
 }
 
 template <int N>
-dsp_status launch_general_n(dsp_context ctx, const FluxParams& p, long long layers, int maxm, const double* tabs,
-                            const JacView* jv, const int* order, int* heads) {
+dsp_status launch_general_n(dsp_context ctx, const FluxParams& p, long long layers, int maxm, int batch,
+                            const double* tabs, const JacView* jv, const int* order, int* heads) {
   if (p.flags & DSP_FLAG_SPHERICAL_BEAM)
-    return launch_general_chunk<N, true>(ctx, p, layers, maxm, tabs, jv, order, heads);
-  return launch_general_chunk<N, false>(ctx, p, layers, maxm, tabs, jv, order, heads);
+    return launch_general_chunk<N, true>(ctx, p, layers, maxm, batch, tabs, jv, order, heads);
+  return launch_general_chunk<N, false>(ctx, p, layers, maxm, batch, tabs, jv, order, heads);
 }
 
-dsp_status launch_general(dsp_context ctx, int N, const FluxParams& p, long long layers, int maxm,
+dsp_status launch_general(dsp_context ctx, int N, const FluxParams& p, long long layers, int maxm, int batch,
                           const double* tabs, const JacView* jv, const int* order, int* heads) {
   switch (N) {
-    case 4: return launch_general_n<4>(ctx, p, layers, maxm, tabs, jv, order, heads);
-    case 6: return launch_general_n<6>(ctx, p, layers, maxm, tabs, jv, order, heads);
-    case 8: return launch_general_n<8>(ctx, p, layers, maxm, tabs, jv, order, heads);
-    case 10: return launch_general_n<10>(ctx, p, layers, maxm, tabs, jv, order, heads);
-    case 12: return launch_general_n<12>(ctx, p, layers, maxm, tabs, jv, order, heads);
-    case 14: return launch_general_n<14>(ctx, p, layers, maxm, tabs, jv, order, heads);
-    case 16: return launch_general_n<16>(ctx, p, layers, maxm, tabs, jv, order, heads);
-    case 32: return launch_general_n<32>(ctx, p, layers, maxm, tabs, jv, order, heads);
-    case 64: return launch_general_n<64>(ctx, p, layers, maxm, tabs, jv, order, heads);
+    case 4: return launch_general_n<4>(ctx, p, layers, maxm, batch, tabs, jv, order, heads);
+    case 6: return launch_general_n<6>(ctx, p, layers, maxm, batch, tabs, jv, order, heads);
+    case 8: return launch_general_n<8>(ctx, p, layers, maxm, batch, tabs, jv, order, heads);
+    case 10: return launch_general_n<10>(ctx, p, layers, maxm, batch, tabs, jv, order, heads);
+    case 12: return launch_general_n<12>(ctx, p, layers, maxm, batch, tabs, jv, order, heads);
+    case 14: return launch_general_n<14>(ctx, p, layers, maxm, batch, tabs, jv, order, heads);
+    case 16: return launch_general_n<16>(ctx, p, layers, maxm, batch, tabs, jv, order, heads);
+    case 32: return launch_general_n<32>(ctx, p, layers, maxm, batch, tabs, jv, order, heads);
+    case 64: return launch_general_n<64>(ctx, p, layers, maxm, batch, tabs, jv, order, heads);
   }
   return fail(ctx, DSP_ERR_UNSUPPORTED, "unsupported num_streams");
 }
@@ -299,6 +307,24 @@ __global__ void gen_fill_nan_kernel(const int* ids, int count, int ntau, int num
 struct DevFlux {
   double* f[8];
 };
+
+// Instances of an N-stream boundary-value launch that fill the GPU twice over.
+template <int N>
+int64_t bvp_fill(int sm_count) { return (int64_t)2 * BCfg<N>::MINB * BCfg<N>::TPW * sm_count; }
+int64_t general_fill(int N, int sm_count) {
+  switch (N) {
+    case 4: return bvp_fill<4>(sm_count);
+    case 6: return bvp_fill<6>(sm_count);
+    case 8: return bvp_fill<8>(sm_count);
+    case 10: return bvp_fill<10>(sm_count);
+    case 12: return bvp_fill<12>(sm_count);
+    case 14: return bvp_fill<14>(sm_count);
+    case 16: return bvp_fill<16>(sm_count);
+    case 32: return bvp_fill<32>(sm_count);
+    case 64: return bvp_fill<64>(sm_count);
+  }
+  return 1;
+}
 
 inline size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
@@ -738,6 +764,8 @@ dsp_status general_solve(dsp_context ctx, const dsp_general_batch* bin, const ds
     int64_t surf_doubles = 0;  // bidirectional surface tables, one per slot
     int64_t be_doubles = 0;    // Buras-Emde tables, one per slot (all of one NT)
     int maxm = 0;
+    int batch = 1;             // azimuth modes per launch
+    int nt_max = 0;            // largest number of output depths
     // persistent boundary-value launches: the slots by descending layer count
     std::vector<int32_t> order;
   };
@@ -778,7 +806,7 @@ dsp_status general_solve(dsp_context ctx, const dsp_general_batch* bin, const ds
       if (hN[i] != N) continue;
       const int L = hL[i] > 0 ? hL[i] : 0;
       const int NT = user_tau ? b.num_user_tau : L + 1;
-      const int64_t rec = GenLayout::make(L, N, NT).stride + ptab_doubles(N) + (brdf ? brdf_stride(N, numu_eff) : 0) +
+      const int64_t rec = GenLayout::make(L, N, NT).stride + ptab_doubles(N) + (int64_t)ntau_need * numu_eff + (brdf ? brdf_stride(N, numu_eff) : 0) +
                           (becorr ? becor_stride(ntau_need, na) : 0);
       const size_t ib = (size_t)(rec + (int64_t)L * per_layer) * sizeof(double);
       if (!c.ids.empty() && bytes + ib > budget) flush();
@@ -789,6 +817,7 @@ dsp_status general_solve(dsp_context ctx, const dsp_general_batch* bin, const ds
       if (brdf) c.surf_doubles += brdf_stride(N, numu_eff);
       if (becorr) c.be_doubles += becor_stride(ntau_need, na);
       c.layers += L;
+      if (NT > c.nt_max) c.nt_max = NT;
       bytes += ib;
       int naz = N - 1;
       if (!dev)
@@ -799,6 +828,30 @@ dsp_status general_solve(dsp_context ctx, const dsp_general_batch* bin, const ds
       if (naz > c.maxm) c.maxm = naz;
     }
     flush();
+  }
+  // per mode: the layer and boundary-value records, the solution, the spherical
+  // records, P_l^m at the angles and the mode's intensities
+  auto mode_doubles = [&](const Chunk& c) -> int64_t {
+    return c.layers * (glrec_stride(c.N, numu_eff) + brec_stride(c.N) + c.N + sph_per_layer(c.N)) +
+           (int64_t)c.ids.size() * ptab_doubles(c.N) + ((int64_t)c.ids.size() * c.nt_max * numu_eff + 3) / 4 * 4;
+  };
+  auto fixed_doubles = [&](const Chunk& c) -> int64_t {
+    return c.inst_doubles + c.surf_doubles + c.be_doubles + c.layers * jac_per_layer(c.N);
+  };
+  // Azimuth modes per launch.  The modes of an instance are independent up to the
+  // convergence test, and a mode's boundary-value problem is a serial chain over
+  // the layers, so a chunk that does not fill the GPU runs as many modes side by
+  // side as do (one column at 32 streams: 32 launches of one busy warp -> one
+  // launch of 32, 25 -> 2 ms), within the workspace budget.  With a convergence
+  // criterion at most 4, so that few modes are computed past the end of a series.
+  for (Chunk& c : chunks) {
+    const int64_t fill = general_fill(c.N, ctx->sm_count), nc = (int64_t)c.ids.size();
+    int64_t mb = (fill + nc - 1) / nc;
+    const int64_t room = (int64_t)(budget / sizeof(double)) - fixed_doubles(c);
+    mb = std::min<int64_t>(mb, room / std::max<int64_t>(mode_doubles(c), 1));
+    if (b.accuracy_fourier_series > 0.0) mb = std::min<int64_t>(mb, 4);
+    if (brdf) mb = 1;
+    c.batch = (int)std::max<int64_t>(1, std::min<int64_t>(mb, c.maxm + 1));
   }
   if (chunks.empty()) goto copy_back;
   // the size-class queue of each chunk the schedule runs persistently
@@ -816,11 +869,7 @@ dsp_status general_solve(dsp_context ctx, const dsp_general_batch* bin, const ds
     for (const Chunk& c : chunks) {
       meta_need += align256(c.ids.size() * 4) + align256(c.ids.size() * 8) + align256((c.ids.size() + 1) * 8) +
                    align256(c.layers * 4) + align256(c.order.size() * 4) + align256((c.maxm + 1) * 4);
-      const int64_t lstride = glrec_stride(c.N, numu_eff);
-      const size_t w =
-          (size_t)(c.inst_doubles + c.surf_doubles + c.be_doubles + (int64_t)c.ids.size() * ptab_doubles(c.N) +
-                   c.layers * (lstride + brec_stride(c.N) + c.N + sph_per_layer(c.N) + jac_per_layer(c.N))) *
-          sizeof(double);
+      const size_t w = (size_t)(fixed_doubles(c) + c.batch * mode_doubles(c)) * sizeof(double);
       if (w > ws_need) ws_need = w;
     }
     if ((st = ensure(ctx, &ctx->meta, &ctx->meta_bytes, meta_need, "chunk index")) != DSP_OK) return st;
@@ -915,38 +964,45 @@ dsp_status general_solve(dsp_context ctx, const dsp_general_batch* bin, const ds
       g.lstride = glrec_stride(c.N, numu_eff);
       p.n = (int)nc;
       p.N = c.N;
+      // the instance records, the Jacobians' vectors, the surface and Buras-Emde
+      // tables, then each per-mode area for the modes of a launch
       double* w = static_cast<double*>(ctx->ws);
-      p.inst_rec = w;
-      p.layer_rec = w + c.inst_doubles;
-      p.bvp_rec = p.layer_rec + c.layers * g.lstride;
-      g.cc = p.bvp_rec + c.layers * brec_stride(c.N);
-      // after the solution coefficients: the spherical records
-      p.sph = spherical ? g.cc + c.layers * c.N : nullptr;
+      auto take = [&](int64_t doubles) {
+        double* r = w;
+        w += doubles;
+        return r;
+      };
+      p.inst_rec = take(c.inst_doubles);
       JacView jv;
       if (jac) {
-        // then the Jacobians' vectors
-        jv.cv = jrecs ? g.cc + c.layers * (c.N + sph_per_layer(c.N)) : nullptr;
+        jv.cv = jrecs ? take(c.layers * jac_per_layer(c.N)) : nullptr;
         jv.ndof = jdof;
         jv.ndof_out = (int)jdof_o;
         for (int f = 0; f < 6; ++f) jv.out[f] = djac[f];
       }
-      // after every per-layer area: the surface tables of the chunk's slots
-      double* const wend = static_cast<double*>(ctx->ws) + c.inst_doubles +
-                           c.layers * (g.lstride + brec_stride(c.N) + c.N + sph_per_layer(c.N) + jac_per_layer(c.N));
-      g.brdf = brdf ? wend : nullptr;
-      g.becor = becorr ? wend + c.surf_doubles : nullptr;
-      g.ptab = wend + c.surf_doubles + c.be_doubles;
+      g.brdf = brdf ? take(c.surf_doubles) : nullptr;
+      g.becor = becorr ? take(c.be_doubles) : nullptr;
+      g.ms_layer = c.layers * g.lstride;
+      g.ms_bvp = c.layers * brec_stride(c.N);
+      g.ms_cc = c.layers * c.N;
+      g.ms_sph = c.layers * sph_per_layer(c.N);
+      g.ms_ptab = (int64_t)nc * ptab_doubles(c.N);
+      g.ms_int = ((int64_t)nc * c.nt_max * numu_eff + 3) / 4 * 4;
+      g.nt_max = c.nt_max;
+      p.layer_rec = take(c.batch * g.ms_layer);
+      p.bvp_rec = take(c.batch * g.ms_bvp);
+      g.cc = take(c.batch * g.ms_cc);
+      p.sph = spherical ? take(c.batch * g.ms_sph) : nullptr;
+      g.ptab = take(c.batch * g.ms_ptab);
+      g.imode = take(c.batch * g.ms_int);
       const double* tabs = nullptr;
       if ((st = get_mode_tables(ctx, c.N, &tabs)) != DSP_OK) return st;
       if (ctx->debug & DSP_DEBUG_POISON_SCRATCH) {
-        const size_t wb = (size_t)(c.inst_doubles + c.surf_doubles + c.be_doubles + (int64_t)nc * ptab_doubles(c.N) +
-                                   c.layers * (g.lstride + brec_stride(c.N) + c.N + sph_per_layer(c.N) +
-                                               jac_per_layer(c.N))) *
-                          sizeof(double);
+        const size_t wb = (size_t)(fixed_doubles(c) + c.batch * mode_doubles(c)) * sizeof(double);
         e = cudaMemsetAsync(ctx->ws, 0xFF, wb, s);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "scratch poison");
       }
-      if ((st = launch_general(ctx, c.N, p, c.layers, c.maxm, tabs, jac ? &jv : nullptr, order, heads)) != DSP_OK)
+      if ((st = launch_general(ctx, c.N, p, c.layers, c.maxm, c.batch, tabs, jac ? &jv : nullptr, order, heads)) != DSP_OK)
         return st;
     }
   }

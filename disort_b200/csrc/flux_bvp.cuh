@@ -50,7 +50,7 @@ struct BCfg {
   // so that 8 lanes reading one row each with 16-byte loads meet no conflict
   static constexpr int LDM = HP % 4 == 2 ? HP : HP + 2;
   static constexpr int MAT = H * LDM;
-  static constexpr int NV = 5 * HP + 2;         // vectors of a layer record
+  static constexpr int NV = 7 * HP + 2;         // vectors of a layer record
   static constexpr int SB = 2 * HP + 4;         // pivot-row buffer of a sweep
   // team shared memory (doubles)
   static constexpr int O_X = 0;                 // X^T: row c = column c of X
@@ -72,6 +72,9 @@ struct BCfg {
   static constexpr int MINB_REGS = H <= 8 ? 16 : (H <= 16 ? 12 : 8);
   static constexpr int MINB = MINB_SMEM < MINB_REGS ? MINB_SMEM : MINB_REGS;
   static constexpr bool ROLL = H > 16;          // 64 streams: rolled outer loops
+  // the lane's row of the identity in registers: diagonal elements as products
+  // (the FP64 pipe has room) instead of selects by lane
+  static constexpr bool IDREG = H <= 8;
 };
 
 // Negative inverse of a symmetric positive definite matrix with unit diagonal
@@ -84,7 +87,7 @@ struct BCfg {
 // alignment).  With a unit diagonal every pivot is <= 1, so the pivot lane can
 // take the common update with 1 - 1/pivot in the place of the multiplier
 // without losing digits: v - v (1 - p) = v p, p >= 1.
-template <int H, int SB>
+template <int H, int SB, bool CHECK>
 __device__ __forceinline__ void sweep_step(double* a, const int j, const int k, const bool odd, const bool store,
                                            double* buf, bool& singular) {
   double* b = buf + (odd ? SB : 0);
@@ -96,8 +99,11 @@ __device__ __forceinline__ void sweep_step(double* a, const int j, const int k, 
   __syncwarp();
   const double* v = b + k + o;
   const double d = v[0];
-  if (d == 0.0) singular = true;  // a zero pivot: its row and column are left out
-  const double p = d == 0.0 ? 0.0 : rcp_newton(d);
+  double p = rcp_newton(d);
+  if (CHECK && d == 0.0) {  // a zero pivot: its row and column are left out
+    singular = true;
+    p = 0.0;
+  }
   const double c = a[0] * p;
   const double cc = j == k ? 1.0 - p : c;
   const double2* v2 = reinterpret_cast<const double2*>(v);
@@ -114,18 +120,18 @@ __device__ __forceinline__ void sweep_step(double* a, const int j, const int k, 
   a[H - 1] = j == k ? -p : c;
 }
 
-template <int H, int SB, bool ROLL>
+template <int H, int SB, bool ROLL, bool CHECK = false>
 __device__ __forceinline__ void sweep_inverse(double* a, const int j, const bool store, double* buf, bool& singular) {
   if constexpr (ROLL) {
     static_assert(!ROLL || H % 2 == 0, "steps in pairs");
 #pragma unroll 1
     for (int k = 0; k < H; k += 2) {
-      sweep_step<H, SB>(a, j, k, false, store, buf, singular);
-      sweep_step<H, SB>(a, j, k + 1, true, store, buf, singular);
+      sweep_step<H, SB, CHECK>(a, j, k, false, store, buf, singular);
+      sweep_step<H, SB, CHECK>(a, j, k + 1, true, store, buf, singular);
     }
   } else {
 #pragma unroll
-    for (int k = 0; k < H; ++k) sweep_step<H, SB>(a, j, k, (k & 1) != 0, store, buf, singular);
+    for (int k = 0; k < H; ++k) sweep_step<H, SB, CHECK>(a, j, k, (k & 1) != 0, store, buf, singular);
   }
   __syncwarp();
 }
@@ -208,7 +214,8 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
   double* const vd = ve + HP;
 
   const bool ifb = (p.flags & DSP_FLAG_INDEX_FROM_BOTTOM) != 0;
-  const int m = GEN ? p.g.m : 0;
+  const int mrow = GEN ? (int)blockIdx.y : 0;
+  const int m = GEN ? p.g.m + mrow : 0;
   // i: status / input / output index, L: layers, NT: output levels
   const int sl = slot >= 0 ? slot : 0;
   const int i = GEN ? p.g.ids[sl] : sl;
@@ -218,8 +225,8 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
   const double* const rec = p.inst_rec + (GEN ? p.g.inst_off[sl] : (long long)i * p.il.stride);
   const long long lay0 = GEN ? p.g.lay_off[sl] : (long long)i * p.L;
   const long long lstride = GEN ? p.g.lstride : (long long)lrec_stride(N);
-  const double* const lrec0 = p.layer_rec + lay0 * lstride;
-  double* const brec0 = p.bvp_rec + lay0 * brec_stride(N);
+  const double* const lrec0 = p.layer_rec + (GEN ? mrow * p.g.ms_layer : 0ll) + lay0 * lstride;
+  double* const brec0 = p.bvp_rec + (GEN ? mrow * p.g.ms_bvp : 0ll) + lay0 * brec_stride(N);
   auto oidx = [&](int lev) {
     if constexpr (GEN) return (long long)i * p.g.ntau_out + (ifb ? NT - 1 - lev : lev);
     else return (long long)i * NT + (ifb ? L - lev : lev);
@@ -251,40 +258,47 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
   const bool beam = fbeam > 0.0;
   const double* const taus = rec + il.tau_s;
   const double* const btr = rec + il.btr;
-  const double* const dtau_s = rec + il.dtau_s;
   const double dj = p.tables[tab_dsim(N) + j];
-  bool singular = false, sg = false;
+  bool singular = false;
 
   // the layer record of layer l: X^T and the vectors, Y^T
   auto load_x = [&](int l) {
     if (l < ncut) {
       const double* lr = lrec0 + (long long)l * lstride;
-      team_copy_rows_async<TEAM>(Xs, LDM, lr + mod_X(N), HP, H, HP, t);
-      team_copy_async<TEAM>(vec, lr + mod_k(N), C::NV, t);
+      team_copy_mat<TEAM, HP, H, LDM>(Xs, lr + mod_X(N), t);
+      team_copy_vec<TEAM, C::NV>(vec, lr + mod_k(N), t);
     }
     cp_async_commit();
   };
   auto load_y = [&](int l) {
-    if (l < ncut) team_copy_rows_async<TEAM>(Ys, LDM, lrec0 + (long long)l * lstride + mod_Y(N), HP, H, HP, t);
+    if (l < ncut) team_copy_mat<TEAM, HP, H, LDM>(Ys, lrec0 + (long long)l * lstride + mod_Y(N), t);
     cp_async_commit();
   };
-  // per-layer scalars: dtau, scaled depths and beam factors of the two boundaries
-  struct Scal { double dt, t0, t1, b0, b1; };
-  auto load_s = [&](int l) {
-    Scal s{0.0, 0.0, 0.0, 0.0, 0.0};
-    if (l < ncut) {
-      s.dt = dtau_s[l];
+  // per-layer scalars, loaded one layer ahead: scaled depths and beam factors of
+  // the two boundaries; going up also 1 - omega and the unscaled depths
+  struct Scal { double t0, t1, b0, b1, w1, u0, u1; };
+  auto load_s = [&](int l, bool up) {
+    Scal s{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    if (l >= 0 && l < ncut) {
       s.t0 = taus[l];
       s.t1 = taus[l + 1];
       if (beam) {
         s.b0 = btr[l];
         s.b1 = btr[l + 1];
       }
+      if (up) {
+        const int lin = ifb ? L - 1 - l : l;
+        s.w1 = 1.0 - (GEN ? p.g.ssa[p.g.in_off[i] + lin] : p.ssa(i, lin));
+        if (!GEN && beam) {
+          s.u0 = rec[il.tauc + l];
+          s.u1 = rec[il.tauc + l + 1];
+        }
+      }
     }
     return s;
   };
   // pseudo-spherical beam: the record [c1 | d1 | xba | Chapman factor] of layer l
-  auto SR = [&](int l) { return p.sph + (lay0 + l) * sph_stride(N); };
+  auto SR = [&](int l) { return p.sph + (GEN ? mrow * p.g.ms_sph : 0ll) + (lay0 + l) * sph_stride(N); };
   // lane j's particular solution (c, d) at scaled depth tau of layer l; `bt` the
   // beam factor there (computeBeamSourceSpherical's form when SPH)
   auto particular = [&](int l, double tau, double bt, double& c, double& d) {
@@ -294,24 +308,24 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
       if constexpr (SPH) {
         const double* sr = SR(l < ncut ? l : 0);
         const double e = exp(-sr[sph_xba(N)] * tau);
-        c = e * fma(sr[j], tau, vec[HP + j]);
-        d = e * fma(sr[H + j], tau, vec[2 * HP + j]);
+        c = e * fma(sr[j], tau, vec[3 * HP + j]);
+        d = e * fma(sr[H + j], tau, vec[4 * HP + j]);
       } else {
-        c = vec[HP + j] * bt;
-        d = vec[2 * HP + j] * bt;
+        c = vec[3 * HP + j] * bt;
+        d = vec[4 * HP + j] * bt;
       }
     }
     if (thermal) {
-      const double x0 = vec[5 * HP], x1 = vec[5 * HP + 1];
-      c = fma(vec[3 * HP + j], fma(x1, tau, x0), c);
-      d = fma(vec[4 * HP + j], x1, d);
+      const double x0 = vec[7 * HP], x1 = vec[7 * HP + 1];
+      c = fma(vec[5 * HP + j], fma(x1, tau, x0), c);
+      d = fma(vec[6 * HP + j], x1, d);
     }
   };
 
   // ------------------------------------------------------------------- down
   load_x(0);
   load_y(0);
-  Scal sc = load_s(0);
+  Scal sc = load_s(0, false);
   // odd h: the pad element of every gathered vector and row stays 0
   if (own) {
     for (int r = 0; r < HP; ++r) As[j * LDM + r] = r == j ? 1.0 : 0.0;
@@ -322,19 +336,22 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
     for (int v = 0; v < C::NG; ++v) vg[v * HP + H] = 0.0;
   __syncwarp();
 
-  double a[H];
+  double a[H], id[C::IDREG ? H : 1];
+  if constexpr (C::IDREG) {
+#pragma unroll
+    for (int r = 0; r < H; ++r) id[r] = r == j ? 1.0 : 0.0;
+  }
   for (int l = 0; l < Lw; ++l) {
     const bool on = l < ncut;
     const Scal s = sc;
-    sc = load_s(l + 1);
+    sc = load_s(l + 1, false);
     cp_async_wait<1>();
     __syncwarp();
-    const double k = vec[j];
-    const double ex = exp(-k * s.dt);
-    const double fx = -expm1(-2.0 * k * s.dt);
+    const double ex = vec[HP + j], fx = vec[2 * HP + j];
     double ct, dt_, cb, db;
     particular(l, s.t0, s.b0, ct, dt_);
     particular(l, s.t1, s.b1, cb, db);
+    DSP_PHASE(0)
     // I + M = I + X^T A X, column j
     const double* xj = Xs + j * LDM;
     double diag = 0.0;
@@ -358,7 +375,13 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
 #pragma unroll
         for (int r = 0; r < H; ++r) {
           a[r] = dot_reg<H>(tv, Xs + r * LDM);
-          if (r == j) diag = 1.0 + a[r];
+          if constexpr (C::IDREG) {
+            a[r] += id[r];
+            diag = fma(a[r], id[r], diag);
+          } else if (r == j) {
+            a[r] += 1.0;
+            diag = a[r];
+          }
         }
       }
     }
@@ -372,12 +395,14 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
     __syncwarp();
 #pragma unroll
     for (int r = 0; r < H; ++r) {
-      const double v = ROLL ? As[r * LDM + j] : a[r];
-      a[r] = r == j ? 1.0 : v * (s1 * vsc[r]);
+      if constexpr (ROLL) a[r] = r == j ? 1.0 : As[r * LDM + j] * (s1 * vsc[r]);
+      else a[r] *= s1 * vsc[r];
     }
     // X and the vectors are used up: the next layer's start loading
     load_x(l + 1);
-    sweep_inverse<H, SB, ROLL>(a, j, own, sbuf, sg);
+    DSP_PHASE(1)
+    sweep_inverse<H, SB, ROLL>(a, j, own, sbuf, singular);
+    DSP_PHASE(2)
     double* const br = brec0 + (long long)(on ? l : 0) * brec_stride(N);
 #pragma unroll
     for (int r = 0; r < H; ++r) {
@@ -389,10 +414,14 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
     const double q = ex * rj;
     // Z = (1 - E^2) + 2 E H E
     const double ex2 = 2.0 * ex;
+    diag = 0.0;
 #pragma unroll
     for (int r = 0; r < H; ++r) {
       a[r] *= ex2 * ve[r];
-      if (r == j) {
+      if constexpr (C::IDREG) {
+        a[r] = fma(fx, id[r], a[r]);
+        diag = fma(a[r], id[r], diag);
+      } else if (r == j) {
         a[r] += fx;
         diag = a[r];
       }
@@ -405,10 +434,10 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
     }
     __syncwarp();
 #pragma unroll
-    for (int r = 0; r < H; ++r) a[r] = r == j ? 1.0 : a[r] * (s2 * vsc[r]);
-    sweep_inverse<H, SB, ROLL>(a, j, own, sbuf, sg);
-    if (on && sg) singular = true;
-    sg = false;
+    for (int r = 0; r < H; ++r) a[r] *= s2 * vsc[r];
+    DSP_PHASE(3)
+    sweep_inverse<H, SB, ROLL>(a, j, own, sbuf, singular);
+    DSP_PHASE(4)
 #pragma unroll
     for (int r = 0; r < H; ++r) {
       a[r] = -a[r] * (s2 * vsc[r]);
@@ -418,7 +447,7 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
     if (own) {
       vgam[j] = gb;
 #pragma unroll
-      for (int r = 0; r < H; ++r) Ws[j * LDM + r] = r == j ? fma(2.0, a[r], -1.0) : 2.0 * a[r];
+      for (int r = 0; r < H; ++r) Ws[j * LDM + r] = C::IDREG ? fma(2.0, a[r], -id[C::IDREG ? r : 0]) : (r == j ? fma(2.0, a[r], -1.0) : 2.0 * a[r]);
     }
     cp_async_wait<1>();  // Y of this layer
     __syncwarp();
@@ -451,11 +480,10 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
     }
     __syncwarp();
     load_y(l + 1);
+    DSP_PHASE(5)
   }
   cp_async_wait<0>();
   __syncwarp();
-  DSP_PHASE(20)
-
   // ----------------------------------------------------------------- surface
   // up = R down + src at the bottom, psi = A phi + g:
   // [(I - R) + (I + R) A] phi = 2 src - (I + R) g.
@@ -473,8 +501,8 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
     if (act && beam) {
       const double* sr = SR(ncut - 1);
       const double tau = taus[ncut], e = exp(-sr[sph_xba(N)] * tau), bt = btr[ncut];
-      dc = vec[HP + j] * bt - e * fma(sr[j], tau, vec[HP + j]);
-      dd = vec[2 * HP + j] * bt - e * fma(sr[H + j], tau, vec[2 * HP + j]);
+      dc = vec[3 * HP + j] * bt - e * fma(sr[j], tau, vec[3 * HP + j]);
+      dd = vec[4 * HP + j] * bt - e * fma(sr[H + j], tau, vec[4 * HP + j]);
     }
     if (own) {
       vw1[j] = dc;
@@ -529,7 +557,7 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
       __syncwarp();
 #pragma unroll
       for (int r = 0; r < H; ++r) a[r] = r == j ? 1.0 : a[r] * (s1 * vsc[r]);
-      sweep_inverse<H, SB, ROLL>(a, j, own, sbuf, singular);
+      sweep_inverse<H, SB, ROLL, true>(a, j, own, sbuf, singular);
 #pragma unroll
       for (int r = 0; r < H; ++r) {
         a[r] = -a[r] * (s1 * vsc[r]);
@@ -611,20 +639,19 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
     }
     __syncwarp();
   }
-  DSP_PHASE(21)
+  DSP_PHASE(6)
 
   // --------------------------------------------------------------------- up
   bool nonfinite = false;
-  auto ssa_of = [&](int l) {
-    const int lin = ifb ? L - 1 - l : l;
-    return GEN ? p.g.ssa[p.g.in_off[i] + lin] : p.ssa(i, lin);
-  };
+  const double wd = own ? 0.5 * p.tables[tab_wt(N) + j] / dj : 0.0;  // w / (2 d) of stream j
+  const double muj = p.tables[tab_mu(N) + j];
+  const double rumu0 = beam ? 1.0 / umu0 : 0.0;
   // fluxes at output level lu of layer l from the modal amplitudes (c, d) of the
   // homogeneous part there (computeFluxes, FluxSolver.cpp:1138-1287;
   // DisortSolver.cpp:1980-2124); `put`: this team has the level
-  auto eval_level = [&](int l, int lu, double utaupr, double utau, double c, double d, bool put) {
+  auto eval_level = [&](int l, int lu, double utaupr, double utau, double w1, double c, double d, bool put) {
     const double ch = SPH && beam && put ? SR(l)[sph_ch(N)] : 1.0;
-    const double fact = beam ? exp(-utaupr / (SPH ? ch : umu0)) : 0.0;
+    const double fact = beam ? (SPH ? exp(-utaupr / ch) : exp(-utaupr * rumu0)) : 0.0;
     double cp, dp;
     particular(l, utaupr, fact, cp, dp);
     __syncwarp();
@@ -634,9 +661,8 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
     }
     __syncwarp();
     const double ph = dot_col<H>(Xs + j, LDM, vgam), ps = dot_col<H>(Ys + j, LDM, vd);
-    const double wd = own ? 0.5 * p.tables[tab_wt(N) + j] / dj : 0.0, md = own ? p.tables[tab_mu(N) + j] : 0.0;
     double su = wd * (ph + ps), sd = wd * (ph - ps);
-    double fu = md * su, fd = md * sd;
+    double fu = muj * su, fd = muj * sd;
 #pragma unroll
     for (int off = TEAM / 2; off > 0; off >>= 1) {
       su += __shfl_xor_sync(0xffffffffu, su, off);
@@ -649,16 +675,17 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
       if (beam) {
         dirint = fbeam * fact;
         fldir = umu0 * fbeam * fact;
-        fdir = SPH ? fabs(umu0) * fbeam * exp(-utau / ch) : umu0 * fbeam * exp(-utau / umu0);
+        fdir = SPH ? fabs(umu0) * fbeam * exp(-utau / ch) : umu0 * fbeam * exp(-utau * rumu0);
       }
       fu *= 2.0 * PI;
       fd *= 2.0 * PI;
       const double fdn = (fd + fldir) - fdir;
-      const double ua = (2.0 * PI * (su + sd) + dirint) / (4.0 * PI);
-      const double uaso = dirint / (4.0 * PI);
+      constexpr double R4PI = 1.0 / (4.0 * PI);
+      const double ua = 0.5 * (su + sd) + dirint * R4PI;
+      const double uaso = dirint * R4PI;
       const double uad = 0.5 * sd, uau = 0.5 * su;
-      const double plsorc = thermal ? fma(vec[5 * HP + 1], utaupr, vec[5 * HP]) : 0.0;
-      const double dfdt = (1.0 - ssa_of(l)) * 4.0 * PI * (ua - plsorc);
+      const double plsorc = thermal ? fma(vec[7 * HP + 1], utaupr, vec[7 * HP]) : 0.0;
+      const double dfdt = w1 * 4.0 * PI * (ua - plsorc);
       const double o[8] = {fdir, fdn, fu, dfdt, ua, uad, uau, uaso};
 #pragma unroll
       for (int f = 0; f < 8; ++f)
@@ -689,32 +716,32 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
       const double* lr = lrec0 + (long long)l * lstride;
       const double* br = brec0 + (long long)l * brec_stride(N);
       if (what == 0) {
-        team_copy_rows_async<TEAM>(Ys, LDM, lr + mod_Y(N), HP, H, HP, t);
-        team_copy_rows_async<TEAM>(Xs, LDM, lr + mod_X(N), HP, H, HP, t);
-        team_copy_async<TEAM>(vec, lr + mod_k(N), C::NV, t);
+        team_copy_mat<TEAM, HP, H, LDM>(Ys, lr + mod_Y(N), t);
+        team_copy_mat<TEAM, HP, H, LDM>(Xs, lr + mod_X(N), t);
+        team_copy_vec<TEAM, C::NV>(vec, lr + mod_k(N), t);
       } else {
-        team_copy_rows_async<TEAM>(Ws, LDM, br + brec_G(N), HP, H, HP, t);  // G
-        team_copy_rows_async<TEAM>(As, LDM, br + brec_H(N), HP, H, HP, t);  // H
+        team_copy_mat<TEAM, HP, H, LDM>(Ws, br + brec_G(N), t);  // G
+        team_copy_mat<TEAM, HP, H, LDM>(As, br + brec_H(N), t);  // H
       }
     }
     cp_async_commit();
   };
   load_up(Lw - 1, 0);
   load_up(Lw - 1, 1);
-  sc = load_s(Lw - 1);
+  sc = load_s(Lw - 1, true);
   double r_next = Lw - 1 < ncut && own ? brec0[(long long)(Lw - 1) * brec_stride(N) + brec_r(N) + j] : 0.0;
   for (int l = Lw - 1; l >= 0; --l) {
     const bool on = l < ncut;
     const Scal s = sc;
     const double rj = r_next;
     if (l > 0) {
-      sc = load_s(l - 1);
+      sc = load_s(l - 1, true);
       r_next = l - 1 < ncut && own ? brec0[(long long)(l - 1) * brec_stride(N) + brec_r(N) + j] : 0.0;
     }
     cp_async_wait<0>();
     __syncwarp();
-    const double k = vec[j];
-    const double ex = exp(-k * s.dt);
+    DSP_PHASE(7)
+    const double ex = vec[HP + j];
     double ct, dt_, cb, db;
     particular(l, s.t0, s.b0, ct, dt_);
     particular(l, s.t1, s.b1, cb, db);
@@ -731,14 +758,15 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
     // G and H are used up
     load_up(l - 1, 1);
     const double phi = dot_col<H>(Xs + j, LDM, vw1);
+    DSP_PHASE(8)
     if constexpr (GEN) {
       if (on && own) {
-        double* cc = p.g.cc + (lay0 + l) * N;
+        double* cc = p.g.cc + mrow * p.g.ms_cc + (lay0 + l) * N;
         cc[j] = b;
         cc[H + j] = av;
       }
       if (m == 0) {
-        const double fx = -expm1(-2.0 * k * s.dt);
+        const double k = vec[j], fx = vec[2 * HP + j];
         for (int lu = 0; lu < NTw; ++lu) {
           const bool put = on && lu < NT && (int)lyr_l[lu] == l;
           if (!__any_sync(0xffffffffu, put)) continue;
@@ -747,20 +775,20 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
           // C inside the layer from its values at the two boundaries (no cancellation)
           double cu = c;
           if (fx > 0.0) cu = (c * (e1 * -expm1(-2.0 * k * x2)) + chom_b * (e2 * -expm1(-2.0 * k * x1))) / fx;
-          eval_level(l, lu, tu, put ? utau_l[lu] : 0.0, cu, e2 * b - e1 * av, put);
+          eval_level(l, lu, tu, put ? utau_l[lu] : 0.0, s.w1, cu, e2 * b - e1 * av, put);
         }
       }
     } else {
-      eval_level(l, l + 1, s.t1, on ? rec[il.tauc + l + 1] : 0.0, chom_b, b - ex * av, on);
-      if (l == 0) eval_level(0, 0, s.t0, on ? rec[il.tauc] : 0.0, c, ex * b - av, on);
+      eval_level(l, l + 1, s.t1, s.u1, s.w1, chom_b, b - ex * av, on);
+      if (l == 0) eval_level(0, 0, s.t0, s.u0, s.w1, c, ex * b - av, on);
     }
     __syncwarp();
     if (on && own) ve[j] = phi;
     load_up(l - 1, 0);
     __syncwarp();
+    DSP_PHASE(9)
   }
   cp_async_wait<0>();
-  DSP_PHASE(22)
   DSP_PHASE_END
   if (act) {
     if (singular && t == 0) set_status(p.status, i, DSP_ERR_SINGULAR);
@@ -778,12 +806,13 @@ __global__ void __launch_bounds__(32, BCfg<N>::MINB) flux_bvp_kernel(FluxParams 
 
 // Persistent form (general solver): a resident grid whose warps take chunk slots
 // from a work queue -- `order`, the chunk's slots by descending layer count (the
-// size classes), consumed through the counter `head` -- so that the longest
+// size classes), consumed through one counter per mode -- so that the longest
 // instances start first, the instances of a warp have about the same depth and
 // the tail of the launch is short.
 template <int N, bool SPH = false>
-__global__ void __launch_bounds__(32, BCfg<N>::MINB) gen_bvp_persistent_kernel(FluxParams p, const int* order, int* head) {
+__global__ void __launch_bounds__(32, BCfg<N>::MINB) gen_bvp_persistent_kernel(FluxParams p, const int* order, int* heads) {
   using C = BCfg<N>;
+  int* const head = heads + blockIdx.y;  // one queue per mode of the launch
   for (;;) {
     int k = 0;
     if (threadIdx.x == 0) k = atomicAdd(head, C::TPW);

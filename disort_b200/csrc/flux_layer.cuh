@@ -243,6 +243,11 @@ __device__ __forceinline__ void jacobi_rot(double apq, double app, double aqq, d
 }
 
 // One layer task: its instance, layer and addresses.
+template <bool GEN>
+__device__ __forceinline__ int mode_row() { return GEN ? (int)blockIdx.y : 0; }
+template <bool GEN>
+__device__ __forceinline__ int mode_of(const FluxParams& p) { return GEN ? p.g.m + (int)blockIdx.y : 0; }
+
 template <int N, bool GEN>
 struct LayerTask {
   int i, lc;          // input / status index, layer (top down)
@@ -264,7 +269,7 @@ __device__ __forceinline__ LayerTask<N, GEN> layer_task(const FluxParams& p, lon
     Lin = p.g.Ls[q.i];
     q.il = InstLayout::make(Lin, N);
     q.rec = p.inst_rec + p.g.inst_off[q.slot];
-    q.lrec = p.layer_rec + task * p.g.lstride;
+    q.lrec = p.layer_rec + mode_row<GEN>() * p.g.ms_layer + task * p.g.lstride;
     const int lin = (p.flags & DSP_FLAG_INDEX_FROM_BOTTOM) ? Lin - 1 - q.lc : q.lc;
     q.pml = p.g.pmom + (p.g.in_off[q.i] + lin) * (long long)p.pc;
   } else {
@@ -281,7 +286,7 @@ __device__ __forceinline__ LayerTask<N, GEN> layer_task(const FluxParams& p, lon
   // general solver also skips modes past the instance's last one or after its
   // azimuthal series converged
   q.live = !(p.status && p.status[q.i] == DSP_ERR_INVALID_INPUT) && q.lc < (int)q.rec[H_NCUT];
-  if constexpr (GEN) q.live = q.live && p.g.m <= (int)q.rec[H_NAZ] && q.rec[H_DONE] == 0.0;
+  if constexpr (GEN) q.live = q.live && mode_of<GEN>(p) <= (int)q.rec[H_NAZ] && q.rec[H_DONE] == 0.0;
   return q;
 }
 template <bool GEN>
@@ -292,7 +297,7 @@ __device__ __forceinline__ long long layer_tasks(const FluxParams& p) {
 // P_l^m(-mu0) of an instance
 template <int N, bool GEN>
 __device__ __forceinline__ const double* beam_legendre(const FluxParams& p, const LayerTask<N, GEN>& q) {
-  if constexpr (GEN) return p.g.ptab + q.slot * (long long)(N * (1 + p.g.numu));
+  if constexpr (GEN) return p.g.ptab + mode_row<GEN>() * p.g.ms_ptab + q.slot * (long long)(N * (1 + p.g.numu));
   else return q.rec + q.il.yb;
 }
 
@@ -338,13 +343,14 @@ __global__ void __launch_bounds__(LCfg<N>::CTA, LCfg<N>::MINB) flux_layer_kernel
   constexpr int BPA = NPAIR;  // blocks (a, b) per column pair b
   extern __shared__ double smem[];
   // CTA-level constant tables
+  const int m = mode_of<GEN>(p);
   for (int k = threadIdx.x; k < C::TAB; k += blockDim.x) smem[k] = p.tables[k];
   __syncthreads();
   const double* mu = smem + tab_mu(N);
   const double* wt = smem + tab_wt(N);
   const double* dsim = smem + tab_dsim(N);
   const double* dinv = smem + tab_dinv(N);
-  const double* Y = p.tables + tab_ylm(N);
+  const double* Y = p.tables + (long long)mode_row<GEN>() * tab_size(N) + tab_ylm(N);
 
   const int team = threadIdx.x / TEAM, t = threadIdx.x % TEAM;
   const long long task = (long long)blockIdx.x * C::TPC + team;
@@ -369,7 +375,7 @@ __global__ void __launch_bounds__(LCfg<N>::CTA, LCfg<N>::MINB) flux_layer_kernel
     for (int k = t; k < N; k += TEAM) gl[k] = phase_coeff<GEN>(k, q.pml[k], mode, ws, f, sig);
   }
   team_sync<TEAM>();
-  const int odd0 = GEN ? 1 - (p.g.m & 1) : 1;  // first l of odd l + m
+  const int odd0 = GEN ? 1 - (m & 1) : 1;  // first l of odd l + m
   // ---- -A_s and -B_s from the even and odd phase sums ----------------------
   for (int it = t; it < NN * NN; it += TEAM) {
     const int r = it / NN, c = it % NN;
@@ -392,7 +398,7 @@ __global__ void __launch_bounds__(LCfg<N>::CTA, LCfg<N>::MINB) flux_layer_kernel
   if (beam) {
     // (2 - delta_m0) F0 / 4pi sum_k g'_k P_k^m(mu_r) P_k^m(-mu0) by parity (DisortSolver.cpp:1361-1368)
     const double* yb = beam_legendre<N, GEN>(p, q);
-    const double fac = ((GEN && p.g.m > 0) ? 2.0 * fbeam : fbeam) / (4.0 * 3.14159265358979323846);
+    const double fac = ((GEN && m > 0) ? 2.0 * fbeam : fbeam) / (4.0 * 3.14159265358979323846);
     for (int r = t; r < NN; r += TEAM) {
       double so = 0.0, se = 0.0;
       for (int l = 0; l < N; l += 2) {
@@ -579,8 +585,11 @@ __global__ void __launch_bounds__(LCfg<N>::CTA, LCfg<N>::MINB) flux_layer_kernel
     }
     const double* x = (primary ? MA : T) + c;
     const double* y = (primary ? T : MA) + c;
-    double* vec = q.lrec + mod_k(N);
-    vec[c] = k;
+    double* vec = q.lrec;
+    const double dts = q.rec[q.il.dtau_s + q.lc];
+    vec[mod_k(N) + c] = k;
+    vec[mod_E(N) + c] = exp(-k * dts);
+    vec[mod_F(N) + c] = -expm1(-2.0 * k * dts);
     if (beam) {
       double umu0 = q.rec[H_UMU0];
       bool res = false;
@@ -591,8 +600,8 @@ __global__ void __launch_bounds__(LCfg<N>::CTA, LCfg<N>::MINB) flux_layer_kernel
         // angles, up and down, for the user-angle interpolation and
         // flux_sph_source_kernel (DisortSolver.cpp:1524-1527)
         const double dm = 0.5 * mu[c] / dsim[c];
-        vec[HP + c] = dm * (b1[c] + b2[c]);
-        vec[2 * HP + c] = dm * (b1[c] - b2[c]);
+        vec[mod_cb(N) + c] = dm * (b1[c] + b2[c]);
+        vec[mod_db(N) + c] = dm * (b1[c] - b2[c]);
       } else {
         double al = 0.0, be = 0.0;
         for (int r = 0; r < NN; ++r) {
@@ -600,17 +609,17 @@ __global__ void __launch_bounds__(LCfg<N>::CTA, LCfg<N>::MINB) flux_layer_kernel
           be += y[r * NS] * b2[r];
         }
         const double r0 = 1.0 / umu0, den = k * k - r0 * r0;
-        vec[HP + c] = (k * al - be * r0) / den;
-        vec[2 * HP + c] = (k * be - al * r0) / den;
+        vec[mod_cb(N) + c] = (k * al - be * r0) / den;
+        vec[mod_db(N) + c] = (k * be - al * r0) / den;
       }
     }
-    if ((p.flags & DSP_FLAG_THERMAL) && (!GEN || p.g.m == 0)) {
+    if ((p.flags & DSP_FLAG_THERMAL) && m == 0) {
       double v = 0.0;
       for (int r = 0; r < NN; ++r) v += x[r * NS] * (dsim[r] / mu[r]);
       v = 2.0 * (1.0 - ws) * v / k;
-      vec[3 * HP + c] = v;
-      vec[4 * HP + c] = v / k;
-      if (c == 0) thermal_source(q, vec[5 * HP], vec[5 * HP + 1]);
+      vec[mod_ct(N) + c] = v;
+      vec[mod_dt(N) + c] = v / k;
+      if (c == 0) thermal_source(q, vec[mod_xr(N)], vec[mod_xr(N) + 1]);
     }
   }
   team_sync<TEAM>();
@@ -688,10 +697,27 @@ __global__ void __launch_bounds__(128) flux_layer_front_kernel(FluxParams p, Con
   constexpr int NN = N / 2;
   using HO = Handoff<NN>;
   constexpr int TRI = HO::TRI;
+  // P_l^m(mu_i): the flux path's from the constant bank, the general solver's (one
+  // table per mode of the launch) from shared memory, read where it is used
+  // (volatile: kept in registers over the sums, the table would push them to
+  // local memory)
+  __shared__ double ysm[GEN ? N * NN : 1];
+  if constexpr (GEN) {
+    const double* Y = p.tables + (long long)mode_row<GEN>() * tab_size(N) + tab_ylm(N);
+    for (int e = threadIdx.x; e < N * NN; e += blockDim.x) ysm[e] = Y[(e / NN) * N + e % NN];
+    __syncthreads();
+  }
+  const volatile double* const yv = ysm;
+  auto ytab = [&](int l, int i) -> double {
+    if constexpr (GEN) return yv[l * NN + i];
+    else return tc.y[l * NN + i];
+  };
   const long long nt = layer_tasks<GEN>(p);
   const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= nt) return;
-  auto hp = [&](int e) { return handoff_lane<NN>(p.bvp_rec, nt, j, e); };
+  const int m = mode_of<GEN>(p);
+  double* const hand = p.bvp_rec + mode_row<GEN>() * p.g.ms_bvp;
+  auto hp = [&](int e) { return handoff_lane<NN>(hand, nt, j, e); };
   const LayerTask<N, GEN> q = layer_task<N, GEN>(p, j);
   if (!q.live) {
     *hp(HO::S_FLAG) = 0.0;
@@ -710,33 +736,33 @@ __global__ void __launch_bounds__(128) flux_layer_front_kernel(FluxParams p, Con
     for (int a = 0; a < NN; ++a) {
       double z[N];
 #pragma unroll
-      for (int l = 0; l < N; ++l) z[l] = gl[l] * tc.y[l * NN + a];
+      for (int l = 0; l < N; ++l) z[l] = gl[l] * ytab(l, a);
 #pragma unroll
       for (int b = 0; b <= a; ++b) {
         double se = 0.0, so = 0.0;
 #pragma unroll
-        for (int l = 0; l < N; l += 2) se += z[l] * tc.y[l * NN + b];
+        for (int l = 0; l < N; l += 2) se += z[l] * ytab(l, b);
 #pragma unroll
-        for (int l = 1; l < N; l += 2) so += z[l] * tc.y[l * NN + b];
+        for (int l = 1; l < N; l += 2) so += z[l] * ytab(l, b);
         E[tri_idx(a, b)] = se;
         O[tri_idx(a, b)] = so;
       }
     }
     const double fbeam = q.rec[H_FBEAM];
-    const bool swap = GEN && (p.g.m & 1);
+    const bool swap = GEN && (m & 1);
     if (fbeam > 0.0) {
       // (2 - delta_m0) F0 / 4pi sum_k g'_k P_k^m(mu_r) P_k^m(-mu0) by parity (DisortSolver.cpp:1361-1368)
       const double* yb = beam_legendre<N, GEN>(p, q);
 #pragma unroll
       for (int k = 0; k < N; ++k) gl[k] *= yb[k];
-      const double fac = ((GEN && p.g.m > 0) ? 4.0 : 2.0) * fbeam / (4.0 * 3.14159265358979323846);
+      const double fac = ((GEN && m > 0) ? 4.0 : 2.0) * fbeam / (4.0 * 3.14159265358979323846);
 #pragma unroll
       for (int r = 0; r < NN; ++r) {
         double se = 0.0, so = 0.0;
 #pragma unroll
-        for (int l = 0; l < N; l += 2) se += gl[l] * tc.y[l * NN + r];
+        for (int l = 0; l < N; l += 2) se += gl[l] * ytab(l, r);
 #pragma unroll
-        for (int l = 1; l < N; l += 2) so += gl[l] * tc.y[l * NN + r];
+        for (int l = 1; l < N; l += 2) so += gl[l] * ytab(l, r);
         const double dm = tc.dsim[r] * tc.rmu[r] * fac;
         *hp(HO::S_B1 + r) = dm * (swap ? so : se);
         *hp(HO::S_B2 + r) = dm * (swap ? se : so);
@@ -877,7 +903,7 @@ template <int N>
 struct ECfg {
   static constexpr int HP = mod_hp(N);
   static constexpr int RS = 2 * HP + 1;   // staging row: one mode's X and Y
-  static constexpr int VS = 5 * HP + 3;   // staging row: the vectors
+  static constexpr int VS = 7 * HP + 3;   // staging row: the vectors
   static constexpr int WARP = 32 * (RS + VS);
   static constexpr size_t smem_bytes(int cta) { return sizeof(double) * (size_t)(cta / 32) * WARP; }
 };
@@ -901,7 +927,9 @@ __global__ void __launch_bounds__(128) flux_eigen_kernel(FluxParams p, ConstTab<
   // lanes past the end or skipped by the front compute on a valid task's
   // addresses and write nothing (no early exit: the warp writes rows together)
   const long long jj = j < nt ? j : nt - 1;
-  auto hv = [&](int e) { return *handoff_lane<NN>(p.bvp_rec, nt, jj, e); };
+  const int m = mode_of<GEN>(p);
+  double* const hand = p.bvp_rec + mode_row<GEN>() * p.g.ms_bvp;
+  auto hv = [&](int e) { return *handoff_lane<NN>(hand, nt, jj, e); };
   const double flag = hv(HO::S_FLAG);
   const bool act = j < nt && flag != 0.0;  // skipped: cut layer, invalid input, no factorisation
   const unsigned okm = __ballot_sync(0xffffffffu, act);
@@ -918,7 +946,7 @@ __global__ void __launch_bounds__(128) flux_eigen_kernel(FluxParams p, ConstTab<
   const double fbeam = act ? q.rec[H_FBEAM] : 0.0;
   const bool beam = fbeam > 0.0;
   const bool raw = GEN && (p.flags & DSP_FLAG_SPHERICAL_BEAM);
-  const bool thermal = (p.flags & DSP_FLAG_THERMAL) && (!GEN || p.g.m == 0);
+  const bool thermal = (p.flags & DSP_FLAG_THERMAL) && m == 0;
   double r0 = 0.0;
   if (beam) {
     double umu0 = q.rec[H_UMU0];
@@ -936,7 +964,8 @@ __global__ void __launch_bounds__(128) flux_eigen_kernel(FluxParams p, ConstTab<
 #pragma unroll
   for (int k = 0; k < NN; ++k) rdg[k] = 1.0 / L[tri_idx(k, k)];
   const long long ls = GEN ? p.g.lstride : (long long)lrec_stride(N);
-  double* const rec0 = p.layer_rec + j0 * ls;
+  double* const rec0 = p.layer_rec + mode_row<GEN>() * p.g.ms_layer + j0 * ls;
+  const double dts = act ? q.rec[q.il.dtau_s + q.lc] : 0.0;
 #pragma unroll
   for (int c = 0; c < NN; ++c) {
     const double k = mode_k(S[tri_idx(c, c)]);
@@ -973,14 +1002,16 @@ __global__ void __launch_bounds__(128) flux_eigen_kernel(FluxParams p, ConstTab<
       row[HP + NN] = 0.0;
     }
     vrow[c] = k;
+    vrow[HP + c] = exp(-k * dts);
+    vrow[2 * HP + c] = -expm1(-2.0 * k * dts);
     if (beam) {
       if (raw) {
         // pseudo-spherical beam (general solver): the raw source at the quadrature
         // angles, up and down, for the user-angle interpolation and
         // flux_sph_source_kernel (DisortSolver.cpp:1524-1527)
         const double dm = 0.5 * tc.mu[c] * tc.dinv[c], u1 = hv(HO::S_B1 + c), u2 = hv(HO::S_B2 + c);
-        vrow[HP + c] = dm * (u1 + u2);
-        vrow[2 * HP + c] = dm * (u1 - u2);
+        vrow[3 * HP + c] = dm * (u1 + u2);
+        vrow[4 * HP + c] = dm * (u1 - u2);
       } else {
 #pragma unroll
         for (int r = 0; r < NN; ++r) {
@@ -988,14 +1019,14 @@ __global__ void __launch_bounds__(128) flux_eigen_kernel(FluxParams p, ConstTab<
           be += y[r] * hv(HO::S_B2 + r);
         }
         const double den = 1.0 / (k * k - r0 * r0);
-        vrow[HP + c] = (k * al - be * r0) * den;
-        vrow[2 * HP + c] = (k * be - al * r0) * den;
+        vrow[3 * HP + c] = (k * al - be * r0) * den;
+        vrow[4 * HP + c] = (k * be - al * r0) * den;
       }
     }
     if (thermal) {
       ve = ws2 * ve / k;
-      vrow[3 * HP + c] = ve;
-      vrow[4 * HP + c] = ve / k;
+      vrow[5 * HP + c] = ve;
+      vrow[6 * HP + c] = ve / k;
     }
     // X^T row c and Y^T row c of every task: lane group (task, X or Y) x HP
     __syncwarp();
@@ -1008,11 +1039,11 @@ __global__ void __launch_bounds__(128) flux_eigen_kernel(FluxParams p, ConstTab<
           rec0[b * ls + (e < HP ? mod_X(N) + c * HP + e : mod_Y(N) + c * HP + e - HP)] = stg[b * RS + e];
     __syncwarp();
   }
-  if (thermal && act) thermal_source(q, vrow[5 * HP], vrow[5 * HP + 1]);
+  if (thermal && act) thermal_source(q, vrow[7 * HP], vrow[7 * HP + 1]);
   __syncwarp();
   for (int b = 0; b < 32; ++b)
     if ((okm >> b) & 1u)
-      for (int e = lane; e < 5 * HP + 2; e += 32) rec0[b * ls + mod_k(N) + e] = vst[b * VS + e];
+      for (int e = lane; e < 7 * HP + 2; e += 32) rec0[b * ls + mod_k(N) + e] = vst[b * VS + e];
 }
 
 // Host side of the layer stage: launches (through `wrap(kind, launch)`, which may
@@ -1031,24 +1062,24 @@ inline void flux_layer_set_attrs() {
     cudaFuncSetAttribute(flux_layer_kernel<N, GEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem_bytes());
 }
 
-// The layer stage of `tasks` layer tasks.  split: one thread per task (N <= 16
+// The layer stage of `tasks` layer tasks (of each of `modes` azimuth modes).  split: one thread per task (N <= 16
 // only), with `cta` threads per CTA (64 or 128); otherwise the team kernel.
 template <int N, bool GEN = false, class Wrap>
 inline void flux_layer_launch(const FluxParams& p, long long tasks, const double* host_tab, cudaStream_t s,
-                              Wrap&& wrap, bool split = layer_split<N>(), int cta = 128) {
+                              Wrap&& wrap, bool split = layer_split<N>(), int cta = 128, int modes = 1) {
   using C = LCfg<N>;
   if constexpr (layer_split<N>()) {
     if (split || GEN) {
       const int b = cta == 64 ? 64 : 128;
       const ConstTab<N> tc = make_const_tab<N>(host_tab);
-      const unsigned g = (unsigned)((tasks + b - 1) / b);
+      const dim3 g((unsigned)((tasks + b - 1) / b), (unsigned)modes);
       wrap(0, [&] { flux_layer_front_kernel<N, GEN><<<g, b, 0, s>>>(p, tc); });
       wrap(1, [&] { flux_eigen_kernel<N, GEN><<<g, b, ECfg<N>::smem_bytes(b), s>>>(p, tc); });
       return;
     }
   }
   if constexpr (!GEN || !layer_split<N>()) {
-    const unsigned grid = (unsigned)((tasks + C::TPC - 1) / C::TPC);
+    const dim3 grid((unsigned)((tasks + C::TPC - 1) / C::TPC), (unsigned)modes);
     wrap(2, [&] { flux_layer_kernel<N, GEN><<<grid, C::CTA, C::smem_bytes(), s>>>(p); });
   }
 }

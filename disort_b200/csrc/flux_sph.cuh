@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(128) flux_sph_source_kernel(FluxParams p) {
     Lin = p.g.Ls[i];
     il = InstLayout::make(Lin, N);
     rec = p.inst_rec + p.g.inst_off[ci];
-    lrec = p.layer_rec + task * p.g.lstride;
+    lrec = p.layer_rec + blockIdx.y * p.g.ms_layer + task * p.g.lstride;
     const int lin = (p.flags & DSP_FLAG_INDEX_FROM_BOTTOM) ? Lin - 1 - lc : lc;
     pml = p.g.pmom + (p.g.in_off[i] + lin) * (long long)p.pc;
   } else {
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(128) flux_sph_source_kernel(FluxParams p) {
   const double fbeam = rec[H_FBEAM];
   if (!(fbeam > 0.0) || lc >= (int)rec[H_NCUT]) return;
   if constexpr (GEN) {
-    if (p.g.m > (int)rec[H_NAZ] || rec[H_DONE] != 0.0) return;
+    if (p.g.m + (int)blockIdx.y > (int)rec[H_NAZ] || rec[H_DONE] != 0.0) return;
   }
   double* sm = smem + warp * C::WARP_SMEM;
   double* A = sm + C::O_A;
@@ -192,10 +192,12 @@ __global__ void __launch_bounds__(128) flux_sph_source_kernel(FluxParams p) {
   double* z1 = sm + C::O_Z1;
   int* piv = reinterpret_cast<int*>(sm + C::O_PIV);
   const double* mu = p.tables + tab_mu(N);
-  const double* Y = p.tables + tab_ylm(N);  // Y[l * N + i] = P_l^m(mu_i)
+  const double* Y = p.tables + (GEN ? (long long)blockIdx.y * tab_size(N) : 0ll) + tab_ylm(N);  // Y[l * N + i] = P_l^m(mu_i)
   const double* taus = rec + il.tau_s;
   const double* btr = rec + il.btr;
-  double* sr = p.sph + task * sph_stride(N);
+  double* sr = p.sph + (GEN ? blockIdx.y * p.g.ms_sph : 0ll) + task * sph_stride(N);
+  // the Chapman factor of the layer is in the first mode's record
+  const double chf = p.sph[task * sph_stride(N) + sph_ch(N)];
 
   // scaled phase coefficients g'_k (disortSet, FluxSolver.cpp:336-386;
   // DisortSolver.cpp:663-747, where P_0 is normalised to 1)
@@ -244,7 +246,7 @@ __global__ void __launch_bounds__(128) flux_sph_source_kernel(FluxParams p) {
   __syncwarp();
   // attenuation xba = 1 / ch with the reference's guards and dithering
   const double big = sqrt(1.79769313486231570815e+308) / 1.0e10;
-  double xba = 1.0 / sr[sph_ch(N)];
+  double xba = 1.0 / chf;
   if (fabs(xba) > big && taus[lc + 1] > 1.0) xba = 0.0;
   if (fabs(xba * taus[lc + 1]) > log(big)) xba = 0.0;
   if (fabs(xba) > 1.0e-5)
@@ -356,7 +358,10 @@ __global__ void __launch_bounds__(128) flux_sph_source_kernel(FluxParams p) {
     sr[c] = c1;
     sr[NN + c] = d1;
   }
-  if (lane == 0) sr[sph_xba(N)] = xba;
+  if (lane == 0) {
+    sr[sph_xba(N)] = xba;
+    if (GEN && blockIdx.y) sr[sph_ch(N)] = chf;
+  }
 }
 
 }  // namespace dsp

@@ -228,7 +228,7 @@ static __global__ void __launch_bounds__(128) gen_ptab_kernel(FluxParams p) {
   const int slot = (int)(k / na), v = (int)(k % na);
   const int i = g.ids[slot];
   const double x = v == 0 ? -p.umu0(i) : g.umu.row(i)[v - 1];
-  legendre_column(g.m, x, p.N - 1, g.ptab + k * p.N, 1);
+  legendre_column(g.m + (int)blockIdx.y, x, p.N - 1, g.ptab + blockIdx.y * g.ms_ptab + k * p.N, 1);
 }
 
 // Eigenvectors and sources of every layer at the user polar angles for mode m
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(128) gen_angle_kernel(FluxParams p) {
   if (!q.live) return;
   const int st0 = p.status ? p.status[q.i] : 0;
   if (st0 == DSP_ERR_EIGEN) return;
-  const int m = p.g.m, numu = p.g.numu;
+  const int m = mode_of<true>(p), numu = p.g.numu;
   const double ws = q.rec[q.il.ssa_s + q.lc];
   {
     const int mode = (int)q.rec[q.il.mode + q.lc];
@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(128) gen_angle_kernel(FluxParams p) {
     xr1 = q.lrec[mod_xr(N) + 1];
   }
   const double dj = p.tables[tab_dsim(N) + j], wd = p.tables[tab_wt(N) + j] / dj;
-  const double* const Y = p.tables + tab_ylm(N);
+  const double* const Y = p.tables + (long long)mode_row<true>() * tab_size(N) + tab_ylm(N);
   const double* const yb = beam_legendre<N, true>(p, q);
   const double fact = 2.0 * (m == 0 ? 1.0 : 2.0) * fbeam / (4.0 * 3.14159265358979323846);
   const int odd0 = 1 - (m & 1);  // first l of odd l + m
@@ -357,11 +357,165 @@ __global__ void __launch_bounds__(128) gen_angle_kernel(FluxParams p) {
 }
 
 // Intensities at the user angles for mode m (computeUserIntensities,
-// DisortSolver.cpp:2938-3268): one warp per instance, a lane per (level, angle)
-// pair, looping over the layers between the level and the boundary.
+// DisortSolver.cpp:2938-3226): the formal solution along one user angle, layer by
+// layer from the boundary the radiation comes from.  A team of pow2ceil(h) lanes
+// per (slot, angle), lane j on eigenmode j: its share of the intensity at the
+// layer's far side follows from the near side by I <- I exp(-dtau/|mu|) + (the
+// layer's own), so every layer is passed once for all output depths, with one
+// exponential and two reciprocals per lane; the lanes are summed only at the
+// output depths (there with the part of the layer up to the depth).  I_m goes to
+// imode; gen_fourier_kernel adds the modes up.
+template <int N>
+struct ICfg {
+  static constexpr int H = N / 2, TEAM = pow2ceil(H), TPC = 128 / TEAM;
+};
 template <int N>
 __global__ void __launch_bounds__(128) gen_intensity_kernel(FluxParams p) {
-  constexpr int NN = N / 2;
+  using C = ICfg<N>;
+  constexpr int H = C::H, TEAM = C::TEAM;
+  constexpr double PI = 3.14159265358979323846;
+  const GenView& g = p.g;
+  const int t = threadIdx.x % TEAM, j = t < H ? t : H - 1;
+  const bool own = t < H;
+  const unsigned msk = team_mask<TEAM>();
+  const int numu = g.numu;
+  const long long item = (long long)blockIdx.x * C::TPC + threadIdx.x / TEAM;
+  if (item >= (long long)p.n * numu) return;
+  const int slot = (int)(item / numu), iu = (int)(item % numu);
+  const int i = g.ids[slot];
+  const int L = g.Ls[i];
+  const int NT = g.user_tau ? g.user_tau : L + 1;
+  const int mrow = (int)blockIdx.y, m = g.m + mrow;
+  const int st0 = p.status ? p.status[i] : 0;
+  if (st0 == DSP_ERR_INVALID_INPUT || st0 == DSP_ERR_EIGEN) return;
+  const double* const rec = p.inst_rec + g.inst_off[slot];
+  if (m > (int)rec[H_NAZ] || rec[H_DONE] != 0.0) return;
+  const GenLayout gly = GenLayout::make(L, N, NT);
+  const InstLayout& il = gly.il;
+  const int ncut = (int)rec[H_NCUT];
+  const bool lyrcut = rec[H_LYRCUT] != 0.0;
+  const bool thermal = (p.flags & DSP_FLAG_THERMAL) != 0 && m == 0;
+  const bool dlbc = (p.flags & DSP_FLAG_DIFFUSION_LOWER_BC) != 0;
+  const double fbeam = rec[H_FBEAM], umu0 = rec[H_UMU0];
+  const bool beam = fbeam > 0.0;
+  const double* const taus = rec + il.tau_s;
+  const double* const btr = rec + il.btr;
+  const double* const utaus = rec + gly.utaus;
+  const double* const lyr = rec + gly.lyr;
+  const double* const lrec0 = p.layer_rec + mrow * g.ms_layer + g.lay_off[slot] * g.lstride;
+  const double* const cc0 = g.cc + mrow * g.ms_cc + g.lay_off[slot] * N;
+  const double umv = g.umu.row(i)[iu];
+  const bool neg = umv < 0.0;
+  const double nu = fabs(umv);
+  double* const out = g.imode + mrow * g.ms_int + (long long)slot * g.nt_max * numu + iu;
+  auto total = [&](double v) {
+#pragma unroll
+    for (int off = TEAM / 2; off > 0; off >>= 1) v += __shfl_xor_sync(msk, v, off, TEAM);
+    return v;
+  };
+
+  // boundary radiation at the angle (DisortSolver.cpp:3180-3226)
+  double bnd = 0.0;
+  if (neg) {
+    if (m == 0) bnd = rec[H_FISOT] + rec[H_PTOP];
+  } else if (dlbc) {
+    if (!lyrcut && m == 0) bnd = rec[H_PBOT] + umv * rec[H_PBOTD];
+  } else if (!lyrcut) {
+    const double* const mu = p.tables + tab_mu(N);
+    const double* const wt = p.tables + tab_wt(N);
+    // the downward intensities at the bottom come with the boundary-value solution
+    const double dfu = own ? p.bvp_rec[mrow * g.ms_bvp + (g.lay_off[slot] + ncut - 1) * brec_stride(N) + brec_dn(N) + j] : 0.0;
+    const double muw = mu[j] * wt[j];
+    if (g.brdf) {
+      // bidirectional surface at user angles; the isotropic bottom flux enters at
+      // every mode, as the reference adds it (DisortSolver.cpp:3213-3220)
+      const double* ur = g.brdf + (long long)slot * brdf_stride(N, numu) + (H + iu) * brdf_row(N);
+      const double refl = total((m == 0 ? 2.0 : 1.0) * ur[1 + j] * muw * dfu);
+      bnd = refl + umu0 * fbeam / PI * ur[0] * btr[L] + (m == 0 ? ur[H + 1] * rec[H_PBOT] : 0.0) + rec[H_FISOB];
+    } else if (m == 0) {
+      // Lambertian surface at user angles: set for mu > 0 only (DisortSolver.cpp:2655-2662)
+      const double alb = rec[H_ALB];
+      const double refl = total(2.0 * muw * dfu);
+      const double rho = umv > 0.0 ? alb : 0.0, em = umv > 0.0 ? 1.0 - alb : 0.0;
+      bnd = rho * refl + umu0 * fbeam / PI * rho * btr[L] + em * rec[H_PBOT] + rec[H_FISOB];
+    }
+  }
+
+  // output depths below the cut carry zeros
+  for (int lu = t; lu < NT; lu += TEAM)
+    if (lyrcut && (int)lyr[lu] >= ncut) out[(long long)lu * numu] = 0.0;
+  const int my_lyr = t < NT ? (int)lyr[t] : -1;  // the first TEAM depths' layers, kept
+  const double rnu = 1.0 / nu, rmu0 = beam ? 1.0 / umu0 : 0.0;
+  const double bden = neg ? 1.0 - nu * rmu0 : 1.0 + nu * rmu0;
+  const bool bres = fabs(bden) < 0.0001;
+  const double rbden = bres ? 0.0 : 1.0 / bden;
+  // lane j's share of the intensity, and the beam and thermal parts (every lane the same)
+  double acc = 0.0, accs = 0.0;
+  for (int s = 0; s < ncut; ++s) {
+    const int l = neg ? s : ncut - 1 - s;
+    const double* const lr = lrec0 + (long long)l * g.lstride;
+    const double* const gu = lr + glrec_gu(N) + (long long)iu * N;
+    const double* const zu = lr + glrec_gu(N) + (long long)numu * N;
+    const double* const x = cc0 + (long long)l * N;
+    const double k = lr[mod_k(N) + j], wk = lr[mod_E(N) + j];
+    const double gb = own ? gu[j] * x[j] : 0.0, ga = own ? gu[H + j] * x[H + j] : 0.0;
+    const double tt = taus[l], tb = taus[l + 1], dt = tb - tt;
+    const double e = exp(-dt * rnu);
+    const double t0 = neg ? tt : tb;  // the near side, where the radiation enters
+    // the mode that grows towards the far side (down: a from the top; up: b from the
+    // bottom) meets the resonance k = 1/|mu|
+    const double gn = neg ? ga : gb, gf = neg ? gb : ga;
+    const double den = 1.0 - nu * k;
+    const bool res = fabs(den) < 0.0001;
+    const double rn = res ? 0.0 : rcp_newton(den), rf = rcp_newton(1.0 + nu * k);
+    const double b0 = beam ? btr[l] : 0.0, b1 = beam ? btr[l + 1] : 0.0;
+    const double zb = beam ? zu[iu] : 0.0, z0 = thermal ? zu[numu + iu] : 0.0, z1 = thermal ? zu[2 * numu + iu] : 0.0;
+    // output depths in this layer: the part of the layer on the boundary side
+    for (int base = 0; base < NT; base += TEAM) {
+      const int v = base == 0 ? my_lyr : (base + t < NT ? (int)lyr[base + t] : -1);
+      unsigned hit = __ballot_sync(msk, v == l) >> (threadIdx.x & 31u & ~(unsigned)(TEAM - 1));
+      if constexpr (TEAM < 32) hit &= (1u << TEAM) - 1u;
+      while (hit) {
+        const int lu = base + __ffs(hit) - 1;
+        hit &= hit - 1u;
+        const double ut = utaus[lu];
+        const double d = neg ? ut - t0 : t0 - ut;  // depth from the near side
+        double v1 = acc, v2 = accs, ed = 1.0;
+        if (fabs(d) >= 1e-6) {
+          ed = exp(-d * rnu);
+          // the near mode at the depth (1 at the near side), the far mode there and
+          // at the near side (wk)
+          const double en = exp(-k * d), ef = exp(-k * (neg ? tb - ut : ut - tt));
+          v1 = acc * ed + gn * (res ? d * rnu * ed : (en - ed) * rn) + gf * ((ef - wk * ed) * rf);
+          v2 = accs * ed;
+          if (beam) {
+            const double exp0 = exp(-ut * rmu0);
+            v2 += zb * (bres ? d * rmu0 * exp0 : (exp0 - (neg ? b0 : b1) * ed) * rbden);
+          }
+          if (thermal) v2 += z0 * (1.0 - ed) + z1 * ((ut + umv) - (t0 + umv) * ed);
+        }
+        const double dist = neg ? ut : taus[L] - ut;
+        const double I = total(v1) + v2 + (bnd != 0.0 ? bnd * exp(-dist * rnu) : 0.0);
+        if (t == 0) out[(long long)lu * numu] = I;
+      }
+    }
+    // across the layer
+    acc = acc * e + gn * (res ? dt * rnu * e : (wk - e) * rn) + gf * ((1.0 - wk * e) * rf);
+    if (beam) {
+      const double bn = neg ? b0 : b1, bf = neg ? b1 : b0;
+      accs = accs * e + zb * (bres ? dt * rmu0 * exp(-tb * rmu0) : (bf - bn * e) * rbden);
+    } else {
+      accs *= e;
+    }
+    if (thermal) accs += z0 * (1.0 - e) + z1 * (((neg ? tb : tt) + umv) - (t0 + umv) * e);
+  }
+}
+
+// The Fourier sum over the modes of a launch (DisortSolver.cpp:3228-3266), one
+// warp per instance, a lane per (level, angle) pair; in mode order, with the
+// azimuthal convergence test after each mode (:337-347), so that a mode past
+// the convergence adds nothing even when it was computed with the others.
+static __global__ void __launch_bounds__(128) gen_fourier_kernel(FluxParams p, int modes) {
   constexpr double PI = 3.14159265358979323846;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slot = blockIdx.x * 4 + warp;
@@ -370,224 +524,74 @@ __global__ void __launch_bounds__(128) gen_intensity_kernel(FluxParams p) {
   const int i = g.ids[slot];
   const int L = g.Ls[i];
   const int NT = g.user_tau ? g.user_tau : L + 1;
-  const int m = g.m, numu = g.numu, nphi = g.nphi;
+  const int numu = g.numu, nphi = g.nphi, nk = NT * numu;
   const bool ifb = (p.flags & DSP_FLAG_INDEX_FROM_BOTTOM) != 0;
-  auto orow = [&](int lu) { return (long long)i * g.ntau_out + (ifb ? NT - 1 - lu : lu); };
+  auto elem = [&](int k) {
+    const int lu = k / numu, iu = k % numu;
+    return ((long long)i * g.ntau_out + (ifb ? NT - 1 - lu : lu)) * g.numu_out + iu;
+  };
   const int st0 = p.status ? p.status[i] : 0;
   if (st0 == DSP_ERR_INVALID_INPUT || st0 == DSP_ERR_EIGEN) {
-    if (m == 0) {
+    if (g.m == 0) {
       const double qnan = __longlong_as_double(0x7ff8000000000000ll);
-      for (int k = lane; k < NT * numu; k += 32) {
-        const int lu = k / numu, iu = k % numu;
-        g.out_iavg[orow(lu) * g.numu_out + iu] = qnan;
-        for (int j = 0; j < nphi; ++j) g.out_int[(orow(lu) * g.numu_out + iu) * nphi + j] = qnan;
+      for (int k = lane; k < nk; k += 32) {
+        const long long o2 = elem(k);
+        g.out_iavg[o2] = qnan;
+        for (int j = 0; j < nphi; ++j) g.out_int[o2 * nphi + j] = qnan;
       }
     }
     return;
   }
-  const double* rec = p.inst_rec + g.inst_off[slot];
-  if (m > (int)rec[H_NAZ] || rec[H_DONE] != 0.0) return;
-  const GenLayout gly = GenLayout::make(L, N, NT);
-  const InstLayout& il = gly.il;
-  const double* mu = p.tables + tab_mu(N);
-  const double* wt = p.tables + tab_wt(N);
-  const int ncut = (int)rec[H_NCUT];
-  const bool lyrcut = rec[H_LYRCUT] != 0.0;
-  const bool thermal = (p.flags & DSP_FLAG_THERMAL) != 0 && m == 0;
-  const bool dlbc = (p.flags & DSP_FLAG_DIFFUSION_LOWER_BC) != 0;
-  const double fbeam = rec[H_FBEAM], umu0 = rec[H_UMU0], alb = rec[H_ALB];
-  const bool beam = fbeam > 0.0;
-  const double* taus = rec + il.tau_s;
-  const double* dts = rec + il.dtau_s;
-  const double* btr = rec + il.btr;
-  const double* utaus = rec + gly.utaus;
-  const double* lyr = rec + gly.lyr;
-  const double* lrec0 = p.layer_rec + g.lay_off[slot] * g.lstride;
-  const double* cc0 = g.cc + g.lay_off[slot] * N;
-  auto LR = [&](int l) { return lrec0 + (long long)l * g.lstride; };
-  const double* um = g.umu.row(i);
-
-  // reflected field: the downward intensities at the bottom come with the
-  // boundary-value solution
-  double bsum = 0.0;
-  // bidirectional surface: this mode's table; its user rows receive the
-  // reflected sum of each user angle in their last slot
-  double* sft = g.brdf ? g.brdf + (long long)slot * brdf_stride(N, g.numu) : nullptr;
-  const bool lambert_bnd = (m == 0) && !lyrcut && !dlbc && !sft;
-  if ((sft && !lyrcut) || lambert_bnd) {
-    const double dfu = lane < NN ? p.bvp_rec[(g.lay_off[slot] + ncut - 1) * brec_stride(N) + brec_dn(N) + lane] : 0.0;
-    const double muw = lane < NN ? mu[lane] * wt[lane] : 0.0;
-    const double cpl = m == 0 ? 2.0 : 1.0;
-    auto total = [](double v) {
+  double* const rec = p.inst_rec + g.inst_off[slot];
+  const int naz = (int)rec[H_NAZ];
+  if (rec[H_DONE] != 0.0) return;
+  double kconv = rec[H_KCONV];
+  const double* const ph = g.phi.row(i);
+  const double phi0 = g.phi0(i);
+  for (int mi = 0; mi < modes; ++mi) {
+    const int m = g.m + mi;
+    if (m > naz) break;
+    const double* const im = g.imode + mi * g.ms_int + (long long)slot * g.nt_max * numu;
+    double maxr = 0.0;
+    for (int j0 = 0; j0 < nphi || j0 == 0; j0 += 32) {
+      const int nj = nphi - j0 < 32 ? nphi - j0 : 32;
+      double cm = 1.0;
+      if (m > 0 && lane < nj) cm = cos(static_cast<double>(m) * ((ph[j0 + lane] - phi0) * PI / 180.0));
+      for (int kb = 0; kb < nk; kb += 32) {
+        const int k = kb + lane;
+        const double I = k < nk ? im[k] : 0.0;
+        const long long o2 = k < nk ? elem(k) : 0;
+        if (m == 0 && j0 == 0 && k < nk) g.out_iavg[o2] = I;
+        for (int j = 0; j < nj; ++j) {
+          const double az = I * __shfl_sync(0xffffffffu, cm, j);
+          if (k >= nk) continue;
+          double& acc = g.out_int[o2 * nphi + j0 + j];
+          const double v = m == 0 ? az : acc + az;
+          acc = v;
+          const double uu = fabs(v);
+          double ratio;
+          if (uu == 0.0) ratio = 1.0 + fabs(az);
+          else if (fabs(az) == 0.0) ratio = 0.0;
+          else ratio = fabs(az) / uu;
+          maxr = fmax(maxr, ratio);
+        }
+      }
+    }
+    if (m > 0 && g.accur > 0.0) {
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-      return v;
-    };
-    if (lambert_bnd) {
-      // sum_iq 2 mu w dfuint (DisortSolver.cpp:3180-3218)
-      bsum = total(2.0 * muw * dfu);
-    } else {
-      // sum_iq (1 + delta_m0) R_m(mu_u, mu_iq) mu_iq w_iq dfuint(iq) per user angle
-      for (int iu = 0; iu < numu; ++iu) {
-        double* ur = sft + (NN + iu) * brdf_row(N);
-        const double v = total(lane < NN ? cpl * ur[1 + lane] * muw * dfu : 0.0);
-        if (lane == 0) ur[NN + 2] = v;
-      }
-      __syncwarp();
-    }
-  }
-
-  double maxr = 0.0;
-  for (int k = lane; k < NT * numu; k += 32) {
-    const int lu = k / numu, iu = k % numu;
-    const double umv = um[iu];
-    const int y = (int)lyr[lu];
-    double I = 0.0;
-    if (!(lyrcut && y >= ncut)) {
-      const double ut = utaus[lu];
-      const double exp0 = beam ? exp(-ut / umu0) : 0.0;
-      const bool neg = umv < 0.0;
-      const int ls = neg ? 0 : y + 1, le = neg ? y - 1 : ncut - 1;
-      const double sgn = neg ? -1.0 : 1.0;
-      double palint = 0.0, plkint = 0.0;
-      // layers entirely between the level and the boundary
-      for (int lc = ls; lc <= le; ++lc) {
-        const double* lr = LR(lc);
-        const double* gu = lr + glrec_gu(N) + iu * N;
-        const double* x = cc0 + (long long)lc * N;
-        const double* kk = lr + mod_k(N);
-        const double dt = dts[lc];
-        const double e1 = exp((ut - taus[lc]) / umv);
-        const double e2 = exp((ut - taus[lc + 1]) / umv);
-        if (thermal) {
-          const double f0n = sgn * (e1 - e2);
-          const double f1n = sgn * ((taus[lc] + umv) * e1 - (taus[lc + 1] + umv) * e2);
-          const double* zu = lr + glrec_gu(N) + numu * N + numu;
-          plkint += zu[iu] * f0n + zu[numu + iu] * f1n;
-        }
-        if (beam) {
-          const double den = 1.0 + umv / umu0;
-          double expn;
-          if (fabs(den) < 0.0001) expn = (dt / umu0) * exp0;
-          else expn = (e1 * btr[lc] - e2 * btr[lc + 1]) * sgn / den;
-          palint += lr[glrec_gu(N) + numu * N + iu] * expn;
-        }
-#pragma unroll 4
-        for (int iq = 0; iq < NN; ++iq) {
-          const double k = kk[iq], wk = exp(-k * dt);
-          // b: exp(-k (tau_bot - tau)), a: exp(-k (tau - tau_top))
-          double den = 1.0 - umv * k, expn;
-          if (fabs(den) < 0.0001) expn = (dt / umv) * e2;
-          else expn = sgn * (e1 * wk - e2) / den;
-          palint += (gu[iq] * x[iq]) * expn;
-          den = 1.0 + umv * k;
-          if (fabs(den) < 0.0001) expn = -(dt / umv) * e1;
-          else expn = sgn * (e1 - e2 * wk) / den;
-          palint += (gu[NN + iq] * x[NN + iq]) * expn;
-        }
-      }
-      // the part of the level's own layer on the boundary side
-      const double dt1 = ut - taus[y], dt2 = ut - taus[y + 1];
-      if ((fabs(dt1) >= 1e-6 || !neg) && (fabs(dt2) >= 1e-6 || neg)) {
-        const double* lr = LR(y);
-        const double* gu = lr + glrec_gu(N) + iu * N;
-        const double* x = cc0 + (long long)y * N;
-        const double* kk = lr + mod_k(N);
-        const double e1c = neg ? exp(dt1 / umv) : 0.0;
-        const double e2c = neg ? 0.0 : exp(dt2 / umv);
-        if (beam) {
-          const double den = 1.0 + umv / umu0;
-          double expn;
-          if (fabs(den) < 0.0001) expn = (dt1 / umu0) * exp0;
-          else if (neg) expn = (exp0 - btr[y] * e1c) / den;
-          else expn = (exp0 - btr[y + 1] * e2c) / den;
-          palint += lr[glrec_gu(N) + numu * N + iu] * expn;
-        }
-        const double dty = dts[y];
-#pragma unroll 4
-        for (int iq = 0; iq < NN; ++iq) {
-          const double k = kk[iq], wk = exp(-k * dty);
-          double den = 1.0 - umv * k, expn;
-          if (fabs(den) < 0.0001) expn = -dt2 / umv * e2c;
-          else if (neg) expn = (exp(k * dt2) - wk * e1c) / den;
-          else expn = (exp(k * dt2) - e2c) / den;
-          palint += (gu[iq] * x[iq]) * expn;
-          den = 1.0 + umv * k;
-          if (fabs(den) < 0.0001) expn = -(dt1 / umv) * e1c;
-          else if (neg) expn = (exp(-k * dt1) - e1c) / den;
-          else expn = (exp(-k * dt1) - wk * e2c) / den;
-          palint += (gu[NN + iq] * x[NN + iq]) * expn;
-        }
-        if (thermal) {
-          const double expn = neg ? e1c : e2c;
-          const double fact = neg ? taus[y] + umv : taus[y + 1] + umv;
-          const double f0n = 1.0 - expn;
-          const double f1n = ut + umv - fact * expn;
-          const double* zu = lr + glrec_gu(N) + numu * N + numu;
-          plkint += zu[iu] * f0n + zu[numu + iu] * f1n;
-        }
-      }
-      // boundary terms
-      double bndint = 0.0;
-      bool bnd_skip = false;
-      if (neg && m == 0) {
-        bndint = (rec[H_FISOT] + rec[H_PTOP]) * exp(ut / umv);
-      } else if (!neg) {
-        if (dlbc) {
-          if (lyrcut || m > 0) bnd_skip = true;
-          else bndint = (rec[H_PBOT] + umv * rec[H_PBOTD]) * exp((ut - taus[L]) / umv);
-        } else if (lyrcut || (m > 0 && !sft)) {
-          bnd_skip = true;
-        } else if (sft) {
-          // bidirectional surface at user angles (DisortSolver.cpp:3213-3220); the
-          // isotropic bottom flux enters at every mode, as the reference adds it
-          const double* ur = sft + (NN + iu) * brdf_row(N);
-          const double bnddir = umu0 * fbeam / PI * ur[0] * btr[L];
-          const double emit = m == 0 ? ur[NN + 1] * rec[H_PBOT] : 0.0;
-          bndint = (ur[NN + 2] + bnddir + emit + rec[H_FISOB]) * exp((ut - taus[L]) / umv);
-        } else {
-          // Lambertian surface at user angles: set for mu > 0 only (DisortSolver.cpp:2655-2662)
-          const double rho = umv > 0.0 ? alb : 0.0, em = umv > 0.0 ? 1.0 - alb : 0.0;
-          const double bnddir = umu0 * fbeam / PI * rho * btr[L];
-          bndint = (rho * bsum + bnddir + em * rec[H_PBOT] + rec[H_FISOB]) * exp((ut - taus[L]) / umv);
-        }
-      }
-      I = bnd_skip ? palint + plkint : palint + plkint + bndint;
-    }
-    // accumulate the Fourier series (DisortSolver.cpp:3228-3266)
-    const long long o2 = orow(lu) * g.numu_out + iu;
-    if (m == 0) {
-      g.out_iavg[o2] = I;
-      for (int j = 0; j < nphi; ++j) g.out_int[o2 * nphi + j] = I;
-    } else {
-      const double* ph = g.phi.row(i);
-      const double phi0 = g.phi0(i);
-      for (int j = 0; j < nphi; ++j) {
-        const double phirad = (ph[j] - phi0) * PI / 180.0;
-        const double az = I * cos(static_cast<double>(m) * phirad);
-        double& acc = g.out_int[o2 * nphi + j];
-        acc += az;
-        const double uu = fabs(acc);
-        double ratio;
-        if (uu == 0.0) ratio = 1.0 + fabs(az);
-        else if (fabs(az) == 0.0) ratio = 0.0;
-        else ratio = fabs(az) / uu;
-        maxr = fmax(maxr, ratio);
-      }
-    }
-  }
-  // azimuthal convergence (DisortSolver.cpp:337-347)
-  if (m > 0 && g.accur > 0.0) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) maxr = fmax(maxr, __shfl_xor_sync(0xffffffffu, maxr, off));
-    if (lane == 0) {
-      double* wrec = p.inst_rec + g.inst_off[slot];
-      double kconv = wrec[H_KCONV];
+      for (int off = 16; off > 0; off >>= 1) maxr = fmax(maxr, __shfl_xor_sync(0xffffffffu, maxr, off));
       if (maxr <= g.accur) kconv += 1.0;
-      wrec[H_KCONV] = kconv;
-      if (kconv >= 2.0) wrec[H_DONE] = 1.0;
+      if (kconv >= 2.0) {
+        __syncwarp();
+        if (lane == 0) {
+          rec[H_KCONV] = kconv;
+          rec[H_DONE] = 1.0;
+        }
+        return;
+      }
     }
   }
+  if (lane == 0) rec[H_KCONV] = kconv;
 }
 
 }  // namespace dsp

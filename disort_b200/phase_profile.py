@@ -7,11 +7,9 @@ Solves the thermal sweep (20,000 bands x 60 layers x 16 streams by default)
 twice through the tracing build of libdsp.so (lib/phase/libdsp.so) with device
 pointers, and prints each phase's share of the boundary-value kernel's
 warp-time and its cycles per instance.  The phases are the kernel's DSP_PHASE
-markers (csrc/flux_bvp_reg.cuh): going down, per layer the new rows, per pivot
-step the pivot search (with the previous step's row updates) and the pivot-row
-broadcast, the last step's updates, the multiplier stores and the column phase;
-going up, the wait for the records, the triangular solve, the next records'
-prefetch and the fluxes.
+markers (csrc/flux_bvp.cuh): going down, per layer the wait for the record with the
+exponentials, I + M, its inverse, Z, its inverse and the new admittance; the
+surface; going up, the wait for the records, the solution and the fluxes.
 """
 from __future__ import annotations
 
@@ -21,10 +19,9 @@ import sys
 
 import numpy as np
 
-PHASES = [(0, "rows (new continuity / boundary rows)"), (7, "pivot search (+ previous step's updates)"),
-          (8, "pivot row broadcast"), (1, "last step's updates"), (9, "multiplier stores"),
-          (2, "column phase (x_{l+1} block, rhs)"), (4, "up: wait for records"), (5, "up: U x = c - V x_next"),
-          (6, "up: record prefetch"), (3, "up: fluxes")]
+PHASES = [(0, "down: wait for the record, exponentials"), (1, "down: I + X^T A X"), (2, "down: inverse H"),
+          (3, "down: H out, Z"), (4, "down: inverse G"), (5, "down: G out, Y (2G - I) Y^T"), (6, "surface"),
+          (7, "up: wait for the records"), (8, "up: solution"), (9, "up: fluxes, next records")]
 
 
 def main(n_bands: int = 20000) -> None:
