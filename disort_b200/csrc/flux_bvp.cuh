@@ -23,7 +23,8 @@
 //   phi_t = X (c + c_t).
 // I + M and Z are symmetric positive definite whatever the layer (M is a
 // congruence of A, and Z < 2), so both are inverted without pivoting, and no
-// growing exponential is formed.  Two h x h inverses and four h^3 products per
+// growing exponential is formed.  (Unphysical moments above 1 can break that; the
+// sweeps then run on an indefinite matrix, scaled by the absolute diagonal.)  Two h x h inverses and four h^3 products per
 // layer take the place of the N-column elimination of a 3h-row panel, about a
 // tenth of its operations; near omega' = 1 (k -> 0) nothing cancels, because
 // 1 - E^2 comes from expm1.
@@ -386,7 +387,7 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
       }
     }
     const double gam = dot_row<H>(xj, vg);
-    const double s1 = rsqrt(diag);
+    const double s1 = rsqrt(fabs(diag));
     if (own) {
       vw1[j] = gam - dt_ - ct;
       vsc[j] = s1;
@@ -426,7 +427,7 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
         diag = a[r];
       }
     }
-    const double s2 = rsqrt(diag);
+    const double s2 = rsqrt(fabs(diag));
     __syncwarp();  // every lane has read the first scale
     if (own) {
       vsc[j] = s2;
@@ -548,7 +549,7 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
         }
       }
       rhs = 2.0 * (sh - 2.0 * f * dj * dsrc) - vg[j];
-      const double s1 = rsqrt(diag);
+      const double s1 = rsqrt(fabs(diag));
       __syncwarp();
       if (own) {
         vsc[j] = s1;

@@ -17,8 +17,13 @@
 // beta = Y^T D M^{-1} (q+ - q-), q+- the source at the up/down quadrature angles,
 //   c = (k alpha - beta/mu0) / (k^2 - mu0^{-2}),
 //   d = (k beta - alpha/mu0) / (k^2 - mu0^{-2}).
-// When -B_s is not positive definite, -A_s = L L^T and S = L^T (-B_s) L give
-// the same modes with the two forms exchanged (X = L^{-T} U K^{1/2}, Y = L U K^{-1/2}).
+// U and K are the left singular vectors and values of L^T R, -A_s = R R^T, which a
+// one-sided Jacobi iteration finds without forming S: its rotations act on the
+// columns of L^T R only (no eigenvector matrix is accumulated), and the small
+// singular values keep their relative accuracy.  When -A_s is not positive
+// definite S is diagonalised instead, and when -B_s is not, -A_s = L L^T and
+// S = L^T (-B_s) L give the same modes with the two forms exchanged
+// (X = L^{-T} U K^{1/2}, Y = L U K^{-1/2}).
 // The quadrature is symmetric (mu_{h+j} = -mu_j, P_l^m(-mu) = (-1)^{l+m} P_l^m(mu)),
 // so -B_s holds the phase sums of odd l + m only and -A_s those of even l + m:
 //   alpha -/+ beta = M^{-1} (O W - I), M^{-1} (E W - I),
@@ -82,13 +87,15 @@ __host__ __device__ constexpr int tri_idx(int r, int c) {
 // blocks of 32 layer tasks, element e of the block's lane k at
 // 32 HS b + e w + k (w = tasks in the block), so that a warp of the
 // one-thread-per-task kernels reads or writes an element of 32 tasks in one
-// coalesced access.  Per task: flag (0 skipped, 1 primary factorisation,
-// 2 fallback), S and the Cholesky factor L (packed lower), and with a beam the
-// source vectors D M^{-1} (q+ + q-), D M^{-1} (q+ - q-).
+// coalesced access.  Per task: flag (0 skipped; 1: L^T R by columns; 2: -A_s is
+// indefinite, S = L^T (-A_s) L; 3: -B_s is, L is the factor of -A_s and
+// S = L^T (-B_s) L; S packed lower in the place of L^T R), the Cholesky factor L
+// (packed lower), and with a beam the source vectors D M^{-1} (q+ + q-),
+// D M^{-1} (q+ - q-).
 template <int NN>
 struct Handoff {
   static constexpr int TRI = NN * (NN + 1) / 2;
-  static constexpr int S_FLAG = 0, S_S = 1, S_L = 1 + TRI, S_B1 = 1 + 2 * TRI, S_B2 = S_B1 + NN;
+  static constexpr int S_FLAG = 0, S_F = 1, S_L = S_F + NN * NN, S_B1 = S_L + TRI, S_B2 = S_B1 + NN;
   static constexpr int HS = S_B2 + NN;
 };
 
@@ -567,6 +574,8 @@ __global__ void __launch_bounds__(LCfg<N>::CTA, LCfg<N>::MINB) flux_layer_kernel
   // ---- modes and particular solutions, one thread per mode ------------------
   for (int c = t; c < NN; c += TEAM) {
     const double k = mode_k(Sc[c * NS + c]);
+    // lambda < 0 beyond rounding: M is indefinite, and its inverse carries the sign
+    const bool lneg = Sc[c * NS + c] < -1e-10;
     const double sk = sqrt(k), rsk = 1.0 / sk;
     // T: L^{-T} u, MA: L u (MA is dead once S is formed)
     for (int r = NN - 1; r >= 0; --r) {
@@ -587,9 +596,11 @@ __global__ void __launch_bounds__(LCfg<N>::CTA, LCfg<N>::MINB) flux_layer_kernel
     const double* y = (primary ? T : MA) + c;
     double* vec = q.lrec;
     const double dts = q.rec[q.il.dtau_s + q.lc];
-    vec[mod_k(N) + c] = k;
-    vec[mod_E(N) + c] = exp(-k * dts);
-    vec[mod_F(N) + c] = -expm1(-2.0 * k * dts);
+    const double ks = lneg && !primary ? -k : k;  // (the reference's a and b change roles)
+    vec[mod_k(N) + c] = ks;
+    const double em = expm1(-ks * dts);  // E - 1; 1 - E^2 = -em (2 + em)
+    vec[mod_E(N) + c] = 1.0 + em;
+    vec[mod_F(N) + c] = -em * (2.0 + em);
     if (beam) {
       double umu0 = q.rec[H_UMU0];
       bool res = false;
@@ -608,17 +619,18 @@ __global__ void __launch_bounds__(LCfg<N>::CTA, LCfg<N>::MINB) flux_layer_kernel
           al += x[r * NS] * b1[r];
           be += y[r * NS] * b2[r];
         }
-        const double r0 = 1.0 / umu0, den = k * k - r0 * r0;
-        vec[mod_cb(N) + c] = (k * al - be * r0) / den;
-        vec[mod_db(N) + c] = (k * be - al * r0) / den;
+        const double r0 = 1.0 / umu0, ka = lneg && primary ? -k : k, kb = lneg && !primary ? -k : k;
+        const double den = ka * kb - r0 * r0;
+        vec[mod_cb(N) + c] = (kb * al - be * r0) / den;
+        vec[mod_db(N) + c] = (ka * be - al * r0) / den;
       }
     }
     if ((p.flags & DSP_FLAG_THERMAL) && m == 0) {
       double v = 0.0;
       for (int r = 0; r < NN; ++r) v += x[r * NS] * (dsim[r] / mu[r]);
-      v = 2.0 * (1.0 - ws) * v / k;
+      v = 2.0 * (1.0 - ws) * v / (lneg && primary ? -k : k);
       vec[mod_ct(N) + c] = v;
-      vec[mod_dt(N) + c] = v / k;
+      vec[mod_dt(N) + c] = v / (lneg && !primary ? -k : k);
       if (c == 0) thermal_source(q, vec[mod_xr(N)], vec[mod_xr(N) + 1]);
     }
   }
@@ -657,39 +669,100 @@ __device__ __forceinline__ void jacobi_rot_rsq(double apq, double app, double aq
   tt = rot ? sv * g : 0.0;
 }
 
-// Cholesky of a packed lower triangle in place; false when a pivot is not
-// positive (the factor is then not used).  The updates are subtracted in the
-// order of the right-looking form and the column is divided by its pivot, as
-// the reference's LLT does: at omega' = 1 one pivot is rounding noise around
-// zero, and the factor's other entries should carry the same rounding.
+// Pivot of a Cholesky factorisation, d0 the diagonal element it started from: at
+// omega' = 1 the last pivot of -A_s is zero to rounding, of either sign, and is
+// taken as 1e-18 d0 (k ~ 1e-9); NaN or a negative pivot beyond rounding: 0, the
+// matrix is indefinite.
+__device__ __forceinline__ double chol_pivot(double s, double d0) {
+  return s > 1e-18 * d0 ? s : (s > -1e-12 * d0 ? 1e-18 * d0 : 0.0);
+}
+
+// Cholesky of a packed lower triangle in place; false when the matrix is
+// indefinite (the factor is then not used).
 template <int NN>
 __device__ __forceinline__ bool chol_packed(double* A) {
   bool ok = true;
 #pragma unroll
   for (int j = 0; j < NN; ++j) {
-    double s = A[tri_idx(j, j)];
+    const double d0 = A[tri_idx(j, j)];
+    double s = d0;
 #pragma unroll
     for (int k = 0; k < j; ++k) s -= A[tri_idx(j, k)] * A[tri_idx(j, k)];
+    s = chol_pivot(s, d0);
     ok = ok && s > 0.0;
-    const double ljj = sqrt(ok ? s : 1.0);
-    A[tri_idx(j, j)] = ljj;
+    const double r = rsqrt(ok ? s : 1.0);
+    A[tri_idx(j, j)] = ok ? s * r : 1.0;
 #pragma unroll
     for (int i = j + 1; i < NN; ++i) {
       double t = A[tri_idx(i, j)];
 #pragma unroll
       for (int k = 0; k < j; ++k) t -= A[tri_idx(i, k)] * A[tri_idx(j, k)];
-      A[tri_idx(i, j)] = t / ljj;
+      A[tri_idx(i, j)] = t * r;
     }
   }
   return ok;
+}
+
+// The front's hand-off of a task with exactly one of -B_s (okb) and -A_s positive
+// definite: S = L^T M L with the definite one's factor L and the other as M.  Rare
+// (phase functions with unphysical moments): local memory and rolled loops.
+template <int N, bool GEN>
+__device__ __noinline__ void layer_front_indefinite(const FluxParams& p, const LayerTask<N, GEN>& q, double* hand,
+                                                    long long nt, long long j, bool okb) {
+  constexpr int NN = N / 2;
+  using HO = Handoff<NN>;
+  const int m = mode_of<GEN>(p);
+  const double* tab = p.tables + mode_row<GEN>() * (long long)tab_size(N);
+  const double* Y = tab + tab_ylm(N);
+  double M[2][HO::TRI], gl[N];  // -B_s, -A_s
+  const double ws = q.rec[q.il.ssa_s + q.lc], f = q.rec[q.il.fsc + q.lc], sig = q.rec[q.il.sig + q.lc];
+  const int mode = (int)q.rec[q.il.mode + q.lc];
+  for (int k = 0; k < N; ++k) gl[k] = phase_coeff<GEN>(k, q.pml[k], mode, ws, f, sig);
+  for (int r = 0; r < NN; ++r)
+    for (int c = 0; c <= r; ++c) {
+      double sum[2] = {0.0, 0.0};  // odd, even l + m
+      for (int l = 0; l < N; ++l) sum[1 - ((l + m) & 1)] += gl[l] * Y[l * N + r] * Y[l * N + c];
+      const double rm = 1.0 / tab[tab_mu(N) + r];
+      for (int h = 0; h < 2; ++h)
+        M[h][tri_idx(r, c)] = -tab[tab_dsim(N) + r] * ((tab[tab_wt(N) + c] * sum[h]) * rm - (r == c ? rm : 0.0)) *
+                              tab[tab_dinv(N) + c];
+    }
+  double* const L = okb ? M[0] : M[1];
+  const double* const I = okb ? M[1] : M[0];
+  for (int c = 0; c < NN; ++c) {
+    const double d0 = L[tri_idx(c, c)];
+    double v = d0;
+    for (int k = 0; k < c; ++k) v -= L[tri_idx(c, k)] * L[tri_idx(c, k)];
+    const double ljj = sqrt(chol_pivot(v, d0));
+    L[tri_idx(c, c)] = ljj;
+    for (int r = c + 1; r < NN; ++r) {
+      double t = L[tri_idx(r, c)];
+      for (int k = 0; k < c; ++k) t -= L[tri_idx(r, k)] * L[tri_idx(c, k)];
+      L[tri_idx(r, c)] = t / ljj;
+    }
+  }
+  for (int c = 0; c < NN; ++c) {
+    double t[NN];  // (M L)[:, c]
+    for (int r = 0; r < NN; ++r) {
+      t[r] = 0.0;
+      for (int k = c; k < NN; ++k) t[r] += I[tri_idx(r, k)] * L[tri_idx(k, c)];
+    }
+    for (int r = c; r < NN; ++r) {
+      double v = 0.0;
+      for (int k = r; k < NN; ++k) v += L[tri_idx(k, r)] * t[k];
+      *handoff_lane<NN>(hand, nt, j, HO::S_F + tri_idx(r, c)) = v;
+    }
+  }
+  for (int e = 0; e < HO::TRI; ++e) *handoff_lane<NN>(hand, nt, j, HO::S_L + e) = L[e];
+  *handoff_lane<NN>(hand, nt, j, HO::S_FLAG) = okb ? 2.0 : 3.0;
 }
 
 // ---------------------------------------------------------------------------
 // Front of a split layer stage, one thread per layer task: scaled phase
 // coefficients (disortSet, FluxSolver.cpp:336-386), the phase sums, alpha -/+ beta
 // in the symmetric form of the reference (FluxSolver.cpp:466-514), the Cholesky
-// factorisation of -B_s, else of -A_s (:521-558), S = L^T M L and the beam's
-// source vectors, written to the hand-off.  Every matrix is a packed symmetric
+// factors of -B_s and -A_s (:521-558), L^T R and the beam's source vectors,
+// written to the hand-off.  Every matrix is a packed symmetric
 // h x h in registers; the tables are constant-bank operands.
 // ---------------------------------------------------------------------------
 template <int N, bool GEN>
@@ -787,118 +860,177 @@ __global__ void __launch_bounds__(128) flux_layer_front_kernel(FluxParams p, Con
         X[tri_idx(r, c)] = -tc.dsim[r] * a * tc.dinv[c];
       }
   };
-  // ---- Cholesky of -B_s, else of -A_s --------------------------------------
-  double Lf[TRI];
+  // ---- Cholesky factors L of -B_s and R of -A_s, F = L^T R -------------------
+  double Lf[TRI], R[TRI];
   minus_s(O, Lf);
-  const bool primary = chol_packed<NN>(Lf);
-  if (!primary) {
-    minus_s(E, Lf);
-    if (!chol_packed<NN>(Lf)) {
-      set_status(p.status, q.i, DSP_ERR_EIGEN);
-      *hp(HO::S_FLAG) = 0.0;
-      return;
-    }
+  minus_s(E, R);
+  const bool okb = chol_packed<NN>(Lf), oka = chol_packed<NN>(R);
+  if (okb && oka) {
+#pragma unroll
+    for (int c = 0; c < NN; ++c)
+#pragma unroll
+      for (int r = 0; r < NN; ++r) {
+        double v = 0.0;
+#pragma unroll
+        for (int k = (r > c ? r : c); k < NN; ++k) v += Lf[tri_idx(k, r)] * R[tri_idx(k, c)];
+        *hp(HO::S_F + c * NN + r) = v;
+      }
+#pragma unroll
+    for (int e = 0; e < TRI; ++e) *hp(HO::S_L + e) = Lf[e];
+    *hp(HO::S_FLAG) = 1.0;
+    return;
   }
-  // ---- S = L^T M L, M = -A_s (primary) or -B_s (fallback), by columns ----
-  double M[TRI];
+  if (!okb && !oka) {
+    set_status(p.status, q.i, DSP_ERR_EIGEN);
+    *hp(HO::S_FLAG) = 0.0;
+    return;
+  }
+  layer_front_indefinite<N, GEN>(p, q, hand, nt, j, okb);
+}
+
+// Tangent of the Jacobi angle that makes two columns of squared norms app, aqq and
+// inner product apq orthogonal (0 where they are to rounding): the smaller root t
+// of t^2 + 2 th t - 1, th = (aqq - app) / (2 apq).  In single precision: the
+// rotation built from it is orthogonal to double precision whatever t is
+// (rsqrt_near1), and an angle off by 1e-7 of itself leaves 1e-7 of the inner
+// product, which the next sweep's quadratic convergence absorbs.
+// far: the pair was rotated by more than 1e-8 or was further than 1e-8 from
+// orthogonal.
+__device__ __forceinline__ float jacobi_tan(double apq, double app, double aqq, bool& far) {
+  const double g2 = apq * apq, ab = app * aqq;
+  const bool need = g2 > DSP_JACOBI_TOL2 * ab;
+  const float d = static_cast<float>(aqq - app), e = 2.0f * static_cast<float>(apq);
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fmaf(d, d, e * e)));
+  const float t = __fdividef(fabsf(e), fabsf(d) + r);  // NaN when both vanish
+  const bool use = need && t <= 1.0f;
+  far = use && (t > 1e-8f || g2 > 1e-16 * ab);
+  const bool same = (d < 0.0f) == (e < 0.0f);  // sgn(th), sgn(0) = +1
+  return use ? (same ? t : -t) : 0.0f;
+}
+
+// 1/sqrt(x) for x in [1, 2]: the single-precision value y refined by one step of
+// the third-order iteration y (1 + e/2 + 3 e^2/8), e = 1 - x y^2 (e ~ 2^-22, error
+// ~ e^3; Muller et al., Handbook of Floating-Point Arithmetic, section 4.7).
+__device__ __forceinline__ double rsqrt_near1(double x) {
+  const double y = static_cast<double>(rsqrtf(static_cast<float>(x)));
+  const double e = fma(-x * y, y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// One round of a one-sided Jacobi sweep in odd-even order: the pairs (p, p + 1),
+// p = ODD, ODD + 2, ..., of the columns of F are rotated to be orthogonal and change
+// places, so that n rounds bring every two columns together, always in the same
+// registers.  nrm: the columns' squared norms.  Returns whether a pair was rotated
+// by more than 1e-8 or its columns were further than 1e-8 from orthogonal: when
+// none of a sweep's was, what is left is below rounding (quadratic convergence,
+// and the angles' 1e-7).  live: false leaves the columns in place, up to sign.
+template <int NN, int ODD>
+__device__ __forceinline__ bool onesided_round(double (*F)[NN], double* nrm, bool live) {
+  constexpr int NPAIR = (NN - ODD) / 2;
+  bool more = false;
+  // the rotations of the round's pairs side by side (their serial chains overlap)
+  double cs[NPAIR > 0 ? NPAIR : 1], sn[NPAIR > 0 ? NPAIR : 1];
 #pragma unroll
-  for (int e = 0; e < TRI; ++e) E[e] = primary ? E[e] : O[e];
-  minus_s(E, M);
+  for (int a = 0; a < NPAIR; ++a) {
+    const int p = 2 * a + ODD, q = p + 1;
+    double d0 = 0.0, d1 = 0.0;
 #pragma unroll
-  for (int c = 0; c < NN; ++c) {
-    double t[NN];  // (M L)[:, c]; L[k][c] = 0 for k < c
+    for (int r = 0; r < NN; r += 2) {
+      d0 = fma(F[p][r], F[q][r], d0);
+      if (r + 1 < NN) d1 = fma(F[p][r + 1], F[q][r + 1], d1);
+    }
+    const double g = d0 + d1, np = nrm[p], nq = nrm[q];
+    bool far;
+    const float tf = jacobi_tan(g, np, nq, far);
+    const double t = tf;
+    more = more || far;
+    const double c = rsqrt_near1(fma(t, t, 1.0));
+    cs[a] = live ? c : 0.0;  // a finished task's columns stay in place (one changes sign)
+    sn[a] = live ? t * c : 1.0;
+    nrm[q] = fma(-t, g, np);
+    nrm[p] = fma(t, g, nq);
+  }
+#pragma unroll
+  for (int a = 0; a < NPAIR; ++a) {
+    const int p = 2 * a + ODD, q = p + 1;
 #pragma unroll
     for (int r = 0; r < NN; ++r) {
-      double s = 0.0;
-#pragma unroll
-      for (int k = c; k < NN; ++k) s += M[tri_idx(r, k)] * Lf[tri_idx(k, c)];
-      t[r] = s;
-    }
-#pragma unroll
-    for (int r = c; r < NN; ++r) {
-      double s = 0.0;
-#pragma unroll
-      for (int k = r; k < NN; ++k) s += Lf[tri_idx(k, r)] * t[k];
-      *hp(HO::S_S + tri_idx(r, c)) = s;
+      const double x = F[p][r], y = F[q][r];
+      F[q][r] = fma(cs[a], x, -(sn[a] * y));
+      F[p][r] = fma(sn[a], x, cs[a] * y);
     }
   }
-#pragma unroll
-  for (int e = 0; e < TRI; ++e) *hp(HO::S_L + e) = Lf[e];
-  *hp(HO::S_FLAG) = primary ? 1.0 : 2.0;
+  return more;
 }
 
-// Rotation of the pair (p, q) applied to S (packed lower, both sides) and to the
-// columns p, q of V; the same update as the team form's 2x2 blocks:
-// column p' = c col p - s col q, column q' = s col p + c col q, and on the
-// diagonal block a_pp - t a_pq, a_qq + t a_pq, a_pq -> 0.
+// One-sided Jacobi iteration on the columns of F, in registers.  Two rounds are the
+// body of a rolled loop (a sweep unrolled overflows the instruction cache: 1.8 of
+// 5.5 stalled cycles per instruction; the round-robin order, rolled, moves every
+// column between registers).  A warp runs until its last active task has
+// converged, 3 to 5 sweeps; a task that has is left as it is, so that its result
+// does not depend on the others of its warp.
 template <int NN>
-__device__ __forceinline__ void jacobi_apply(double* S, double* V, int p, int q, double c, double s,
-                                             double t) {
-  const double apq = S[tri_idx(p, q)];
-#pragma unroll
-  for (int k = 0; k < NN; ++k) {
-    if (k == p || k == q) continue;
-    const double x = S[tri_idx(k, p)], y = S[tri_idx(k, q)];
-    S[tri_idx(k, p)] = c * x - s * y;
-    S[tri_idx(k, q)] = s * x + c * y;
-  }
-  S[tri_idx(p, p)] -= t * apq;
-  S[tri_idx(q, q)] += t * apq;
-  S[tri_idx(p, q)] = (t != 0.0) ? 0.0 : apq;
-#pragma unroll
-  for (int k = 0; k < NN; ++k) {
-    const double x = V[k * NN + p], y = V[k * NN + q];
-    V[k * NN + p] = c * x - s * y;
-    V[k * NN + q] = s * x + c * y;
-  }
-}
-
-// The sweeps of the one-thread-per-task eigensolver on S (packed lower) and the
-// eigenvector matrix V (row-major), every index a compile-time constant (rounds
-// and pairs unrolled).  The sweeps, the round-robin pair order, the rotation
-// angle (as jacobi_rot) and the stopping rule (a sweep is run while some pair
-// still needs a rotation, at most 20) are those of the team form in
-// flux_layer_kernel; a warp runs until its last active task has converged, and
-// a converged task's rotations are the identity.  Called by all 32 lanes.
-template <int NN>
-__device__ __forceinline__ void jacobi_sweeps(double* S, double* V, bool act) {
-  constexpr int NNP = NN + (NN & 1), NPAIR = NNP / 2;
+__device__ __forceinline__ void onesided_jacobi(double (*F)[NN], bool act) {
+  bool live = act;
   for (int sweep = 0; sweep < 20; ++sweep) {
+    double nrm[NN];
 #pragma unroll
-    for (int r = 0; r < NNP - 1; ++r) {
-      double c[NPAIR], s[NPAIR], tt[NPAIR];
+    for (int c = 0; c < NN; ++c) {
+      nrm[c] = 0.0;
 #pragma unroll
-      for (int a = 0; a < NPAIR; ++a) {
-        const int pp = rr_player<NNP>(r, a), qq = rr_player<NNP>(r, NNP - 1 - a);
-        c[a] = 1.0;
-        s[a] = 0.0;
-        tt[a] = 0.0;
-        if (pp < NN && qq < NN)
-          jacobi_rot_rsq(S[tri_idx(pp, qq)], S[tri_idx(pp, pp)], S[tri_idx(qq, qq)], c[a], s[a], tt[a]);
-      }
-#pragma unroll
-      for (int a = 0; a < NPAIR; ++a) {
-        const int pp = rr_player<NNP>(r, a), qq = rr_player<NNP>(r, NNP - 1 - a);
-        if (pp < NN && qq < NN) jacobi_apply<NN>(S, V, pp, qq, c[a], s[a], tt[a]);
-      }
+      for (int r = 0; r < NN; ++r) nrm[c] = fma(F[c][r], F[c][r], nrm[c]);
     }
     bool more = false;
-#pragma unroll
-    for (int r = 1; r < NN; ++r)
-#pragma unroll
-      for (int q = 0; q < r; ++q)
-        if (jacobi_needed(S[tri_idx(r, q)], S[tri_idx(r, r)], S[tri_idx(q, q)])) more = true;
-    if (!__any_sync(0xffffffffu, act && more)) break;
+#pragma unroll 1
+    for (int r = 0; r < NN; r += 2) {
+      more = onesided_round<NN, 0>(F, nrm, live) || more;
+      more = onesided_round<NN, 1>(F, nrm, live) || more;
+    }
+    live = live && more;
+    if (!__any_sync(0xffffffffu, live)) break;
   }
 }
 
-// Eigensolver and output of the split layer stage, one thread per layer task: S
-// from the hand-off into registers, jacobi_sweeps, then mode by mode X and Y
-// (from the eigenvector and the Cholesky factor), k and the particular solutions
-// in the modes.  The layer record is staged per warp in shared memory and written
-// with consecutive lanes on consecutive doubles.  (An eigensolver that writes its
-// vectors to the hand-off for a third launch to read again spent a third of the
-// layer stage on those reads.)
+// Cyclic two-sided Jacobi on a packed symmetric matrix, for the rare task whose
+// -A_s or -B_s is indefinite (local memory, rolled loops).  V: eigenvectors by
+// columns, d: eigenvalues.
+template <int NN>
+__device__ __noinline__ void jacobi_two_sided(double* S, double* V, double* d) {
+  for (int e = 0; e < NN * NN; ++e) V[e] = e / NN == e % NN ? 1.0 : 0.0;
+  for (int sweep = 0; sweep < 20; ++sweep) {
+    bool more = false;
+    for (int q = 1; q < NN; ++q)
+      for (int p = 0; p < q; ++p) {
+        const double apq = S[tri_idx(q, p)];
+        double c, s, t;
+        jacobi_rot_rsq(apq, S[tri_idx(p, p)], S[tri_idx(q, q)], c, s, t);
+        if (t == 0.0) continue;
+        more = true;
+        S[tri_idx(p, p)] -= t * apq;
+        S[tri_idx(q, q)] += t * apq;
+        S[tri_idx(q, p)] = 0.0;
+        for (int k = 0; k < NN; ++k) {
+          if (k != p && k != q) {
+            const double x = S[tri_idx(k, p)], y = S[tri_idx(k, q)];
+            S[tri_idx(k, p)] = c * x - s * y;
+            S[tri_idx(k, q)] = s * x + c * y;
+          }
+          const double x = V[p * NN + k], y = V[q * NN + k];
+          V[p * NN + k] = c * x - s * y;
+          V[q * NN + k] = s * x + c * y;
+        }
+      }
+    if (!more) break;
+  }
+  for (int k = 0; k < NN; ++k) d[k] = S[tri_idx(k, k)];
+}
+
+// Eigensolver and output of the split layer stage, one thread per layer task: F
+// from the hand-off into registers, onesided_jacobi, then mode by mode X and Y
+// (from the singular vector and the Cholesky factor), k and the particular
+// solutions in the modes.  The layer record is staged per warp in shared memory
+// and written with consecutive lanes on consecutive doubles.
 template <int N>
 struct ECfg {
   static constexpr int HP = mod_hp(N);
@@ -934,14 +1066,42 @@ __global__ void __launch_bounds__(128) flux_eigen_kernel(FluxParams p, ConstTab<
   const bool act = j < nt && flag != 0.0;  // skipped: cut layer, invalid input, no factorisation
   const unsigned okm = __ballot_sync(0xffffffffu, act);
   if (okm == 0u) return;  // warp-uniform
-  double S[HO::TRI], V[NN * NN];
+  double F[NN][NN], kk[NN];
+  const bool regular = flag < 1.5;
 #pragma unroll
-  for (int e = 0; e < HO::TRI; ++e) S[e] = act ? hv(HO::S_S + e) : 0.0;
+  for (int c = 0; c < NN; ++c)
 #pragma unroll
-  for (int e = 0; e < NN * NN; ++e) V[e] = (e / NN == e % NN) ? 1.0 : 0.0;
-  jacobi_sweeps<NN>(S, V, act);
+    for (int r = 0; r < NN; ++r) F[c][r] = act && regular ? hv(HO::S_F + c * NN + r) : 0.0;
+  onesided_jacobi<NN>(F, act && regular);
+#pragma unroll
+  for (int c = 0; c < NN; ++c) {
+    double n2 = 0.0;
+#pragma unroll
+    for (int r = 0; r < NN; ++r) n2 = fma(F[c][r], F[c][r], n2);
+    const double rs = n2 > 0.0 ? rsqrt(n2) : 0.0;
+    kk[c] = fmax(n2 * rs, 1e-9);
+#pragma unroll
+    for (int r = 0; r < NN; ++r) F[c][r] *= rs;
+  }
+  // eigenvalues lambda = k^2 are negative only where -A_s (bit set in nega) or -B_s
+  // (negb) is indefinite; k = sqrt|lambda| as in the reference, the inverses of the
+  // particular solutions carry the sign, and with -B_s the reference's a and b
+  // change roles, which is the mode of -k
+  unsigned nega = 0u, negb = 0u;
+  if (act && !regular) {
+    double S[HO::TRI], V[NN * NN], d[NN];
+    for (int e = 0; e < HO::TRI; ++e) S[e] = hv(HO::S_F + e);
+    jacobi_two_sided<NN>(S, V, d);
+#pragma unroll
+    for (int c = 0; c < NN; ++c) {
+      kk[c] = mode_k(d[c]);
+      if (d[c] < 0.0) (flag < 2.5 ? nega : negb) |= 1u << c;
+#pragma unroll
+      for (int r = 0; r < NN; ++r) F[c][r] = V[c * NN + r];
+    }
+  }
 
-  const bool primary = flag == 1.0;
+  const bool primary = flag < 2.5;
   const LayerTask<N, GEN> q = layer_task<N, GEN>(p, jj);
   const double fbeam = act ? q.rec[H_FBEAM] : 0.0;
   const bool beam = fbeam > 0.0;
@@ -952,7 +1112,7 @@ __global__ void __launch_bounds__(128) flux_eigen_kernel(FluxParams p, ConstTab<
     double umu0 = q.rec[H_UMU0];
     bool res = false;
 #pragma unroll
-    for (int c = 0; c < NN; ++c) res = res || beam_resonant(mode_k(S[tri_idx(c, c)]), umu0);
+    for (int c = 0; c < NN; ++c) res = res || beam_resonant(kk[c], umu0);
     if (res) umu0 = 0.999 * umu0;
     r0 = 1.0 / umu0;
   }
@@ -962,18 +1122,17 @@ __global__ void __launch_bounds__(128) flux_eigen_kernel(FluxParams p, ConstTab<
   for (int e = 0; e < HO::TRI; ++e) L[e] = act ? hv(HO::S_L + e) : 1.0;
   double rdg[NN];
 #pragma unroll
-  for (int k = 0; k < NN; ++k) rdg[k] = 1.0 / L[tri_idx(k, k)];
+  for (int k = 0; k < NN; ++k) rdg[k] = rcp_newton(L[tri_idx(k, k)]);
   const long long ls = GEN ? p.g.lstride : (long long)lrec_stride(N);
   double* const rec0 = p.layer_rec + mode_row<GEN>() * p.g.ms_layer + j0 * ls;
   const double dts = act ? q.rec[q.il.dtau_s + q.lc] : 0.0;
 #pragma unroll
   for (int c = 0; c < NN; ++c) {
-    const double k = mode_k(S[tri_idx(c, c)]);
-    const double sk = sqrt(k), rsk = 1.0 / sk;
+    const double k = kk[c], rsk = rsqrt(k), sk = k * rsk;
     double x[NN], y[NN];
     // y = L^{-T} u, x = L u
 #pragma unroll
-    for (int r = 0; r < NN; ++r) y[r] = V[r * NN + c];
+    for (int r = 0; r < NN; ++r) y[r] = F[c][r];
 #pragma unroll
     for (int e = NN - 1; e >= 0; --e) {
       y[e] *= rdg[e];
@@ -984,7 +1143,7 @@ __global__ void __launch_bounds__(128) flux_eigen_kernel(FluxParams p, ConstTab<
     for (int r = 0; r < NN; ++r) {
       double s = 0.0;
 #pragma unroll
-      for (int e = 0; e <= r; ++e) s += L[tri_idx(r, e)] * V[e * NN + c];
+      for (int e = 0; e <= r; ++e) s += L[tri_idx(r, e)] * F[c][e];
       x[r] = s;
     }
     double ve = 0.0, al = 0.0, be = 0.0;
@@ -1001,9 +1160,11 @@ __global__ void __launch_bounds__(128) flux_eigen_kernel(FluxParams p, ConstTab<
       row[NN] = 0.0;
       row[HP + NN] = 0.0;
     }
-    vrow[c] = k;
-    vrow[HP + c] = exp(-k * dts);
-    vrow[2 * HP + c] = -expm1(-2.0 * k * dts);
+    const double ks = (negb >> c) & 1u ? -k : k;
+    vrow[c] = ks;
+    const double em = expm1(-ks * dts);  // E - 1; 1 - E^2 = -em (2 + em)
+    vrow[HP + c] = 1.0 + em;
+    vrow[2 * HP + c] = -em * (2.0 + em);
     if (beam) {
       if (raw) {
         // pseudo-spherical beam (general solver): the raw source at the quadrature
@@ -1018,15 +1179,17 @@ __global__ void __launch_bounds__(128) flux_eigen_kernel(FluxParams p, ConstTab<
           al += x[r] * hv(HO::S_B1 + r);
           be += y[r] * hv(HO::S_B2 + r);
         }
-        const double den = 1.0 / (k * k - r0 * r0);
-        vrow[3 * HP + c] = (k * al - be * r0) * den;
-        vrow[4 * HP + c] = (k * be - al * r0) * den;
+        const double ka = (nega >> c) & 1u ? -k : k, kb = (negb >> c) & 1u ? -k : k;
+        const double den = rcp_newton(ka * kb - r0 * r0);
+        vrow[3 * HP + c] = (kb * al - be * r0) * den;
+        vrow[4 * HP + c] = (ka * be - al * r0) * den;
       }
     }
     if (thermal) {
-      ve = ws2 * ve / k;
+      const double rk = rsk * rsk;
+      ve = ws2 * ve * ((nega >> c) & 1u ? -rk : rk);
       vrow[5 * HP + c] = ve;
-      vrow[6 * HP + c] = ve / k;
+      vrow[6 * HP + c] = ve * ((negb >> c) & 1u ? -rk : rk);
     }
     // X^T row c and Y^T row c of every task: lane group (task, X or Y) x HP
     __syncwarp();

@@ -59,3 +59,24 @@ def test_conservative_columns_conserve_the_net_flux(N):
     net = got["flux_up"] - got["flux_down"] - got["flux_direct_beam"]
     incoming = np.pi * 0.3 + got["flux_direct_beam"][:, :1]
     assert np.max(np.abs(net - net[:, :1]) / incoming) <= 1e-13 * 300
+
+
+@pytest.mark.parametrize("N", [4, 6, 8, 14, 16, 32, 64])
+@pytest.mark.parametrize("which", [0, 1])
+def test_indefinite_layers(N, which):
+    """Layers whose phase moments make -A_s (an even moment far above 1) or -B_s (an
+    odd one) indefinite: the eigensolver's other branch.  Unphysical but accepted,
+    as by the oracle, which is the checker at its own double-extended distance
+    (such columns amplify rounding)."""
+    w = columns(N, 5, 3, 11 * N + which, True, ssa=0.9)
+    w["arrays"]["delta_tau"] = np.clip(w["arrays"]["delta_tau"], 0.01, 0.5)
+    pm = w["arrays"]["phase_function_moments"]
+    pm[:, :, 1:] *= 0.2
+    pm[::2, 1, 2 if which == 0 else 1] = 1.6
+    got, gst, rc = gpu_lib.flux_solve(w)
+    ref, rst = oracle_lib.flux_solve(w, ext=True)
+    dbl, _ = oracle_lib.flux_solve(w)
+    assert rc == 0 and np.array_equal(gst, rst)
+    for f in capi.FLUX_OUT_FIELDS:
+        spread = np.max(np.abs(dbl[f] - ref[f]) / (np.abs(ref[f]) + 1e-3))
+        np.testing.assert_allclose(got[f], ref[f], rtol=1e-9 + 4.0 * spread, atol=1e-12 + 4e-3 * spread, err_msg=f)
