@@ -30,8 +30,9 @@
 //   O_ij, E_ij = sum_{l + m odd, even} g'_l P_l^m(mu_i) P_l^m(mu_j).
 //
 // N <= 16: one thread per layer task, every matrix in registers (front kernel,
-// then the eigensolver with the record's output).  Larger N (and, on the flux
-// path, when a schedule asks for it): a team of threads per task in shared memory.
+// then the eigensolver with the record's output); on the flux path, when a schedule
+// asks for it, a team of threads per task in shared memory.  N = 32, 64: a team of
+// lanes per task, two columns per lane in registers.
 #pragma once
 
 #include "dsp_device.cuh"
@@ -1209,28 +1210,514 @@ __global__ void __launch_bounds__(128) flux_eigen_kernel(FluxParams p, ConstTab<
       for (int e = lane; e < 7 * HP + 2; e += 32) rec0[b * ls + mod_k(N) + e] = vst[b * VS + e];
 }
 
+// ---------------------------------------------------------------------------
+// Layer stage of 32 and 64 streams: a team of h/2 lanes per layer task, two
+// columns of h rows per lane in registers (two tasks per warp at 64 streams, four
+// at 32).  The same steps as the one-thread stage: phase sums column by column,
+// Cholesky factors of -B_s and -A_s with the pivot column exchanged through shared
+// memory, F = L^T R, one-sided Jacobi in odd-even order, where a lane's two columns
+// are the even rounds' pair and the odd rounds' pair takes the next lane's first
+// column by shuffles, and the modes from the triangular factor.
+// What bounds it: FP64 issue in the Jacobi rounds (about 5 h + 20 instructions per
+// lane and round for two tasks a warp).  The team form it replaced (shared-memory
+// two-sided Jacobi with a barrier per round, 128 threads a task at 64 streams) took
+// 8.7 ms for 192 x 91 layers at 64 streams.
+// ---------------------------------------------------------------------------
+template <int N>
+struct WCfg {
+  static constexpr int H = N / 2, TEAM = H / 2, TPW = 32 / TEAM;
+  static constexpr int LDM = H + 2;            // row stride: an odd number of 16-byte words
+  static constexpr int MAT = H * LDM;
+  static constexpr int O_L = 0;                // Cholesky factor L, row-major
+  static constexpr int O_R = O_L + MAT;        // -A_s and its factor; then X^T, Y^T on their way out
+  static constexpr int O_C = O_R + MAT;        // pivot column, twice (rotated reads), two buffers
+  static constexpr int O_GL = O_C + 2 * (2 * H + 4);  // g'_l [N]
+  static constexpr int O_B1 = O_GL + N;        // D M^{-1} (q+ + q-), D M^{-1} (q+ - q-), D M^{-1} 1
+  static constexpr int O_B2 = O_B1 + H;
+  static constexpr int O_E = O_B2 + H;
+  static constexpr int SIZE = O_E + H;
+  static constexpr int STRIDE = SIZE + ((2 - SIZE) % 16 + 16) % 16;  // teams 4 banks apart
+  static constexpr size_t smem_bytes() { return sizeof(double) * (size_t)(TPW * STRIDE); }
+  static constexpr int MINB = H == 32 ? 6 : 10;
+};
+
+// Cholesky factor of the symmetric matrix whose columns 2t, 2t + 1 lane t holds in
+// c0, c1 (rows in order), written row-major to `out` (stride LDM, upper part zero).
+// Right-looking; in step k register i of a column is row k + i, the update shifting
+// it by one row.  Returns false (to every lane of the team) if it is indefinite.
+template <int H, int LDM, int TEAM>
+__device__ __forceinline__ bool team_chol_columns(double* c0, double* c1, double* out, double* cbuf, int t,
+                                                  unsigned msk) {
+  bool ok = true;
+  double d00 = 0.0, d01 = 0.0;  // the original diagonal elements of the lane's columns
+#pragma unroll
+  for (int r = 0; r < H; ++r) {
+    if (r == 2 * t) d00 = c0[r];
+    if (r == 2 * t + 1) d01 = c1[r];
+  }
+#pragma unroll 1
+  for (int k2 = 0; k2 < H; k2 += 2) {
+#pragma unroll
+    for (int odd = 0; odd < 2; ++odd) {
+      const int k = k2 + odd;
+      const bool mine = t == k2 / 2;
+      double* const buf = cbuf + odd * (2 * H + 4);
+      if (mine) {
+        // register 0 is the pivot
+        const double* c = odd ? c1 : c0;
+        const double s = chol_pivot(c[0], odd ? d01 : d00);
+        const double r = s > 0.0 ? rsqrt(s) : 0.0;
+#pragma unroll
+        for (int i = 0; i < H; ++i) {
+          const double v = i == 0 ? s * r : c[i] * r;
+          buf[i] = v;  // rows k .. k + H - 1: past the matrix the registers hold zeros
+          if (k + i < H) out[(k + i) * LDM + k] = v;
+        }
+        for (int i = 0; i < k; ++i) out[i * LDM + k] = 0.0;
+      }
+      __syncwarp(msk);
+      ok = ok && buf[0] > 0.0;
+      // rows of the lane's columns in this step's numbering: column c is row c - k
+      const int a0 = 2 * t - k, a1 = a0 + 1;
+      const double l0 = a0 > 0 ? buf[a0] : 0.0, l1 = a1 > 0 ? buf[a1] : 0.0;
+      const double2* b2 = reinterpret_cast<const double2*>(buf);
+      {
+        const double2 w = b2[0];
+        c0[0] = fma(-l0, w.y, c0[1]);
+        c1[0] = fma(-l1, w.y, c1[1]);
+      }
+#pragma unroll
+      for (int i = 2; i < H; i += 2) {
+        const double2 w = b2[i / 2];
+        c0[i - 1] = fma(-l0, w.x, c0[i]);
+        c1[i - 1] = fma(-l1, w.x, c1[i]);
+        c0[i] = fma(-l0, w.y, c0[i + 1]);
+        c1[i] = fma(-l1, w.y, c1[i + 1]);
+      }
+      c0[H - 1] = 0.0;
+      c1[H - 1] = 0.0;
+    }
+  }
+  __syncwarp(msk);
+  return ok;
+}
+
+// The modes of a task with exactly one of -B_s (okb) and -A_s positive definite, by
+// one lane in global scratch (rare: unphysical moments): the eigenvectors of S by
+// columns at V, its eigenvalues at d, the factor at L (row-major, stride LDM).
+template <int H, int LDM>
+__device__ __noinline__ void team_indefinite(const double* gl, const double* Y, const double* tab, int N, int m,
+                                             bool okb, double* L, double* M, double* V, double* d) {
+  double* const S = M + H * H;  // scratch: M [H][H], S [H][H]
+  for (int r = 0; r < H; ++r)
+    for (int c = 0; c <= r; ++c) {
+      double sum[2] = {0.0, 0.0};  // odd, even l + m
+      for (int l = 0; l < N; ++l) sum[1 - ((l + m) & 1)] += gl[l] * Y[l * N + r] * Y[l * N + c];
+      const double rm = 1.0 / tab[r], dl = r == c ? rm : 0.0;
+      const double sc = -tab[tab_dsim(N) + r] * tab[tab_dinv(N) + c];
+      const double vb = sc * (tab[tab_wt(N) + c] * sum[0] * rm - dl), va = sc * (tab[tab_wt(N) + c] * sum[1] * rm - dl);
+      L[r * LDM + c] = okb ? vb : va;
+      M[r * H + c] = M[c * H + r] = okb ? va : vb;
+    }
+  for (int c = 0; c < H; ++c) {
+    const double d0 = L[c * LDM + c];
+    double v = d0;
+    for (int k = 0; k < c; ++k) v -= L[c * LDM + k] * L[c * LDM + k];
+    const double ljj = sqrt(chol_pivot(v, d0));
+    L[c * LDM + c] = ljj;
+    for (int r = 0; r < c; ++r) L[r * LDM + c] = 0.0;
+    for (int r = c + 1; r < H; ++r) {
+      double t = L[r * LDM + c];
+      for (int k = 0; k < c; ++k) t -= L[r * LDM + k] * L[c * LDM + k];
+      L[r * LDM + c] = t / ljj;
+    }
+  }
+  for (int c = 0; c < H; ++c) {  // V as scratch: (M L)[:, c] in its first row
+    for (int r = 0; r < H; ++r) {
+      double v = 0.0;
+      for (int k = c; k < H; ++k) v += M[r * H + k] * L[k * LDM + c];
+      V[r] = v;
+    }
+    for (int r = c; r < H; ++r) {
+      double v = 0.0;
+      for (int k = r; k < H; ++k) v += L[k * LDM + r] * V[k];
+      S[r * H + c] = S[c * H + r] = v;
+    }
+  }
+  for (int e = 0; e < H * H; ++e) V[e] = e / H == e % H ? 1.0 : 0.0;
+  for (int sweep = 0; sweep < 20; ++sweep) {
+    bool more = false;
+    for (int q = 1; q < H; ++q)
+      for (int p = 0; p < q; ++p) {
+        const double apq = S[q * H + p];
+        double c, s, t;
+        jacobi_rot_rsq(apq, S[p * H + p], S[q * H + q], c, s, t);
+        if (t == 0.0) continue;
+        more = true;
+        for (int k = 0; k < H; ++k) {
+          if (k != p && k != q) {
+            const double x = S[k * H + p], y = S[k * H + q];
+            S[k * H + p] = S[p * H + k] = c * x - s * y;
+            S[k * H + q] = S[q * H + k] = s * x + c * y;
+          }
+          const double x = V[p * H + k], y = V[q * H + k];
+          V[p * H + k] = c * x - s * y;
+          V[q * H + k] = s * x + c * y;
+        }
+        S[p * H + p] -= t * apq;
+        S[q * H + q] += t * apq;
+        S[q * H + p] = S[p * H + q] = 0.0;
+      }
+    if (!more) break;
+  }
+  for (int k = 0; k < H; ++k) d[k] = S[k * H + k];
+}
+
+template <int N, bool GEN>
+__global__ void __launch_bounds__(32, WCfg<N>::MINB) flux_layer_warp_kernel(FluxParams p) {
+  using C = WCfg<N>;
+  constexpr int H = C::H, TEAM = C::TEAM, LDM = C::LDM;
+  extern __shared__ double smem[];
+  const int t = threadIdx.x % TEAM;
+  const unsigned msk = 0xffffffffu;  // the warp's teams go together
+  double* const sm = smem + (threadIdx.x / TEAM) * C::STRIDE;
+  double* const Ls = sm + C::O_L;
+  double* const Rs = sm + C::O_R;
+  double* const cb = sm + C::O_C;
+  double* const gl = sm + C::O_GL;
+  double* const b1 = sm + C::O_B1;
+  double* const b2 = sm + C::O_B2;
+  double* const ev = sm + C::O_E;
+  const int m = mode_of<GEN>(p);
+  const double* const tab = p.tables;
+  const double* const Y = tab + (long long)mode_row<GEN>() * tab_size(N) + tab_ylm(N);
+  const long long nt = layer_tasks<GEN>(p);
+  const long long task = (long long)blockIdx.x * C::TPW + threadIdx.x / TEAM;
+  // a team without a task computes on the last one's inputs and writes nothing
+  const LayerTask<N, GEN> q = layer_task<N, GEN>(p, task < nt ? task : nt - 1);
+  bool act = task < nt && q.live;
+  if (!__any_sync(msk, act)) return;
+  const double ws = q.rec[q.il.ssa_s + q.lc];
+  {
+    const int mode = (int)q.rec[q.il.mode + q.lc];
+    const double f = q.rec[q.il.fsc + q.lc], sig = q.rec[q.il.sig + q.lc];
+    for (int k = t; k < N; k += TEAM) gl[k] = phase_coeff<GEN>(k, q.pml[k], mode, ws, f, sig);
+  }
+  __syncwarp(msk);
+  const int odd0 = 1 - (m & 1);  // first l of odd l + m
+  const double fbeam = act ? q.rec[H_FBEAM] : 0.0;
+  const bool beam = fbeam > 0.0;
+  for (int r = t; r < H; r += TEAM) {
+    const double dm = tab[tab_dsim(N) + r] / tab[r];
+    ev[r] = dm;
+    double so = 0.0, se = 0.0;
+    if (beam) {
+      // (2 - delta_m0) F0 / 4pi sum_k g'_k P_k^m(mu_r) P_k^m(-mu0) by parity (DisortSolver.cpp:1361-1368)
+      const double* yb = beam_legendre<N, GEN>(p, q);
+      const double fac = ((GEN && m > 0) ? 4.0 : 2.0) * fbeam / (4.0 * 3.14159265358979323846);
+      for (int l = 0; l < N; l += 2) {
+        so += gl[l + odd0] * Y[(l + odd0) * N + r] * yb[l + odd0];
+        se += gl[l + 1 - odd0] * Y[(l + 1 - odd0) * N + r] * yb[l + 1 - odd0];
+      }
+      so *= dm * fac;
+      se *= dm * fac;
+    }
+    b1[r] = se;
+    b2[r] = so;
+  }
+  // ---- columns 2t, 2t + 1 of -A_s (into R) and -B_s (into L) -----------------
+  const double w0 = tab[tab_wt(N) + 2 * t], w1 = tab[tab_wt(N) + 2 * t + 1];
+  const double i0 = tab[tab_dinv(N) + 2 * t], i1 = tab[tab_dinv(N) + 2 * t + 1];
+  bool ok[2];
+  double F0[H], F1[H];
+#pragma unroll 1
+  for (int part = 0; part < 2; ++part) {  // 0: -A_s (even sums), 1: -B_s (odd sums)
+#pragma unroll
+    for (int r = 0; r < H; ++r) F0[r] = F1[r] = 0.0;
+    const int l0 = part == 0 ? 1 - odd0 : odd0;
+#pragma unroll 1
+    for (int l = l0; l < N; l += 2) {
+      const double* y = Y + l * N;
+      const double z0 = gl[l] * y[2 * t], z1 = gl[l] * y[2 * t + 1];
+      const double2* y2 = reinterpret_cast<const double2*>(y);
+#pragma unroll
+      for (int r = 0; r < H; r += 2) {
+        const double2 v = y2[r / 2];
+        F0[r] = fma(v.x, z0, F0[r]);
+        F0[r + 1] = fma(v.y, z0, F0[r + 1]);
+        F1[r] = fma(v.x, z1, F1[r]);
+        F1[r + 1] = fma(v.y, z1, F1[r + 1]);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < H; ++r) {
+      const double dm = ev[r];  // d_r / mu_r
+      F0[r] = -dm * (w0 * F0[r] - (r == 2 * t ? 1.0 : 0.0)) * i0;
+      F1[r] = -dm * (w1 * F1[r] - (r == 2 * t + 1 ? 1.0 : 0.0)) * i1;
+    }
+    ok[part] = team_chol_columns<H, LDM, TEAM>(F0, F1, part == 0 ? Rs : Ls, cb, t, msk);
+  }
+  const bool okb = ok[1], oka = ok[0];
+  if (act && !okb && !oka) {
+    if (t == 0) set_status(p.status, q.i, DSP_ERR_EIGEN);
+    act = false;
+  }
+  const bool regular = okb && oka;
+  // ---- F = L^T R, columns 2t, 2t + 1 ----------------------------------------
+#pragma unroll
+  for (int r = 0; r < H; ++r) F0[r] = F1[r] = 0.0;
+#pragma unroll 1
+  for (int k = 0; k < H; ++k) {
+    const double r0 = Rs[k * LDM + 2 * t], r1 = Rs[k * LDM + 2 * t + 1];
+    const double2* l2 = reinterpret_cast<const double2*>(Ls + k * LDM);
+#pragma unroll
+    for (int r = 0; r < H; r += 2) {
+      const double2 v = l2[r / 2];
+      F0[r] = fma(v.x, r0, F0[r]);
+      F0[r + 1] = fma(v.y, r0, F0[r + 1]);
+      F1[r] = fma(v.x, r1, F1[r]);
+      F1[r + 1] = fma(v.y, r1, F1[r + 1]);
+    }
+  }
+  // ---- one-sided Jacobi -------------------------------------------------------
+  auto dot = [](const double* x, const double* y) {
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+#pragma unroll
+    for (int r = 0; r < H; r += 4) {
+      s0 = fma(x[r], y[r], s0);
+      s1 = fma(x[r + 1], y[r + 1], s1);
+      s2 = fma(x[r + 2], y[r + 2], s2);
+      s3 = fma(x[r + 3], y[r + 3], s3);
+    }
+    return (s0 + s1) + (s2 + s3);
+  };
+  bool live = act && regular;
+  const bool last = t == TEAM - 1;
+#pragma unroll 1
+  for (int sweep = 0; sweep < 20; ++sweep) {
+    double n0 = dot(F0, F0), n1 = dot(F1, F1);
+    bool more = false;
+#pragma unroll 1
+    for (int rd = 0; rd < H; rd += 2) {
+      {  // even round: the lane's own pair, changing places
+        bool far;
+        const double g = dot(F0, F1);
+        const double tn = jacobi_tan(g, n0, n1, far);
+        more = more || far;
+        const double cc = rsqrt_near1(fma(tn, tn, 1.0));
+        const double c = live ? cc : 0.0, s = live ? tn * cc : 1.0;
+        const double q0 = n0, q1 = n1;
+        n1 = live ? fma(-tn, g, q0) : q1;
+        n0 = live ? fma(tn, g, q1) : q0;
+#pragma unroll
+        for (int r = 0; r < H; ++r) {
+          const double x = F0[r], y = F1[r];
+          F1[r] = fma(c, x, -(s * y));
+          F0[r] = fma(s, x, c * y);
+        }
+      }
+      {  // odd round: the second column with the next lane's first, changing places
+        double G[H];
+#pragma unroll
+        for (int r = 0; r < H; ++r) G[r] = __shfl_down_sync(msk, F0[r], 1, TEAM);
+        const double ng = __shfl_down_sync(msk, n0, 1, TEAM);
+        bool far;
+        const double g = dot(F1, G);
+        const double tn = jacobi_tan(g, n1, ng, far);
+        const bool rot = live && !last;
+        more = more || (far && !last);
+        const double cc = rsqrt_near1(fma(tn, tn, 1.0));
+        const double c = rot ? cc : 0.0, s = rot ? tn * cc : 1.0;
+        const double qn = rot ? fma(-tn, g, n1) : ng;  // squared norm of the column handed on
+        n1 = rot ? fma(tn, g, ng) : n1;
+#pragma unroll
+        for (int r = 0; r < H; ++r) {
+          const double x = F1[r], y = G[r];
+          G[r] = fma(c, x, -(s * y));
+          F1[r] = fma(s, x, c * y);
+          const double back = __shfl_up_sync(msk, G[r], 1, TEAM);
+          F0[r] = t == 0 ? F0[r] : back;
+        }
+        const double nb = __shfl_up_sync(msk, qn, 1, TEAM);
+        n0 = t == 0 ? n0 : nb;
+      }
+    }
+    // the task's verdict is the team's
+    const unsigned tm = __ballot_sync(msk, live && more);
+    const unsigned team_bits = (TEAM == 32 ? 0xffffffffu : ((1u << TEAM) - 1u)) << (threadIdx.x & 31u & ~(unsigned)(TEAM - 1));
+    live = live && (tm & team_bits) != 0u;
+    if (!__any_sync(msk, live)) break;
+  }
+  double k0 = dot(F0, F0), k1 = dot(F1, F1);
+  {
+    const double r0 = k0 > 0.0 ? rsqrt(k0) : 0.0, r1 = k1 > 0.0 ? rsqrt(k1) : 0.0;
+    k0 = fmax(k0 * r0, 1e-9);
+    k1 = fmax(k1 * r1, 1e-9);
+#pragma unroll
+    for (int r = 0; r < H; ++r) {
+      F0[r] *= r0;
+      F1[r] *= r1;
+    }
+  }
+  // lambda = k^2 negative: -A_s (na) or -B_s (nb) indefinite; see flux_eigen_kernel
+  bool na0 = false, na1 = false, nb0 = false, nb1 = false;
+  if (__any_sync(msk, act && !regular)) {
+    if (act && !regular) {
+      double* const scr = p.bvp_rec + mode_row<GEN>() * p.g.ms_bvp + task * brec_stride(N);  // dead until the boundary-value kernel
+      if (t == 0)
+        team_indefinite<H, LDM>(gl, Y, tab, N, m, okb, Ls, scr, scr + 2 * H * H, scr + 3 * H * H);
+      __threadfence_block();
+    }
+    __syncwarp(msk);
+    if (act && !regular) {
+      const double* const scr = p.bvp_rec + mode_row<GEN>() * p.g.ms_bvp + task * brec_stride(N);
+      const double *V = scr + 2 * H * H, *d = scr + 3 * H * H;
+      const double d0 = d[2 * t], d1 = d[2 * t + 1];
+      k0 = mode_k(d0);
+      k1 = mode_k(d1);
+      na0 = okb && d0 < 0.0;
+      na1 = okb && d1 < 0.0;
+      nb0 = !okb && d0 < 0.0;
+      nb1 = !okb && d1 < 0.0;
+#pragma unroll
+      for (int r = 0; r < H; ++r) {
+        F0[r] = V[(2 * t) * H + r];
+        F1[r] = V[(2 * t + 1) * H + r];
+      }
+    }
+    __syncwarp(msk);
+  }
+  const bool primary = okb;  // L factors -B_s
+  // ---- x = L u / sqrt(k) (primary; else sqrt(k) L u / k) and its sums ----------
+  const double rs0 = rsqrt(k0), rs1 = rsqrt(k1), sk0 = k0 * rs0, sk1 = k1 * rs1;
+  // sums of the form with L u (lu) and with L^{-T} u (li): with b1, b2 and D M^{-1} 1
+  double lu_b[2] = {0.0, 0.0}, li_b[2] = {0.0, 0.0}, lu_e[2] = {0.0, 0.0}, li_e[2] = {0.0, 0.0};
+  const double* const blu = primary ? b1 : b2;  // X goes with b1, Y with b2
+  const double* const bli = primary ? b2 : b1;
+  double* const outlu = q.lrec + (primary ? mod_X(N) : mod_Y(N));
+  double* const outli = q.lrec + (primary ? mod_Y(N) : mod_X(N));
+#pragma unroll 1
+  for (int r = 0; r < H; ++r) {
+    const double2* l2 = reinterpret_cast<const double2*>(Ls + r * LDM);
+    double a0 = 0.0, a1 = 0.0, c0 = 0.0, c1 = 0.0;
+#pragma unroll
+    for (int e = 0; e < H; e += 2) {
+      const double2 v = l2[e / 2];
+      a0 = fma(v.x, F0[e], a0);
+      c0 = fma(v.y, F0[e + 1], c0);
+      a1 = fma(v.x, F1[e], a1);
+      c1 = fma(v.y, F1[e + 1], c1);
+    }
+    const double x0 = (a0 + c0) * rs0, x1 = (a1 + c1) * rs1;
+    Rs[(2 * t) * LDM + r] = x0;
+    Rs[(2 * t + 1) * LDM + r] = x1;
+    lu_b[0] = fma(x0, blu[r], lu_b[0]);
+    lu_b[1] = fma(x1, blu[r], lu_b[1]);
+    lu_e[0] = fma(x0, ev[r], lu_e[0]);
+    lu_e[1] = fma(x1, ev[r], lu_e[1]);
+  }
+  __syncwarp(msk);
+  if (act)
+    for (int e = t; e < H * H / 2; e += TEAM) {
+      const int c = e / (H / 2), r = 2 * (e % (H / 2));
+      *reinterpret_cast<double2*>(outlu + c * H + r) = *reinterpret_cast<const double2*>(Rs + c * LDM + r);
+    }
+  __syncwarp(msk);
+  // ---- L^{-T} u sqrt(k): back substitution, fully unrolled ----------------------
+#pragma unroll
+  for (int e = H - 1; e >= 0; --e) {
+    const double2* l2 = reinterpret_cast<const double2*>(Ls + e * LDM);
+    const double rd = rcp_newton(Ls[e * LDM + e]);
+    const double y0 = F0[e] * rd, y1 = F1[e] * rd;
+#pragma unroll
+    for (int r = 0; r < e; r += 2) {
+      const double2 v = l2[r / 2];
+      F0[r] = fma(-v.x, y0, F0[r]);
+      F1[r] = fma(-v.x, y1, F1[r]);
+      if (r + 1 < e) {
+        F0[r + 1] = fma(-v.y, y0, F0[r + 1]);
+        F1[r + 1] = fma(-v.y, y1, F1[r + 1]);
+      }
+    }
+    const double z0 = y0 * sk0, z1 = y1 * sk1;
+    Rs[(2 * t) * LDM + e] = z0;
+    Rs[(2 * t + 1) * LDM + e] = z1;
+    li_b[0] = fma(z0, bli[e], li_b[0]);
+    li_b[1] = fma(z1, bli[e], li_b[1]);
+    li_e[0] = fma(z0, ev[e], li_e[0]);
+    li_e[1] = fma(z1, ev[e], li_e[1]);
+  }
+  __syncwarp(msk);
+  if (!act) return;
+  for (int e = t; e < H * H / 2; e += TEAM) {
+    const int c = e / (H / 2), r = 2 * (e % (H / 2));
+    *reinterpret_cast<double2*>(outli + c * H + r) = *reinterpret_cast<const double2*>(Rs + c * LDM + r);
+  }
+  // ---- k, E, F and the particular solutions --------------------------------------
+  double umu0 = q.rec[H_UMU0];
+  if (beam) {
+    const bool res = beam_resonant(k0, umu0) || beam_resonant(k1, umu0);
+    const unsigned tmask = team_mask<TEAM>();
+    if (__any_sync(tmask, res)) umu0 = 0.999 * umu0;
+  }
+  const double dts = q.rec[q.il.dtau_s + q.lc], r0 = beam ? 1.0 / umu0 : 0.0;
+  const bool thermal = (p.flags & DSP_FLAG_THERMAL) && m == 0;
+#pragma unroll
+  for (int v = 0; v < 2; ++v) {
+    const int c = 2 * t + v;
+    const double k = v ? k1 : k0;
+    const bool na = v ? na1 : na0, nb = v ? nb1 : nb0;
+    const double ka = na ? -k : k, kb = nb ? -k : k;
+    const double em = expm1(-kb * dts);  // E - 1; 1 - E^2 = -em (2 + em)
+    q.lrec[mod_k(N) + c] = kb;
+    q.lrec[mod_E(N) + c] = 1.0 + em;
+    q.lrec[mod_F(N) + c] = -em * (2.0 + em);
+    if (beam) {
+      if (GEN && (p.flags & DSP_FLAG_SPHERICAL_BEAM)) {
+        // pseudo-spherical beam: the raw source at the quadrature angles (DisortSolver.cpp:1524-1527)
+        const double dm = 0.5 / ev[c];
+        q.lrec[mod_cb(N) + c] = dm * (b1[c] + b2[c]);
+        q.lrec[mod_db(N) + c] = dm * (b1[c] - b2[c]);
+      } else {
+        const double al = primary ? lu_b[v] : li_b[v], be = primary ? li_b[v] : lu_b[v];
+        const double den = ka * kb - r0 * r0;
+        q.lrec[mod_cb(N) + c] = (kb * al - be * r0) / den;
+        q.lrec[mod_db(N) + c] = (ka * be - al * r0) / den;
+      }
+    }
+    if (thermal) {
+      const double ct = 2.0 * (1.0 - ws) * (primary ? lu_e[v] : li_e[v]) / ka;
+      q.lrec[mod_ct(N) + c] = ct;
+      q.lrec[mod_dt(N) + c] = ct / kb;
+    }
+  }
+  if (thermal && t == 0) thermal_source(q, q.lrec[mod_xr(N)], q.lrec[mod_xr(N) + 1]);
+}
+
 // Host side of the layer stage: launches (through `wrap(kind, launch)`, which may
 // time them; kind 0: front, 1: eigensolver, 2: team kernel) the two launches of a split stage or the team kernel; `host_tab` is a
 // host copy of the (mode's) tab_* tables of N.
 template <int N, bool GEN = false>
 inline void flux_layer_set_attrs() {
-  using C = LCfg<N>;
   if constexpr (layer_split<N>()) {
     static_assert(Handoff<N / 2>::HS <= brec_stride(N), "the hand-off must fit in the boundary-value records");
     cudaFuncSetAttribute(flux_eigen_kernel<N, GEN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)ECfg<N>::smem_bytes(128));
   }
-  // the team kernel serves every N of the flux path (N <= 16: when a schedule asks for it)
-  if constexpr (!GEN || !layer_split<N>())
-    cudaFuncSetAttribute(flux_layer_kernel<N, GEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem_bytes());
+  // the team kernel: N <= 16 on the flux path, when a schedule asks for it
+  if constexpr (!GEN && layer_split<N>())
+    cudaFuncSetAttribute(flux_layer_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LCfg<N>::smem_bytes());
+  if constexpr (!layer_split<N>())
+    cudaFuncSetAttribute(flux_layer_warp_kernel<N, GEN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)WCfg<N>::smem_bytes());
 }
 
-// The layer stage of `tasks` layer tasks (of each of `modes` azimuth modes).  split: one thread per task (N <= 16
+// The layer stage of `tasks` layer tasks (of each of `modes` azimuth modes).  N >= 32:
+// the warp kernel.  split: one thread per task (N <= 16
 // only), with `cta` threads per CTA (64 or 128); otherwise the team kernel.
 template <int N, bool GEN = false, class Wrap>
 inline void flux_layer_launch(const FluxParams& p, long long tasks, const double* host_tab, cudaStream_t s,
                               Wrap&& wrap, bool split = layer_split<N>(), int cta = 128, int modes = 1) {
-  using C = LCfg<N>;
   if constexpr (layer_split<N>()) {
     if (split || GEN) {
       const int b = cta == 64 ? 64 : 128;
@@ -1240,10 +1727,15 @@ inline void flux_layer_launch(const FluxParams& p, long long tasks, const double
       wrap(1, [&] { flux_eigen_kernel<N, GEN><<<g, b, ECfg<N>::smem_bytes(b), s>>>(p, tc); });
       return;
     }
-  }
-  if constexpr (!GEN || !layer_split<N>()) {
-    const dim3 grid((unsigned)((tasks + C::TPC - 1) / C::TPC), (unsigned)modes);
-    wrap(2, [&] { flux_layer_kernel<N, GEN><<<grid, C::CTA, C::smem_bytes(), s>>>(p); });
+    if constexpr (!GEN) {
+      using C = LCfg<N>;
+      const unsigned grid = (unsigned)((tasks + C::TPC - 1) / C::TPC);
+      wrap(2, [&] { flux_layer_kernel<N><<<grid, C::CTA, C::smem_bytes(), s>>>(p); });
+    }
+  } else {
+    using C = WCfg<N>;
+    const dim3 grid((unsigned)((tasks + C::TPW - 1) / C::TPW), (unsigned)modes);
+    wrap(2, [&] { flux_layer_warp_kernel<N, GEN><<<grid, 32, C::smem_bytes(), s>>>(p); });
   }
 }
 
