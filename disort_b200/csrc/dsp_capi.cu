@@ -216,6 +216,10 @@ dsp_status dsp_context_destroy(dsp_context ctx) {
   if (ctx->s_in) cudaStreamDestroy(ctx->s_in);
   if (ctx->s_out) cudaStreamDestroy(ctx->s_out);
   if (ctx->s_c2) cudaStreamDestroy(ctx->s_c2);
+  for (auto& b : ctx->pin) {
+    if (b.p) cudaFreeHost(b.p);
+    if (b.ev) cudaEventDestroy(b.ev);
+  }
   if (ctx->ws) cudaFree(ctx->ws);
   if (ctx->stage_in) cudaFree(ctx->stage_in);
   if (ctx->stage_out) cudaFree(ctx->stage_out);
@@ -399,6 +403,11 @@ dsp_status flux_solve(dsp_context ctx, const dsp_flux_batch* batch_in, const dsp
   // ---- stage host inputs into device memory --------------------------------
   dsp_darray* arr = batch_arrays(&b);
   const double* host_in[kFluxArrays] = {};  // per-instance host arrays still to be copied
+  const size_t arr_bytes = ((size_t)n * nlev * sizeof(double) + 255) / 256 * 256;
+  const size_t jac_bytes = jac ? ((size_t)n * nlev * (L + 2) * sizeof(double) + 255) / 256 * 256 : 0;
+  const size_t st_bytes = ((size_t)n * sizeof(int32_t) + 255) / 256 * 256;
+  const size_t out_bytes = (dev ? 0 : 8 * arr_bytes + 6 * jac_bytes) + st_bytes;
+  bool small = false;  // a host batch that goes through pinned staging
   {
     size_t need = 0;
     for (int k = 0; k < kFluxArrays; ++k) {
@@ -410,6 +419,9 @@ dsp_status flux_solve(dsp_context ctx, const dsp_flux_batch* batch_in, const dsp
     }
     if ((st = ensure(ctx, &ctx->stage_in, &ctx->stage_in_bytes, need + 256, "input staging")) != DSP_OK) return st;
     char* cur = static_cast<char*>(ctx->stage_in);
+    small = !dev && need <= kSmallHostBytes && out_bytes <= kSmallHostBytes;
+    char* pin = nullptr;
+    if (small && (st = pin_acquire(ctx, 0, need, &pin)) != DSP_OK) return st;
     for (int k = 0; k < kFluxArrays; ++k) {
       if (!arr[k].ptr) {
         if (kScalarField[k]) {  // absent scalar: the DisortFluxConfig default
@@ -420,7 +432,9 @@ dsp_status flux_solve(dsp_context ctx, const dsp_flux_batch* batch_in, const dsp
       }
       if (dev) continue;
       const size_t elems = arr[k].stride == 0 ? (size_t)cnt[k] : (size_t)((n - 1) * arr[k].stride + cnt[k]);
-      if (arr[k].stride == 0) {  // shared by every instance: copied now
+      if (small) {
+        std::memcpy(pin + (cur - static_cast<char*>(ctx->stage_in)), arr[k].ptr, elems * sizeof(double));
+      } else if (arr[k].stride == 0) {  // shared by every instance: copied now
         e = cudaMemcpyAsync(cur, arr[k].ptr, elems * sizeof(double), cudaMemcpyHostToDevice, s);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMemcpyAsync(input)");
       } else {  // per instance: copied piece by piece below
@@ -428,6 +442,11 @@ dsp_status flux_solve(dsp_context ctx, const dsp_flux_batch* batch_in, const dsp
       }
       arr[k].ptr = reinterpret_cast<const double*>(cur);
       cur += ((elems * sizeof(double) + 255) / 256) * 256;
+    }
+    if (small) {
+      e = cudaMemcpyAsync(ctx->stage_in, pin, need, cudaMemcpyHostToDevice, s);
+      if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMemcpyAsync(input)");
+      pin_mark(ctx, 0, s);
     }
   }
   // ---- outputs -----------------------------------------------------------
@@ -444,11 +463,7 @@ dsp_status flux_solve(dsp_context ctx, const dsp_flux_batch* batch_in, const dsp
                            out->mean_intensity_direct_beam};
     for (int f = 0; f < 8; ++f)
       if (!host_out[f]) return fail(ctx, DSP_ERR_INVALID_INPUT, "every output array is required");
-    const size_t arr_bytes = ((size_t)n * nlev * sizeof(double) + 255) / 256 * 256;
-    const size_t jac_bytes = jac ? ((size_t)n * nlev * ndof * sizeof(double) + 255) / 256 * 256 : 0;
-    const size_t st_bytes = ((size_t)n * sizeof(int32_t) + 255) / 256 * 256;
-    const size_t need = (dev ? 0 : 8 * arr_bytes + 6 * jac_bytes) + st_bytes;
-    if ((st = ensure(ctx, &ctx->stage_out, &ctx->stage_out_bytes, need, "output staging")) != DSP_OK) return st;
+    if ((st = ensure(ctx, &ctx->stage_out, &ctx->stage_out_bytes, out_bytes, "output staging")) != DSP_OK) return st;
     char* cur = static_cast<char*>(ctx->stage_out);
     for (int f = 0; f < 8; ++f) {
       if (dev) dout[f] = host_out[f];
@@ -486,10 +501,7 @@ dsp_status flux_solve(dsp_context ctx, const dsp_flux_batch* batch_in, const dsp
   const size_t sph_d = spherical ? (size_t)L * sph_stride(N) : 0;
   sz.bvp += jcv_d + sph_d;
   const size_t inst_doubles = sz.inst + sz.layer + sz.bvp;
-  size_t budget = workspace_budget();
-  size_t freeb = 0, totalb = 0;
-  if (cudaMemGetInfo(&freeb, &totalb) == cudaSuccess && freeb / 2 < budget + ctx->ws_bytes)
-    budget = (freeb + ctx->ws_bytes) / 2;
+  const size_t budget = call_budget(ctx, (size_t)n * sz.per_inst_bytes());
   int64_t chunk = (int64_t)(budget / sz.per_inst_bytes());
   if (chunk < 1) chunk = 1;
   if (chunk > n) chunk = n;
@@ -553,6 +565,24 @@ dsp_status flux_solve(dsp_context ctx, const dsp_flux_batch* batch_in, const dsp
     const size_t ws_need = (size_t)chunk * inst_doubles * sizeof(double) + 1024;
     if ((st = ensure(ctx, &ctx->ws, &ctx->ws_bytes, ws_need, "workspace")) != DSP_OK) return st;
     return run_range(0, n, s, static_cast<double*>(ctx->ws), chunk);
+  }
+  if (small) {  // one copy each way, the outputs laid out as in the staging area
+    const size_t ws_need = (size_t)chunk * inst_doubles * sizeof(double) + 1024;
+    if ((st = ensure(ctx, &ctx->ws, &ctx->ws_bytes, ws_need, "workspace")) != DSP_OK) return st;
+    if ((st = run_range(0, n, s, static_cast<double*>(ctx->ws), chunk)) != DSP_OK) return st;
+    char* pin = nullptr;
+    if ((st = pin_acquire(ctx, 1, out_bytes, &pin)) != DSP_OK) return st;
+    e = cudaMemcpyAsync(pin, ctx->stage_out, out_bytes, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "flux solve");
+    auto at = [&](const void* dp) { return pin + (static_cast<const char*>(dp) - static_cast<char*>(ctx->stage_out)); };
+    double* const ho[8] = {out->flux_direct_beam, out->flux_down, out->flux_up, out->flux_tau_divergence,
+                           out->mean_intensity, out->mean_intensity_down, out->mean_intensity_up,
+                           out->mean_intensity_direct_beam};
+    for (int f = 0; f < 8; ++f) std::memcpy(ho[f], at(dout[f]), (size_t)n * nlev * sizeof(double));
+    for (int f = 0; f < 6 && jac; ++f) std::memcpy(hjac[f], at(djac[f]), (size_t)n * nlev * ndof * sizeof(double));
+    if (out->status) std::memcpy(out->status, at(dstatus), (size_t)n * sizeof(int32_t));
+    return DSP_OK;
   }
 
   // ---- host buffers: copies overlapped with the solves ----------------------

@@ -620,9 +620,14 @@ dsp_status general_solve(dsp_context ctx, const dsp_general_batch* bin, const ds
       need += (!sc[k]->ptr) ? 256 : (dev ? 0 : align256(darray_elems(*sc[k], 1) * sizeof(double)));
     if ((st = ensure(ctx, &ctx->stage_in, &ctx->stage_in_bytes, need + 256, "input staging")) != DSP_OK) return st;
     char* cur = static_cast<char*>(ctx->stage_in);
+    // small inputs go through pinned staging with one copy
+    const bool pack = need <= kSmallHostBytes;
+    char* pin = nullptr;
+    if (pack && (st = pin_acquire(ctx, 0, need, &pin)) != DSP_OK) return st;
     auto put = [&](const void* src, size_t bytes) -> const void* {
       void* dst = cur;
-      if (bytes) e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
+      if (pack) std::memcpy(pin + (cur - static_cast<char*>(ctx->stage_in)), src, bytes);
+      else if (bytes) e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
       cur += align256(bytes);
       return dst;
     };
@@ -674,6 +679,10 @@ dsp_status general_solve(dsp_context ctx, const dsp_general_batch* bin, const ds
         dsc[k].ptr = static_cast<const double*>(put(sc[k]->ptr, darray_elems(*sc[k], 1) * sizeof(double)));
       }
     }
+    if (pack && cur > static_cast<char*>(ctx->stage_in)) {
+      e = cudaMemcpyAsync(ctx->stage_in, pin, cur - static_cast<char*>(ctx->stage_in), cudaMemcpyHostToDevice, s);
+      pin_mark(ctx, 0, s);
+    }
     if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMemcpyAsync(input)");
   }
 
@@ -690,6 +699,7 @@ dsp_status general_solve(dsp_context ctx, const dsp_general_batch* bin, const ds
   double* const hjac[6] = {jac ? jac->flux_up : nullptr, jac ? jac->flux_down : nullptr,
                            jac ? jac->mean_intensity : nullptr, jac ? jac->mean_intensity_down : nullptr,
                            jac ? jac->mean_intensity_up : nullptr, jac ? jac->flux_divergence : nullptr};
+  size_t out_bytes = 0;  // staging area up to the end of the status
   {
     const size_t need = (dev ? 0 : 8 * align256(flux_elems * 8) + align256(int_elems * 8) + align256(iavg_elems * 8) +
                                        6 * align256(jac_elems * 8)) +
@@ -721,14 +731,19 @@ dsp_status general_solve(dsp_context ctx, const dsp_general_batch* bin, const ds
     }
     dstatus = (dev && out->status) ? out->status : reinterpret_cast<int32_t*>(cur);
     cur += align256(n * sizeof(int32_t));
+    out_bytes = cur - static_cast<char*>(ctx->stage_out);
     double** dfp = reinterpret_cast<double**>(cur);
     cur += align256(8 * sizeof(double*));
     int32_t* dskip = reinterpret_cast<int32_t*>(cur);
-    e = cudaMemcpyAsync(dfp, dflux, sizeof(dflux), cudaMemcpyHostToDevice, s);
-    for (int f = 0; f < 8 && e == cudaSuccess; ++f) e = cudaMemsetAsync(dflux[f], 0, flux_elems * 8, s);
-    if (e == cudaSuccess && dint) e = cudaMemsetAsync(dint, 0, int_elems * 8, s);
-    if (e == cudaSuccess && diavg) e = cudaMemsetAsync(diavg, 0, iavg_elems * 8, s);
-    for (int f = 0; f < 6 && jac && e == cudaSuccess; ++f) e = cudaMemsetAsync(djac[f], 0, jac_elems * 8, s);
+    if (dev) {
+      for (int f = 0; f < 8 && e == cudaSuccess; ++f) e = cudaMemsetAsync(dflux[f], 0, flux_elems * 8, s);
+      if (e == cudaSuccess && dint) e = cudaMemsetAsync(dint, 0, int_elems * 8, s);
+      if (e == cudaSuccess && diavg) e = cudaMemsetAsync(diavg, 0, iavg_elems * 8, s);
+      for (int f = 0; f < 6 && jac && e == cudaSuccess; ++f) e = cudaMemsetAsync(djac[f], 0, jac_elems * 8, s);
+      if (e == cudaSuccess) e = cudaMemsetAsync(dstatus, 0, n * sizeof(int32_t), s);
+    } else {
+      e = cudaMemsetAsync(ctx->stage_out, 0, out_bytes, s);
+    }
     if (e != cudaSuccess) return cuda_fail(ctx, e, "output initialisation");
 
     // status: 0, or the verdict on instances no kernel takes
@@ -739,9 +754,12 @@ dsp_status general_solve(dsp_context ctx, const dsp_general_batch* bin, const ds
       else if (!supported_nstr(hN[i])) hst[i] = DSP_ERR_UNSUPPORTED;
       if (hst[i]) skip.push_back(i);
     }
-    e = cudaMemcpyAsync(dstatus, hst.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // hst leaves scope
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "status initialisation");
+    if (!skip.empty()) {
+      e = cudaMemcpyAsync(dfp, dflux, sizeof(dflux), cudaMemcpyHostToDevice, s);
+      if (e == cudaSuccess) e = cudaMemcpyAsync(dstatus, hst.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, s);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // hst leaves scope
+      if (e != cudaSuccess) return cuda_fail(ctx, e, "status initialisation");
+    }
     if (!skip.empty()) {
       e = cudaMemcpyAsync(dskip, skip.data(), skip.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s);
       if (e == cudaSuccess) {
@@ -771,11 +789,11 @@ dsp_status general_solve(dsp_context ctx, const dsp_general_batch* bin, const ds
   };
   std::vector<Chunk> chunks;
   size_t budget = workspace_budget();
-  {
-    size_t freeb = 0, totalb = 0;
-    if (cudaMemGetInfo(&freeb, &totalb) == cudaSuccess && freeb / 2 < budget + ctx->ws_bytes)
-      budget = (freeb + ctx->ws_bytes) / 2;
-  }
+  // (planned within the configured budget; when that would have the workspace grow,
+  // the free memory is queried and the plan made again within what it allows)
+  bool queried = false;
+plan:
+  chunks.clear();
   const double* h_fbeam = (!dev && b.direct_beam_flux.ptr) ? b.direct_beam_flux.ptr : nullptr;
   const double* h_umu0 = (!dev && b.direct_beam_mu.ptr) ? b.direct_beam_mu.ptr : nullptr;
   const double* h_mu = (!dev && user_mu) ? b.mu_user.ptr : nullptr;
@@ -854,6 +872,17 @@ dsp_status general_solve(dsp_context ctx, const dsp_general_batch* bin, const ds
     c.batch = (int)std::max<int64_t>(1, std::min<int64_t>(mb, c.maxm + 1));
   }
   if (chunks.empty()) goto copy_back;
+  if (!queried) {
+    size_t most = 0;
+    for (const Chunk& c : chunks)
+      most = std::max(most, (size_t)(fixed_doubles(c) + c.batch * mode_doubles(c)) * sizeof(double));
+    const size_t allowed = call_budget(ctx, most + 1024);
+    queried = true;
+    if (allowed < budget) {
+      budget = allowed;
+      goto plan;
+    }
+  }
   // the size-class queue of each chunk the schedule runs persistently
   for (Chunk& c : chunks) {
     const int meanL = c.ids.empty() ? 0 : (int)(c.layers / (int64_t)c.ids.size());
@@ -874,7 +903,9 @@ dsp_status general_solve(dsp_context ctx, const dsp_general_batch* bin, const ds
     }
     if ((st = ensure(ctx, &ctx->meta, &ctx->meta_bytes, meta_need, "chunk index")) != DSP_OK) return st;
     if ((st = ensure(ctx, &ctx->ws, &ctx->ws_bytes, ws_need + 1024, "workspace")) != DSP_OK) return st;
-    std::vector<char> hmeta(meta_need);
+    // built in pinned staging: no wait for its copy
+    char* hmeta = nullptr;
+    if ((st = pin_acquire(ctx, 0, meta_need, &hmeta)) != DSP_OK) return st;
     std::vector<size_t> moff(chunks.size());
     {
       size_t o = 0;
@@ -882,23 +913,24 @@ dsp_status general_solve(dsp_context ctx, const dsp_general_batch* bin, const ds
         const Chunk& c = chunks[k];
         moff[k] = o;
         const size_t nc = c.ids.size();
-        std::memcpy(hmeta.data() + o, c.ids.data(), nc * 4);
+        std::memcpy(hmeta + o, c.ids.data(), nc * 4);
         o += align256(nc * 4);
-        std::memcpy(hmeta.data() + o, c.inst_off.data(), nc * 8);
+        std::memcpy(hmeta + o, c.inst_off.data(), nc * 8);
         o += align256(nc * 8);
-        std::memcpy(hmeta.data() + o, c.lay_off.data(), (nc + 1) * 8);
+        std::memcpy(hmeta + o, c.lay_off.data(), (nc + 1) * 8);
         o += align256((nc + 1) * 8);
-        int32_t* li = reinterpret_cast<int32_t*>(hmeta.data() + o);
+        int32_t* li = reinterpret_cast<int32_t*>(hmeta + o);
         for (size_t ci = 0; ci < nc; ++ci)
           for (int64_t l = c.lay_off[ci]; l < c.lay_off[ci + 1]; ++l) li[l] = (int32_t)ci;
         o += align256(c.layers * 4);
-        if (!c.order.empty()) std::memcpy(hmeta.data() + o, c.order.data(), c.order.size() * 4);
+        if (!c.order.empty()) std::memcpy(hmeta + o, c.order.data(), c.order.size() * 4);
         o += align256(c.order.size() * 4);
-        o += align256((c.maxm + 1) * 4);  // queue counters, one per mode, zero
+        std::memset(hmeta + o, 0, (c.maxm + 1) * 4);  // queue counters, one per mode
+        o += align256((c.maxm + 1) * 4);
       }
     }
-    e = cudaMemcpyAsync(ctx->meta, hmeta.data(), meta_need, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // hmeta leaves scope
+    e = cudaMemcpyAsync(ctx->meta, hmeta, meta_need, cudaMemcpyHostToDevice, s);
+    pin_mark(ctx, 0, s);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "chunk index upload");
 
     FluxParams p;
@@ -1009,6 +1041,22 @@ dsp_status general_solve(dsp_context ctx, const dsp_general_batch* bin, const ds
 
 copy_back:
   if (dev) return DSP_OK;
+  if (out_bytes <= kSmallHostBytes) {  // one copy through pinned staging
+    char* pin = nullptr;
+    if ((st = pin_acquire(ctx, 1, out_bytes, &pin)) != DSP_OK) return st;
+    e = cudaMemcpyAsync(pin, ctx->stage_out, out_bytes, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "general solve");
+    auto get = [&](void* dst, const void* dp, size_t bytes) {
+      std::memcpy(dst, pin + (static_cast<const char*>(dp) - static_cast<char*>(ctx->stage_out)), bytes);
+    };
+    for (int f = 0; f < 8; ++f) get(out->flux[f], dflux[f], flux_elems * 8);
+    if (dint) get(out->intensity, dint, int_elems * 8);
+    if (diavg) get(out->intensity_azimuth_avg, diavg, iavg_elems * 8);
+    for (int f = 0; f < 6 && jac; ++f) get(hjac[f], djac[f], jac_elems * 8);
+    if (out->status) get(out->status, dstatus, n * sizeof(int32_t));
+    return DSP_OK;
+  }
   for (int f = 0; f < 8; ++f) {
     e = cudaMemcpyAsync(out->flux[f], dflux[f], flux_elems * 8, cudaMemcpyDeviceToHost, s);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMemcpyAsync(output)");

@@ -42,6 +42,14 @@ struct dsp_context_s {
   void* meta = nullptr;                // general solver: chunk index arrays
   double* flux_defaults = nullptr;     // defaults of absent flux-batch scalars (device, uploaded once)
   size_t meta_bytes = 0;
+  // small host-buffer solves: pinned staging, [0] on the way in (also the general
+  // solver's chunk index), [1] on the way out; `ev` marks its last copy
+  struct Pinned {
+    void* p = nullptr;
+    size_t bytes = 0;
+    cudaEvent_t ev = nullptr;
+    bool busy = false;
+  } pin[2];
   // host-buffer solves: copy streams and events of the copy/compute pipeline
   cudaStream_t s_in = nullptr, s_out = nullptr;
   cudaStream_t s_c2 = nullptr;  // second solve stream of the host-buffer pipeline
@@ -172,6 +180,56 @@ inline dsp_status ensure(dsp_context ctx, void** buf, size_t* have, size_t need,
   }
   *have = alloc;
   return DSP_OK;
+}
+
+// Host batches whose inputs and outputs are each at most this go through pinned
+// staging with one copy each way: a copy of a few KB from the caller's pageable
+// arrays costs 5-8 us apiece whatever its size, and a call has 20 to 30 of them;
+// above, packing on the host costs more than it saves.
+inline constexpr size_t kSmallHostBytes = size_t(512) << 10;
+
+// The pinned buffer k of the context, at least `need` bytes, its last copy done.
+inline dsp_status pin_acquire(dsp_context ctx, int k, size_t need, char** out) {
+  dsp_context_s::Pinned& b = ctx->pin[k];
+  if (b.busy) {
+    cudaEventSynchronize(b.ev);
+    b.busy = false;
+  }
+  if (b.bytes < need) {
+    if (b.p) cudaFreeHost(b.p);
+    b.p = nullptr;
+    b.bytes = 0;
+    const size_t alloc = need + need / 4 + 4096;
+    if (cudaHostAlloc(&b.p, alloc, cudaHostAllocDefault) != cudaSuccess) {
+      cudaGetLastError();
+      b.p = nullptr;
+      return fail(ctx, DSP_ERR_NO_MEMORY, "pinned staging allocation failed");
+    }
+    b.bytes = alloc;
+  }
+  if (!b.ev && cudaEventCreateWithFlags(&b.ev, cudaEventDisableTiming) != cudaSuccess)
+    return fail(ctx, DSP_ERR_CUDA, "pinned staging event");
+  *out = static_cast<char*>(b.p);
+  return DSP_OK;
+}
+// Marks the buffer in use until the work queued on `s` so far is done.
+inline void pin_mark(dsp_context ctx, int k, cudaStream_t s) {
+  cudaEventRecord(ctx->pin[k].ev, s);
+  ctx->pin[k].busy = true;
+}
+
+// Workspace bytes a call may use: the configured budget, or less when the device is
+// short of memory.  The query of the free memory (0.1-0.6 ms, more under load) is
+// only made when the call would have the workspace grow: `want` is what it takes
+// within the configured budget.
+inline size_t workspace_budget();
+inline size_t call_budget(dsp_context ctx, size_t want) {
+  size_t budget = workspace_budget();
+  if (std::min(want, budget) <= ctx->ws_bytes) return budget;
+  size_t freeb = 0, totalb = 0;
+  if (cudaMemGetInfo(&freeb, &totalb) == cudaSuccess && freeb / 2 < budget + ctx->ws_bytes)
+    budget = (freeb + ctx->ws_bytes) / 2;
+  return budget;
 }
 
 // Gauss-Legendre nodes/weights on (0,1) by Newton iteration (the reference's
