@@ -450,7 +450,9 @@ __global__ void __launch_bounds__(128) gen_intensity_kernel(FluxParams p) {
   const bool bres = fabs(bden) < 0.0001;
   const double rbden = bres ? 0.0 : 1.0 / bden;
   // lane j's share of the intensity, and the beam and thermal parts (every lane the same)
-  double acc = 0.0, accs = 0.0;
+  // (accr: the beam's part at an angle that resonates with mu0, where the reference's
+  // limit carries the attenuation of the output depth, DisortSolver.cpp:3010-3030)
+  double acc = 0.0, accs = 0.0, accr = 0.0;
   for (int s = 0; s < ncut; ++s) {
     const int l = neg ? s : ncut - 1 - s;
     const double* const lr = lrec0 + (long long)l * g.lstride;
@@ -481,17 +483,16 @@ __global__ void __launch_bounds__(128) gen_intensity_kernel(FluxParams p) {
         const double ut = utaus[lu];
         const double d = neg ? ut - t0 : t0 - ut;  // depth from the near side
         double v1 = acc, v2 = accs, ed = 1.0;
+        const double exp0 = beam ? exp(-ut * rmu0) : 0.0;
+        if (bres) v2 += accr * exp0;
         if (fabs(d) >= 1e-6) {
           ed = exp(-d * rnu);
           // the near mode at the depth (1 at the near side), the far mode there and
           // at the near side (wk)
           const double en = exp(-k * d), ef = exp(-k * (neg ? tb - ut : ut - tt));
           v1 = acc * ed + gn * (res ? d * rnu * ed : (en - ed) * rn) + gf * ((ef - wk * ed) * rf);
-          v2 = accs * ed;
-          if (beam) {
-            const double exp0 = exp(-ut * rmu0);
-            v2 += zb * (bres ? d * rmu0 * exp0 : (exp0 - (neg ? b0 : b1) * ed) * rbden);
-          }
+          v2 = fma(accs, ed, bres ? accr * exp0 : 0.0);
+          if (beam) v2 += zb * (bres ? d * rmu0 * exp0 : (exp0 - (neg ? b0 : b1) * ed) * rbden);
           if (thermal) v2 += z0 * (1.0 - ed) + z1 * ((ut + umv) - (t0 + umv) * ed);
         }
         const double dist = neg ? ut : taus[L] - ut;
@@ -503,7 +504,8 @@ __global__ void __launch_bounds__(128) gen_intensity_kernel(FluxParams p) {
     acc = acc * e + gn * (res ? dt * rnu * e : (wk - e) * rn) + gf * ((1.0 - wk * e) * rf);
     if (beam) {
       const double bn = neg ? b0 : b1, bf = neg ? b1 : b0;
-      accs = accs * e + zb * (bres ? dt * rmu0 * exp(-tb * rmu0) : (bf - bn * e) * rbden);
+      if (bres) accr = fma(zb, dt * rmu0, accr);
+      accs = accs * e + zb * ((bf - bn * e) * rbden);  // (rbden is 0 at resonance)
     } else {
       accs *= e;
     }
