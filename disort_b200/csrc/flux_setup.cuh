@@ -1,8 +1,10 @@
 // flux_setup.cuh — per-instance setup: validation, delta-M / delta-M+ scaling,
 // optical-depth scans, absorption cut, beam transmission and level Planck values.
 //
-// One warp per instance; lanes run over layers/levels, lane 0 does the scans in
-// the reference's sequential order so cumulative depths round identically.
+// One warp per instance; lanes run over layers/levels.  The cumulative depths are
+// summed in the reference's sequential order, so they round identically: the warp
+// stages 32 layers in shared memory and every lane runs the same short chain of
+// additions, keeping the sums at its own layer (setup_scan).
 #pragma once
 
 #include "dsp_device.cuh"
@@ -86,8 +88,66 @@ static __global__ void __launch_bounds__(256) hg_moments_kernel(DArr g, long lon
   out[t] = gk;
 }
 
+// Cumulative optical depths, the absorption cut and the beam transmission at the
+// level boundaries (disortSet, FluxSolver.cpp:312-331, 391-412, 429-435;
+// DisortSolver.cpp:749-790).  The sums form a serial chain of L additions; what
+// bounded the stage when lane 0 walked the layers was not that chain but a global
+// load, a store and a double-precision exponential and division per step behind
+// it.  Here the chain reads broadcasts from shared memory and all lanes do the
+// loads, stores and exponentials: 60,000 columns of 40 layers SETUP_A, one column
+// of 60 layers SETUP_B.  Entries of btr past the absorption cut stay zero, as on a
+// freshly constructed reference solver.  `st` is 96 doubles of the warp's own.
+struct SetupScan {
+  double total_abs;  // absorption optical depth of the column
+  int ncut;          // layers above the absorption cut
+};
+template <class FD, class FS>
+__device__ __forceinline__ SetupScan setup_scan(double* rec, const InstLayout& il, int L, double fbeam, double umu0,
+                                                double* st, int lane, const FD& dtau_at, const FS& ssa_at) {
+  constexpr double abscut = 10.0;
+  double tauc = 0.0, taus = 0.0, abstau = 0.0;
+  int ncut = L;
+  if (lane == 0) {
+    rec[il.tauc] = 0.0;
+    rec[il.tau_s] = 0.0;
+    rec[il.btr] = fbeam > 0.0 ? 1.0 : 0.0;
+  }
+  for (int l0 = 0; l0 < L; l0 += 32) {
+    const int lc = l0 + lane, nl = L - l0 < 32 ? L - l0 : 32;
+    __syncwarp();
+    if (lc < L) {
+      st[lane] = dtau_at(lc);
+      st[32 + lane] = 1.0 - ssa_at(lc);
+      st[64 + lane] = rec[il.dtau_s + lc];  // this lane's own store
+    }
+    __syncwarp();
+    double my_tauc = 0.0, my_taus = 0.0;
+    bool above = false;
+#pragma unroll 8
+    for (int j = 0; j < nl; ++j) {
+      const bool in = abstau < abscut;
+      if (in) ncut = l0 + j + 1;
+      abstau += st[32 + j] * st[j];
+      tauc += st[j];
+      taus += st[64 + j];  // without scaling the scaled depths are the depths
+      if (j == lane) {
+        my_tauc = tauc;
+        my_taus = taus;
+        above = in;
+      }
+    }
+    if (lc < L) {
+      rec[il.tauc + lc + 1] = my_tauc;
+      rec[il.tau_s + lc + 1] = my_taus;
+      rec[il.btr + lc + 1] = (fbeam > 0.0 && above) ? exp(-my_taus / umu0) : 0.0;
+    }
+  }
+  return {abstau, ncut};
+}
+
 // Four instances per 128-thread CTA, one warp each.
 static __global__ void __launch_bounds__(128) flux_setup_kernel(FluxParams p) {
+  __shared__ double stage[4][96];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i = blockIdx.x * 4 + warp;
   if (i >= p.n) return;
@@ -181,50 +241,31 @@ static __global__ void __launch_bounds__(128) flux_setup_kernel(FluxParams p) {
     rec[il.sig + lc] = sig;
     rec[il.mode + lc] = mode;
   }
-  // Planck at the levels (computeIsotropicSource, FluxSolver.cpp:748-752)
+  // Planck at the levels and the two boundaries (computeIsotropicSource, FluxSolver.cpp:748-752)
   if (thermal)
-    for (int lev = lane; lev <= L; lev += 32) rec[il.pkag + lev] = planck2(wlo, whi, temp_at(lev), p.pk);
+    for (int lev = lane; lev < L + 3; lev += 32) {
+      const double B = planck2(wlo, whi, lev <= L ? temp_at(lev) : lev == L + 1 ? ttop : tbot, p.pk);
+      if (lev <= L) rec[il.pkag + lev] = B;
+      else if (lev == L + 1) rec[H_PTOP] = B * emis;
+      else rec[H_PBOT] = B;
+    }
+
+  const SetupScan sc = setup_scan(rec, il, L, fbeam, umu0, stage[warp], lane, dtau_at, ssa_at);
   __syncwarp();
 
   if (lane == 0) {
-    // cumulative depths, absorption cut (FluxSolver.cpp:312-331, 429-435)
-    const double abscut = 10.0;
-    double tauc = 0.0, taus = 0.0, abstau = 0.0;
-    int ncut = L;
-    rec[il.tauc] = 0.0;
-    rec[il.tau_s] = 0.0;
-    for (int lc = 0; lc < L; ++lc) {
-      if (abstau < abscut) ncut = lc + 1;
-      abstau += (1.0 - ssa_at(lc)) * dtau_at(lc);
-      tauc = tauc + dtau_at(lc);
-      rec[il.tauc + lc + 1] = tauc;
-      if (!deltam && !dmplus) taus = tauc;
-      else taus = taus + rec[il.dtau_s + lc];
-      rec[il.tau_s + lc + 1] = taus;
-    }
-    // beam transmission for lc < ncut of the absorption loop (FluxSolver.cpp:391-412);
-    // later entries stay zero, as on a freshly constructed reference solver
-    for (int lev = 0; lev <= L; ++lev) rec[il.btr + lev] = 0.0;
-    if (fbeam > 0.0) {
-      rec[il.btr] = 1.0;
-      for (int lc = 0; lc < ncut; ++lc) rec[il.btr + lc + 1] = exp(-rec[il.tau_s + lc + 1] / umu0);
-    }
-    const bool lyrcut = (abstau >= abscut && !thermal && L > 1);
-    if (!lyrcut) ncut = L;
-    double ptop = 0.0, pbot = 0.0, pbotd = 0.0;
-    if (thermal) {
-      ptop = planck2(wlo, whi, ttop, p.pk) * emis;
-      pbot = planck2(wlo, whi, tbot, p.pk);
-      if (dlbc) {
-        const double bl = planck2(wlo, whi, temp_at(L - 1), p.pk);
-        const double dl = rec[il.dtau_s + L - 1];
-        if (dl > 0.0) pbotd = (pbot - bl) / dl;
-      }
+    const bool lyrcut = (sc.total_abs >= 10.0 && !thermal && L > 1);
+    const int ncut = lyrcut ? sc.ncut : L;
+    double pbotd = 0.0;
+    if (!thermal) {
+      rec[H_PTOP] = 0.0;
+      rec[H_PBOT] = 0.0;
+    } else if (dlbc) {
+      const double dl = rec[il.dtau_s + L - 1];
+      if (dl > 0.0) pbotd = (rec[H_PBOT] - rec[il.pkag + L - 1]) / dl;
     }
     rec[H_NCUT] = ncut;
     rec[H_LYRCUT] = lyrcut ? 1.0 : 0.0;
-    rec[H_PTOP] = ptop;
-    rec[H_PBOT] = pbot;
     rec[H_PBOTD] = pbotd;
     rec[H_DELTAM] = deltam ? 1.0 : 0.0;
     rec[H_DMPLUS] = dmplus ? 1.0 : 0.0;

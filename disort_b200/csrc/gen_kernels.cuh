@@ -17,6 +17,7 @@ namespace dsp {
 // decisions of DisortSolver::solve, :21-234).  Validation follows
 // DisortConfig::validate (DisortConfig.cpp:72-249).
 static __global__ void __launch_bounds__(128) gen_setup_kernel(FluxParams p) {
+  __shared__ double stage[4][96];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slot = blockIdx.x * 4 + warp;
   if (slot >= p.n) return;
@@ -46,6 +47,7 @@ static __global__ void __launch_bounds__(128) gen_setup_kernel(FluxParams p) {
     for (int k = 0; k < 16; ++k) rec[k] = 0.0;
     rec[H_NT] = NT;
   }
+  __syncwarp();  // other lanes store boundary Planck terms into the header below
 
   // ---- validate (DisortConfig.cpp:72-249) -------------------------------
   bool bad = L <= 0 || nmom < 0 || pc < (nmom > N ? nmom : N) + 1;
@@ -135,44 +137,27 @@ static __global__ void __launch_bounds__(128) gen_setup_kernel(FluxParams p) {
     rec[il.sig + lc] = sig;
     rec[il.mode + lc] = mode;
   }
+  // Planck at the levels and the two boundaries (DisortSolver.cpp:186-202)
   if (thermal)
-    for (int lev = lane; lev <= L; lev += 32) rec[il.pkag + lev] = planck2(wlo, whi, temp_at(lev), p.pk);
+    for (int lev = lane; lev < L + 3; lev += 32) {
+      const double B = planck2(wlo, whi, lev <= L ? temp_at(lev) : lev == L + 1 ? ttop : tbot, p.pk);
+      if (lev <= L) rec[il.pkag + lev] = B;
+      else if (lev == L + 1) rec[H_PTOP] = B * emis;
+      else rec[H_PBOT] = B;
+    }
+  const SetupScan sc = setup_scan(rec, il, L, fbeam, umu0, stage[warp], lane, dtau_at, ssa_at);
   __syncwarp();
 
   if (lane == 0) {
-    const double abscut = 10.0;
-    double tauc = 0.0, taus = 0.0, abstau = 0.0;
-    int ncut = L;
-    rec[il.tauc] = 0.0;
-    rec[il.tau_s] = 0.0;
-    for (int lc = 0; lc < L; ++lc) {
-      if (abstau < abscut) ncut = lc + 1;
-      abstau += (1.0 - ssa_at(lc)) * dtau_at(lc);
-      tauc = tauc + dtau_at(lc);
-      rec[il.tauc + lc + 1] = tauc;
-      if (!deltam && !dmplus) taus = tauc;
-      else taus = taus + rec[il.dtau_s + lc];
-      rec[il.tau_s + lc + 1] = taus;
-    }
-    // beam transmission for lc < ncut of the absorption loop (DisortSolver.cpp:749-790);
-    // later entries stay zero, as on a freshly constructed reference solver
-    for (int lev = 0; lev <= L; ++lev) rec[il.btr + lev] = 0.0;
-    if (fbeam > 0.0) {
-      rec[il.btr] = 1.0;
-      for (int lc = 0; lc < ncut; ++lc) rec[il.btr + lc + 1] = exp(-rec[il.tau_s + lc + 1] / umu0);
-    }
-    const bool lyrcut = (abstau >= abscut && !thermal && L > 1);
-    if (!lyrcut) ncut = L;
-    // boundary Planck terms (DisortSolver.cpp:186-202)
-    double ptop = 0.0, pbot = 0.0, pbotd = 0.0;
-    if (thermal) {
-      ptop = planck2(wlo, whi, ttop, p.pk) * emis;
-      pbot = planck2(wlo, whi, tbot, p.pk);
-      if (dlbc) {
-        const double bl = planck2(wlo, whi, temp_at(L - 1), p.pk);
-        const double dl = rec[il.dtau_s + L - 1];
-        if (dl > 0.0) pbotd = (pbot - bl) / dl;
-      }
+    const bool lyrcut = (sc.total_abs >= 10.0 && !thermal && L > 1);
+    const int ncut = lyrcut ? sc.ncut : L;
+    double pbotd = 0.0;
+    if (!thermal) {
+      rec[H_PTOP] = 0.0;
+      rec[H_PBOT] = 0.0;
+    } else if (dlbc) {
+      const double dl = rec[il.dtau_s + L - 1];
+      if (dl > 0.0) pbotd = (rec[H_PBOT] - rec[il.pkag + L - 1]) / dl;
     }
     // highest azimuth mode (DisortSolver.cpp:218-234).  The reference reads
     // mu_user[1] and mu_user[2] (one past the index it means); entries past the
@@ -187,8 +172,6 @@ static __global__ void __launch_bounds__(128) gen_setup_kernel(FluxParams p) {
     const int naz = (indep || g.numu == 0) ? 0 : N - 1;
     rec[H_NCUT] = ncut;
     rec[H_LYRCUT] = lyrcut ? 1.0 : 0.0;
-    rec[H_PTOP] = ptop;
-    rec[H_PBOT] = pbot;
     rec[H_PBOTD] = pbotd;
     rec[H_DELTAM] = deltam ? 1.0 : 0.0;
     rec[H_DMPLUS] = dmplus ? 1.0 : 0.0;
