@@ -33,8 +33,7 @@ using namespace dsp_tc;
 
 namespace {
 
-constexpr int STAGES = 4;
-constexpr int DW_SPLITS = 8;
+constexpr int kSMs = 148;
 
 __device__ __forceinline__ float gelu_f(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f)); }
 __device__ __forceinline__ float gelu_grad_f(float z) {
@@ -42,133 +41,231 @@ __device__ __forceinline__ float gelu_grad_f(float z) {
 }
 
 // ---------------------------------------------------------------- epilogues
-struct EpiStore {  // C = acc
-  float* C;
-  int M, N;
-  __device__ void apply(int row, int col0, const float (&v)[16], int) const {
-    if (row >= M) return;
+// Arrays are 16-byte aligned with row lengths that are multiples of 16, unless said
+// otherwise.  A slice passes through the warp's 4 KB of shared memory: 2 KB of FP32
+// rows, 1 KB of BF16 rows, 1 KB of BF16 columns (tc_gemm.cuh).  The 16-byte pieces
+// of a row are permuted so that neither side of the exchange has bank conflicts.
+__device__ __forceinline__ float4* stage_f32(const EpiSlice& t, int row, int piece) {
+  return reinterpret_cast<float4*>(t.stage + row * 64 + ((piece ^ (row >> 1)) & 3) * 16);
+}
+__device__ __forceinline__ uint4* stage_bf16(const EpiSlice& t, int row, int piece) {
+  return reinterpret_cast<uint4*>(t.stage + 2048 + row * 32 + ((piece ^ (row >> 2)) & 1) * 16);
+}
+__device__ __forceinline__ uint32_t* stage_cols(const EpiSlice& t) {
+  return reinterpret_cast<uint32_t*>(t.stage + 3072);
+}
+__device__ __forceinline__ void load16(const float* p, float (&v)[16]) {
 #pragma unroll
-    for (int j = 0; j < 16; ++j)
-      if (col0 + j < N) C[(long long)row * N + col0 + j] = v[j];
+  for (int j = 0; j < 16; j += 4) {
+    const float4 q = *reinterpret_cast<const float4*>(p + j);
+    v[j] = q.x, v[j + 1] = q.y, v[j + 2] = q.z, v[j + 3] = q.w;
   }
-};
+}
+// this lane's row to the stage, and from it
+__device__ __forceinline__ void put_f32(const EpiSlice& t, const float (&v)[16]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) *stage_f32(t, t.lane, j) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+}
+__device__ __forceinline__ void get_f32(const EpiSlice& t, float (&v)[16]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float4 q = *stage_f32(t, t.lane, j);
+    v[4 * j] = q.x, v[4 * j + 1] = q.y, v[4 * j + 2] = q.z, v[4 * j + 3] = q.w;
+  }
+}
+// BF16 of this lane's row to the stage, as a row and (COLS) as 16 columns of 32 rows:
+// lanes 2r and 2r + 1 trade halves, so that each word holds two rows of one column
+template <bool COLS>
+__device__ __forceinline__ void put_bf16(const EpiSlice& t, const float (&v)[16]) {
+  uint32_t h[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+    h[j] = *reinterpret_cast<const uint32_t*>(&b);
+  }
+  *stage_bf16(t, t.lane, 0) = make_uint4(h[0], h[1], h[2], h[3]);
+  *stage_bf16(t, t.lane, 1) = make_uint4(h[4], h[5], h[6], h[7]);
+  if (COLS) {
+    const bool odd = t.lane & 1;
+    uint32_t* const w = stage_cols(t) + (odd ? 16 : 0) + (t.lane >> 1);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const uint32_t other = __shfl_xor_sync(0xffffffffu, h[j], 1);
+      w[j * 32] = odd ? __byte_perm(other, h[j], 0x7632) : __byte_perm(h[j], other, 0x5410);
+    }
+  }
+}
+// the staged slice to rows of N elements of an M-row array, four (FP32) or two (BF16)
+// lanes per row
+template <class F>
+__device__ __forceinline__ void rows_f32(const EpiSlice& t, int M, const F& f) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int r = k * 8 + (t.lane >> 2);
+    if (t.row0 + r < M) f(t.row0 + r, t.col0 + (t.lane & 3) * 4, stage_f32(t, r, t.lane & 3));
+  }
+}
+__device__ __forceinline__ void rows_bf16(const EpiSlice& t, int M, int N, bf16* p) {
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int r = k * 16 + (t.lane >> 1);
+    if (t.row0 + r < M)
+      *reinterpret_cast<uint4*>(p + (long long)(t.row0 + r) * N + t.col0 + (t.lane & 1) * 8) = *stage_bf16(t, r, t.lane & 1);
+  }
+}
+// the staged columns to rows col0.. of the transposed copy; M a multiple of 128
+__device__ __forceinline__ void cols_bf16(const EpiSlice& t, int M, bf16* p) {
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int c = k * 8 + (t.lane >> 2), piece = t.lane & 3;
+    *reinterpret_cast<uint4*>(p + (long long)(t.col0 + c) * M + t.row0 + piece * 8) =
+        reinterpret_cast<const uint4*>(stage_cols(t))[c * 4 + piece];
+  }
+}
 
-struct EpiStoreBias {  // C = acc + b, columns < N only
+struct EpiStore {  // C = acc (+ bias), columns < N
   float* C;
-  const float* bias;
+  const float* bias;  // null, or padded to a multiple of 64
   int M, N;
-  __device__ void apply(int row, int col0, const float (&v)[16], int) const {
-    if (row >= M) return;
+  bool wide;  // N a multiple of 4 and C 16-byte aligned
+  __device__ void apply(const EpiSlice& t, const float (&v)[16], float&) const {
+    if (t.col0 >= N) return;
+    float z[16];
+    if (bias) load16(bias + t.col0, z);
 #pragma unroll
-    for (int j = 0; j < 16; ++j)
-      if (col0 + j < N) C[(long long)row * N + col0 + j] = v[j] + bias[col0 + j];
+    for (int j = 0; j < 16; ++j) z[j] = bias ? v[j] + z[j] : v[j];
+    put_f32(t, z);
+    __syncwarp();
+    rows_f32(t, M, [&](int row, int col, const float4* q) {
+      float* const c = C + (long long)row * N + col;
+      if (wide && col < N) {
+        *reinterpret_cast<float4*>(c) = *q;
+      } else if (!wide) {
+        const float e[4] = {q->x, q->y, q->z, q->w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (col + j < N) c[j] = e[j];
+      }
+    });
   }
+  __device__ void finish(float) const {}
 };
 
 struct EpiHidden {  // Z = acc + b; H = GELU(Z); optional Z (FP32) and H^T
   const float* bias;
   float* Z;
   bf16* H;
-  bf16* Ht;
+  bf16* Ht;  // with M a multiple of 128
   int M, N;
-  __device__ void apply(int row, int col0, const float (&v)[16], int) const {
-    if (row >= M) return;
+  __device__ void apply(const EpiSlice& t, const float (&v)[16], float&) const {
     float z[16];
-    __align__(16) bf16 h[16];
+    load16(bias + t.col0, z);
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      z[j] = v[j] + bias[col0 + j];
-      h[j] = __float2bfloat16(gelu_f(z[j]));
-    }
-    const long long o = (long long)row * N + col0;
-    if (Z) {
+    for (int j = 0; j < 16; ++j) z[j] = v[j] + z[j];
+    if (Z) put_f32(t, z);
 #pragma unroll
-      for (int j = 0; j < 16; j += 4)
-        *reinterpret_cast<float4*>(Z + o + j) = make_float4(z[j], z[j + 1], z[j + 2], z[j + 3]);
-    }
-    *reinterpret_cast<uint4*>(H + o) = *reinterpret_cast<const uint4*>(h);
-    *reinterpret_cast<uint4*>(H + o + 8) = *reinterpret_cast<const uint4*>(h + 8);
-    if (Ht) {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) Ht[(long long)(col0 + j) * M + row] = h[j];
-    }
+    for (int j = 0; j < 16; ++j) z[j] = gelu_f(z[j]);
+    if (Ht) put_bf16<true>(t, z);
+    else put_bf16<false>(t, z);
+    __syncwarp();
+    if (Z)
+      rows_f32(t, M, [&](int row, int col, const float4* q) {
+        *reinterpret_cast<float4*>(Z + (long long)row * N + col) = *q;
+      });
+    rows_bf16(t, M, N, H);
+    if (Ht) cols_bf16(t, M, Ht);
   }
+  __device__ void finish(float) const {}
 };
 
-struct EpiOut {  // P = acc + b; training: dZ = dLoss/dP (BF16, and transposed), loss sum
+struct EpiOut {  // P = acc + b; dZ = dLoss/dP (BF16, and transposed), loss sum; M a multiple of 128
   const float* bias;
-  float* P;
   const float* Y;   // [M][nout]
-  const float* hw;  // [M][nheads] or null
+  const float* hw;  // [M][nheads]
   bf16* dZ;
   bf16* dZt;
   float* loss;
   int M, N, nout, nheads;
   float gscale;
-  __device__ void apply(int row, int col0, const float (&v)[16], int) const {
-    if (row >= M) return;
-    float lsum = 0.0f;
+  __device__ void apply(const EpiSlice& t, const float (&v)[16], float& lsum) const {
+    if (t.col0 >= N) return;
+    // head h and output k of each column; the columns past the last head are padding
+    const int nreal = nheads * nout - t.col0;
+    float p[16], y[16];
+    // targets, 16 lanes per row
+    {
+      const int j = t.lane & 15, k = (t.col0 + j) % nout;
+#pragma unroll
+      for (int it = 0; it < 16; ++it) {
+        const int r = it * 2 + (t.lane >> 4);
+        y[it] = j < nreal ? Y[(long long)(t.row0 + r) * nout + k] : 0.0f;
+      }
+#pragma unroll
+      for (int it = 0; it < 16; ++it)
+        reinterpret_cast<float*>(stage_f32(t, it * 2 + (t.lane >> 4), j >> 2))[j & 3] = y[it];
+    }
+    __syncwarp();
+    get_f32(t, y);
+    load16(bias + t.col0, p);
+    const float* const hrow = hw + (long long)(t.row0 + t.lane) * nheads;
+    int h = t.col0 / nout, k = t.col0 - h * nout;
+    float w = nreal > 0 ? hrow[h] : 0.0f;
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
-      const int n = col0 + j;
-      if (n >= N) continue;
-      const float p = v[j] + bias[n];
-      if (P) P[(long long)row * N + n] = p;
-      if (dZ) {
-        float g = 0.0f;
-        if (n < nheads * nout) {
-          const int h = n / nout, k = n - h * nout;
-          const float d = p - Y[(long long)row * nout + k];
-          const float w = hw ? hw[(long long)row * nheads + h] : 1.0f;
-          g = gscale * w * d;
-          lsum += w * d * d;
-        }
-        const bf16 gb = __float2bfloat16(g);
-        dZ[(long long)row * N + n] = gb;
-        dZt[(long long)n * M + row] = gb;
+      const float d = j < nreal ? (v[j] + p[j]) - y[j] : 0.0f;
+      lsum += w * d * d;
+      p[j] = gscale * w * d;
+      if (++k == nout && j + 1 < nreal) {
+        k = 0;
+        w = hrow[++h];
       }
     }
-    if (dZ && loss) {
-      // one atomic per warp when the whole warp holds rows (training batches are
-      // multiples of 128 rows); otherwise one per thread
-      if (__activemask() == 0xffffffffu) {
+    put_bf16<true>(t, p);
+    __syncwarp();
+    rows_bf16(t, M, N, dZ);
+    cols_bf16(t, M, dZt);
+  }
+  __device__ void finish(float lsum) const {
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, off);
-        if ((threadIdx.x & 31) == 0) atomicAdd(loss, lsum);
-      } else {
-        atomicAdd(loss, lsum);
-      }
-    }
+    for (int off = 16; off > 0; off >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, off);
+    if ((threadIdx.x & 31) == 0) atomicAdd(loss, lsum);
   }
 };
 
-struct EpiBwdX {  // dZ_prev = acc * GELU'(Z_prev), BF16 and transposed
+struct EpiBwdX {  // dZ_prev = acc * GELU'(Z_prev), BF16 and transposed; M a multiple of 128
   const float* Zp;
   bf16* dZ;
   bf16* dZt;
   int M, N;
-  __device__ void apply(int row, int col0, const float (&v)[16], int) const {
-    if (row >= M) return;
-    const long long o = (long long)row * N + col0;
-    __align__(16) bf16 g[16];
+  __device__ void apply(const EpiSlice& t, const float (&v)[16], float&) const {
+    rows_f32(t, M, [&](int row, int col, float4* q) {
+      *q = *reinterpret_cast<const float4*>(Zp + (long long)row * N + col);
+    });
+    __syncwarp();
+    float z[16];
+    get_f32(t, z);
 #pragma unroll
-    for (int j = 0; j < 16; ++j) g[j] = __float2bfloat16(v[j] * gelu_grad_f(Zp[o + j]));
-    *reinterpret_cast<uint4*>(dZ + o) = *reinterpret_cast<const uint4*>(g);
-    *reinterpret_cast<uint4*>(dZ + o + 8) = *reinterpret_cast<const uint4*>(g + 8);
-#pragma unroll
-    for (int j = 0; j < 16; ++j) dZt[(long long)(col0 + j) * M + row] = g[j];
+    for (int j = 0; j < 16; ++j) z[j] = v[j] * gelu_grad_f(z[j]);
+    put_bf16<true>(t, z);
+    __syncwarp();
+    rows_bf16(t, M, N, dZ);
+    cols_bf16(t, M, dZt);
   }
+  __device__ void finish(float) const {}
 };
 
 struct EpiDW {  // dW += acc (split-K partial sums)
   float* dW;
   int M, N;
-  __device__ void apply(int row, int col0, const float (&v)[16], int) const {
-    if (row >= M) return;
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-      if (col0 + j < N) atomicAdd(dW + (long long)row * N + col0 + j, v[j]);
+  __device__ void apply(const EpiSlice& t, const float (&v)[16], float&) const {
+    if (t.col0 >= N) return;
+    put_f32(t, v);
+    __syncwarp();
+    rows_f32(t, M, [&](int row, int col, const float4* q) {
+      atomicAdd(reinterpret_cast<float4*>(dW + (long long)row * N + col), *q);
+    });
   }
+  __device__ void finish(float) const {}
 };
 
 // ---------------------------------------------------------------- small kernels
@@ -185,30 +282,57 @@ __global__ void gather_rows_kernel(const bf16* X, const float* Y, const float* H
     for (int k = threadIdx.x; k < nheads; k += blockDim.x) HWp[r * nheads + k] = HW[src * nheads + k];
 }
 
-// dst[c][r] = src[r][c] for an R x C BF16 block (32 x 32 tiles)
-__global__ void transpose_bf16_kernel(const bf16* src, bf16* dst, int R, int C) {
-  __shared__ bf16 t[32][33];
-  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-    const int r = r0 + k, c = c0 + threadIdx.x;
-    if (r < R && c < C) t[k][threadIdx.x] = src[(long long)r * C + c];
+// dst[c][r] = src[r][c] for an R x C BF16 block, R and C multiples of 64: 64 x 64
+// tiles, read and written in 16-byte pieces (4,096 x 704: 8.5 -> 4.4 us)
+__global__ void __launch_bounds__(256) transpose_bf16_kernel(const bf16* src, bf16* dst, int R, int C) {
+  __shared__ uint16_t t[64][66];
+  const int c0 = blockIdx.x * 64, r0 = blockIdx.y * 64;
+  const int row = threadIdx.x >> 3, piece = (threadIdx.x & 7) * 8;
+#pragma unroll
+  for (int k = 0; k < 64; k += 32) {
+    const uint4 q = *reinterpret_cast<const uint4*>(src + (long long)(r0 + row + k) * C + c0 + piece);
+    uint32_t* const d = reinterpret_cast<uint32_t*>(&t[row + k][piece]);
+    d[0] = q.x, d[1] = q.y, d[2] = q.z, d[3] = q.w;
   }
   __syncthreads();
-  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-    const int c = c0 + k, r = r0 + threadIdx.x;
-    if (r < R && c < C) dst[(long long)c * R + r] = t[threadIdx.x][k];
+#pragma unroll
+  for (int k = 0; k < 64; k += 32) {
+    uint32_t q[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      q[j] = (uint32_t)t[piece + 2 * j][row + k] | ((uint32_t)t[piece + 2 * j + 1][row + k] << 16);
+    *reinterpret_cast<uint4*>(dst + (long long)(c0 + row + k) * R + r0 + piece) = make_uint4(q[0], q[1], q[2], q[3]);
   }
 }
 
-// db[n] = sum_m dZt[n][m]: one warp per n
-__global__ void bias_grad_kernel(const bf16* dZt, float* db, int N, int M) {
-  const int n = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
-  if (n >= N) return;
+// db[n] = sum_m dZt[n][m] of up to kBiasLayers layers in one launch: one warp per n,
+// 16 bytes per lane and load (five layers of 4,096 rows: 50 -> 6.5 us).  M is a multiple
+// of 128.
+constexpr int kBiasLayers = 16;
+struct BiasGrads {
+  const bf16* dZt[kBiasLayers];
+  float* db[kBiasLayers];
+  int end[kBiasLayers];  // rows of this layer and the ones before it
+  int n;
+};
+__global__ void __launch_bounds__(256) bias_grad_kernel(const __grid_constant__ BiasGrads g, int M) {
+  int n = blockIdx.x * 8 + (threadIdx.x >> 5), layer = 0;
+  const int lane = threadIdx.x & 31;
+  if (n >= g.end[g.n - 1]) return;
+  while (n >= g.end[layer]) ++layer;
+  if (layer > 0) n -= g.end[layer - 1];
+  const uint4* const row = reinterpret_cast<const uint4*>(g.dZt[layer] + (long long)n * M);
   float s = 0.0f;
-  for (int m = lane; m < M; m += 32) s += __bfloat162float(dZt[(long long)n * M + m]);
+#pragma unroll 4
+  for (int m = lane; m < M / 8; m += 32) {
+    const uint4 q = row[m];
+    const uint32_t u[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) s += __uint_as_float(u[j] << 16) + __uint_as_float(u[j] & 0xffff0000u);
+  }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  if (lane == 0) db[n] = s;
+  if (lane == 0) g.db[layer][n] = s;
 }
 
 // Adam on FP32 masters [rows][cols]; entries outside [rows_real) x [cols_real)
@@ -314,34 +438,67 @@ bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, ui
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-inline int bn_for(int n) { return (n % 128 == 0) ? 128 : 64; }
+inline int pad64(int x) { return (x + 63) / 64 * 64; }
+
+// Tile width of n output columns (the box of B's tensor map has as many rows): 128,
+// unless half of a last tile would be padding and there are few of them.  The weight
+// gradient of 704 columns takes 13.6 us in 64-column tiles and 10.5 us in 128-column
+// ones; 192 columns stay at 64, where 4,096 rows give 96 tiles instead of 64.
+inline int bn_for(int n) {
+  const int p = pad64(n);
+  return (p % 128 == 0 || p >= 512) ? 128 : 64;
+}
 
 template <int BN, class Epi>
-cudaError_t launch_gemm_bn(const CUtensorMap& A, const CUtensorMap& B, int a_row0, int b_row0, int M, int N, int K,
-                           int splits, const Epi& epi, int* err, cudaStream_t s) {
-  using C = GemmCfg<BN, STAGES>;
+cudaError_t launch_gemm_bn(const CUtensorMap& A, const CUtensorMap& B, int a_row0, int b_row0, const GemmTiles& tiles,
+                           const Epi& epi, int* err, cudaStream_t s) {
+  using C = GemmCfg<BN>;
   static bool attr = false;
   if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(tc_gemm_tn_kernel<BN, STAGES, Epi>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem_bytes());
+    cudaError_t e = cudaFuncSetAttribute(tc_gemm_tn_kernel<BN, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)C::smem_bytes());
     if (e != cudaSuccess) return e;
     attr = true;
   }
-  const int kt = (K + 63) / 64;
-  const int per = (kt + splits - 1) / splits;
-  dim3 grid((M + 127) / 128, (N + BN - 1) / BN, splits);
-  tc_gemm_tn_kernel<BN, STAGES, Epi><<<grid, 128, C::smem_bytes(), s>>>(A, B, a_row0, b_row0, kt, per, epi, err);
-  return cudaGetLastError();
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(std::min(tiles.count(), kSMs));
+  lc.blockDim = dim3(C::THREADS);
+  lc.dynamicSmemBytes = C::smem_bytes();
+  lc.stream = s;
+  // barriers, tensor memory and the launch itself under the end of the kernel in front
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = at;
+  lc.numAttrs = 1;
+  return cudaLaunchKernelEx(&lc, tc_gemm_tn_kernel<BN, Epi>, A, B, a_row0, b_row0, tiles, epi, err);
 }
 
+// `split`: share K out over the SMs that the output's tiles leave idle (the epilogue
+// accumulates atomically).
 template <class Epi>
 cudaError_t launch_gemm(const CUtensorMap& A, const CUtensorMap& B, int a_row0, int b_row0, int M, int N, int K,
-                        int splits, const Epi& epi, int* err, cudaStream_t s) {
-  if (bn_for(N) == 128) return launch_gemm_bn<128>(A, B, a_row0, b_row0, M, N, K, splits, epi, err, s);
-  return launch_gemm_bn<64>(A, B, a_row0, b_row0, M, N, K, splits, epi, err, s);
+                        bool split, const Epi& epi, int* err, cudaStream_t s) {
+  const int bn = bn_for(N);
+  GemmTiles t{(M + 127) / 128, (N + bn - 1) / bn, 1, (K + 63) / 64, (K + 63) / 64};
+  if (split && t.m * t.n < kSMs) {
+    t.k_per_split = (t.k + kSMs / (t.m * t.n) - 1) / (kSMs / (t.m * t.n));
+    t.splits = (t.k + t.k_per_split - 1) / t.k_per_split;
+  }
+  // 256 columns where they take no more rounds of the SMs than twice as many tiles of
+  // half the width: the large GEMMs are bound by L2, and A is then read half as often
+  // (65,536 rows, 512
+  // columns, K = 512: 75 -> 66 us)
+  if (bn == 128 && !split && N % 256 == 0) {
+    const int wide = t.m * (N / 256);
+    if (2 * ((wide + kSMs - 1) / kSMs) <= (t.m * t.n + kSMs - 1) / kSMs) {
+      t.n = N / 256;
+      return launch_gemm_bn<256>(A, B, a_row0, b_row0, t, epi, err, s);
+    }
+  }
+  return bn == 128 ? launch_gemm_bn<128>(A, B, a_row0, b_row0, t, epi, err, s)
+                   : launch_gemm_bn<64>(A, B, a_row0, b_row0, t, epi, err, s);
 }
-
-inline int pad64(int x) { return (x + 63) / 64 * 64; }
 
 struct Layer {
   int in_pad = 0, out_pad = 0, in_real = 0, out_real = 0;
@@ -365,7 +522,6 @@ struct dsp_emu_s {
   std::vector<float*> Z;
   std::vector<bf16*> H, Ht, dZ, dZt;
   bf16 *X0t = nullptr, *dZo = nullptr, *dZot = nullptr;
-  float* P = nullptr;
   float* loss_d = nullptr;
   int* err_d = nullptr;
   float* grad_flat = nullptr;  // contiguous dW/db of all layers
@@ -423,8 +579,8 @@ dsp_status train_pass(dsp_emu e, const CUtensorMap& xmap, const bf16* xsrc, int 
   cudaError_t ce;
   // X^T of the batch for dW_1
   {
-    dim3 blk(32, 8), grd((e->in_pad + 31) / 32, (B + 31) / 32);
-    transpose_bf16_kernel<<<grd, blk, 0, s>>>(xsrc + (int64_t)a_row0 * e->in_pad, e->X0t, B, e->in_pad);
+    dim3 grd(e->in_pad / 64, B / 64);
+    transpose_bf16_kernel<<<grd, 256, 0, s>>>(xsrc + (int64_t)a_row0 * e->in_pad, e->X0t, B, e->in_pad);
   }
   // forward
   for (int i = 0; i < nl; ++i) {
@@ -433,11 +589,11 @@ dsp_status train_pass(dsp_emu e, const CUtensorMap& xmap, const bf16* xsrc, int 
     const int r0 = (i == 0) ? a_row0 : 0;
     if (i < nl - 1) {
       EpiHidden ep{l.b, e->Z[i], e->H[i], e->Ht[i], B, l.out_pad};
-      ce = launch_gemm(am, l.mapW, r0, 0, B, l.out_pad, l.in_pad, 1, ep, e->err_d, s);
+      ce = launch_gemm(am, l.mapW, r0, 0, B, l.out_pad, l.in_pad, false, ep, e->err_d, s);
     } else {
-      EpiOut ep{l.b, e->P, Yb, HWb, e->dZo, e->dZot, e->loss_d, B, l.out_pad, e->cfg.n_out, e->cfg.n_heads,
+      EpiOut ep{l.b, Yb, HWb, e->dZo, e->dZot, e->loss_d, B, l.out_pad, e->cfg.n_out, e->cfg.n_heads,
                 2.0f / (float)(e->cfg.n_out * B)};
-      ce = launch_gemm(am, l.mapW, r0, 0, B, l.out_pad, l.in_pad, 1, ep, e->err_d, s);
+      ce = launch_gemm(am, l.mapW, r0, 0, B, l.out_pad, l.in_pad, false, ep, e->err_d, s);
     }
     if (ce != cudaSuccess) return check_err(e, ce, "forward GEMM");
   }
@@ -449,16 +605,25 @@ dsp_status train_pass(dsp_emu e, const CUtensorMap& xmap, const bf16* xsrc, int 
     const CUtensorMap& dzt = (i == nl - 1) ? e->mapdZot : e->mapdZt[i];
     const CUtensorMap& xt = (i == 0) ? e->mapX0t : e->mapHt[i - 1];
     EpiDW ew{l.dW, l.out_pad, l.in_pad};
-    ce = launch_gemm(dzt, xt, 0, 0, l.out_pad, l.in_pad, B, DW_SPLITS, ew, e->err_d, s);
+    ce = launch_gemm(dzt, xt, 0, 0, l.out_pad, l.in_pad, B, true, ew, e->err_d, s);
     if (ce != cudaSuccess) return check_err(e, ce, "weight-gradient GEMM");
-    const bf16* dzt_ptr = (i == nl - 1) ? e->dZot : e->dZt[i];
-    bias_grad_kernel<<<(l.out_pad + 7) / 8, 256, 0, s>>>(dzt_ptr, l.db, l.out_pad, B);
     if (i > 0) {
       const CUtensorMap& dz = (i == nl - 1) ? e->mapdZo : e->mapdZ[i];
       EpiBwdX ex{e->Z[i - 1], e->dZ[i - 1], e->dZt[i - 1], B, l.in_pad};
-      ce = launch_gemm(dz, l.mapWt, 0, 0, B, l.in_pad, l.out_pad, 1, ex, e->err_d, s);
+      ce = launch_gemm(dz, l.mapWt, 0, 0, B, l.in_pad, l.out_pad, false, ex, e->err_d, s);
       if (ce != cudaSuccess) return check_err(e, ce, "input-gradient GEMM");
     }
+  }
+  for (int i0 = 0; i0 < nl; i0 += kBiasLayers) {
+    BiasGrads g{};
+    g.n = std::min(kBiasLayers, nl - i0);
+    for (int k = 0; k < g.n; ++k) {
+      g.dZt[k] = (i0 + k == nl - 1) ? e->dZot : e->dZt[i0 + k];
+      g.db[k] = e->L[i0 + k].db;
+      g.end[k] = e->L[i0 + k].out_pad + (k > 0 ? g.end[k - 1] : 0);
+    }
+    bias_grad_kernel<<<(g.end[g.n - 1] + 7) / 8, 256, 0, s>>>(g, B);
+    if ((ce = cudaGetLastError()) != cudaSuccess) return check_err(e, ce, "bias gradients");
   }
   return DSP_OK;
 }
@@ -570,10 +735,9 @@ dsp_status dsp_emu_create(int32_t device, void* stream, const dsp_emu_config* cf
     e->X0t = dalloc<bf16>(e, (size_t)e->in_pad * B);
     e->dZo = dalloc<bf16>(e, (size_t)B * e->out_pad);
     e->dZot = dalloc<bf16>(e, (size_t)e->out_pad * B);
-    e->P = dalloc<float>(e, (size_t)B * e->out_pad);
     e->loss_d = dalloc<float>(e, 1);
     e->err_d = dalloc<int>(e, 1);
-    ok = e->X0t && e->dZo && e->dZot && e->P && e->loss_d && e->err_d;
+    ok = e->X0t && e->dZo && e->dZot && e->loss_d && e->err_d;
     ok = ok && make_map(&e->mapX0t, e->X0t, e->in_pad, B, bn_for(e->in_pad)) &&
          make_map(&e->mapdZo, e->dZo, B, e->out_pad, 128) && make_map(&e->mapdZot, e->dZot, e->out_pad, B, 128);
   }
@@ -721,14 +885,15 @@ dsp_status dsp_emu_forward(dsp_emu e, const uint16_t* feats, int64_t rows, float
       cudaError_t ce;
       if (i < e->nl - 1) {
         EpiHidden ep{l.b, nullptr, nxt, nullptr, m, l.out_pad};
-        ce = launch_gemm(am, l.mapW, a0, 0, m, l.out_pad, l.in_pad, 1, ep, e->err_d, s);
+        ce = launch_gemm(am, l.mapW, a0, 0, m, l.out_pad, l.in_pad, false, ep, e->err_d, s);
         std::swap(cur, nxt);
         std::swap(mc, mn);
       } else {
         // predictions of the real head outputs only: compact [rows][n_heads*n_out]
         const int nreal = e->cfg.n_heads * e->cfg.n_out;
-        EpiStoreBias eb{preds + r0 * (int64_t)nreal, l.b, m, nreal};
-        ce = launch_gemm(am, l.mapW, a0, 0, m, l.out_pad, l.in_pad, 1, eb, e->err_d, s);
+        float* const out = preds + r0 * (int64_t)nreal;
+        EpiStore eb{out, l.b, m, nreal, nreal % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0};
+        ce = launch_gemm(am, l.mapW, a0, 0, m, l.out_pad, l.in_pad, false, eb, e->err_d, s);
       }
       if (ce != cudaSuccess) return check_err(e, ce, "inference GEMM");
     }
@@ -785,8 +950,8 @@ dsp_status dsp_emu_gemm_bf16(dsp_emu e, const uint16_t* A, const uint16_t* B, fl
   CUtensorMap ma, mb;
   if (!make_map(&ma, A, M, K, 128) || !make_map(&mb, B, N, K, bn_for(N)))
     return efail(e, DSP_ERR_INVALID_INPUT, "GEMM tensor maps");
-  EpiStore ep{Cm, M, N};
-  cudaError_t ce = launch_gemm(ma, mb, 0, 0, M, N, K, 1, ep, e->err_d, e->stream);
+  EpiStore ep{Cm, nullptr, M, N, N % 4 == 0 && (reinterpret_cast<uintptr_t>(Cm) & 15) == 0};
+  cudaError_t ce = launch_gemm(ma, mb, 0, 0, M, N, K, false, ep, e->err_d, e->stream);
   if (ce != cudaSuccess) return check_err(e, ce, "GEMM launch");
   return read_err_flag(e);
 }

@@ -94,8 +94,8 @@ static __global__ void __launch_bounds__(256) hg_moments_kernel(DArr g, long lon
 // bounded the stage when lane 0 walked the layers was not that chain but a global
 // load, a store and a double-precision exponential and division per step behind
 // it.  Here the chain reads broadcasts from shared memory and all lanes do the
-// loads, stores and exponentials: 60,000 columns of 40 layers SETUP_A, one column
-// of 60 layers SETUP_B.  Entries of btr past the absorption cut stay zero, as on a
+// loads, stores and exponentials: 60,000 columns of 40 layers 0.63 -> 0.28 ms, 20,000
+// of 60 layers 0.173 -> 0.106 ms.  Entries of btr past the absorption cut stay zero, as on a
 // freshly constructed reference solver.  `st` is 96 doubles of the warp's own.
 struct SetupScan {
   double total_abs;  // absorption optical depth of the column

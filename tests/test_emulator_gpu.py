@@ -50,6 +50,27 @@ def test_tc_gemm_matches_fp64(emu_small, M, N, K):
     assert err < 1e-5, err
 
 
+@pytest.mark.parametrize("M,N,K", [
+    (1, 1, 8), (127, 65, 72),            # one tile, ragged in all three
+    (148 * 128 + 1, 64, 64),             # a second round of the SMs with one tile in it
+    (300, 704, 200), (130, 500, 64),     # 128-column tiles, the last one half empty / ragged
+    (148 * 128, 256, 136),               # 256-column tiles, one round
+    (148 * 128 * 2 - 5, 512, 704)])      # 256-column tiles, four rounds, ragged rows
+def test_tc_gemm_tiles(emu_small, M, N, K):
+    """Every tile width and several rounds of a CTA, against FP64.  FP32 accumulation of K
+    products, rounded or truncated: |error| <= K 2^-23 sum |a||b|."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    A = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
+    B = torch.randn((N, K), generator=g, device="cuda").to(torch.bfloat16)
+    C = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
+    emu_small.gemm(A, B, C)
+    torch.cuda.synchronize()
+    a, b = A.double(), B.double()
+    bound = K * 2.0 ** -23 * (a.abs() @ b.abs().T)
+    assert bool(((C.double() - a @ b.T).abs() <= bound).all())
+
+
 def test_bounded_wait_times_out_and_the_emulator_stays_usable(emu_small):
     """A device wait on an mbarrier that nothing arrives on (no copy or MMA in
     flight) gives up after its cycle limit; the host reads DSP_ERR_TIMEOUT from
