@@ -75,10 +75,14 @@ dsp_status launch_flux_chunk(dsp_context ctx, const FluxParams& p, cudaStream_t 
     if (!attr) {
       cudaFuncSetAttribute(flux_bvp_kernel<N, false, SPH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)C::smem_bytes());
+      cudaFuncSetAttribute(flux_bvp_kernel<N, false, SPH, C::LEAN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)C::smem_bytes());
       attr = true;
     }
     KernelTimer kt(ctx, "flux_bvp_kernel", s);
-    flux_bvp_kernel<N, false, SPH><<<(p.n + C::TPW - 1) / C::TPW, 32, C::smem_bytes(), s>>>(p);
+    const int grid = (p.n + C::TPW - 1) / C::TPW;
+    if (jv) flux_bvp_kernel<N, false, SPH, C::LEAN><<<grid, 32, C::smem_bytes(), s>>>(p);
+    else flux_bvp_kernel<N, false, SPH><<<grid, 32, C::smem_bytes(), s>>>(p);
   }
   if (jv) {
     using C = JCfg<N>;

@@ -127,6 +127,16 @@ __host__ __device__ constexpr int brec_r(int N) { return 2 * (N / 2) * mod_hp(N)
 __host__ __device__ constexpr int brec_dn(int N) { return brec_r(N) + mod_hp(N); }
 __host__ __device__ constexpr int brec_inv(int N) { return brec_r(N) + 2 * mod_hp(N); }
 __host__ __device__ constexpr int brec_stride(int N) { return round4(N * (2 * N + 2)); }
+// Flux solves of few streams keep, instead, per layer what the upward pass needs of it
+// (flux_bvp.cuh): W [h][HP] | per stream the constant, the two flux functionals and g
+// [h][4] | what the fluxes of the bottom level add to phi [HP] | Planck source at the
+// bottom and the top.
+__host__ __device__ constexpr int trec_v(int N) { return (N / 2) * mod_hp(N); }
+__host__ __device__ constexpr int trec_dphi(int N) { return trec_v(N) + 2 * N; }
+__host__ __device__ constexpr int trec_pl(int N) { return trec_dphi(N) + mod_hp(N); }
+__host__ __device__ constexpr int trec_stride(int N) { return round4(trec_pl(N) + 2); }
+static_assert(trec_stride(4) <= brec_stride(4) && trec_stride(6) <= brec_stride(6) && trec_stride(16) <= brec_stride(16),
+              "transmission record");
 static_assert(mod_size(4) <= lrec_stride(4) && mod_size(6) <= lrec_stride(6) && mod_size(14) <= lrec_stride(14) &&
                   mod_size(64) <= lrec_stride(64),
               "layer record");

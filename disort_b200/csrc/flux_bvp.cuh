@@ -29,6 +29,19 @@
 // tenth of its operations; near omega' = 1 (k -> 0) nothing cancels, because
 // 1 - E^2 comes from expm1.
 //
+// Fluxes alone need less on the way up (LEAN, up to 16 streams).  Substituted into
+// one another, the three equations are
+//   phi_t = W phi_b + f,  W = 2 V G Y^T,  V = X H E,  f = X (c_t - r) + 2 V G (q - c_b),
+// and the fluxes of a level are sums w (phi +- psi), w mu (phi +- psi) with
+// psi = A phi + g, so that psi takes two vectors A w, A w mu and g.  The way down then
+// stores W, f, these two and g (96 doubles a layer at 16 streams) where the general
+// form stores G, H and r (136) and reads them and the layer record (190) again on the
+// way up; one product with W per layer, from registers, takes the place of six
+// matrix-vector products in a chain.  Two more h^3 products per layer pay for it:
+// 60,000 columns of 40 layers at 4 streams 0.80 -> 0.55 ms, 20,000 of 60 at 16 streams
+// 1.89 -> 1.51 ms, one of 60 layers 240 -> 211 us.  With 32 streams the products cost what the way up gains
+// (its share of a layer is 20 %, 11 % at 64).
+//
 // Mapping: lane j of a team owns column j; products read the other operand from
 // shared memory as broadcasts (one 16-byte word of each team per instruction),
 // the inverses are symmetric sweeps whose pivot row is exchanged through shared
@@ -61,7 +74,7 @@ struct BCfg {
   static constexpr int O_V = O_W + MAT;         // layer-record vectors
   static constexpr int O_S = O_V + NV;          // 2 pivot-row buffers
   static constexpr int O_G = O_S + 2 * SB;      // gathered vectors, HP each:
-  static constexpr int NG = 7;                  // g, w1, w2, gamma, scale, E / phi, D
+  static constexpr int NG = 9;                  // g, w1, w2, gamma, scale, E / phi, D / w, w mu, d
   static constexpr int SIZE = O_G + NG * HP;
   // teams of a warp start 4 banks apart: their broadcasts are conflict-free
   static constexpr int STRIDE = TPW == 1 ? SIZE : SIZE + ((2 - SIZE) % 16 + 16) % 16;
@@ -76,6 +89,8 @@ struct BCfg {
   // the lane's row of the identity in registers: diagonal elements as products
   // (the FP64 pipe has room) instead of selects by lane
   static constexpr bool IDREG = H <= 8;
+  // fluxes without Jacobians: transmission records instead of G, H, r
+  static constexpr bool LEAN = H <= 8;
 };
 
 // Negative inverse of a symmetric positive definite matrix with unit diagonal
@@ -189,7 +204,7 @@ __device__ __forceinline__ void axpy_row(double* acc, const double* row, const d
 }
 
 // The instances of one warp: team `team` solves chunk slot `slot` (-1: none).
-template <int N, bool GEN, bool SPH>
+template <int N, bool GEN, bool SPH, bool LEAN>
 __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
   using C = BCfg<N>;
   constexpr int H = C::H, HP = C::HP, TEAM = C::TEAM, LDM = C::LDM, SB = C::SB;
@@ -213,6 +228,8 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
   double* const vsc = vgam + HP;
   double* const ve = vsc + HP;  // E going down, phi going up
   double* const vd = ve + HP;
+  double* const vwm = vd + HP;
+  double* const vdp = vwm + HP;
 
   const bool ifb = (p.flags & DSP_FLAG_INDEX_FROM_BOTTOM) != 0;
   const int mrow = GEN ? (int)blockIdx.y : 0;
@@ -227,7 +244,8 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
   const long long lay0 = GEN ? p.g.lay_off[sl] : (long long)i * p.L;
   const long long lstride = GEN ? p.g.lstride : (long long)lrec_stride(N);
   const double* const lrec0 = p.layer_rec + (GEN ? mrow * p.g.ms_layer : 0ll) + lay0 * lstride;
-  double* const brec0 = p.bvp_rec + (GEN ? mrow * p.g.ms_bvp : 0ll) + lay0 * brec_stride(N);
+  constexpr int BSTRIDE = LEAN ? trec_stride(N) : brec_stride(N);
+  double* const brec0 = p.bvp_rec + (GEN ? mrow * p.g.ms_bvp : 0ll) + lay0 * BSTRIDE;
   auto oidx = [&](int lev) {
     if constexpr (GEN) return (long long)i * p.g.ntau_out + (ifb ? NT - 1 - lev : lev);
     else return (long long)i * NT + (ifb ? L - lev : lev);
@@ -260,6 +278,9 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
   const double* const taus = rec + il.tau_s;
   const double* const btr = rec + il.btr;
   const double dj = p.tables[tab_dsim(N) + j];
+  const double wd = own ? 0.5 * p.tables[tab_wt(N) + j] / dj : 0.0;  // w / (2 d) of stream j
+  const double muj = p.tables[tab_mu(N) + j];
+  const double rumu0 = beam ? 1.0 / umu0 : 0.0;
   bool singular = false;
 
   // the layer record of layer l: X^T and the vectors, Y^T
@@ -335,6 +356,10 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
   }
   if (HP != H && t == 0)
     for (int v = 0; v < C::NG; ++v) vg[v * HP + H] = 0.0;
+  if (LEAN && own) {
+    vd[j] = wd;
+    vwm[j] = wd * muj;
+  }
   __syncwarp();
 
   double a[H], id[C::IDREG ? H : 1];
@@ -352,6 +377,11 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
     double ct, dt_, cb, db;
     particular(l, s.t0, s.b0, ct, dt_);
     particular(l, s.t1, s.b1, cb, db);
+    double pl0 = 0.0, pl1 = 0.0;  // Planck source at the top and the bottom
+    if (LEAN && thermal) {
+      pl0 = fma(vec[7 * HP + 1], s.t0, vec[7 * HP]);
+      pl1 = fma(vec[7 * HP + 1], s.t1, vec[7 * HP]);
+    }
     DSP_PHASE(0)
     // I + M = I + X^T A X, column j
     const double* xj = Xs + j * LDM;
@@ -400,19 +430,56 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
       else a[r] *= s1 * vsc[r];
     }
     // X and the vectors are used up: the next layer's start loading
-    load_x(l + 1);
+    if constexpr (!LEAN) load_x(l + 1);
     DSP_PHASE(1)
     sweep_inverse<H, SB, ROLL>(a, j, own, sbuf, singular);
     DSP_PHASE(2)
-    double* const br = brec0 + (long long)(on ? l : 0) * brec_stride(N);
+    double* const br = brec0 + (long long)(on ? l : 0) * BSTRIDE;
 #pragma unroll
     for (int r = 0; r < H; ++r) {
       a[r] = -a[r] * (s1 * vsc[r]);
-      if (on && own) br[brec_H(N) + r * HP + j] = a[r];
+      if (!LEAN && on && own) br[brec_H(N) + r * HP + j] = a[r];
     }
-    const double rj = ct + dot_reg<H>(a, vw1);
-    if (on && own) br[brec_r(N) + j] = rj;
+    const double hv = dot_reg<H>(a, vw1);
+    const double rj = ct + hv;
+    if (!LEAN && on && own) br[brec_r(N) + j] = rj;
     const double q = ex * rj;
+    double xh = 0.0;  // X (r - c_t)
+    double dphi = 0.0;
+    bool past = false;
+    if constexpr (LEAN) {
+      // V = X H E, column j, into the place of A
+      double v[H];
+#pragma unroll
+      for (int r = 0; r < H; ++r) v[r] = 0.0;
+#pragma unroll
+      for (int r = 0; r < H; ++r) axpy_row<H>(v, Xs + r * LDM, a[r]);
+      if (own) vgam[j] = hv;
+      __syncwarp();
+      xh = dot_col<H>(Xs + j, LDM, vgam);
+      if (on && own) {
+#pragma unroll
+        for (int r = 0; r < H; ++r) As[j * LDM + r] = ex * v[r];
+      }
+      // below the absorption cut of a thermal column the boundary-value problem has no
+      // beam (btr = 0), but the reference's fluxes there still add its particular
+      // solution: X c to phi and Y d to psi of the bottom level
+      if constexpr (!SPH) {
+        past = __any_sync(0xffffffffu, on && thermal && beam && s.b1 == 0.0);
+        if (past) {
+          const double fact = on && beam && s.b1 == 0.0 ? exp(-s.t1 * rumu0) : 0.0;
+          __syncwarp();
+          if (own) {
+            vgam[j] = vec[3 * HP + j] * fact;
+            vdp[j] = vec[4 * HP + j] * fact;
+          }
+          __syncwarp();
+          dphi = dot_col<H>(Xs + j, LDM, vgam);
+        }
+      }
+      __syncwarp();
+      load_x(l + 1);
+    }
     // Z = (1 - E^2) + 2 E H E
     const double ex2 = 2.0 * ex;
     diag = 0.0;
@@ -442,11 +509,13 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
 #pragma unroll
     for (int r = 0; r < H; ++r) {
       a[r] = -a[r] * (s2 * vsc[r]);
-      if (on && own) br[brec_G(N) + r * HP + j] = a[r];
+      if (!LEAN && on && own) br[brec_G(N) + r * HP + j] = a[r];
     }
-    const double gb = cb + db + 2.0 * dot_reg<H>(a, vw2);
+    const double y = dot_reg<H>(a, vw2);  // G (q - c_b)
+    const double gb = cb + db + 2.0 * y;
     if (own) {
       vgam[j] = gb;
+      if (LEAN) vw1[j] = y;
 #pragma unroll
       for (int r = 0; r < H; ++r) Ws[j * LDM + r] = C::IDREG ? fma(2.0, a[r], -id[C::IDREG ? r : 0]) : (r == j ? fma(2.0, a[r], -1.0) : 2.0 * a[r]);
     }
@@ -460,6 +529,20 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
 #pragma unroll(ROLL ? 2 : H)
       for (int r = 0; r < H; ++r) axpy_row<H>(tv, Ws + r * LDM, Ys[r * LDM + j]);
       const double gn = dot_col<H>(Ys + j, LDM, vgam);
+      double f = 0.0;
+      if constexpr (LEAN) {
+        f = fma(2.0, dot_col<H>(As + j, LDM, vw1), -xh);
+        // column j of W: 2 G Y^T = (2 G - I) Y^T + Y^T
+        double wt[H];
+#pragma unroll
+        for (int r = 0; r < H; ++r) wt[r] = 0.0;
+#pragma unroll
+        for (int r = 0; r < H; ++r) axpy_row<H>(wt, As + r * LDM, tv[r] + Ys[r * LDM + j]);
+        if (on && own) {
+#pragma unroll
+          for (int r = 0; r < H; ++r) br[r * HP + j] = wt[r];
+        }
+      }
       double w[H];
 #pragma unroll
       for (int r = 0; r < H; ++r) w[r] = 0.0;
@@ -472,6 +555,16 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
       } else {
 #pragma unroll
         for (int r = 0; r < H; ++r) axpy_row<H>(w, Ys + r * LDM, tv[r]);
+      }
+      if constexpr (LEAN) {
+        if (on && own) {
+          double2* const o = reinterpret_cast<double2*>(br + trec_v(N) + 4 * j);
+          o[0] = make_double2(f, past ? gn + dot_col<H>(Ys + j, LDM, vdp) : gn);
+          if (thermal && beam) br[trec_dphi(N) + j] = dphi;
+          o[1] = make_double2(dot_reg<H>(w, vd), dot_reg<H>(w, vwm));
+          if (j == 0) *reinterpret_cast<double2*>(br + trec_pl(N)) = make_double2(pl0, pl1);
+        }
+        __syncwarp();  // every lane is done with V
       }
       if (on && own) {
 #pragma unroll
@@ -492,7 +585,7 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
   if constexpr (GEN)
     if (p.g.brdf && !lyrcut && !dlbc) sft = p.g.brdf + (long long)sl * brdf_stride(N, p.g.numu);
   const double alb = m == 0 && act && !lyrcut && !dlbc && !sft ? rec[H_ALB] : 0.0;
-  double* const bl = brec0 + (long long)(ncut > 0 ? ncut - 1 : 0) * brec_stride(N);  // the last layer's record
+  double* const bl = brec0 + (long long)(ncut > 0 ? ncut - 1 : 0) * BSTRIDE;  // the last layer's record
   // pseudo-spherical beam: the reference reflects Z0 times the beam factor at the
   // user angles (DisortSolver.cpp:3180-3218), not the solution at that depth; the
   // difference, in the downward intensities at the bottom
@@ -562,7 +655,7 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
 #pragma unroll
       for (int r = 0; r < H; ++r) {
         a[r] = -a[r] * (s1 * vsc[r]);
-        if (act && own) bl[brec_inv(N) + r * HP + j] = a[r];
+        if (!LEAN && act && own) bl[brec_inv(N) + r * HP + j] = a[r];
       }
     } else {
       // bidirectional surface: R_rc = (1 + delta_m0) d_r rho_rc d_c, not
@@ -626,7 +719,7 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
 #pragma unroll
       for (int c = 0; c < H; ++c) {
         a[c] = Xs[j * LDM + c];
-        if (act && own) bl[brec_inv(N) + c * HP + j] = a[c];
+        if (!LEAN && act && own) bl[brec_inv(N) + c * HP + j] = a[c];
       }
     }
     __syncwarp();
@@ -644,9 +737,26 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
 
   // --------------------------------------------------------------------- up
   bool nonfinite = false;
-  const double wd = own ? 0.5 * p.tables[tab_wt(N) + j] / dj : 0.0;  // w / (2 d) of stream j
-  const double muj = p.tables[tab_mu(N) + j];
-  const double rumu0 = beam ? 1.0 / umu0 : 0.0;
+  // the eight outputs of a level from its angular sums (mean intensities su, sd, fluxes
+  // fu, fd), the beam factor `fact` and the Planck source
+  auto level_out = [&](double (&o)[8], double su, double sd, double fu, double fd, double fact, double ch,
+                       double utau, double w1, double plsorc) {
+    double dirint = 0.0, fldir = 0.0, fdir = 0.0;
+    if (beam) {
+      dirint = fbeam * fact;
+      fldir = umu0 * fbeam * fact;
+      fdir = SPH ? fabs(umu0) * fbeam * exp(-utau / ch) : umu0 * fbeam * exp(-utau * rumu0);
+    }
+    fu *= 2.0 * PI;
+    fd *= 2.0 * PI;
+    const double fdn = (fd + fldir) - fdir;
+    constexpr double R4PI = 1.0 / (4.0 * PI);
+    const double ua = 0.5 * (su + sd) + dirint * R4PI;
+    const double uaso = dirint * R4PI;
+    const double uad = 0.5 * sd, uau = 0.5 * su;
+    const double dfdt = w1 * 4.0 * PI * (ua - plsorc);
+    o[0] = fdir, o[1] = fdn, o[2] = fu, o[3] = dfdt, o[4] = ua, o[5] = uad, o[6] = uau, o[7] = uaso;
+  };
   // fluxes at output level lu of layer l from the modal amplitudes (c, d) of the
   // homogeneous part there (computeFluxes, FluxSolver.cpp:1138-1287;
   // DisortSolver.cpp:1980-2124); `put`: this team has the level
@@ -672,22 +782,8 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
       fd += __shfl_xor_sync(0xffffffffu, fd, off);
     }
     if (put) {
-      double dirint = 0.0, fldir = 0.0, fdir = 0.0;
-      if (beam) {
-        dirint = fbeam * fact;
-        fldir = umu0 * fbeam * fact;
-        fdir = SPH ? fabs(umu0) * fbeam * exp(-utau / ch) : umu0 * fbeam * exp(-utau * rumu0);
-      }
-      fu *= 2.0 * PI;
-      fd *= 2.0 * PI;
-      const double fdn = (fd + fldir) - fdir;
-      constexpr double R4PI = 1.0 / (4.0 * PI);
-      const double ua = 0.5 * (su + sd) + dirint * R4PI;
-      const double uaso = dirint * R4PI;
-      const double uad = 0.5 * sd, uau = 0.5 * su;
-      const double plsorc = thermal ? fma(vec[7 * HP + 1], utaupr, vec[7 * HP]) : 0.0;
-      const double dfdt = w1 * 4.0 * PI * (ua - plsorc);
-      const double o[8] = {fdir, fdn, fu, dfdt, ua, uad, uau, uaso};
+      double o[8];
+      level_out(o, su, sd, fu, fd, fact, ch, utau, w1, thermal ? fma(vec[7 * HP + 1], utaupr, vec[7 * HP]) : 0.0);
 #pragma unroll
       for (int f = 0; f < 8; ++f)
         if ((f & (TEAM - 1)) == t) {
@@ -711,6 +807,103 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
         if ((int)lyr_l[lu] > ncut - 1)
           for (int f = 0; f < 8; ++f) outp[f][oidx(lu)] = 0.0;
   }
+  if constexpr (LEAN) {
+    // what the lane needs of layer l, loaded two layers ahead: row j of W, f, g, the
+    // flux functionals of its bottom level
+    struct Up { double2 w[HP / 2], fg, u; double dphi; };
+    auto load_rec = [&](int l) {
+      Up q{};
+      if (l >= 0 && l < ncut) {
+        const double* br = brec0 + (long long)l * BSTRIDE;
+        const double2* row = reinterpret_cast<const double2*>(br + j * HP);
+#pragma unroll
+        for (int k = 0; k < HP / 2; ++k) q.w[k] = row[k];
+        const double2* v = reinterpret_cast<const double2*>(br + trec_v(N) + 4 * j);
+        q.fg = v[0];
+        if (own) q.u = v[1];
+        if (thermal && beam) q.dphi = br[trec_dphi(N) + j];
+      }
+      return q;
+    };
+    // TEAM consecutive levels are put out together, one per lane: their sums (kept when
+    // the sweep passes the level) and scalars, loaded a group ahead
+    struct Lev { double t1, u1, w1, pl, ch; };
+    auto load_lev = [&](int base) {
+      const int lev = base + t, la = lev > 0 ? lev - 1 : 0;  // the layer above
+      Lev v{0.0, 0.0, 0.0, 0.0, 1.0};
+      if (base >= 0 && lev <= ncut && act) {
+        v.w1 = 1.0 - p.ssa(i, ifb ? L - 1 - la : la);
+        if (thermal) v.pl = brec0[(long long)la * BSTRIDE + trec_pl(N) + (lev > 0 ? 1 : 0)];
+        if (beam) {
+          v.t1 = taus[lev];
+          v.u1 = rec[il.tauc + lev];
+          if (SPH) v.ch = SR(la)[sph_ch(N)];
+        }
+      }
+      return v;
+    };
+    const double wdm = wd * muj;
+    double su = 0.0, sd = 0.0, fu = 0.0, fd = 0.0;
+    Lev lev = load_lev(Lw & ~(TEAM - 1));
+    // level lu from this lane's phi (+ dphi), with psi's part sum u phi + w g
+    auto level = [&](int lu, double phi, double dphi, double g, double u0, double u1) {
+      double p0 = wd * (phi + dphi), p1 = wdm * (phi + dphi), q0 = fma(u0, phi, wd * g), q1 = fma(u1, phi, wdm * g);
+#pragma unroll
+      for (int off = TEAM / 2; off > 0; off >>= 1) {
+        p0 += __shfl_xor_sync(0xffffffffu, p0, off);
+        p1 += __shfl_xor_sync(0xffffffffu, p1, off);
+        q0 += __shfl_xor_sync(0xffffffffu, q0, off);
+        q1 += __shfl_xor_sync(0xffffffffu, q1, off);
+      }
+      if ((lu & (TEAM - 1)) == t) {
+        su = p0 + q0;
+        sd = p0 - q0;
+        fu = p1 + q1;
+        fd = p1 - q1;
+      }
+      if ((lu & (TEAM - 1)) == 0) {
+        if (act && lu + t <= ncut) {
+          double o[8];
+          const double fact = beam ? (SPH ? exp(-lev.t1 / lev.ch) : exp(-lev.t1 * rumu0)) : 0.0;
+          level_out(o, su, sd, fu, fd, fact, lev.ch, lev.u1, lev.w1, lev.pl);
+#pragma unroll
+          for (int f = 0; f < 8; ++f) {
+            outp[f][oidx(lu + t)] = o[f];
+            if (!isfinite(o[f])) nonfinite = true;
+          }
+        }
+        lev = load_lev(lu - TEAM);
+      }
+    };
+    double phi = ve[j];
+    // one layer from its record, which then takes the one two layers up (two of them in
+    // turn: a register move would wait for the load)
+    auto step = [&](int l, Up& c) {
+      double* const buf = l & 1 ? vgam : ve;
+      if (own) buf[j] = phi;
+      __syncwarp();
+      level(l + 1, phi, c.dphi, c.fg.y, c.u.x, c.u.y);
+      double s0 = c.fg.x, s1 = 0.0;
+#pragma unroll
+      for (int k = 0; k < H; k += 2) {
+        const double2 v = reinterpret_cast<const double2*>(buf)[k / 2];
+        s0 = fma(c.w[k / 2].x, v.x, s0);
+        if (k + 1 < H) s1 = fma(c.w[k / 2].y, v.y, s1);
+      }
+      if (l < ncut) phi = s0 + s1;
+      c = load_rec(l - 2);
+    };
+    Up q = load_rec(Lw - 1), q2 = load_rec(Lw - 2);
+    int l = Lw - 1;
+    for (; l > 0; l -= 2) {
+      step(l, q);
+      step(l - 1, q2);
+    }
+    if (l == 0) step(0, q);
+    // the top: A = I, g = -2 d (incoming)
+    const double inc = act ? rec[H_FISOT] + rec[H_PTOP] : 0.0;
+    level(0, phi, 0.0, own ? -2.0 * dj * inc : 0.0, wd, wdm);
+  } else {
   const int NTw = GEN && m == 0 ? (int)__reduce_max_sync(0xffffffffu, act ? (unsigned)NT : 0u) : 0;
   auto load_up = [&](int l, int what) {
     if (l >= 0 && l < ncut) {
@@ -790,6 +983,7 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
     DSP_PHASE(9)
   }
   cp_async_wait<0>();
+  }  // !LEAN
   DSP_PHASE_END
   if (act) {
     if (singular && t == 0) set_status(p.status, i, DSP_ERR_SINGULAR);
@@ -798,11 +992,12 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
 }
 
 // One team per instance, in chunk-slot order.
-template <int N, bool GEN = false, bool SPH = false>
+// JAC: the Jacobian kernel follows and reads the records of the general form.
+template <int N, bool GEN = false, bool SPH = false, bool JAC = false>
 __global__ void __launch_bounds__(32, BCfg<N>::MINB) flux_bvp_kernel(FluxParams p) {
   using C = BCfg<N>;
   const int slot = blockIdx.x * C::TPW + threadIdx.x / C::TEAM;
-  bvp_warp<N, GEN, SPH>(p, slot < p.n ? slot : -1);
+  bvp_warp<N, GEN, SPH, !GEN && !JAC && C::LEAN>(p, slot < p.n ? slot : -1);
 }
 
 // Persistent form (general solver): a resident grid whose warps take chunk slots
@@ -820,7 +1015,7 @@ __global__ void __launch_bounds__(32, BCfg<N>::MINB) gen_bvp_persistent_kernel(F
     k = __shfl_sync(0xffffffffu, k, 0);
     if (k >= p.n) break;
     k += threadIdx.x / C::TEAM;
-    bvp_warp<N, true, SPH>(p, k < p.n ? order[k] : -1);
+    bvp_warp<N, true, SPH, false>(p, k < p.n ? order[k] : -1);
     __syncwarp();  // the shared memory serves the next instances
   }
 }

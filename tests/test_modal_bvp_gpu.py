@@ -51,6 +51,29 @@ def test_partial_warps_and_extreme_layers(N, n, L):
         assert_parity(got, ref, f"N={N} n={n} L={L} thermal={thermal}")
 
 
+@pytest.mark.parametrize("N", [n for n in capi.SUPPORTED_NSTR if n <= 16])
+@pytest.mark.parametrize("n,L", [(1, 1), (2, 8), (9, 17), (35, 40)])
+def test_levels_below_the_absorption_cut(N, n, L):
+    """Thermal columns with a beam, absorbing enough that the cut falls inside them: the
+    boundary-value problem has no beam there, the fluxes still add its particular
+    solution.  The two forms of the upward pass (fluxes alone, and before Jacobians)
+    against the oracle; level groups of every length."""
+    w = columns(N, n, L, 11 * N + n, True)
+    w["arrays"]["delta_tau"] = np.where(w["arrays"]["delta_tau"] > 0, w["arrays"]["delta_tau"] * 4.0, 0.0)
+    for extra in (0, capi.FLAG_INDEX_FROM_BOTTOM):
+        got, gst, rc = gpu_lib.flux_solve(w, extra)
+        jac = gpu_lib.flux_solve_jac(w, extra)
+        ref, rst = oracle_lib.flux_solve(w, extra_flags=extra, ext=True)
+        assert rc == 0 and not gst.any() and not rst.any()
+        for form, out in (("fluxes", got), ("before Jacobians", jac[0])):
+            # the divergence is 4 pi (1 - omega) (mean intensity - Planck): it has the
+            # parity of the mean intensity, not of its own difference
+            div = np.abs(out["flux_tau_divergence"] - ref["flux_tau_divergence"])
+            assert (div <= 1e-9 * (4 * np.pi * ref["mean_intensity"] + np.abs(ref["flux_tau_divergence"])) + 1e-12).all()
+            rest = dict(out, flux_tau_divergence=ref["flux_tau_divergence"])
+            assert_parity(rest, ref, f"{form} N={N} n={n} L={L} flags={extra}")
+
+
 @pytest.mark.parametrize("N", capi.SUPPORTED_NSTR)
 def test_conservative_columns_conserve_the_net_flux(N):
     w = columns(N, 9, 12, 7 * N, False, ssa=1.0)
