@@ -84,7 +84,12 @@ dsp_status launch_flux_chunk(dsp_context ctx, const FluxParams& p, cudaStream_t 
     if (jv) flux_bvp_kernel<N, false, SPH, C::LEAN><<<grid, 32, C::smem_bytes(), s>>>(p);
     else flux_bvp_kernel<N, false, SPH><<<grid, 32, C::smem_bytes(), s>>>(p);
   }
-  if (jv) {
+  if (jv && BCfg<N>::LEAN) {
+    if constexpr (BCfg<N>::LEAN) {
+      KernelTimer kt(ctx, "flux_jac_kernel", s);
+      flux_jac_lean_kernel<N><<<p.n, JLCfg<N>::KB, JLCfg<N>::smem_bytes(), s>>>(p, *jv);
+    }
+  } else if (jv) {
     using C = JCfg<N>;
     static bool attr = false;
     if (!attr) {

@@ -135,6 +135,15 @@ __host__ __device__ constexpr int trec_v(int N) { return (N / 2) * mod_hp(N); }
 __host__ __device__ constexpr int trec_dphi(int N) { return trec_v(N) + 2 * N; }
 __host__ __device__ constexpr int trec_pl(int N) { return trec_dphi(N) + mod_hp(N); }
 __host__ __device__ constexpr int trec_stride(int N) { return round4(trec_pl(N) + 2); }
+// With Jacobians to follow (flux_jac.cuh): R [h][HP] | per stream what a thermal source's
+// value at the top, at the bottom and its slope add to f, then to g [h][6] | inverse of
+// the surface system [h][HP] (the last layer's).
+__host__ __device__ constexpr int tjac_R(int N) { return trec_stride(N); }
+__host__ __device__ constexpr int tjac_s(int N) { return tjac_R(N) + (N / 2) * mod_hp(N); }
+__host__ __device__ constexpr int tjac_inv(int N) { return round4(tjac_s(N) + 3 * N); }
+__host__ __device__ constexpr int tjac_stride(int N) { return round4(tjac_inv(N) + (N / 2) * mod_hp(N)); }
+static_assert(tjac_stride(4) <= brec_stride(4) && tjac_stride(6) <= brec_stride(6) && tjac_stride(16) <= brec_stride(16),
+              "Jacobian record");
 static_assert(trec_stride(4) <= brec_stride(4) && trec_stride(6) <= brec_stride(6) && trec_stride(16) <= brec_stride(16),
               "transmission record");
 static_assert(mod_size(4) <= lrec_stride(4) && mod_size(6) <= lrec_stride(6) && mod_size(14) <= lrec_stride(14) &&

@@ -204,7 +204,7 @@ __device__ __forceinline__ void axpy_row(double* acc, const double* row, const d
 }
 
 // The instances of one warp: team `team` solves chunk slot `slot` (-1: none).
-template <int N, bool GEN, bool SPH, bool LEAN>
+template <int N, bool GEN, bool SPH, bool LEAN, bool JAC = false>
 __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
   using C = BCfg<N>;
   constexpr int H = C::H, HP = C::HP, TEAM = C::TEAM, LDM = C::LDM, SB = C::SB;
@@ -244,7 +244,7 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
   const long long lay0 = GEN ? p.g.lay_off[sl] : (long long)i * p.L;
   const long long lstride = GEN ? p.g.lstride : (long long)lrec_stride(N);
   const double* const lrec0 = p.layer_rec + (GEN ? mrow * p.g.ms_layer : 0ll) + lay0 * lstride;
-  constexpr int BSTRIDE = LEAN ? trec_stride(N) : brec_stride(N);
+  constexpr int BSTRIDE = LEAN ? (JAC ? tjac_stride(N) : trec_stride(N)) : brec_stride(N);
   double* const brec0 = p.bvp_rec + (GEN ? mrow * p.g.ms_bvp : 0ll) + lay0 * BSTRIDE;
   auto oidx = [&](int lev) {
     if constexpr (GEN) return (long long)i * p.g.ntau_out + (ifb ? NT - 1 - lev : lev);
@@ -378,6 +378,11 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
     particular(l, s.t0, s.b0, ct, dt_);
     particular(l, s.t1, s.b1, cb, db);
     double pl0 = 0.0, pl1 = 0.0;  // Planck source at the top and the bottom
+    double jc = 0.0, jd = 0.0;    // thermal (c, d) of a unit source
+    if (JAC) {
+      jc = vec[5 * HP + j];
+      jd = vec[6 * HP + j];
+    }
     if (LEAN && thermal) {
       pl0 = fma(vec[7 * HP + 1], s.t0, vec[7 * HP]);
       pl1 = fma(vec[7 * HP + 1], s.t1, vec[7 * HP]);
@@ -447,6 +452,8 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
     double xh = 0.0;  // X (r - c_t)
     double dphi = 0.0;
     bool past = false;
+    // for the Jacobians: R, and hv, X hv of a unit source's value at the top and slope
+    double rr[JAC ? H : 1], hv0 = 0.0, hv2 = 0.0, xj0 = 0.0, xj2 = 0.0;
     if constexpr (LEAN) {
       // V = X H E, column j, into the place of A
       double v[H];
@@ -455,6 +462,29 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
 #pragma unroll
       for (int r = 0; r < H; ++r) axpy_row<H>(v, Xs + r * LDM, a[r]);
       if (own) vgam[j] = hv;
+      if constexpr (JAC) {
+        if (own) {
+#pragma unroll
+          for (int r = 0; r < H; ++r) Ws[j * LDM + r] = v[r];  // X H
+          sbuf[j] = -jc;
+          sbuf[HP + j] = -jd;
+        }
+        __syncwarp();
+        hv0 = dot_reg<H>(a, sbuf);
+        hv2 = dot_reg<H>(a, sbuf + HP);
+#pragma unroll
+        for (int r = 0; r < H; ++r) rr[r] = 0.0;
+#pragma unroll
+        for (int r = 0; r < H; ++r) axpy_row<H>(rr, Ws + r * LDM, Xs[r * LDM + j]);  // X H X^T
+        __syncwarp();
+        if (own) {
+          sbuf[j] = hv0;
+          sbuf[HP + j] = hv2;
+        }
+        __syncwarp();
+        xj0 = dot_col<H>(Xs + j, LDM, sbuf);
+        xj2 = dot_col<H>(Xs + j, LDM, sbuf + HP);
+      }
       __syncwarp();
       xh = dot_col<H>(Xs + j, LDM, vgam);
       if (on && own) {
@@ -532,6 +562,50 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
       double f = 0.0;
       if constexpr (LEAN) {
         f = fma(2.0, dot_col<H>(As + j, LDM, vw1), -xh);
+        if constexpr (JAC) {
+          // unit sources: y = G (E (c_t + hv) - c_b), f = 2 V y - X hv, g' = Y (c_b + d + 2 y)
+          double *const b0 = sbuf, *const b1 = b0 + HP, *const b2 = b1 + HP;
+          if (own) {
+            b0[j] = ex * (jc + hv0);
+            b1[j] = -jc;
+            b2[j] = ex * hv2;
+          }
+          __syncwarp();
+          const double y0 = dot_reg<H>(a, b0), y1 = dot_reg<H>(a, b1), y2 = dot_reg<H>(a, b2);
+          __syncwarp();
+          if (own) {
+            b0[j] = 2.0 * y0;
+            b1[j] = 2.0 * y1;
+            b2[j] = 2.0 * y2;
+          }
+          __syncwarp();
+          const double f0 = dot_col<H>(As + j, LDM, b0) - xj0, f1 = dot_col<H>(As + j, LDM, b1),
+                       f2 = dot_col<H>(As + j, LDM, b2) - xj2;
+          __syncwarp();
+          if (own) {
+            b1[j] += jc;
+            b2[j] += jd;
+          }
+          __syncwarp();
+          if (on && own) {
+            double2* const o = reinterpret_cast<double2*>(br + tjac_s(N) + 6 * j);
+            o[0] = make_double2(f0, f1);
+            o[1] = make_double2(f2, dot_col<H>(Ys + j, LDM, b0));
+            o[2] = make_double2(dot_col<H>(Ys + j, LDM, b1), dot_col<H>(Ys + j, LDM, b2));
+          }
+          // R = X H X^T - V (2 G) V^T, 2 G V^T = (2 G - I) V^T + V^T
+          double gv[H];
+#pragma unroll
+          for (int r = 0; r < H; ++r) gv[r] = 0.0;
+#pragma unroll
+          for (int r = 0; r < H; ++r) axpy_row<H>(gv, Ws + r * LDM, As[r * LDM + j]);
+#pragma unroll
+          for (int r = 0; r < H; ++r) axpy_row<H>(rr, As + r * LDM, -(gv[r] + As[r * LDM + j]));
+          if (on && own) {
+#pragma unroll
+            for (int r = 0; r < H; ++r) br[tjac_R(N) + r * HP + j] = rr[r];
+          }
+        }
         // column j of W: 2 G Y^T = (2 G - I) Y^T + Y^T
         double wt[H];
 #pragma unroll
@@ -655,7 +729,7 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
 #pragma unroll
       for (int r = 0; r < H; ++r) {
         a[r] = -a[r] * (s1 * vsc[r]);
-        if (!LEAN && act && own) bl[brec_inv(N) + r * HP + j] = a[r];
+        if ((!LEAN || JAC) && act && own) bl[(JAC ? tjac_inv(N) : brec_inv(N)) + r * HP + j] = a[r];
       }
     } else {
       // bidirectional surface: R_rc = (1 + delta_m0) d_r rho_rc d_c, not
@@ -992,12 +1066,12 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
 }
 
 // One team per instance, in chunk-slot order.
-// JAC: the Jacobian kernel follows and reads the records of the general form.
+// JAC (up to 16 streams): flux_jac_lean_kernel follows and reads its part of the records.
 template <int N, bool GEN = false, bool SPH = false, bool JAC = false>
-__global__ void __launch_bounds__(32, BCfg<N>::MINB) flux_bvp_kernel(FluxParams p) {
+__global__ void __launch_bounds__(32, JAC ? 8 : BCfg<N>::MINB) flux_bvp_kernel(FluxParams p) {
   using C = BCfg<N>;
   const int slot = blockIdx.x * C::TPW + threadIdx.x / C::TEAM;
-  bvp_warp<N, GEN, SPH, !GEN && !JAC && C::LEAN>(p, slot < p.n ? slot : -1);
+  bvp_warp<N, GEN, SPH, !GEN && C::LEAN, JAC>(p, slot < p.n ? slot : -1);
 }
 
 // Persistent form (general solver): a resident grid whose warps take chunk slots

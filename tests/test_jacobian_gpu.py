@@ -91,6 +91,15 @@ def test_deep_column_more_degrees_of_freedom_than_a_pass():
     check(w, label="L=90")
 
 
+@pytest.mark.parametrize("L", [1, 62, 63, 64, 127])
+@pytest.mark.parametrize("nstr", [4, 14])
+def test_degrees_of_freedom_at_the_edges_of_a_pass(nstr, L):
+    """63 to 129 degrees of freedom: the last pass holds one, two or all of its threads,
+    and starts at the layer above its first level."""
+    w = workloads.thermal_sweep(n_bands=3, num_layers=L, num_streams=nstr, seed=L)
+    check(w, label=f"N={nstr} L={L}")
+
+
 def test_jacobian_device_pointers_equal_host_pointers_and_edge_cases():
     w = workloads.subset(workloads.thermal_sweep(), np.arange(0, 20000, 1000))
     w["arrays"]["single_scat_albedo"] = w["arrays"]["single_scat_albedo"].copy()
