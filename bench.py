@@ -242,15 +242,6 @@ def committed_traffic(workload_name: str, kernel: str):
         return None
 
 
-def general_traffic(kernel: str, n: int, launches: int):
-    """Average DRAM bytes per launch of the general path's boundary-value kernel
-    on n instances, from the committed per-instance ncu figure."""
-    if kernel != "gen_bvp_kernel" or launches <= 0:
-        return None
-    per = committed_traffic("general_mix", "gen_bvp_kernel_bytes_per_instance")
-    return None if per is None else per * n / launches
-
-
 def run_e2e(args, ctx, w, douts, stream, dev, world):
     """Same solve through the C ABI with pinned host buffers: inputs up, results
     down, inside the timed region.  Returns (solves/s, h2d bytes, d2h bytes,
@@ -497,7 +488,8 @@ GENERAL_METRIC = "solves/s (general mix: N 4-64, L 10-120, DM+, beam, 3 tau x 5 
 def general_batch(n: int, seed: int):
     insts, flags = workloads.general_mix(n, seed=seed)
     d = capi.pack_general(insts, flags)
-    fl = {"gen_layer_kernel": 0.0, "gen_bvp_kernel": 0.0, "gen_intensity_kernel": 0.0, "total": 0.0}
+    fl = {"gen_layer_kernel": 0.0, "gen_angle_kernel": 0.0, "gen_bvp_kernel": 0.0, "gen_intensity_kernel": 0.0,
+          "total": 0.0}
     for c in insts:
         ncut = flops.absorption_cut(c["delta_tau"], c["single_scat_albedo"], False)
         modes = 1 if abs(1.0 - c["direct_beam_mu"]) < 1e-5 else c["num_streams"]
@@ -753,9 +745,7 @@ def measure_general(ctx, stream, dev, n, seed, steps, warmup, world=1, rank=0, e
                 "peak_source": "measured on this GPU by disort_b200/csrc/fp64_peak.cu (FP64 FMA chains, burst)",
                 "flops_per_step": fl[dom], "flops_total_per_step": fl["total"],
                 "avg_launch_ms": dom_ms / max(1, dom_launches),
-                "traffic": general_traffic(dom, n, dom_launches),
-                "traffic_source": "profiles/traffic.json (ncu DRAM bytes per instance-solve of the boundary-value "
-                                  "kernels on a 512-instance mix, x instances / launches)",
+                "traffic": None,  # not captured for the mix
                 "kernel_ms_per_step": {k: v[0] / args.steps for k, v in ktimes.items()},
                 "all_kernels_tflops": fl["total"] * args.steps / (ms_max / 1000.0) / 1e12}
     cpu, parity = None, None

@@ -2,7 +2,7 @@
 
 The engine has more than one way to launch some of its stages; which is faster
 depends on the stream count N and the layer count L of the instances:
-  - flux path, N <= 16: the layer stage as three one-thread-per-task launches
+  - flux path, N <= 16: the layer stage as two one-thread-per-task launches
     (eigensolver in registers; 64 or 128 threads per CTA) or as one team per
     layer task (eigensolver in shared memory);
   - general path: the boundary-value kernel as one CTA or team per instance in

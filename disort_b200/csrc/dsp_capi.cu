@@ -84,20 +84,20 @@ dsp_status launch_flux_chunk(dsp_context ctx, const FluxParams& p, cudaStream_t 
     if (jv) flux_bvp_kernel<N, false, SPH, C::LEAN><<<grid, 32, C::smem_bytes(), s>>>(p);
     else flux_bvp_kernel<N, false, SPH><<<grid, 32, C::smem_bytes(), s>>>(p);
   }
-  if (jv && BCfg<N>::LEAN) {
+  if (jv) {
     if constexpr (BCfg<N>::LEAN) {
       KernelTimer kt(ctx, "flux_jac_kernel", s);
       flux_jac_lean_kernel<N><<<p.n, JLCfg<N>::KB, JLCfg<N>::smem_bytes(), s>>>(p, *jv);
+    } else {
+      using C = JCfg<N>;
+      static bool attr = false;
+      if (!attr) {
+        cudaFuncSetAttribute(flux_jac_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem_bytes());
+        attr = true;
+      }
+      KernelTimer kt(ctx, "flux_jac_kernel", s);
+      flux_jac_kernel<N><<<p.n, C::KB, C::smem_bytes(), s>>>(p, *jv);
     }
-  } else if (jv) {
-    using C = JCfg<N>;
-    static bool attr = false;
-    if (!attr) {
-      cudaFuncSetAttribute(flux_jac_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem_bytes());
-      attr = true;
-    }
-    KernelTimer kt(ctx, "flux_jac_kernel", s);
-    flux_jac_kernel<N><<<p.n, C::KB, C::smem_bytes(), s>>>(p, *jv);
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(ctx, e, "flux kernel launch");

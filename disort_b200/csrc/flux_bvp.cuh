@@ -977,6 +977,7 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
     // the top: A = I, g = -2 d (incoming)
     const double inc = act ? rec[H_FISOT] + rec[H_PTOP] : 0.0;
     level(0, phi, 0.0, own ? -2.0 * dj * inc : 0.0, wd, wdm);
+    DSP_PHASE(9)
   } else {
   const int NTw = GEN && m == 0 ? (int)__reduce_max_sync(0xffffffffu, act ? (unsigned)NT : 0u) : 0;
   auto load_up = [&](int l, int what) {

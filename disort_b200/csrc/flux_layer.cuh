@@ -42,9 +42,9 @@ namespace dsp {
 template <int N>
 struct LCfg {
   static constexpr int NN = N / 2;
-  // 64 streams: a 128-thread team per layer (two threads per stream)
-  static constexpr int TEAM = N >= 64 ? 2 * N : (pow2ceil(N) < 4 ? 4 : pow2ceil(N));
-  static constexpr int CTA = TEAM >= 32 ? TEAM : 128;
+  static_assert(N <= 16, "the team kernel serves N <= 16 on the flux path");
+  static constexpr int TEAM = pow2ceil(N);
+  static constexpr int CTA = 128;
   static constexpr int TPC = CTA / TEAM;
   static constexpr int NNP = NN + (NN & 1);
   static constexpr int NPAIR = NNP / 2;
@@ -60,8 +60,7 @@ struct LCfg {
   static constexpr int O_GL = O_T + MAT;   // g'_l [N]
   static constexpr int O_B1 = O_GL + N;    // beam source sums, D M^{-1} (q+ +/- q-) [NN] each
   static constexpr int O_B2 = O_B1 + NN;
-  static constexpr int O_ROT = O_B2 + NN;  // c, s, t per pair
-  static constexpr int O_MISC = O_ROT + 3 * NPAIR;  // flags
+  static constexpr int O_MISC = O_B2 + NN;  // flags
   static constexpr int TEAM_SMEM = round4(O_MISC + 8);
   static constexpr int TAB = tab_ylm(N);   // mu, wt, dsim, dinv; the Legendre table is read through L1
   static constexpr size_t smem_bytes() { return sizeof(double) * (size_t)(TAB + TPC * TEAM_SMEM); }
@@ -144,42 +143,10 @@ __device__ __forceinline__ int rr_player(int r, int j) {
   return j == 0 ? 0 : 1 + x;
 }
 
-// Cholesky of the lower triangle of M (NN x NN, stride NS) into Lc; false if
-// not SPD.  `flag` is team scratch; every thread leaves through a team
-// barrier, so the caller may reuse it immediately.
-template <int NN, int NS, int TEAM>
-__device__ bool team_cholesky(const double* M, double* Lc, double* flag, int t) {
-  for (int i = t; i < NN * NS; i += TEAM) Lc[i] = 0.0;
-  if (t == 0) flag[0] = 0.0;
-  team_sync<TEAM>();
-  for (int j = 0; j < NN; ++j) {
-    if (t == 0) {
-      double d = M[j * NS + j];
-      for (int k = 0; k < j; ++k) d -= Lc[j * NS + k] * Lc[j * NS + k];
-      if (!(d > 0.0)) flag[0] = 1.0;
-      else Lc[j * NS + j] = sqrt(d);
-    }
-    team_sync<TEAM>();
-    const bool failed = flag[0] != 0.0;
-    team_sync<TEAM>();
-    if (failed) return false;
-    const double ljj = Lc[j * NS + j];
-    for (int i = t; i < NN; i += TEAM)
-      if (i > j) {
-        double s = M[i * NS + j];
-        for (int k = 0; k < j; ++k) s -= Lc[i * NS + k] * Lc[j * NS + k];
-        Lc[i * NS + j] = s / ljj;
-      }
-    team_sync<TEAM>();
-  }
-  return true;
-}
-
-
-
-// Right-looking Cholesky with row i held by thread i (sub-warp teams): column
-// j's entries are broadcast by shuffles, no barriers.  Same contract as
-// team_cholesky.
+// Right-looking Cholesky of the lower triangle of M (NN x NN, stride NS) into Lc,
+// row i held by thread i (sub-warp teams): column j's entries are broadcast by
+// shuffles.  False if M is not positive definite; every thread leaves through a
+// team barrier.
 template <int NN, int NS, int TEAM>
 __device__ bool team_cholesky_reg(const double* M, double* Lc, int t) {
   static_assert(TEAM <= 32, "shuffle Cholesky needs a sub-warp team");
@@ -205,12 +172,6 @@ __device__ bool team_cholesky_reg(const double* M, double* Lc, int t) {
     for (int k = t + 1; k < NN; ++k) Lc[t * NS + k] = 0.0;
   team_sync<TEAM>();
   return ok;
-}
-
-template <int NN, int NS, int TEAM>
-__device__ __forceinline__ bool team_chol(const double* M, double* Lc, double* flag, int t) {
-  if constexpr (TEAM <= 32) return team_cholesky_reg<NN, NS, TEAM>(M, Lc, t);
-  else return team_cholesky<NN, NS, TEAM>(M, Lc, flag, t);
 }
 
 // Whether the Jacobi rotation of pair (p, q) is applied: |apq| above 1e-15 of
@@ -343,7 +304,7 @@ __device__ __forceinline__ void thermal_source(const Q& q, double& xr0, double& 
 // ---------------------------------------------------------------------------
 // Layer stage with a team of threads per task, matrices in shared memory.
 // ---------------------------------------------------------------------------
-template <int N, bool GEN = false>
+template <int N>
 __global__ void __launch_bounds__(LCfg<N>::CTA, LCfg<N>::MINB) flux_layer_kernel(FluxParams p) {
   using C = LCfg<N>;
   constexpr int NN = C::NN, TEAM = C::TEAM, NNP = C::NNP, NPAIR = C::NPAIR, NS = C::NS, BPT = C::BPT;
@@ -351,19 +312,18 @@ __global__ void __launch_bounds__(LCfg<N>::CTA, LCfg<N>::MINB) flux_layer_kernel
   constexpr int BPA = NPAIR;  // blocks (a, b) per column pair b
   extern __shared__ double smem[];
   // CTA-level constant tables
-  const int m = mode_of<GEN>(p);
   for (int k = threadIdx.x; k < C::TAB; k += blockDim.x) smem[k] = p.tables[k];
   __syncthreads();
   const double* mu = smem + tab_mu(N);
   const double* wt = smem + tab_wt(N);
   const double* dsim = smem + tab_dsim(N);
   const double* dinv = smem + tab_dinv(N);
-  const double* Y = p.tables + (long long)mode_row<GEN>() * tab_size(N) + tab_ylm(N);
+  const double* Y = p.tables + tab_ylm(N);
 
   const int team = threadIdx.x / TEAM, t = threadIdx.x % TEAM;
   const long long task = (long long)blockIdx.x * C::TPC + team;
-  if (task >= layer_tasks<GEN>(p)) return;
-  const LayerTask<N, GEN> q = layer_task<N, GEN>(p, task);
+  if (task >= layer_tasks<false>(p)) return;
+  const LayerTask<N, false> q = layer_task<N, false>(p, task);
   if (!q.live) return;
   double* sm = smem + C::TAB + team * C::TEAM_SMEM;
   double* MA = sm + C::O_A;
@@ -374,24 +334,22 @@ __global__ void __launch_bounds__(LCfg<N>::CTA, LCfg<N>::MINB) flux_layer_kernel
   double* gl = sm + C::O_GL;
   double* b1 = sm + C::O_B1;
   double* b2 = sm + C::O_B2;
-  double* rot = sm + C::O_ROT;
   double* misc = sm + C::O_MISC;
   const double ws = q.rec[q.il.ssa_s + q.lc];
   {
     const int mode = (int)q.rec[q.il.mode + q.lc];
     const double f = q.rec[q.il.fsc + q.lc], sig = q.rec[q.il.sig + q.lc];
-    for (int k = t; k < N; k += TEAM) gl[k] = phase_coeff<GEN>(k, q.pml[k], mode, ws, f, sig);
+    for (int k = t; k < N; k += TEAM) gl[k] = phase_coeff<false>(k, q.pml[k], mode, ws, f, sig);
   }
   team_sync<TEAM>();
-  const int odd0 = GEN ? 1 - (m & 1) : 1;  // first l of odd l + m
   // ---- -A_s and -B_s from the even and odd phase sums ----------------------
   for (int it = t; it < NN * NN; it += TEAM) {
     const int r = it / NN, c = it % NN;
     if (c > r) continue;
     double so = 0.0, se = 0.0;
     for (int l = 0; l < N; l += 2) {
-      so += (gl[l + odd0] * Y[(l + odd0) * N + r]) * Y[(l + odd0) * N + c];
-      se += (gl[l + 1 - odd0] * Y[(l + 1 - odd0) * N + r]) * Y[(l + 1 - odd0) * N + c];
+      so += (gl[l + 1] * Y[(l + 1) * N + r]) * Y[(l + 1) * N + c];
+      se += (gl[l] * Y[(l) * N + r]) * Y[(l) * N + c];
     }
     const double rm = 1.0 / mu[r], dl = r == c ? rm : 0.0;
     const double vb = -dsim[r] * ((wt[c] * so) * rm - dl) * dinv[c];
@@ -405,13 +363,13 @@ __global__ void __launch_bounds__(LCfg<N>::CTA, LCfg<N>::MINB) flux_layer_kernel
   const bool beam = fbeam > 0.0;
   if (beam) {
     // (2 - delta_m0) F0 / 4pi sum_k g'_k P_k^m(mu_r) P_k^m(-mu0) by parity (DisortSolver.cpp:1361-1368)
-    const double* yb = beam_legendre<N, GEN>(p, q);
-    const double fac = ((GEN && m > 0) ? 2.0 * fbeam : fbeam) / (4.0 * 3.14159265358979323846);
+    const double* yb = beam_legendre<N, false>(p, q);
+    const double fac = fbeam / (4.0 * 3.14159265358979323846);
     for (int r = t; r < NN; r += TEAM) {
       double so = 0.0, se = 0.0;
       for (int l = 0; l < N; l += 2) {
-        so += gl[l + odd0] * Y[(l + odd0) * N + r] * yb[l + odd0];
-        se += gl[l + 1 - odd0] * Y[(l + 1 - odd0) * N + r] * yb[l + 1 - odd0];
+        so += gl[l + 1] * Y[(l + 1) * N + r] * yb[l + 1];
+        se += gl[l] * Y[(l) * N + r] * yb[l];
       }
       const double dm = dsim[r] / mu[r];
       b1[r] = dm * (2.0 * fac * se);
@@ -420,8 +378,8 @@ __global__ void __launch_bounds__(LCfg<N>::CTA, LCfg<N>::MINB) flux_layer_kernel
   }
   team_sync<TEAM>();
   // ---- Cholesky of -B_s, else of -A_s (:521-558) ---------------------------
-  bool primary = team_chol<NN, NS, TEAM>(MB, LC, misc, t);
-  if (!primary && !team_chol<NN, NS, TEAM>(MA, LC, misc, t)) {
+  bool primary = team_cholesky_reg<NN, NS, TEAM>(MB, LC, t);
+  if (!primary && !team_cholesky_reg<NN, NS, TEAM>(MA, LC, t)) {
     if (t == 0) set_status(p.status, q.i, DSP_ERR_EIGEN);
     return;
   }
@@ -462,31 +420,14 @@ __global__ void __launch_bounds__(LCfg<N>::CTA, LCfg<N>::MINB) flux_layer_kernel
           jacobi_rot(Sc[pp * NS + qq], Sc[pp * NS + pp], Sc[qq * NS + qq], c, sn, tt);
         }
       }
-      if constexpr (TEAM > 32) {
-        if (t < NPAIR) {
-          rot[3 * t] = c;
-          rot[3 * t + 1] = sn;
-          rot[3 * t + 2] = tt;
-        }
-        team_sync<TEAM>();
-      }
 #pragma unroll
       for (int k = 0; k < BPT; ++k) {
         const int blk = t + k * TEAM;
         const bool act = blk < NPAIR * NPAIR;
         const int a = act ? blk / NPAIR : 0, b = act ? blk % NPAIR : 0;  // NPAIR is a power of two or small
-        double ca, sa, ta, cb, sb;
-        if constexpr (TEAM <= 32) {
-          const unsigned m = team_mask<TEAM>();
-          ca = __shfl_sync(m, c, a, TEAM);
-          sa = __shfl_sync(m, sn, a, TEAM);
-          ta = __shfl_sync(m, tt, a, TEAM);
-          cb = __shfl_sync(m, c, b, TEAM);
-          sb = __shfl_sync(m, sn, b, TEAM);
-        } else {
-          ca = rot[3 * a]; sa = rot[3 * a + 1]; ta = rot[3 * a + 2];
-          cb = rot[3 * b]; sb = rot[3 * b + 1];
-        }
+        const unsigned m = team_mask<TEAM>();
+        const double ca = __shfl_sync(m, c, a, TEAM), sa = __shfl_sync(m, sn, a, TEAM), ta = __shfl_sync(m, tt, a, TEAM);
+        const double cb = __shfl_sync(m, c, b, TEAM), sb = __shfl_sync(m, sn, b, TEAM);
         if (!act) continue;
         const int pa = rr_player<NNP>(r, a), qa = rr_player<NNP>(r, NNP - 1 - a);
         const int pb = rr_player<NNP>(r, b), qb = rr_player<NNP>(r, NNP - 1 - b);
@@ -607,26 +548,17 @@ __global__ void __launch_bounds__(LCfg<N>::CTA, LCfg<N>::MINB) flux_layer_kernel
       bool res = false;
       for (int e = 0; e < NN; ++e) res = res || beam_resonant(mode_k(Sc[e * NS + e]), umu0);
       if (res) umu0 = 0.999 * umu0;
-      if (GEN && (p.flags & DSP_FLAG_SPHERICAL_BEAM)) {
-        // pseudo-spherical beam (general solver): the raw source at the quadrature
-        // angles, up and down, for the user-angle interpolation and
-        // flux_sph_source_kernel (DisortSolver.cpp:1524-1527)
-        const double dm = 0.5 * mu[c] / dsim[c];
-        vec[mod_cb(N) + c] = dm * (b1[c] + b2[c]);
-        vec[mod_db(N) + c] = dm * (b1[c] - b2[c]);
-      } else {
-        double al = 0.0, be = 0.0;
-        for (int r = 0; r < NN; ++r) {
-          al += x[r * NS] * b1[r];
-          be += y[r * NS] * b2[r];
-        }
-        const double r0 = 1.0 / umu0, ka = lneg && primary ? -k : k, kb = lneg && !primary ? -k : k;
-        const double den = ka * kb - r0 * r0;
-        vec[mod_cb(N) + c] = (kb * al - be * r0) / den;
-        vec[mod_db(N) + c] = (ka * be - al * r0) / den;
+      double al = 0.0, be = 0.0;
+      for (int r = 0; r < NN; ++r) {
+        al += x[r * NS] * b1[r];
+        be += y[r * NS] * b2[r];
       }
+      const double r0 = 1.0 / umu0, ka = lneg && primary ? -k : k, kb = lneg && !primary ? -k : k;
+      const double den = ka * kb - r0 * r0;
+      vec[mod_cb(N) + c] = (kb * al - be * r0) / den;
+      vec[mod_db(N) + c] = (ka * be - al * r0) / den;
     }
-    if ((p.flags & DSP_FLAG_THERMAL) && m == 0) {
+    if (p.flags & DSP_FLAG_THERMAL) {
       double v = 0.0;
       for (int r = 0; r < NN; ++r) v += x[r * NS] * (dsim[r] / mu[r]);
       v = 2.0 * (1.0 - ws) * v / (lneg && primary ? -k : k);
@@ -1694,9 +1626,9 @@ __global__ void __launch_bounds__(32, WCfg<N>::MINB) flux_layer_warp_kernel(Flux
   if (thermal && t == 0) thermal_source(q, q.lrec[mod_xr(N)], q.lrec[mod_xr(N) + 1]);
 }
 
-// Host side of the layer stage: launches (through `wrap(kind, launch)`, which may
-// time them; kind 0: front, 1: eigensolver, 2: team kernel) the two launches of a split stage or the team kernel; `host_tab` is a
-// host copy of the (mode's) tab_* tables of N.
+// Host side of the layer stage, launched through `wrap(kind, launch)`, which may time
+// it (kind 0: front, 1: eigensolver, 2: one kernel); `host_tab` is a host copy of the
+// (mode's) tab_* tables of N.
 template <int N, bool GEN = false>
 inline void flux_layer_set_attrs() {
   if constexpr (layer_split<N>()) {
@@ -1713,8 +1645,9 @@ inline void flux_layer_set_attrs() {
 }
 
 // The layer stage of `tasks` layer tasks (of each of `modes` azimuth modes).  N >= 32:
-// the warp kernel.  split: one thread per task (N <= 16
-// only), with `cta` threads per CTA (64 or 128); otherwise the team kernel.
+// the warp kernel.  N <= 16: front and eigensolver, one thread per task, with `cta`
+// threads per CTA (64 or 128), or, when a schedule of the flux path asks for it, the
+// team kernel.
 template <int N, bool GEN = false, class Wrap>
 inline void flux_layer_launch(const FluxParams& p, long long tasks, const double* host_tab, cudaStream_t s,
                               Wrap&& wrap, bool split = layer_split<N>(), int cta = 128, int modes = 1) {

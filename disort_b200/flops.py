@@ -1,16 +1,19 @@
-"""Algorithmic FP64 operation counts of one DISORT solve (the roofline numerator).
+"""FP64 operation counts of one DISORT solve (the roofline numerators), by kernel.
 
-The counts are those of the reference algorithm (DisORT++ FluxSolver.cpp), not
-of this engine's kernels:
+Counted is what the algorithm in use cannot do without, h = N/2, a multiplication and
+an addition as two operations:
 
-* per layer (m = 0): phase matrix N^3; Cholesky, S = L^T A L, symmetric QR with
-  vectors and eigenvector recovery 16.33 NN^3 + 6 NN^2; beam and thermal particular
-  solutions (2/3 N^3 + 4 N^2) each when present;
-* boundary-value problem: the LINPACK band factorisation count
-  sum_k 2 lm_k min(ml+mu, n-k) with ml = mu = 3NN-1, n = N ncut (structural zeros
-  inside the band included, as sgbfa performs them), plus the band solve
-  2 sum lm_k + 2 sum (min(k, ml+mu+1) - 1);
-* fluxes: (L+1)(2 N^2 + 8 N).
+* layer stage: the two halves of the phase matrix 2 N h^2, two Cholesky factors and
+  their product 5/3 h^3; the eigenvectors of the h x h product as a symmetric QR
+  iteration would need them, 16.33 h^3 + 6 h^2 (the Jacobi sweeps take more), recovery
+  of X and Y 2 h^3, particular solutions 8 h^2 each;
+* boundary-value problem, modal form (csrc/flux_bvp.cuh): per layer two symmetric
+  inverses 2 h^3 each and four h^3 products of 2 operations, 12 h^3 in all, or six
+  (16 h^3) with transmission records (N <= 16, fluxes only), and its matrix-vector
+  products, 24 h^2.  The band factorisation of the reference (FluxSolver.cpp:838-1131)
+  needs about ten times as many; band_lu_flops counts those for comparison.
+* general path, per azimuth mode: the same; the user angles 2 (N - m) h + 4 h^2 per
+  layer and angle; intensities 8 N per layer, output depth and angle.
 
 Transcendental calls (exp, sqrt, log, pow) are not counted.
 """
@@ -19,14 +22,22 @@ from __future__ import annotations
 import functools
 
 
-def layer_flops(N: int, beam: bool, thermal: bool) -> float:
-    NN = N // 2
-    f = N ** 3 + 16.33 * NN ** 3 + 6 * NN ** 2
-    if beam:
-        f += (2.0 / 3.0) * N ** 3 + 4 * N ** 2
-    if thermal:
-        f += (2.0 / 3.0) * N ** 3 + 4 * N ** 2
-    return f
+def front_flops(N: int, nact: int | None = None) -> float:
+    """Phase sums and factors of one layer with nact active Legendre orders."""
+    h = N / 2
+    return 2.0 * (N if nact is None else nact) * h * h + 5.0 / 3.0 * h ** 3
+
+
+def eigen_flops(N: int, sources: int) -> float:
+    """Eigenvectors, X and Y, and the particular solutions of one layer."""
+    h = N / 2
+    return 18.33 * h ** 3 + 6 * h * h + sources * 8 * h * h
+
+
+def modal_bvp_flops(N: int, lean: bool) -> float:
+    """Both passes over one layer."""
+    h = N / 2
+    return (16.0 if lean else 12.0) * h ** 3 + 24 * h * h
 
 
 @functools.lru_cache(maxsize=None)
@@ -46,16 +57,15 @@ def band_lu_flops(N: int, ncut: int) -> float:
     return fac + sol
 
 
-def flux_flops(N: int, L: int) -> float:
-    return (L + 1) * (2.0 * N * N + 8.0 * N)
-
-
 def flux_solve_flops(N: int, L: int, beam: bool, thermal: bool, ncut: int | None = None) -> dict:
     """FLOPs of one flux solve split by the engine kernel that performs each part."""
     nc = L if ncut is None else ncut
-    lay = nc * layer_flops(N, beam, thermal)
-    bvp = band_lu_flops(N, nc) + flux_flops(N, L)
-    return {"flux_layer_kernel": lay, "flux_bvp_kernel": bvp, "total": lay + bvp}
+    front, eigen = nc * front_flops(N), nc * eigen_flops(N, int(beam) + int(thermal))
+    if N > 16:  # one kernel for the layer stage
+        front, eigen = front + eigen, 0.0
+    bvp = nc * modal_bvp_flops(N, N <= 16) + (L + 1) * 8.0 * N
+    return {"flux_layer_kernel": front, "flux_eigen_kernel": eigen, "flux_bvp_kernel": bvp,
+            "total": front + eigen + bvp}
 
 
 def absorption_cut(dtau, ssa, thermal: bool) -> int:
@@ -72,33 +82,16 @@ def absorption_cut(dtau, ssa, thermal: bool) -> int:
 
 def general_solve_flops(N: int, L: int, ncut: int, modes: int, numu: int, ntau: int, beam: bool,
                         thermal: bool) -> dict:
-    """FLOPs of one general (DisortSolver) solve, split by engine kernel.
-
-    Per azimuth mode m with nact = N - m active Legendre orders, per kept layer:
-    phase matrix 2 NN N nact, the eigensystem as in layer_flops, the beam source
-    (2/3 N^3 + 4 N^2), the thermal source at m = 0, interpEigenvec 2 nact N^2 +
-    2 numu nact N and interpSource (2 nact N + 2 numu nact per source); per mode the
-    band LU, mode-0 fluxes at the ntau output depths, and the user intensities
-    8 N ntau numu ncut.
-    """
-    NN = N // 2
-    lay = bvp = inten = 0.0
+    """FLOPs of one general (DisortSolver) solve, split by engine kernel."""
+    h = N / 2
+    lay = angle = bvp = inten = 0.0
     for m in range(modes):
         nact = N - m
-        per = 2.0 * NN * N * nact + 16.33 * NN ** 3 + 6 * NN ** 2
-        if beam:
-            per += (2.0 / 3.0) * N ** 3 + 4 * N ** 2
-        if thermal and m == 0:
-            per += (2.0 / 3.0) * N ** 3 + 4 * N ** 2
-        if numu:
-            per += 2.0 * nact * N * N + 2.0 * numu * nact * N
-            nsrc = (1 if beam else 0) + (2 if thermal and m == 0 else 0)
-            per += nsrc * (2.0 * nact * N + 2.0 * numu * nact)
-        lay += ncut * per
-        bvp += band_lu_flops(N, ncut)
+        lay += ncut * (front_flops(N, nact) + eigen_flops(N, int(beam) + int(thermal and m == 0)))
+        angle += ncut * numu * (2.0 * nact * h + 4.0 * h * h)
+        bvp += ncut * modal_bvp_flops(N, False)
         if m == 0:
-            bvp += ntau * (2.0 * N * N + 8.0 * N)
-        if numu:
-            inten += 8.0 * N * ntau * numu * ncut
-    return {"gen_layer_kernel": lay, "gen_bvp_kernel": bvp, "gen_intensity_kernel": inten,
-            "total": lay + bvp + inten}
+            bvp += ntau * (8.0 * h * h + 8.0 * N)
+        inten += 8.0 * N * ntau * numu * ncut
+    return {"gen_layer_kernel": lay, "gen_angle_kernel": angle, "gen_bvp_kernel": bvp,
+            "gen_intensity_kernel": inten, "total": lay + angle + bvp + inten}

@@ -298,7 +298,7 @@ dsp_status dsp_context_set_debug(dsp_context ctx, uint32_t flags);
  * per solver).  An entry applies to instances with num_streams == N and
  * min_layers <= num_layers <= max_layers; the first matching entry wins, and
  * without one the built-in choice stands.  Fields (0 = built-in choice):
- *   layer_stage  flux path, N <= 16: 1 = three one-thread-per-task launches
+ *   layer_stage  flux path, N <= 16: 1 = two one-thread-per-task launches
  *                (register-resident eigensolver), 2 = one team per layer task
  *                (shared-memory eigensolver);
  *   layer_cta    threads per CTA of the one-thread-per-task launches: 64 or 128;

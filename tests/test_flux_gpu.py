@@ -405,3 +405,21 @@ def test_branch_free_pivot_reciprocal_against_division():
     y, q = yd.cpu().numpy(), qd.cpu().numpy()
     ulp = np.abs(y - q) / np.spacing(np.abs(q))
     assert np.all(np.isfinite(y)) and float(ulp.max()) <= 2.0, float(ulp.max())
+
+
+@pytest.mark.parametrize("n", [1, 720, 760])
+def test_small_host_batches_equal_device_pointers(n):
+    """Host batches of up to 512 KB each way share one staging copy; 720 columns of 10
+    layers put out 509 KB, 760 go the way of larger batches.  Bit for bit the results
+    of device pointers on both sides of the line, also with Jacobians."""
+    w = workloads.thermal_sweep(n_bands=n, num_layers=10, num_streams=4, seed=n)
+    host, hst, rc = gpu_lib.flux_solve(w)
+    dev, dst = gpu_lib.flux_solve_device(w)[:2]
+    assert rc == 0 and np.array_equal(hst, dst)
+    for f in capi.FLUX_OUT_FIELDS:
+        assert np.array_equal(host[f], dev[f]), f
+    if n <= 720:
+        jh = gpu_lib.flux_solve_jac(w)
+        jd = gpu_lib.flux_solve_jac_device(w)
+        for f in jh[2]:
+            assert np.array_equal(jh[2][f], jd[2][f]), f
