@@ -9,7 +9,8 @@ pointers, and prints each phase's share of the boundary-value kernel's
 warp-time and its cycles per instance.  The phases are the kernel's DSP_PHASE
 markers (csrc/flux_bvp.cuh): going down, per layer the wait for the record with the
 exponentials, I + M, its inverse, Z, its inverse and the new admittance; the
-surface; going up, the wait for the records, the solution and the fluxes.
+surface; going up, the wait for the records, the solution and the fluxes (one
+phase with transmission records, up to 16 streams).
 """
 from __future__ import annotations
 
@@ -21,7 +22,7 @@ import numpy as np
 
 PHASES = [(0, "down: wait for the record, exponentials"), (1, "down: I + X^T A X"), (2, "down: inverse H"),
           (3, "down: H out, Z"), (4, "down: inverse G"), (5, "down: G out, Y (2G - I) Y^T"), (6, "surface"),
-          (7, "up: wait for the records"), (8, "up: solution"), (9, "up: fluxes, next records")]
+          (7, "up: wait for the records"), (8, "up: solution"), (9, "up: fluxes, next records (N <= 16: the whole way up)")]
 
 
 def main(n_bands: int = 20000) -> None:
