@@ -76,10 +76,18 @@ struct BCfg {
   static constexpr int O_G = O_S + 2 * SB;      // gathered vectors, HP each:
   static constexpr int NG = 9;                  // g, w1, w2, gamma, scale, E / phi, D / w, w mu, d
   static constexpr int SIZE = O_G + NG * HP;
-  // teams of a warp start 4 banks apart: their broadcasts are conflict-free
-  static constexpr int STRIDE = TPW == 1 ? SIZE : SIZE + ((2 - SIZE) % 16 + 16) % 16;
-  static_assert(STRIDE % 2 == 0 && NV % 2 == 0 && SB % 2 == 0, "16-byte alignment");
-  static constexpr size_t smem_bytes() { return sizeof(double) * (size_t)(TPW * STRIDE); }
+  // start of a team: the teams of a half warp are the width of a row apart, so that
+  // their column reads (8 bytes a lane) fill the banks once, and the two halves 4 banks
+  // apart, so that the broadcasts (16 bytes a team) do not meet either
+  // (20,000 x 60 layers x 16 streams with all teams 4 banks apart 1.51 ms, so 1.38 ms);
+  // STRIDE leaves room for the shift falling back between the halves
+  static constexpr int HALF = TPW > 1 ? TPW / 2 : 1;
+  static constexpr int STRIDE = (SIZE + (HALF - 1) * TEAM + 15) / 16 * 16;
+  __device__ static constexpr int start(int team) {
+    return team * STRIDE + team % HALF * TEAM + team / HALF * 2;
+  }
+  static_assert(NV % 2 == 0 && SB % 2 == 0 && TEAM % 2 == 0, "16-byte alignment");
+  static constexpr size_t smem_bytes() { return sizeof(double) * (size_t)(TPW * STRIDE + (TPW > 1 ? 18 : 0)); }
   // resident warps per SM: as many as shared memory admits (228 KB, 1 KB reserved
   // per CTA), within 128 registers a thread at 16 warps and 255 at 8
   static constexpr int MINB_SMEM = (int)((228u * 1024u) / (smem_bytes() + 1024u));
@@ -214,7 +222,7 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
   const int t = threadIdx.x % TEAM;
   const int j = t < H ? t : H - 1;  // lanes past the last column repeat it
   const bool own = t < H;
-  double* const sm = smem + (threadIdx.x / TEAM) * C::STRIDE;
+  double* const sm = smem + C::start(threadIdx.x / TEAM);
   double* const Xs = sm + C::O_X;
   double* const Ys = sm + C::O_Y;
   double* const As = sm + C::O_A;
