@@ -841,8 +841,11 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
   };
   // fluxes at output level lu of layer l from the modal amplitudes (c, d) of the
   // homogeneous part there (computeFluxes, FluxSolver.cpp:1138-1287;
-  // DisortSolver.cpp:1980-2124); `put`: this team has the level
-  auto eval_level = [&](int l, int lu, double utaupr, double utau, double w1, double c, double d, bool put) {
+  // DisortSolver.cpp:1980-2124); `put`: this team has the level; `top`: the level is the
+  // top of the column, where the downward intensities are the incoming ones (exactly: as
+  // a difference of the modes they are rounding noise of the upward ones)
+  const double incoming = act && m == 0 ? rec[H_FISOT] + rec[H_PTOP] : 0.0;
+  auto eval_level = [&](int l, int lu, double utaupr, double utau, double w1, double c, double d, bool put, bool top) {
     const double ch = SPH && beam && put ? SR(l)[sph_ch(N)] : 1.0;
     const double fact = beam ? (SPH ? exp(-utaupr / ch) : exp(-utaupr * rumu0)) : 0.0;
     double cp, dp;
@@ -854,7 +857,8 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
     }
     __syncwarp();
     const double ph = dot_col<H>(Xs + j, LDM, vgam), ps = dot_col<H>(Ys + j, LDM, vd);
-    double su = wd * (ph + ps), sd = wd * (ph - ps);
+    const double down = top ? 2.0 * dj * incoming : ph - ps, up = top ? 2.0 * ph - down : ph + ps;
+    double su = wd * up, sd = wd * down;
     double fu = muj * su, fd = muj * sd;
 #pragma unroll
     for (int off = TEAM / 2; off > 0; off >>= 1) {
@@ -983,8 +987,7 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
     }
     if (l == 0) step(0, q);
     // the top: A = I, g = -2 d (incoming)
-    const double inc = act ? rec[H_FISOT] + rec[H_PTOP] : 0.0;
-    level(0, phi, 0.0, own ? -2.0 * dj * inc : 0.0, wd, wdm);
+    level(0, phi, 0.0, own ? -2.0 * dj * incoming : 0.0, wd, wdm);
     DSP_PHASE(9)
   } else {
   const int NTw = GEN && m == 0 ? (int)__reduce_max_sync(0xffffffffu, act ? (unsigned)NT : 0u) : 0;
@@ -1052,12 +1055,12 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
           // C inside the layer from its values at the two boundaries (no cancellation)
           double cu = c;
           if (fx > 0.0) cu = (c * (e1 * -expm1(-2.0 * k * x2)) + chom_b * (e2 * -expm1(-2.0 * k * x1))) / fx;
-          eval_level(l, lu, tu, put ? utau_l[lu] : 0.0, s.w1, cu, e2 * b - e1 * av, put);
+          eval_level(l, lu, tu, put ? utau_l[lu] : 0.0, s.w1, cu, e2 * b - e1 * av, put, l == 0 && x1 == 0.0);
         }
       }
     } else {
-      eval_level(l, l + 1, s.t1, s.u1, s.w1, chom_b, b - ex * av, on);
-      if (l == 0) eval_level(0, 0, s.t0, s.u0, s.w1, c, ex * b - av, on);
+      eval_level(l, l + 1, s.t1, s.u1, s.w1, chom_b, b - ex * av, on, false);
+      if (l == 0) eval_level(0, 0, s.t0, s.u0, s.w1, c, ex * b - av, on, true);
     }
     __syncwarp();
     if (on && own) ve[j] = phi;

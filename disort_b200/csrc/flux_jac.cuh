@@ -295,6 +295,8 @@ __global__ void __launch_bounds__(64) flux_jac_kernel(FluxParams p, JacView jv) 
           u[j * KB] = cu + ft * lr[mod_ct(N) + j];
           w[j * KB] = e2v[j] * b[j] - e1v[j] * av[j] + a1 * lr[mod_dt(N) + j];
         }
+        // at the top of the column psi = phi: the incoming field does not depend on k
+        const bool top = l == 0 && x1 == 0.0;
         double su = 0.0, sd = 0.0, fu = 0.0, fd = 0.0;
         for (int r = 0; r < H; ++r) {
           double ph = 0.0, ps = 0.0;
@@ -303,6 +305,7 @@ __global__ void __launch_bounds__(64) flux_jac_kernel(FluxParams p, JacView jv) 
             ph = fma(lr[mod_X(N) + j * HP + r], u[j * KB], ph);
             ps = fma(lr[mod_Y(N) + j * HP + r], w[j * KB], ps);
           }
+          if (top) ps = ph;
           su = fma(wv[r], ph + ps, su);
           sd = fma(wv[r], ph - ps, sd);
           fu = fma(mv[r], ph + ps, fu);
