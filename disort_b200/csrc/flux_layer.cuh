@@ -835,8 +835,9 @@ __device__ __forceinline__ float jacobi_tan(double apq, double app, double aqq, 
   const float d = static_cast<float>(aqq - app), e = 2.0f * static_cast<float>(apq);
   float r;
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fmaf(d, d, e * e)));
-  const float t = __fdividef(fabsf(e), fabsf(d) + r);  // NaN when both vanish
-  const bool use = need && t <= 1.0f;
+  // columns of equal norm turn by 45 degrees; there the approximations give up to 1 + 2^-23
+  const float t = fminf(__fdividef(fabsf(e), fabsf(d) + r), 1.0f);
+  const bool use = need && e != 0.0f;
   far = use && (t > 1e-8f || g2 > 1e-16 * ab);
   const bool same = (d < 0.0f) == (e < 0.0f);  // sgn(th), sgn(0) = +1
   return use ? (same ? t : -t) : 0.0f;
