@@ -503,13 +503,14 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
       // beam (btr = 0), but the reference's fluxes there still add its particular
       // solution: X c to phi and Y d to psi of the bottom level
       if constexpr (!SPH) {
-        past = __any_sync(0xffffffffu, on && thermal && beam && s.b1 == 0.0);
+        const bool mine = on && thermal && beam && s.b1 == 0.0;
+        past = __any_sync(0xffffffffu, mine);
         if (past) {
-          const double fact = on && beam && s.b1 == 0.0 ? exp(-s.t1 * rumu0) : 0.0;
+          const double fact = mine ? exp(-s.t1 * rumu0) : 0.0;
           __syncwarp();
-          if (own) {
-            vgam[j] = vec[3 * HP + j] * fact;
-            vdp[j] = vec[4 * HP + j] * fact;
+          if (own) {  // (a column without a beam has no beam terms in its record)
+            vgam[j] = mine ? vec[3 * HP + j] * fact : 0.0;
+            vdp[j] = mine ? vec[4 * HP + j] * fact : 0.0;
           }
           __syncwarp();
           dphi = dot_col<H>(Xs + j, LDM, vgam);
