@@ -505,7 +505,8 @@ dsp_status flux_solve(dsp_context ctx, const dsp_flux_batch* batch_in, const dsp
   sz.inst += hg_doubles;
   // with Jacobians of a thermal solve: the vectors r of every degree of freedom [L][h][ndof]
   const bool jrecs = jac && thermal;
-  const size_t jcv_d = jrecs ? (size_t)L * (N / 2) * ndof : 0;
+  // (rounded up: a second workspace half starts behind whole instances)
+  const size_t jcv_d = jrecs ? ((size_t)L * (N / 2) * ndof + 3) / 4 * 4 : 0;
   // with the pseudo-spherical beam: the spherical record of every layer
   const size_t sph_d = spherical ? (size_t)L * sph_stride(N) : 0;
   sz.bvp += jcv_d + sph_d;
@@ -543,6 +544,7 @@ dsp_status flux_solve(dsp_context ctx, const dsp_flux_batch* batch_in, const dsp
       p.inst_rec = wsb;
       p.layer_rec = wsb + (size_t)m * sz.inst;
       p.bvp_rec = p.layer_rec + (size_t)m * sz.layer;
+      if (!records_aligned(p)) return fail(ctx, DSP_ERR_UNSUPPORTED, "flux solve: workspace records off 32 bytes");
       for (int f = 0; f < 8; ++f) p.out[f] = dout[f] + off * nlev;
       p.status = dstatus + off;
       // the spherical and Jacobian areas follow the elimination records of the chunk

@@ -847,14 +847,22 @@ plan:
     }
     flush();
   }
+  // The areas of a chunk's workspace, each rounded up to 32 bytes (the records are read
+  // in 16-byte pieces; h = N/2 and the number of degrees of freedom may both be odd).
+  auto up4 = [](int64_t doubles) -> int64_t { return (doubles + 3) / 4 * 4; };
+  auto jac_doubles = [&](const Chunk& c) { return up4(c.layers * jac_per_layer(c.N)); };
+  auto cc_doubles = [&](const Chunk& c) { return up4(c.layers * c.N); };
+  auto sph_doubles = [&](const Chunk& c) { return up4(c.layers * sph_per_layer(c.N)); };
+  auto ptab_area = [&](const Chunk& c) { return up4((int64_t)c.ids.size() * ptab_doubles(c.N)); };
+  auto int_doubles = [&](const Chunk& c) { return up4((int64_t)c.ids.size() * c.nt_max * numu_eff); };
   // per mode: the layer and boundary-value records, the solution, the spherical
   // records, P_l^m at the angles and the mode's intensities
   auto mode_doubles = [&](const Chunk& c) -> int64_t {
-    return c.layers * (glrec_stride(c.N, numu_eff) + brec_stride(c.N) + c.N + sph_per_layer(c.N)) +
-           (int64_t)c.ids.size() * ptab_doubles(c.N) + ((int64_t)c.ids.size() * c.nt_max * numu_eff + 3) / 4 * 4;
+    return c.layers * (glrec_stride(c.N, numu_eff) + brec_stride(c.N)) + cc_doubles(c) + sph_doubles(c) + ptab_area(c) +
+           int_doubles(c);
   };
   auto fixed_doubles = [&](const Chunk& c) -> int64_t {
-    return c.inst_doubles + c.surf_doubles + c.be_doubles + c.layers * jac_per_layer(c.N);
+    return c.inst_doubles + c.surf_doubles + c.be_doubles + jac_doubles(c);
   };
   // Azimuth modes per launch.  The modes of an instance are independent up to the
   // convergence test, and a mode's boundary-value problem is a serial chain over
@@ -1007,7 +1015,7 @@ plan:
       p.inst_rec = take(c.inst_doubles);
       JacView jv;
       if (jac) {
-        jv.cv = jrecs ? take(c.layers * jac_per_layer(c.N)) : nullptr;
+        jv.cv = jrecs ? take(jac_doubles(c)) : nullptr;
         jv.ndof = jdof;
         jv.ndof_out = (int)jdof_o;
         for (int f = 0; f < 6; ++f) jv.out[f] = djac[f];
@@ -1016,10 +1024,10 @@ plan:
       g.becor = becorr ? take(c.be_doubles) : nullptr;
       g.ms_layer = c.layers * g.lstride;
       g.ms_bvp = c.layers * brec_stride(c.N);
-      g.ms_cc = c.layers * c.N;
-      g.ms_sph = c.layers * sph_per_layer(c.N);
-      g.ms_ptab = (int64_t)nc * ptab_doubles(c.N);
-      g.ms_int = ((int64_t)nc * c.nt_max * numu_eff + 3) / 4 * 4;
+      g.ms_cc = cc_doubles(c);
+      g.ms_sph = sph_doubles(c);
+      g.ms_ptab = ptab_area(c);
+      g.ms_int = int_doubles(c);
       g.nt_max = c.nt_max;
       p.layer_rec = take(c.batch * g.ms_layer);
       p.bvp_rec = take(c.batch * g.ms_bvp);
@@ -1027,6 +1035,7 @@ plan:
       p.sph = spherical ? take(c.batch * g.ms_sph) : nullptr;
       g.ptab = take(c.batch * g.ms_ptab);
       g.imode = take(c.batch * g.ms_int);
+      if (!records_aligned(p)) return fail(ctx, DSP_ERR_UNSUPPORTED, "general solve: workspace records off 32 bytes");
       const double* tabs = nullptr;
       if ((st = get_mode_tables(ctx, c.N, &tabs)) != DSP_OK) return st;
       if (ctx->debug & DSP_DEBUG_POISON_SCRATCH) {

@@ -232,6 +232,12 @@ inline size_t call_budget(dsp_context ctx, size_t want) {
   return budget;
 }
 
+// The layer and boundary-value records are read with 16-byte copies: their areas start
+// on 32 bytes, whatever lies before them in the workspace.
+inline bool records_aligned(const dsp::FluxParams& p) {
+  return ((reinterpret_cast<uintptr_t>(p.layer_rec) | reinterpret_cast<uintptr_t>(p.bvp_rec)) & 31u) == 0;
+}
+
 // Gauss-Legendre nodes/weights on (0,1) by Newton iteration (the reference's
 // gaussianQuadrature, FluxSolver.cpp:257-290) and the m = 0 Legendre table at
 // the nodes (Legendre.cpp:74-88).  Computed on the host so the device and the
