@@ -76,17 +76,21 @@ static_assert(H_NSLOTS <= 16, "instance header is 16 doubles");
 
 // General-solver instance record: the InstLayout fields for (L, N), then the
 // output optical depths utau[NT], their scaled values utaus[NT] and the layer
-// of each, lyr[NT] (NT = user taus, or L + 1 levels).
+// of each, lyr[NT] (NT = user taus, or L + 1 levels), and the lowest azimuth mode that
+// has no eigensystem and the lowest whose boundary-value problem was singular (the modes
+// are solved several at a time; what a mode reports counts once the series reaches it).
 struct GenLayout {
   InstLayout il;
-  int utau, utaus, lyr, stride;
+  int utau, utaus, lyr, eig, sing, stride;
   __host__ __device__ static GenLayout make(int L, int N, int NT) {
     GenLayout g;
     g.il = InstLayout::make(L, N);
     g.utau = g.il.stride;
     g.utaus = g.utau + NT;
     g.lyr = g.utaus + NT;
-    g.stride = round4(g.lyr + NT);
+    g.eig = g.lyr + NT;
+    g.sing = g.eig + 1;
+    g.stride = round4(g.sing + 1);
     return g;
   }
 };
@@ -367,6 +371,12 @@ __device__ __forceinline__ void cp_async_wait() {
 
 __device__ __forceinline__ void set_status(int32_t* status, int i, int code) {
   if (status) atomicMax(status + i, code);
+}
+// Lowers the mode number in a GenLayout eig or sing slot to m (non-negative doubles
+// order like their bit patterns).
+constexpr double kNoMode = 1.0e9;
+__device__ __forceinline__ void lower_mode(double* slot, int m) {
+  atomicMin(reinterpret_cast<long long*>(slot), __double_as_longlong((double)m));
 }
 
 }  // namespace dsp

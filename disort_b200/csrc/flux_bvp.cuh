@@ -259,10 +259,13 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
     else return (long long)i * NT + (ifb ? L - lev : lev);
   };
   double* const* outp = GEN ? p.g.out_flux : p.out;
+  const GenLayout gly = GenLayout::make(GEN ? L : 0, N, GEN ? NT : 0);
   bool act = slot >= 0;
   if (act) {
     const int st0 = p.status ? p.status[i] : 0;
-    if (st0 == DSP_ERR_INVALID_INPUT || st0 == DSP_ERR_EIGEN) {
+    // (GEN: an eigensystem missing at a mode says nothing of the modes before it)
+    const bool no_solution = st0 == DSP_ERR_INVALID_INPUT || (GEN ? rec[gly.eig] <= (double)m : st0 == DSP_ERR_EIGEN);
+    if (no_solution) {
       const double qnan = __longlong_as_double(0x7ff8000000000000ll);
       if (m == 0)
         for (int lev = t; lev < NT; lev += TEAM)
@@ -879,7 +882,6 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
         }
     }
   };
-  const GenLayout gly = GenLayout::make(GEN ? L : 0, N, GEN ? NT : 0);
   const double* const utau_l = rec + gly.utau;
   const double* const utaus_l = rec + gly.utaus;
   const double* const lyr_l = rec + gly.lyr;
@@ -1073,7 +1075,10 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
   }  // !LEAN
   DSP_PHASE_END
   if (act) {
-    if (singular && t == 0) set_status(p.status, i, DSP_ERR_SINGULAR);
+    if (singular && t == 0) {
+      if (GEN && m > 0) lower_mode(const_cast<double*>(rec) + gly.sing, m);
+      else set_status(p.status, i, DSP_ERR_SINGULAR);
+    }
     if (nonfinite) set_status(p.status, i, DSP_ERR_NONFINITE);
   }
 }

@@ -258,6 +258,20 @@ __device__ __forceinline__ LayerTask<N, GEN> layer_task(const FluxParams& p, lon
   if constexpr (GEN) q.live = q.live && mode_of<GEN>(p) <= (int)q.rec[H_NAZ] && q.rec[H_DONE] == 0.0;
   return q;
 }
+// The general solver's chunk-local record layout of a task's instance.
+template <int N>
+__device__ __forceinline__ GenLayout task_layout(const FluxParams& p, const LayerTask<N, true>& q) {
+  const int L = p.g.Ls[q.i];
+  return GenLayout::make(L, N, p.g.user_tau ? p.g.user_tau : L + 1);
+}
+// Neither -A_s nor -B_s of the task is positive definite: the instance's status; of a
+// higher azimuth mode only its entry in the record (the series may end before it).
+template <int N, bool GEN>
+__device__ __forceinline__ void no_eigensystem(const FluxParams& p, const LayerTask<N, GEN>& q) {
+  const int m = mode_of<GEN>(p);
+  if constexpr (GEN) lower_mode(const_cast<double*>(q.rec) + task_layout<N>(p, q).eig, m);
+  if (m == 0) set_status(p.status, q.i, DSP_ERR_EIGEN);
+}
 template <bool GEN>
 __device__ __forceinline__ long long layer_tasks(const FluxParams& p) {
   if constexpr (GEN) return p.g.lay_off[p.n];
@@ -814,7 +828,7 @@ __global__ void __launch_bounds__(128) flux_layer_front_kernel(FluxParams p, Con
     return;
   }
   if (!okb && !oka) {
-    set_status(p.status, q.i, DSP_ERR_EIGEN);
+    no_eigensystem<N, GEN>(p, q);
     *hp(HO::S_FLAG) = 0.0;
     return;
   }
@@ -1392,7 +1406,7 @@ __global__ void __launch_bounds__(32, WCfg<N>::MINB) flux_layer_warp_kernel(Flux
   }
   const bool okb = ok[1], oka = ok[0];
   if (act && !okb && !oka) {
-    if (t == 0) set_status(p.status, q.i, DSP_ERR_EIGEN);
+    if (t == 0) no_eigensystem<N, GEN>(p, q);
     act = false;
   }
   const bool regular = okb && oka;

@@ -46,6 +46,8 @@ static __global__ void __launch_bounds__(128) gen_setup_kernel(FluxParams p) {
   if (lane == 0) {
     for (int k = 0; k < 16; ++k) rec[k] = 0.0;
     rec[H_NT] = NT;
+    rec[gly.eig] = kNoMode;
+    rec[gly.sing] = kNoMode;
   }
   __syncwarp();  // other lanes store boundary Planck terms into the header below
 
@@ -242,9 +244,8 @@ __global__ void __launch_bounds__(128) gen_angle_kernel(FluxParams p) {
   if (task >= p.g.lay_off[p.n]) return;
   const LayerTask<N, true> q = layer_task<N, true>(p, task);
   if (!q.live) return;
-  const int st0 = p.status ? p.status[q.i] : 0;
-  if (st0 == DSP_ERR_EIGEN) return;
   const int m = mode_of<true>(p), numu = p.g.numu;
+  if (q.rec[task_layout<N>(p, q).eig] <= (double)m) return;
   const double ws = q.rec[q.il.ssa_s + q.lc];
   {
     const int mode = (int)q.rec[q.il.mode + q.lc];
@@ -370,10 +371,10 @@ __global__ void __launch_bounds__(128) gen_intensity_kernel(FluxParams p) {
   const int NT = g.user_tau ? g.user_tau : L + 1;
   const int mrow = (int)blockIdx.y, m = g.m + mrow;
   const int st0 = p.status ? p.status[i] : 0;
-  if (st0 == DSP_ERR_INVALID_INPUT || st0 == DSP_ERR_EIGEN) return;
+  if (st0 == DSP_ERR_INVALID_INPUT) return;
   const double* const rec = p.inst_rec + g.inst_off[slot];
-  if (m > (int)rec[H_NAZ] || rec[H_DONE] != 0.0) return;
   const GenLayout gly = GenLayout::make(L, N, NT);
+  if (m > (int)rec[H_NAZ] || rec[H_DONE] != 0.0 || rec[gly.eig] <= (double)m) return;
   const InstLayout& il = gly.il;
   const int ncut = (int)rec[H_NCUT];
   const bool lyrcut = rec[H_LYRCUT] != 0.0;
@@ -499,7 +500,8 @@ __global__ void __launch_bounds__(128) gen_intensity_kernel(FluxParams p) {
 // The Fourier sum over the modes of a launch (DisortSolver.cpp:3228-3266), one
 // warp per instance, a lane per (level, angle) pair; in mode order, with the
 // azimuthal convergence test after each mode (:337-347), so that a mode past
-// the convergence adds nothing even when it was computed with the others.
+// the convergence adds nothing even when it was computed with the others.  The series
+// also ends at a mode that has no eigensystem, with the sum of the modes before it.
 static __global__ void __launch_bounds__(128) gen_fourier_kernel(FluxParams p, int modes) {
   constexpr double PI = 3.14159265358979323846;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -530,12 +532,23 @@ static __global__ void __launch_bounds__(128) gen_fourier_kernel(FluxParams p, i
   double* const rec = p.inst_rec + g.inst_off[slot];
   const int naz = (int)rec[H_NAZ];
   if (rec[H_DONE] != 0.0) return;
+  const GenLayout gly = GenLayout::make(L, p.N, NT);
+  const double eig = rec[gly.eig], sing = rec[gly.sing];
   double kconv = rec[H_KCONV];
   const double* const ph = g.phi.row(i);
   const double phi0 = g.phi0(i);
   for (int mi = 0; mi < modes; ++mi) {
     const int m = g.m + mi;
     if (m > naz) break;
+    if (eig <= (double)m) {  // (mode 0: status EIGEN, above)
+      __syncwarp();
+      if (lane == 0) {
+        set_status(p.status, i, DSP_ERR_EIGEN);
+        rec[H_DONE] = 1.0;
+      }
+      return;
+    }
+    if (sing <= (double)m && lane == 0) set_status(p.status, i, DSP_ERR_SINGULAR);
     const double* const im = g.imode + mi * g.ms_int + (long long)slot * g.nt_max * numu;
     double maxr = 0.0;
     for (int j0 = 0; j0 < nphi || j0 == 0; j0 += 32) {
