@@ -416,6 +416,7 @@ dsp_status flux_solve(dsp_context ctx, const dsp_flux_batch* batch_in, const dsp
   const size_t jac_bytes = jac ? ((size_t)n * nlev * (L + 2) * sizeof(double) + 255) / 256 * 256 : 0;
   const size_t st_bytes = ((size_t)n * sizeof(int32_t) + 255) / 256 * 256;
   const size_t out_bytes = (dev ? 0 : 8 * arr_bytes + 6 * jac_bytes) + st_bytes;
+  size_t in_bytes = 0;  // host inputs
   bool small = false;  // a host batch that goes through pinned staging
   {
     size_t need = 0;
@@ -426,6 +427,7 @@ dsp_status flux_solve(dsp_context ctx, const dsp_flux_batch* batch_in, const dsp
       else elems = arr[k].stride == 0 ? (size_t)cnt[k] : (size_t)((n - 1) * arr[k].stride + cnt[k]);
       need += ((elems * sizeof(double) + 255) / 256) * 256;
     }
+    in_bytes = need;
     if ((st = ensure(ctx, &ctx->stage_in, &ctx->stage_in_bytes, need + 256, "input staging")) != DSP_OK) return st;
     char* cur = static_cast<char*>(ctx->stage_in);
     small = !dev && need <= kSmallHostBytes && out_bytes <= kSmallHostBytes;
@@ -597,13 +599,18 @@ dsp_status flux_solve(dsp_context ctx, const dsp_flux_batch* batch_in, const dsp
   }
 
   // ---- host buffers: copies overlapped with the solves ----------------------
-  // The batch is cut into pieces of whole boundary-value waves (the instances
-  // that kernel keeps resident at once), about a quarter of the batch each, the
-  // remainder last.  Piece k's inputs go up on a copy stream, it is solved on
-  // one of two solve streams (alternating, each with its own half of the
-  // workspace) and its outputs come back on a second copy stream, so the next
-  // piece's kernels fill the GPU while a piece's last wave drains.  (With
-  // pageable host memory the copies do not overlap, but the results are the same.)
+  // The batch is cut into up to seven pieces, the remainder last.  Piece k's inputs go
+  // up on a copy stream, it is solved on one of two solve streams (alternating, each
+  // with its own half of the workspace) and its outputs come back on a second copy
+  // stream, so the next piece's kernels fill the GPU while a piece's last wave drains.
+  // (With pageable host memory the copies do not overlap, but the results are the same.)
+  // Pieces are whole boundary-value waves (the instances that kernel keeps resident at
+  // once), about a quarter of the batch each, unless a wave is so many instances that
+  // the copies would wait for the solves (47,000 at 4 streams): then 16 MB of inputs and
+  // outputs, above which the copies (0.3 ms) outweigh a piece's calls and launches.
+  // 45,000 columns of 40 layers at 4 streams: 3.69 ms in waves, 2.89, 2.92, 2.92, 2.94
+  // ms in pieces of 32, 16, 8, 2 MB; 8,191 of 47 at 8 streams 1.16, 1.16, 0.97, 1.15,
+  // 1.22; 3,000 of 60 at 16 streams with all moments 1.75, 1.70, 1.55, 1.56, 2.04.
   double* host_out[8] = {out->flux_direct_beam, out->flux_down, out->flux_up, out->flux_tau_divergence,
                          out->mean_intensity, out->mean_intensity_down, out->mean_intensity_up,
                          out->mean_intensity_direct_beam};
@@ -614,7 +621,11 @@ dsp_status flux_solve(dsp_context ctx, const dsp_flux_batch* batch_in, const dsp
     hs = hst.data();
   }
   constexpr int kMaxPieces = 8;
-  const int64_t wave = std::max<int64_t>(1, bvp_wave(N, ctx->sm_count));
+  constexpr size_t kPieceBytes = 16'000'000;
+  const int64_t parts =
+      std::max<int64_t>(1, std::min<int64_t>(kMaxPieces - 1, (int64_t)((in_bytes + out_bytes) / kPieceBytes)));
+  const int64_t wave = std::min<int64_t>(std::max<int64_t>(1, bvp_wave(N, ctx->sm_count)),
+                                         ((n + parts - 1) / parts + 63) / 64 * 64);
   const int64_t waves = (n + wave - 1) / wave;
   int64_t piece = wave * std::max<int64_t>(1, waves / 4);
   while ((n + piece - 1) / piece > kMaxPieces - 1) piece += wave;
