@@ -24,10 +24,11 @@
 // I + M and Z are symmetric positive definite whatever the layer (M is a
 // congruence of A, and Z < 2), so both are inverted without pivoting, and no
 // growing exponential is formed.  (Unphysical moments above 1 can break that; the
-// sweeps then run on an indefinite matrix, scaled by the absolute diagonal.)  Two h x h inverses and four h^3 products per
-// layer take the place of the N-column elimination of a 3h-row panel, about a
-// tenth of its operations; near omega' = 1 (k -> 0) nothing cancels, because
-// 1 - E^2 comes from expm1.
+// sweeps then run on an indefinite matrix, scaled by the absolute diagonal, whose signs
+// stay; and a mode of -k has a growing E, which leaves G as 1/E^2.)  Two h x h inverses
+// and four h^3 products per layer take the place of the N-column elimination of a 3h-row
+// panel, about a tenth of its operations; near omega' = 1 (k -> 0) nothing cancels,
+// because 1 - E^2 comes from expm1.
 //
 // Fluxes alone need less on the way up (LEAN, up to 16 streams).  Substituted into
 // one another, the three equations are
@@ -102,7 +103,8 @@ struct BCfg {
 };
 
 // Negative inverse of a symmetric positive definite matrix with unit diagonal
-// (the caller scales), columns held by the lanes: symmetric sweeps (Goodnight
+// (the caller scales; +-1 in an indefinite one), columns held by the lanes: symmetric
+// sweeps (Goodnight
 // 1979, The American Statistician 33) of pivots 0..H-1.  In step k lane j's a[i]
 // is row (k + i) mod H of its column: the update shifts it by one row, so every
 // register index is a constant.  By symmetry the pivot column is the pivot row,
@@ -442,7 +444,7 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
     __syncwarp();
 #pragma unroll
     for (int r = 0; r < H; ++r) {
-      if constexpr (ROLL) a[r] = r == j ? 1.0 : As[r * LDM + j] * (s1 * vsc[r]);
+      if constexpr (ROLL) a[r] = r == j ? copysign(1.0, diag) : As[r * LDM + j] * (s1 * vsc[r]);
       else a[r] *= s1 * vsc[r];
     }
     // X and the vectors are used up: the next layer's start loading
@@ -559,11 +561,13 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
       vgam[j] = gb;
       if (LEAN) vw1[j] = y;
 #pragma unroll
-      for (int r = 0; r < H; ++r) Ws[j * LDM + r] = C::IDREG ? fma(2.0, a[r], -id[C::IDREG ? r : 0]) : (r == j ? fma(2.0, a[r], -1.0) : 2.0 * a[r]);
+      for (int r = 0; r < H; ++r) Ws[j * LDM + r] = !LEAN && r == j ? fma(2.0, a[r], -1.0) : 2.0 * a[r];
     }
     cp_async_wait<1>();  // Y of this layer
     __syncwarp();
-    // A' = Y (2 G - I) Y^T, column j; g' = Y gamma'
+    // A' = Y (2 G - I) Y^T, column j; g' = Y gamma'.  (LEAN: 2 G first, I taken off last, as
+    // W and R take 2 G, of which 2 G - I keeps no digits where E > 1, the modes of -k; A'
+    // before W, whose products the next layer does not wait for: 1.47 -> 1.39 ms)
     {
       double tv[H];
 #pragma unroll
@@ -605,28 +609,18 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
             o[1] = make_double2(f2, dot_col<H>(Ys + j, LDM, b0));
             o[2] = make_double2(dot_col<H>(Ys + j, LDM, b1), dot_col<H>(Ys + j, LDM, b2));
           }
-          // R = X H X^T - V (2 G) V^T, 2 G V^T = (2 G - I) V^T + V^T
+          // R = X H X^T - V (2 G) V^T
           double gv[H];
 #pragma unroll
           for (int r = 0; r < H; ++r) gv[r] = 0.0;
 #pragma unroll
           for (int r = 0; r < H; ++r) axpy_row<H>(gv, Ws + r * LDM, As[r * LDM + j]);
 #pragma unroll
-          for (int r = 0; r < H; ++r) axpy_row<H>(rr, As + r * LDM, -(gv[r] + As[r * LDM + j]));
+          for (int r = 0; r < H; ++r) axpy_row<H>(rr, As + r * LDM, -gv[r]);
           if (on && own) {
 #pragma unroll
             for (int r = 0; r < H; ++r) br[tjac_R(N) + r * HP + j] = rr[r];
           }
-        }
-        // column j of W: 2 G Y^T = (2 G - I) Y^T + Y^T
-        double wt[H];
-#pragma unroll
-        for (int r = 0; r < H; ++r) wt[r] = 0.0;
-#pragma unroll
-        for (int r = 0; r < H; ++r) axpy_row<H>(wt, As + r * LDM, tv[r] + Ys[r * LDM + j]);
-        if (on && own) {
-#pragma unroll
-          for (int r = 0; r < H; ++r) br[r * HP + j] = wt[r];
         }
       }
       double w[H];
@@ -640,9 +634,19 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
         for (int r = 0; r < H; ++r) axpy_row<H>(w, Ys + r * LDM, Ws[r * LDM + j]);
       } else {
 #pragma unroll
-        for (int r = 0; r < H; ++r) axpy_row<H>(w, Ys + r * LDM, tv[r]);
+        for (int r = 0; r < H; ++r) axpy_row<H>(w, Ys + r * LDM, LEAN ? tv[r] - Ys[r * LDM + j] : tv[r]);
       }
       if constexpr (LEAN) {
+        // column j of W
+        double wt[H];
+#pragma unroll
+        for (int r = 0; r < H; ++r) wt[r] = 0.0;
+#pragma unroll
+        for (int r = 0; r < H; ++r) axpy_row<H>(wt, As + r * LDM, tv[r]);
+        if (on && own) {
+#pragma unroll
+          for (int r = 0; r < H; ++r) br[r * HP + j] = wt[r];
+        }
         if (on && own) {
           double2* const o = reinterpret_cast<double2*>(br + trec_v(N) + 4 * j);
           o[0] = make_double2(f, past ? gn + dot_col<H>(Ys + j, LDM, vdp) : gn);
@@ -736,7 +740,7 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
       }
       __syncwarp();
 #pragma unroll
-      for (int r = 0; r < H; ++r) a[r] = r == j ? 1.0 : a[r] * (s1 * vsc[r]);
+      for (int r = 0; r < H; ++r) a[r] = r == j ? copysign(1.0, diag) : a[r] * (s1 * vsc[r]);
       sweep_inverse<H, SB, ROLL, true>(a, j, own, sbuf, singular);
 #pragma unroll
       for (int r = 0; r < H; ++r) {
@@ -1035,7 +1039,17 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
     if (own) vw2[j] = ex * b;
     __syncwarp();
     const double c = fma(2.0, dot_col<H>(As + j, LDM, vw2), -rj);  // homogeneous C at the top
-    const double av = c - ex * b;
+    // D_ = sg (E2 bb - E1 aa): for a mode of -k with the decaying exponentials of |k| and
+    // amplitudes from C at the two boundaries (a and b themselves lose E in digits)
+    double aa = c - ex * b, bb = b, ee = ex, sg = 1.0, fx = vec[2 * HP + j];
+    if (vec[j] < 0.0) {
+      const double x = vec[j] * (s.t1 - s.t0);
+      ee = exp(x);
+      fx = -expm1(2.0 * x);
+      bb = fx > 0.1 ? (chom_b - ee * c) / fx : ex * aa;
+      aa = fx > 0.1 ? (c - ee * chom_b) / fx : ex * b;
+      sg = -1.0;
+    }
     if (own) vw1[j] = c + ct;
     __syncwarp();
     // G and H are used up
@@ -1045,11 +1059,11 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
     if constexpr (GEN) {
       if (on && own) {
         double* cc = p.g.cc + mrow * p.g.ms_cc + (lay0 + l) * N;
-        cc[j] = b;
-        cc[H + j] = av;
+        cc[j] = bb;
+        cc[H + j] = aa;
       }
       if (m == 0) {
-        const double k = vec[j], fx = vec[2 * HP + j];
+        const double k = fabs(vec[j]);
         for (int lu = 0; lu < NTw; ++lu) {
           const bool put = on && lu < NT && (int)lyr_l[lu] == l;
           if (!__any_sync(0xffffffffu, put)) continue;
@@ -1058,12 +1072,12 @@ __device__ __forceinline__ void bvp_warp(const FluxParams& p, const int slot) {
           // C inside the layer from its values at the two boundaries (no cancellation)
           double cu = c;
           if (fx > 0.0) cu = (c * (e1 * -expm1(-2.0 * k * x2)) + chom_b * (e2 * -expm1(-2.0 * k * x1))) / fx;
-          eval_level(l, lu, tu, put ? utau_l[lu] : 0.0, s.w1, cu, e2 * b - e1 * av, put, l == 0 && x1 == 0.0);
+          eval_level(l, lu, tu, put ? utau_l[lu] : 0.0, s.w1, cu, sg * (e2 * bb - e1 * aa), put, l == 0 && x1 == 0.0);
         }
       }
     } else {
-      eval_level(l, l + 1, s.t1, s.u1, s.w1, chom_b, b - ex * av, on, false);
-      if (l == 0) eval_level(0, 0, s.t0, s.u0, s.w1, c, ex * b - av, on, true);
+      eval_level(l, l + 1, s.t1, s.u1, s.w1, chom_b, sg * (bb - ee * aa), on, false);
+      if (l == 0) eval_level(0, 0, s.t0, s.u0, s.w1, c, sg * (ee * bb - aa), on, true);
     }
     __syncwarp();
     if (on && own) ve[j] = phi;

@@ -20,6 +20,7 @@
 #pragma once
 
 #include "dsp_device.cuh"
+#include "flux_layer.cuh"
 #include "flux_setup.cuh"
 
 namespace dsp {
@@ -155,7 +156,7 @@ __global__ void __launch_bounds__(64) flux_jac_kernel(FluxParams p, JacView jv) 
       const double* br = brec0 + (long long)l * brec_stride(N);
       double* cvl = cv0 + (long long)l * H * cvs;
       __syncthreads();
-      for (int r = tid; r < H; r += KB) Ev[r] = exp(-lr[mod_k(N) + r] * dtau_s[l]);
+      for (int r = tid; r < H; r += KB) Ev[r] = exp(mode_exponent(lr[mod_k(N) + r], dtau_s[l]));
       __syncthreads();
       double a0, a1;
       coef(l, a0, a1);
@@ -233,7 +234,7 @@ __global__ void __launch_bounds__(64) flux_jac_kernel(FluxParams p, JacView jv) 
       const double* br = brec0 + (long long)l * brec_stride(N);
       const double* cvl = cv0 + (long long)l * H * cvs;
       __syncthreads();
-      for (int r = tid; r < H; r += KB) Ev[r] = exp(-lr[mod_k(N) + r] * dtau_s[l]);
+      for (int r = tid; r < H; r += KB) Ev[r] = exp(mode_exponent(lr[mod_k(N) + r], dtau_s[l]));
       __syncthreads();
       double a0, a1;
       coef(l, a0, a1);
@@ -277,15 +278,16 @@ __global__ void __launch_bounds__(64) flux_jac_kernel(FluxParams p, JacView jv) 
         const double tu = out_taus(lu), x1 = tu - taus[l], x2 = taus[l + 1] - tu;
         __syncthreads();
         for (int r = tid; r < H; r += KB) {
-          e1v[r] = exp(-lr[mod_k(N) + r] * x1);
-          e2v[r] = exp(-lr[mod_k(N) + r] * x2);
+          const double k = fabs(lr[mod_k(N) + r]);
+          e1v[r] = exp(-k * x1);
+          e2v[r] = exp(-k * x2);
         }
         __syncthreads();
         // C from its values at the boundaries (no cancellation), D_ = E2 b - E1 a
         const double ft = a0 + a1 * x1;
 #pragma unroll
         for (int j = 0; j < H; ++j) {
-          const double kj = lr[mod_k(N) + j];
+          const double kr = lr[mod_k(N) + j], kj = fabs(kr);
           double cu = x1 > x2 ? cb[j] : c[j];
           if (x1 != 0.0 && x2 != 0.0) {
             const double fx = -expm1(-2.0 * kj * (taus[l + 1] - taus[l]));
@@ -293,7 +295,13 @@ __global__ void __launch_bounds__(64) flux_jac_kernel(FluxParams p, JacView jv) 
               cu = (c[j] * (e1v[j] * -expm1(-2.0 * kj * x2)) + cb[j] * (e2v[j] * -expm1(-2.0 * kj * x1))) / fx;
           }
           u[j * KB] = cu + ft * lr[mod_ct(N) + j];
-          w[j * KB] = e2v[j] * b[j] - e1v[j] * av[j] + a1 * lr[mod_dt(N) + j];
+          double dj = e2v[j] * b[j] - e1v[j] * av[j];
+          if (kr < 0.0) {  // a mode of -k (flux_bvp.cuh)
+            const double x = kr * (taus[l + 1] - taus[l]), ee = exp(x), fx = -expm1(2.0 * x);
+            dj = fx > 0.1 ? (e1v[j] * (c[j] - ee * cb[j]) - e2v[j] * (cb[j] - ee * c[j])) / fx
+                          : Ev[j] * (e1v[j] * b[j] - e2v[j] * av[j]);
+          }
+          w[j * KB] = dj + a1 * lr[mod_dt(N) + j];
         }
         // at the top of the column psi = phi: the incoming field does not depend on k
         const bool top = l == 0 && x1 == 0.0;

@@ -300,6 +300,10 @@ __device__ __forceinline__ double phase_coeff(int k, double pk, int mode, double
 // solution depends on k^2)
 __device__ __forceinline__ double mode_k(double lambda) { return fmax(sqrt(fabs(lambda)), 1e-9); }
 
+// exponent of a layer's E = exp(-k dtau): for a mode of -k (-B_s indefinite) E grows, no
+// further than E^2 can be formed (its reciprocal is zero to rounding long before)
+__device__ __forceinline__ double mode_exponent(double k, double dtau) { return -fmax(k * dtau, -300.0); }
+
 // the beam's cosine, moved off a resonance mu0 k = 1 (FluxSolver.cpp:610-618)
 __device__ __forceinline__ bool beam_resonant(double k, double umu0) {
   return fabs(1.0 - umu0 * umu0 * k * k) < 1000.0 * 2.220446049250313e-16;
@@ -554,7 +558,7 @@ __global__ void __launch_bounds__(LCfg<N>::CTA, LCfg<N>::MINB) flux_layer_kernel
     const double dts = q.rec[q.il.dtau_s + q.lc];
     const double ks = lneg && !primary ? -k : k;  // (the reference's a and b change roles)
     vec[mod_k(N) + c] = ks;
-    const double em = expm1(-ks * dts);  // E - 1; 1 - E^2 = -em (2 + em)
+    const double em = expm1(mode_exponent(ks, dts));  // E - 1; 1 - E^2 = -em (2 + em)
     vec[mod_E(N) + c] = 1.0 + em;
     vec[mod_F(N) + c] = -em * (2.0 + em);
     if (beam) {
@@ -1110,7 +1114,7 @@ __global__ void __launch_bounds__(128) flux_eigen_kernel(FluxParams p, ConstTab<
     }
     const double ks = (negb >> c) & 1u ? -k : k;
     vrow[c] = ks;
-    const double em = expm1(-ks * dts);  // E - 1; 1 - E^2 = -em (2 + em)
+    const double em = expm1(mode_exponent(ks, dts));  // E - 1; 1 - E^2 = -em (2 + em)
     vrow[HP + c] = 1.0 + em;
     vrow[2 * HP + c] = -em * (2.0 + em);
     if (beam) {
@@ -1615,7 +1619,7 @@ __global__ void __launch_bounds__(32, WCfg<N>::MINB) flux_layer_warp_kernel(Flux
     const double k = v ? k1 : k0;
     const bool na = v ? na1 : na0, nb = v ? nb1 : nb0;
     const double ka = na ? -k : k, kb = nb ? -k : k;
-    const double em = expm1(-kb * dts);  // E - 1; 1 - E^2 = -em (2 + em)
+    const double em = expm1(mode_exponent(kb, dts));  // E - 1; 1 - E^2 = -em (2 + em)
     q.lrec[mod_k(N) + c] = kb;
     q.lrec[mod_E(N) + c] = 1.0 + em;
     q.lrec[mod_F(N) + c] = -em * (2.0 + em);

@@ -443,8 +443,12 @@ __global__ void __launch_bounds__(128) gen_intensity_kernel(FluxParams p) {
     const double* const gu = lr + glrec_gu(N) + (long long)iu * N;
     const double* const zu = lr + glrec_gu(N) + (long long)numu * N;
     const double* const x = cc0 + (long long)l * N;
-    const double k = lr[mod_k(N) + j], wk = lr[mod_E(N) + j];
-    const double gb = own ? gu[j] * x[j] : 0.0, ga = own ? gu[H + j] * x[H + j] : 0.0;
+    // (a mode of -k: the exponentials of |k|, with the signs of its D_, flux_bvp.cuh)
+    const double kr = lr[mod_k(N) + j], k = fabs(kr), we = lr[mod_E(N) + j];
+    const double g0 = own ? gu[j] : 0.0, g1 = own ? gu[H + j] : 0.0;
+    const bool minus = kr < 0.0;
+    const double wk = minus ? rcp_newton(we) : we;
+    const double gb = (minus ? g1 : g0) * x[j], ga = (minus ? g0 : g1) * x[H + j];
     const double tt = taus[l], tb = taus[l + 1], dt = tb - tt;
     const double e = exp(-dt * rnu);
     const double t0 = neg ? tt : tb;  // the near side, where the radiation enters
