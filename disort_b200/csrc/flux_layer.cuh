@@ -21,9 +21,10 @@
 // one-sided Jacobi iteration finds without forming S: its rotations act on the
 // columns of L^T R only (no eigenvector matrix is accumulated), and the small
 // singular values keep their relative accuracy.  When -A_s is not positive
-// definite S is diagonalised instead, and when -B_s is not, -A_s = L L^T and
-// S = L^T (-B_s) L give the same modes with the two forms exchanged
-// (X = L^{-T} U K^{1/2}, Y = L U K^{-1/2}).
+// definite (unphysical moments) S is formed, and its eigenvectors are the left singular
+// vectors of S + shift I, shifted no further than makes it positive definite; when -B_s
+// is not, -A_s = L L^T and S = L^T (-B_s) L give the same modes with the two forms
+// exchanged (X = L^{-T} U K^{1/2}, Y = L U K^{-1/2}).
 // The quadrature is symmetric (mu_{h+j} = -mu_j, P_l^m(-mu) = (-1)^{l+m} P_l^m(mu)),
 // so -B_s holds the phase sums of odd l + m only and -A_s those of even l + m:
 //   alpha -/+ beta = M^{-1} (O W - I), M^{-1} (E W - I),
@@ -89,9 +90,10 @@ __host__ __device__ constexpr int tri_idx(int r, int c) {
 // one-thread-per-task kernels reads or writes an element of 32 tasks in one
 // coalesced access.  Per task: flag (0 skipped; 1: L^T R by columns; 2: -A_s is
 // indefinite, S = L^T (-A_s) L; 3: -B_s is, L is the factor of -A_s and
-// S = L^T (-B_s) L; S packed lower in the place of L^T R), the Cholesky factor L
+// S = L^T (-B_s) L; (S + shift I) / scale in the place of L^T R), the Cholesky factor L
 // (packed lower), and with a beam the source vectors D M^{-1} (q+ + q-),
-// D M^{-1} (q+ - q-).
+// D M^{-1} (q+ - q-).  Shift and scale of an indefinite task are handed on in its layer
+// record, in the place of xr0 and xr1.
 template <int NN>
 struct Handoff {
   static constexpr int TRI = NN * (NN + 1) / 2;
@@ -597,29 +599,6 @@ __global__ void __launch_bounds__(LCfg<N>::CTA, LCfg<N>::MINB) flux_layer_kernel
   }
 }
 
-// The rotation of jacobi_rot from two reciprocal square roots, without branches
-// or divisions (a sweep is then one scheduling region): with
-// r = 1/sqrt(d^2 + e^2), cos 2theta = |d| r and sin 2theta = sgn(d) e r, so
-// h = cos^2 theta = (1 + |d| r) / 2, g = 1/sqrt(h) = 1/cos theta,
-// c = h g, s = sin 2theta g / 2 and t = tan theta = s g (the same angle as
-// jacobi_rot's t = sgn(d) |e| / (|d| + sqrt(d^2 + e^2)); no cancellation for
-// small angles).  A pair whose d^2 + e^2 is below 1e-280 is left unrotated:
-// S's norm is at least its largest eigenvalue, far above that.
-__device__ __forceinline__ void jacobi_rot_rsq(double apq, double app, double aqq, double& c, double& s,
-                                               double& tt) {
-  const double d = aqq - app, e = 2.0 * apq;
-  const double q = fma(d, d, e * e);
-  const bool rot = jacobi_needed(apq, app, aqq) && q > 1e-280;
-  const double r = rsqrt(rot ? q : 1.0);
-  const double num = d > 0.0 ? e : (d < 0.0 ? -e : fabs(e));  // sgn(d) e, sgn(0) = +1
-  const double h = fma(0.5 * fabs(d), r, 0.5);
-  const double g = rsqrt(h);
-  const double sv = (0.5 * num * r) * g;
-  c = rot ? h * g : 1.0;
-  s = rot ? sv : 0.0;
-  tt = rot ? sv * g : 0.0;
-}
-
 // Pivot of a Cholesky factorisation, d0 the diagonal element it started from: at
 // omega' = 1 the last pivot of -A_s is zero to rounding, of either sign, and is
 // taken as 1e-18 d0 (k ~ 1e-9); NaN or a negative pivot beyond rounding: 0, the
@@ -654,9 +633,15 @@ __device__ __forceinline__ bool chol_packed(double* A) {
   return ok;
 }
 
+// An indefinite S is shifted by the first of kFirstShift x its largest row sum, 16 times
+// that, ... that makes it positive definite: not far above its most negative eigenvalue,
+// so that the small eigenvalues keep their digits, and at the row sum at the latest.
+constexpr double kFirstShift = 1.0e-6;
+
 // The front's hand-off of a task with exactly one of -B_s (okb) and -A_s positive
-// definite: S = L^T M L with the definite one's factor L and the other as M.  Rare
-// (phase functions with unphysical moments): local memory and rolled loops.
+// definite: S = L^T M L with the definite one's factor L and the other as M, shifted
+// and scaled for onesided_jacobi.  Rare (phase functions with unphysical moments):
+// local memory and rolled loops.
 template <int N, bool GEN>
 __device__ __noinline__ void layer_front_indefinite(const FluxParams& p, const LayerTask<N, GEN>& q, double* hand,
                                                     long long nt, long long j, bool okb) {
@@ -679,7 +664,7 @@ __device__ __noinline__ void layer_front_indefinite(const FluxParams& p, const L
                               tab[tab_dinv(N) + c];
     }
   double* const L = okb ? M[0] : M[1];
-  const double* const I = okb ? M[1] : M[0];
+  double* const I = okb ? M[1] : M[0];  // the indefinite one, then scratch
   for (int c = 0; c < NN; ++c) {
     const double d0 = L[tri_idx(c, c)];
     double v = d0;
@@ -692,6 +677,7 @@ __device__ __noinline__ void layer_front_indefinite(const FluxParams& p, const L
       L[tri_idx(r, c)] = t / ljj;
     }
   }
+  double S[HO::TRI];
   for (int c = 0; c < NN; ++c) {
     double t[NN];  // (M L)[:, c]
     for (int r = 0; r < NN; ++r) {
@@ -701,9 +687,33 @@ __device__ __noinline__ void layer_front_indefinite(const FluxParams& p, const L
     for (int r = c; r < NN; ++r) {
       double v = 0.0;
       for (int k = r; k < NN; ++k) v += L[tri_idx(k, r)] * t[k];
-      *handoff_lane<NN>(hand, nt, j, HO::S_F + tri_idx(r, c)) = v;
+      S[tri_idx(r, c)] = v;
     }
   }
+  double scale = 0.0;  // largest row sum: no eigenvalue is beyond it
+  for (int r = 0; r < NN; ++r) {
+    double v = 0.0;
+    for (int c = 0; c < NN; ++c) v += fabs(S[tri_idx(r, c)]);
+    scale = fmax(scale, v);
+  }
+  if (!(scale > 0.0)) scale = 1.0;
+  double shift = kFirstShift * scale;
+  for (; shift < scale; shift *= 16.0) {
+    bool ok = true;
+    for (int c = 0; c < NN && ok; ++c)
+      for (int r = c; r < NN; ++r) {
+        double v = S[tri_idx(r, c)] + (r == c ? shift : 0.0);
+        for (int k = 0; k < c; ++k) v -= I[tri_idx(r, k)] * I[tri_idx(c, k)];
+        if (r == c) ok = v > 0.0;
+        I[tri_idx(r, c)] = r == c ? sqrt(fmax(v, 0.0)) : v / I[tri_idx(c, c)];
+      }
+    if (ok) break;
+  }
+  for (int c = 0; c < NN; ++c)
+    for (int r = 0; r < NN; ++r)
+      *handoff_lane<NN>(hand, nt, j, HO::S_F + c * NN + r) = (S[tri_idx(r, c)] + (r == c ? shift : 0.0)) / scale;
+  q.lrec[mod_xr(N)] = shift;
+  q.lrec[mod_xr(N) + 1] = scale;
   for (int e = 0; e < HO::TRI; ++e) *handoff_lane<NN>(hand, nt, j, HO::S_L + e) = L[e];
   *handoff_lane<NN>(hand, nt, j, HO::S_FLAG) = okb ? 2.0 : 3.0;
 }
@@ -944,40 +954,6 @@ __device__ __forceinline__ void onesided_jacobi(double (*F)[NN], bool act) {
   }
 }
 
-// Cyclic two-sided Jacobi on a packed symmetric matrix, for the rare task whose
-// -A_s or -B_s is indefinite (local memory, rolled loops).  V: eigenvectors by
-// columns, d: eigenvalues.
-template <int NN>
-__device__ __noinline__ void jacobi_two_sided(double* S, double* V, double* d) {
-  for (int e = 0; e < NN * NN; ++e) V[e] = e / NN == e % NN ? 1.0 : 0.0;
-  for (int sweep = 0; sweep < 20; ++sweep) {
-    bool more = false;
-    for (int q = 1; q < NN; ++q)
-      for (int p = 0; p < q; ++p) {
-        const double apq = S[tri_idx(q, p)];
-        double c, s, t;
-        jacobi_rot_rsq(apq, S[tri_idx(p, p)], S[tri_idx(q, q)], c, s, t);
-        if (t == 0.0) continue;
-        more = true;
-        S[tri_idx(p, p)] -= t * apq;
-        S[tri_idx(q, q)] += t * apq;
-        S[tri_idx(q, p)] = 0.0;
-        for (int k = 0; k < NN; ++k) {
-          if (k != p && k != q) {
-            const double x = S[tri_idx(k, p)], y = S[tri_idx(k, q)];
-            S[tri_idx(k, p)] = c * x - s * y;
-            S[tri_idx(k, q)] = s * x + c * y;
-          }
-          const double x = V[p * NN + k], y = V[q * NN + k];
-          V[p * NN + k] = c * x - s * y;
-          V[q * NN + k] = s * x + c * y;
-        }
-      }
-    if (!more) break;
-  }
-  for (int k = 0; k < NN; ++k) d[k] = S[tri_idx(k, k)];
-}
-
 // Eigensolver and output of the split layer stage, one thread per layer task: F
 // from the hand-off into registers, onesided_jacobi, then mode by mode X and Y
 // (from the singular vector and the Cholesky factor), k and the particular
@@ -1023,8 +999,8 @@ __global__ void __launch_bounds__(128) flux_eigen_kernel(FluxParams p, ConstTab<
 #pragma unroll
   for (int c = 0; c < NN; ++c)
 #pragma unroll
-    for (int r = 0; r < NN; ++r) F[c][r] = act && regular ? hv(HO::S_F + c * NN + r) : 0.0;
-  onesided_jacobi<NN>(F, act && regular);
+    for (int r = 0; r < NN; ++r) F[c][r] = act ? hv(HO::S_F + c * NN + r) : 0.0;
+  onesided_jacobi<NN>(F, act);
 #pragma unroll
   for (int c = 0; c < NN; ++c) {
     double n2 = 0.0;
@@ -1035,26 +1011,23 @@ __global__ void __launch_bounds__(128) flux_eigen_kernel(FluxParams p, ConstTab<
 #pragma unroll
     for (int r = 0; r < NN; ++r) F[c][r] *= rs;
   }
+  const LayerTask<N, GEN> q = layer_task<N, GEN>(p, jj);
   // eigenvalues lambda = k^2 are negative only where -A_s (bit set in nega) or -B_s
   // (negb) is indefinite; k = sqrt|lambda| as in the reference, the inverses of the
   // particular solutions carry the sign, and with -B_s the reference's a and b
   // change roles, which is the mode of -k
   unsigned nega = 0u, negb = 0u;
   if (act && !regular) {
-    double S[HO::TRI], V[NN * NN], d[NN];
-    for (int e = 0; e < HO::TRI; ++e) S[e] = hv(HO::S_F + e);
-    jacobi_two_sided<NN>(S, V, d);
+    const double shift = q.lrec[mod_xr(N)], scale = q.lrec[mod_xr(N) + 1];
 #pragma unroll
     for (int c = 0; c < NN; ++c) {
-      kk[c] = mode_k(d[c]);
-      if (d[c] < 0.0) (flag < 2.5 ? nega : negb) |= 1u << c;
-#pragma unroll
-      for (int r = 0; r < NN; ++r) F[c][r] = V[c * NN + r];
+      const double lambda = fma(kk[c], scale, -shift);
+      kk[c] = mode_k(lambda);
+      if (lambda < 0.0) (flag < 2.5 ? nega : negb) |= 1u << c;
     }
   }
 
   const bool primary = flag < 2.5;
-  const LayerTask<N, GEN> q = layer_task<N, GEN>(p, jj);
   const double fbeam = act ? q.rec[H_FBEAM] : 0.0;
   const bool beam = fbeam > 0.0;
   const bool raw = GEN && (p.flags & DSP_FLAG_SPHERICAL_BEAM);
@@ -1195,17 +1168,13 @@ struct WCfg {
 // Cholesky factor of the symmetric matrix whose columns 2t, 2t + 1 lane t holds in
 // c0, c1 (rows in order), written row-major to `out` (stride LDM, upper part zero).
 // Right-looking; in step k register i of a column is row k + i, the update shifting
-// it by one row.  Returns false (to every lane of the team) if it is indefinite.
-template <int H, int LDM, int TEAM>
-__device__ __forceinline__ bool team_chol_columns(double* c0, double* c1, double* out, double* cbuf, int t,
-                                                  unsigned msk) {
+// it by one row.  d00, d01: the diagonal elements of the lane's columns (picked out of
+// the registers by lane they would put a column into local memory).  Returns false (to
+// every lane of the team) if it is indefinite.  STORE = false: only the verdict.
+template <int H, int LDM, int TEAM, bool STORE = true>
+__device__ __forceinline__ bool team_chol_columns(double* c0, double* c1, double d00, double d01, double* out,
+                                                  double* cbuf, int t, unsigned msk) {
   bool ok = true;
-  double d00 = 0.0, d01 = 0.0;  // the original diagonal elements of the lane's columns
-#pragma unroll
-  for (int r = 0; r < H; ++r) {
-    if (r == 2 * t) d00 = c0[r];
-    if (r == 2 * t + 1) d01 = c1[r];
-  }
 #pragma unroll 1
   for (int k2 = 0; k2 < H; k2 += 2) {
 #pragma unroll
@@ -1222,9 +1191,10 @@ __device__ __forceinline__ bool team_chol_columns(double* c0, double* c1, double
         for (int i = 0; i < H; ++i) {
           const double v = i == 0 ? s * r : c[i] * r;
           buf[i] = v;  // rows k .. k + H - 1: past the matrix the registers hold zeros
-          if (k + i < H) out[(k + i) * LDM + k] = v;
+          if (STORE && k + i < H) out[(k + i) * LDM + k] = v;
         }
-        for (int i = 0; i < k; ++i) out[i * LDM + k] = 0.0;
+        if constexpr (STORE)
+          for (int i = 0; i < k; ++i) out[i * LDM + k] = 0.0;
       }
       __syncwarp(msk);
       ok = ok && buf[0] > 0.0;
@@ -1253,184 +1223,13 @@ __device__ __forceinline__ bool team_chol_columns(double* c0, double* c1, double
   return ok;
 }
 
-// The modes of a task with exactly one of -B_s (okb) and -A_s positive definite, by
-// one lane in global scratch (rare: unphysical moments): the eigenvectors of S by
-// columns at V, its eigenvalues at d, the factor at L (row-major, stride LDM).
-template <int H, int LDM>
-__device__ __noinline__ void team_indefinite(const double* gl, const double* Y, const double* tab, int N, int m,
-                                             bool okb, double* L, double* M, double* V, double* d) {
-  double* const S = M + H * H;  // scratch: M [H][H], S [H][H]
-  for (int r = 0; r < H; ++r)
-    for (int c = 0; c <= r; ++c) {
-      double sum[2] = {0.0, 0.0};  // odd, even l + m
-      for (int l = 0; l < N; ++l) sum[1 - ((l + m) & 1)] += gl[l] * Y[l * N + r] * Y[l * N + c];
-      const double rm = 1.0 / tab[r], dl = r == c ? rm : 0.0;
-      const double sc = -tab[tab_dsim(N) + r] * tab[tab_dinv(N) + c];
-      const double vb = sc * (tab[tab_wt(N) + c] * sum[0] * rm - dl), va = sc * (tab[tab_wt(N) + c] * sum[1] * rm - dl);
-      L[r * LDM + c] = okb ? vb : va;
-      M[r * H + c] = M[c * H + r] = okb ? va : vb;
-    }
-  for (int c = 0; c < H; ++c) {
-    const double d0 = L[c * LDM + c];
-    double v = d0;
-    for (int k = 0; k < c; ++k) v -= L[c * LDM + k] * L[c * LDM + k];
-    const double ljj = sqrt(chol_pivot(v, d0));
-    L[c * LDM + c] = ljj;
-    for (int r = 0; r < c; ++r) L[r * LDM + c] = 0.0;
-    for (int r = c + 1; r < H; ++r) {
-      double t = L[r * LDM + c];
-      for (int k = 0; k < c; ++k) t -= L[r * LDM + k] * L[c * LDM + k];
-      L[r * LDM + c] = t / ljj;
-    }
-  }
-  for (int c = 0; c < H; ++c) {  // V as scratch: (M L)[:, c] in its first row
-    for (int r = 0; r < H; ++r) {
-      double v = 0.0;
-      for (int k = c; k < H; ++k) v += M[r * H + k] * L[k * LDM + c];
-      V[r] = v;
-    }
-    for (int r = c; r < H; ++r) {
-      double v = 0.0;
-      for (int k = r; k < H; ++k) v += L[k * LDM + r] * V[k];
-      S[r * H + c] = S[c * H + r] = v;
-    }
-  }
-  for (int e = 0; e < H * H; ++e) V[e] = e / H == e % H ? 1.0 : 0.0;
-  for (int sweep = 0; sweep < 20; ++sweep) {
-    bool more = false;
-    for (int q = 1; q < H; ++q)
-      for (int p = 0; p < q; ++p) {
-        const double apq = S[q * H + p];
-        double c, s, t;
-        jacobi_rot_rsq(apq, S[p * H + p], S[q * H + q], c, s, t);
-        if (t == 0.0) continue;
-        more = true;
-        for (int k = 0; k < H; ++k) {
-          if (k != p && k != q) {
-            const double x = S[k * H + p], y = S[k * H + q];
-            S[k * H + p] = S[p * H + k] = c * x - s * y;
-            S[k * H + q] = S[q * H + k] = s * x + c * y;
-          }
-          const double x = V[p * H + k], y = V[q * H + k];
-          V[p * H + k] = c * x - s * y;
-          V[q * H + k] = s * x + c * y;
-        }
-        S[p * H + p] -= t * apq;
-        S[q * H + q] += t * apq;
-        S[q * H + p] = S[p * H + q] = 0.0;
-      }
-    if (!more) break;
-  }
-  for (int k = 0; k < H; ++k) d[k] = S[k * H + k];
-}
-
-template <int N, bool GEN>
-__global__ void __launch_bounds__(32, WCfg<N>::MINB) flux_layer_warp_kernel(FluxParams p) {
-  using C = WCfg<N>;
-  constexpr int H = C::H, TEAM = C::TEAM, LDM = C::LDM;
-  extern __shared__ double smem[];
-  const int t = threadIdx.x % TEAM;
-  const unsigned msk = 0xffffffffu;  // the warp's teams go together
-  double* const sm = smem + (threadIdx.x / TEAM) * C::STRIDE;
-  double* const Ls = sm + C::O_L;
-  double* const Rs = sm + C::O_R;
-  double* const cb = sm + C::O_C;
-  double* const gl = sm + C::O_GL;
-  double* const b1 = sm + C::O_B1;
-  double* const b2 = sm + C::O_B2;
-  double* const ev = sm + C::O_E;
-  const int m = mode_of<GEN>(p);
-  const double* const tab = p.tables;
-  const double* const Y = tab + (long long)mode_row<GEN>() * tab_size(N) + tab_ylm(N);
-  const long long nt = layer_tasks<GEN>(p);
-  const long long task = (long long)blockIdx.x * C::TPW + threadIdx.x / TEAM;
-  // a team without a task computes on the last one's inputs and writes nothing
-  const LayerTask<N, GEN> q = layer_task<N, GEN>(p, task < nt ? task : nt - 1);
-  bool act = task < nt && q.live;
-  if (!__any_sync(msk, act)) return;
-  const double ws = q.rec[q.il.ssa_s + q.lc];
-  {
-    const int mode = (int)q.rec[q.il.mode + q.lc];
-    const double f = q.rec[q.il.fsc + q.lc], sig = q.rec[q.il.sig + q.lc];
-    for (int k = t; k < N; k += TEAM) gl[k] = phase_coeff<GEN>(k, q.pml[k], mode, ws, f, sig);
-  }
-  __syncwarp(msk);
-  const int odd0 = 1 - (m & 1);  // first l of odd l + m
-  const double fbeam = act ? q.rec[H_FBEAM] : 0.0;
-  const bool beam = fbeam > 0.0;
-  for (int r = t; r < H; r += TEAM) {
-    const double dm = tab[tab_dsim(N) + r] / tab[r];
-    ev[r] = dm;
-    double so = 0.0, se = 0.0;
-    if (beam) {
-      // (2 - delta_m0) F0 / 4pi sum_k g'_k P_k^m(mu_r) P_k^m(-mu0) by parity (DisortSolver.cpp:1361-1368)
-      const double* yb = beam_legendre<N, GEN>(p, q);
-      const double fac = ((GEN && m > 0) ? 4.0 : 2.0) * fbeam / (4.0 * 3.14159265358979323846);
-      for (int l = 0; l < N; l += 2) {
-        so += gl[l + odd0] * Y[(l + odd0) * N + r] * yb[l + odd0];
-        se += gl[l + 1 - odd0] * Y[(l + 1 - odd0) * N + r] * yb[l + 1 - odd0];
-      }
-      so *= dm * fac;
-      se *= dm * fac;
-    }
-    b1[r] = se;
-    b2[r] = so;
-  }
-  // ---- columns 2t, 2t + 1 of -A_s (into R) and -B_s (into L) -----------------
-  const double w0 = tab[tab_wt(N) + 2 * t], w1 = tab[tab_wt(N) + 2 * t + 1];
-  const double i0 = tab[tab_dinv(N) + 2 * t], i1 = tab[tab_dinv(N) + 2 * t + 1];
-  bool ok[2];
-  double F0[H], F1[H];
-#pragma unroll 1
-  for (int part = 0; part < 2; ++part) {  // 0: -A_s (even sums), 1: -B_s (odd sums)
-#pragma unroll
-    for (int r = 0; r < H; ++r) F0[r] = F1[r] = 0.0;
-    const int l0 = part == 0 ? 1 - odd0 : odd0;
-#pragma unroll 1
-    for (int l = l0; l < N; l += 2) {
-      const double* y = Y + l * N;
-      const double z0 = gl[l] * y[2 * t], z1 = gl[l] * y[2 * t + 1];
-      const double2* y2 = reinterpret_cast<const double2*>(y);
-#pragma unroll
-      for (int r = 0; r < H; r += 2) {
-        const double2 v = y2[r / 2];
-        F0[r] = fma(v.x, z0, F0[r]);
-        F0[r + 1] = fma(v.y, z0, F0[r + 1]);
-        F1[r] = fma(v.x, z1, F1[r]);
-        F1[r + 1] = fma(v.y, z1, F1[r + 1]);
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < H; ++r) {
-      const double dm = ev[r];  // d_r / mu_r
-      F0[r] = -dm * (w0 * F0[r] - (r == 2 * t ? 1.0 : 0.0)) * i0;
-      F1[r] = -dm * (w1 * F1[r] - (r == 2 * t + 1 ? 1.0 : 0.0)) * i1;
-    }
-    ok[part] = team_chol_columns<H, LDM, TEAM>(F0, F1, part == 0 ? Rs : Ls, cb, t, msk);
-  }
-  const bool okb = ok[1], oka = ok[0];
-  if (act && !okb && !oka) {
-    if (t == 0) no_eigensystem<N, GEN>(p, q);
-    act = false;
-  }
-  const bool regular = okb && oka;
-  // ---- F = L^T R, columns 2t, 2t + 1 ----------------------------------------
-#pragma unroll
-  for (int r = 0; r < H; ++r) F0[r] = F1[r] = 0.0;
-#pragma unroll 1
-  for (int k = 0; k < H; ++k) {
-    const double r0 = Rs[k * LDM + 2 * t], r1 = Rs[k * LDM + 2 * t + 1];
-    const double2* l2 = reinterpret_cast<const double2*>(Ls + k * LDM);
-#pragma unroll
-    for (int r = 0; r < H; r += 2) {
-      const double2 v = l2[r / 2];
-      F0[r] = fma(v.x, r0, F0[r]);
-      F0[r + 1] = fma(v.y, r0, F0[r + 1]);
-      F1[r] = fma(v.x, r1, F1[r]);
-      F1[r + 1] = fma(v.y, r1, F1[r + 1]);
-    }
-  }
-  // ---- one-sided Jacobi -------------------------------------------------------
+// One-sided Jacobi iteration on a team's columns (two per lane) in odd-even order: a
+// lane's two columns are the even rounds' pair, the odd rounds' pair takes the next
+// lane's first column by shuffles.  Leaves the columns normalised and their norms in k0,
+// k1.  live: false leaves the columns in place, up to sign.  The warp goes together.
+template <int H, int TEAM>
+__device__ __forceinline__ void team_onesided_jacobi(double* F0, double* F1, double& k0, double& k1, bool live, int t) {
+  const unsigned msk = 0xffffffffu;
   auto dot = [](const double* x, const double* y) {
     double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
 #pragma unroll
@@ -1442,7 +1241,6 @@ __global__ void __launch_bounds__(32, WCfg<N>::MINB) flux_layer_warp_kernel(Flux
     }
     return (s0 + s1) + (s2 + s3);
   };
-  bool live = act && regular;
   const bool last = t == TEAM - 1;
 #pragma unroll 1
   for (int sweep = 0; sweep < 20; ++sweep) {
@@ -1499,7 +1297,8 @@ __global__ void __launch_bounds__(32, WCfg<N>::MINB) flux_layer_warp_kernel(Flux
     live = live && (tm & team_bits) != 0u;
     if (!__any_sync(msk, live)) break;
   }
-  double k0 = dot(F0, F0), k1 = dot(F1, F1);
+  k0 = dot(F0, F0);
+  k1 = dot(F1, F1);
   {
     const double r0 = k0 > 0.0 ? rsqrt(k0) : 0.0, r1 = k1 > 0.0 ? rsqrt(k1) : 0.0;
     k0 = fmax(k0 * r0, 1e-9);
@@ -1510,35 +1309,218 @@ __global__ void __launch_bounds__(32, WCfg<N>::MINB) flux_layer_warp_kernel(Flux
       F1[r] *= r1;
     }
   }
+}
+
+// Columns 2t, 2t + 1 of -A_s or -B_s, the phase sums over l = l0, l0 + 2, ..., and their
+// diagonal elements once more.
+template <int N>
+__device__ __forceinline__ void team_matrix_columns(double* F0, double* F1, double& d00, double& d01, int l0, const double* gl, const double* ev,
+                                                    const double* Y, const double* tab, int t) {
+  constexpr int H = N / 2;
+  const double w0 = tab[tab_wt(N) + 2 * t], w1 = tab[tab_wt(N) + 2 * t + 1];
+  const double i0 = tab[tab_dinv(N) + 2 * t], i1 = tab[tab_dinv(N) + 2 * t + 1];
+  d00 = d01 = 0.0;
+#pragma unroll
+  for (int r = 0; r < H; ++r) F0[r] = F1[r] = 0.0;
+#pragma unroll 1
+  for (int l = l0; l < N; l += 2) {
+    const double* y = Y + l * N;
+    const double z0 = gl[l] * y[2 * t], z1 = gl[l] * y[2 * t + 1];
+    d00 = fma(y[2 * t], z0, d00);
+    d01 = fma(y[2 * t + 1], z1, d01);
+    const double2* y2 = reinterpret_cast<const double2*>(y);
+#pragma unroll
+    for (int r = 0; r < H; r += 2) {
+      const double2 v = y2[r / 2];
+      F0[r] = fma(v.x, z0, F0[r]);
+      F0[r + 1] = fma(v.y, z0, F0[r + 1]);
+      F1[r] = fma(v.x, z1, F1[r]);
+      F1[r + 1] = fma(v.y, z1, F1[r + 1]);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < H; ++r) {
+    const double dm = ev[r];  // d_r / mu_r
+    F0[r] = -dm * (w0 * F0[r] - (r == 2 * t ? 1.0 : 0.0)) * i0;
+    F1[r] = -dm * (w1 * F1[r] - (r == 2 * t + 1 ? 1.0 : 0.0)) * i1;
+  }
+  d00 = -ev[2 * t] * (w0 * d00 - 1.0) * i0;
+  d01 = -ev[2 * t + 1] * (w1 * d01 - 1.0) * i1;
+}
+
+// Columns 2t, 2t + 1 of A^T C, both in shared memory by rows.
+template <int H, int LDM>
+__device__ __forceinline__ void team_row_products(double* F0, double* F1, const double* A, const double* C, int t) {
+#pragma unroll
+  for (int r = 0; r < H; ++r) F0[r] = F1[r] = 0.0;
+#pragma unroll 1
+  for (int k = 0; k < H; ++k) {
+    const double c0 = C[k * LDM + 2 * t], c1 = C[k * LDM + 2 * t + 1];
+    const double2* a2 = reinterpret_cast<const double2*>(A + k * LDM);
+#pragma unroll
+    for (int r = 0; r < H; r += 2) {
+      const double2 v = a2[r / 2];
+      F0[r] = fma(v.x, c0, F0[r]);
+      F0[r + 1] = fma(v.y, c0, F0[r + 1]);
+      F1[r] = fma(v.x, c1, F1[r]);
+      F1[r + 1] = fma(v.y, c1, F1[r + 1]);
+    }
+  }
+}
+
+// INDEF: the pass over the tasks of which exactly one of -B_s and -A_s is positive
+// definite (rare: unphysical moments).  The ordinary pass marks them in their
+// boundary-value records (dead until the boundary-value kernel) and writes nothing more;
+// this one takes the definite matrix's factor L, forms S = L^T M L of the other one, M,
+// and goes on from S shifted and scaled as in layer_front_indefinite.  A pass of its own
+// costs a launch that finds nothing marked (2 us); as a branch the rare path took registers
+// from the ordinary one (192 x 91 layers at 64 streams 2.85 -> 3.85 ms), and one lane per
+// task with a two-sided Jacobi in global memory took 110 ms for 192 x 16 marked layers.
+template <int N, bool GEN, bool INDEF = false>
+__global__ void __launch_bounds__(32, WCfg<N>::MINB) flux_layer_warp_kernel(FluxParams p) {
+  using C = WCfg<N>;
+  constexpr int H = C::H, TEAM = C::TEAM, LDM = C::LDM;
+  extern __shared__ double smem[];
+  const int t = threadIdx.x % TEAM;
+  const unsigned msk = 0xffffffffu;  // the warp's teams go together
+  double* const sm = smem + (threadIdx.x / TEAM) * C::STRIDE;
+  double* const Ls = sm + C::O_L;
+  double* const Rs = sm + C::O_R;
+  double* const cb = sm + C::O_C;
+  double* const gl = sm + C::O_GL;
+  double* const b1 = sm + C::O_B1;
+  double* const b2 = sm + C::O_B2;
+  double* const ev = sm + C::O_E;
+  const int m = mode_of<GEN>(p);
+  const double* const tab = p.tables;
+  const double* const Y = tab + (long long)mode_row<GEN>() * tab_size(N) + tab_ylm(N);
+  const long long nt = layer_tasks<GEN>(p);
+  const long long task = (long long)blockIdx.x * C::TPW + threadIdx.x / TEAM;
+  // a team without a task computes on the last one's inputs and writes nothing
+  const LayerTask<N, GEN> q = layer_task<N, GEN>(p, task < nt ? task : nt - 1);
+  bool act = task < nt && q.live;
+  double* const mark = p.bvp_rec + mode_row<GEN>() * p.g.ms_bvp + task * brec_stride(N);
+  if constexpr (INDEF) act = act && *mark != 0.0;
+  if (!__any_sync(msk, act)) return;
+  const double ws = q.rec[q.il.ssa_s + q.lc];
+  {
+    const int mode = (int)q.rec[q.il.mode + q.lc];
+    const double f = q.rec[q.il.fsc + q.lc], sig = q.rec[q.il.sig + q.lc];
+    for (int k = t; k < N; k += TEAM) gl[k] = phase_coeff<GEN>(k, q.pml[k], mode, ws, f, sig);
+  }
+  __syncwarp(msk);
+  const int odd0 = 1 - (m & 1);  // first l of odd l + m
+  const double fbeam = act ? q.rec[H_FBEAM] : 0.0;
+  const bool beam = fbeam > 0.0;
+  for (int r = t; r < H; r += TEAM) {
+    const double dm = tab[tab_dsim(N) + r] / tab[r];
+    ev[r] = dm;
+    double so = 0.0, se = 0.0;
+    if (beam) {
+      // (2 - delta_m0) F0 / 4pi sum_k g'_k P_k^m(mu_r) P_k^m(-mu0) by parity (DisortSolver.cpp:1361-1368)
+      const double* yb = beam_legendre<N, GEN>(p, q);
+      const double fac = ((GEN && m > 0) ? 4.0 : 2.0) * fbeam / (4.0 * 3.14159265358979323846);
+      for (int l = 0; l < N; l += 2) {
+        so += gl[l + odd0] * Y[(l + odd0) * N + r] * yb[l + odd0];
+        se += gl[l + 1 - odd0] * Y[(l + 1 - odd0) * N + r] * yb[l + 1 - odd0];
+      }
+      so *= dm * fac;
+      se *= dm * fac;
+    }
+    b1[r] = se;
+    b2[r] = so;
+  }
+  // ---- columns 2t, 2t + 1 of -A_s (into R) and -B_s (into L) -----------------
+  bool ok[2];
+  double F0[H], F1[H];
+#pragma unroll 1
+  for (int part = 0; part < 2; ++part) {  // 0: -A_s (even sums), 1: -B_s (odd sums)
+    double d00, d01;
+    team_matrix_columns<N>(F0, F1, d00, d01, part == 0 ? 1 - odd0 : odd0, gl, ev, Y, tab, t);
+    ok[part] = team_chol_columns<H, LDM, TEAM>(F0, F1, d00, d01, part == 0 ? Rs : Ls, cb, t, msk);
+  }
+  const bool okb = ok[1], oka = ok[0];
   // lambda = k^2 negative: -A_s (na) or -B_s (nb) indefinite; see flux_eigen_kernel
   bool na0 = false, na1 = false, nb0 = false, nb1 = false;
-  if (__any_sync(msk, act && !regular)) {
-    if (act && !regular) {
-      double* const scr = p.bvp_rec + mode_row<GEN>() * p.g.ms_bvp + task * brec_stride(N);  // dead until the boundary-value kernel
-      if (t == 0)
-        team_indefinite<H, LDM>(gl, Y, tab, N, m, okb, Ls, scr, scr + 2 * H * H, scr + 3 * H * H);
-      __threadfence_block();
+  double k0, k1;
+  if constexpr (!INDEF) {
+    if (act && t == 0) {
+      *mark = okb != oka ? 1.0 : 0.0;
+      if (!okb && !oka) no_eigensystem<N, GEN>(p, q);
     }
-    __syncwarp(msk);
-    if (act && !regular) {
-      const double* const scr = p.bvp_rec + mode_row<GEN>() * p.g.ms_bvp + task * brec_stride(N);
-      const double *V = scr + 2 * H * H, *d = scr + 3 * H * H;
-      const double d0 = d[2 * t], d1 = d[2 * t + 1];
-      k0 = mode_k(d0);
-      k1 = mode_k(d1);
-      na0 = okb && d0 < 0.0;
-      na1 = okb && d1 < 0.0;
-      nb0 = !okb && d0 < 0.0;
-      nb1 = !okb && d1 < 0.0;
+    act = act && okb && oka;
+    // ---- F = L^T R, columns 2t, 2t + 1 ----------------------------------------
+    team_row_products<H, LDM>(F0, F1, Ls, Rs, t);
+    team_onesided_jacobi<H, TEAM>(F0, F1, k0, k1, act, t);
+  } else {
+    auto to_rows = [&] {  // the lane's columns as rows 2t, 2t + 1 of Rs
+      __syncwarp(msk);
 #pragma unroll
       for (int r = 0; r < H; ++r) {
-        F0[r] = V[(2 * t) * H + r];
-        F1[r] = V[(2 * t + 1) * H + r];
+        Rs[(2 * t) * LDM + r] = F0[r];
+        Rs[(2 * t + 1) * LDM + r] = F1[r];
       }
+      __syncwarp(msk);
+    };
+    if (!okb)
+      for (int e = t; e < H * H; e += TEAM) Ls[(e / H) * LDM + e % H] = Rs[(e / H) * LDM + e % H];
+    double d00, d01;
+    team_matrix_columns<N>(F0, F1, d00, d01, okb ? 1 - odd0 : odd0, gl, ev, Y, tab, t);
+    to_rows();
+    team_row_products<H, LDM>(F0, F1, Rs, Ls, t);  // M L (M is symmetric)
+    __syncwarp(msk);
+#pragma unroll
+    for (int r = 0; r < H; ++r) {
+      Rs[r * LDM + 2 * t] = F0[r];
+      Rs[r * LDM + 2 * t + 1] = F1[r];
     }
     __syncwarp(msk);
+    team_row_products<H, LDM>(F0, F1, Ls, Rs, t);  // S
+    to_rows();
+    double scale = 0.0, s1 = 0.0;
+#pragma unroll
+    for (int r = 0; r < H; ++r) {
+      scale += fabs(F0[r]);
+      s1 += fabs(F1[r]);
+    }
+    scale = fmax(scale, s1);
+#pragma unroll
+    for (int off = TEAM / 2; off > 0; off >>= 1) scale = fmax(scale, __shfl_xor_sync(msk, scale, off, TEAM));
+    if (!(scale > 0.0)) scale = 1.0;
+    double shift = kFirstShift * scale;
+    auto shifted = [&] {
+#pragma unroll
+      for (int r = 0; r < H; ++r) {
+        F0[r] = Rs[(2 * t) * LDM + r] + (r == 2 * t ? shift : 0.0);
+        F1[r] = Rs[(2 * t + 1) * LDM + r] + (r == 2 * t + 1 ? shift : 0.0);
+      }
+    };
+    bool done = !act;
+#pragma unroll 1
+    while (!__all_sync(msk, done)) {
+      shifted();
+      const bool pd = team_chol_columns<H, LDM, TEAM, false>(F0, F1, Rs[(2 * t) * LDM + 2 * t] + shift,
+                                                             Rs[(2 * t + 1) * LDM + 2 * t + 1] + shift, nullptr, cb, t, msk);
+      if (!done && !pd) shift *= 16.0;
+      done = done || pd || !(shift < scale);
+    }
+    shifted();
+#pragma unroll
+    for (int r = 0; r < H; ++r) {
+      F0[r] /= scale;
+      F1[r] /= scale;
+    }
+    __syncwarp(msk);
+    team_onesided_jacobi<H, TEAM>(F0, F1, k0, k1, act, t);
+    const double d0 = fma(k0, scale, -shift), d1 = fma(k1, scale, -shift);
+    k0 = mode_k(d0);
+    k1 = mode_k(d1);
+    na0 = okb && d0 < 0.0;
+    na1 = okb && d1 < 0.0;
+    nb0 = !okb && d0 < 0.0;
+    nb1 = !okb && d1 < 0.0;
   }
-  const bool primary = okb;  // L factors -B_s
+  const bool primary = !INDEF || okb;  // L factors -B_s
   // ---- x = L u / sqrt(k) (primary; else sqrt(k) L u / k) and its sums ----------
   const double rs0 = rsqrt(k0), rs1 = rsqrt(k1), sk0 = k0 * rs0, sk1 = k1 * rs1;
   // sums of the form with L u (lu) and with L^{-T} u (li): with b1, b2 and D M^{-1} 1
@@ -1658,9 +1640,12 @@ inline void flux_layer_set_attrs() {
   // the team kernel: N <= 16 on the flux path, when a schedule asks for it
   if constexpr (!GEN && layer_split<N>())
     cudaFuncSetAttribute(flux_layer_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LCfg<N>::smem_bytes());
-  if constexpr (!layer_split<N>())
+  if constexpr (!layer_split<N>()) {
     cudaFuncSetAttribute(flux_layer_warp_kernel<N, GEN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)WCfg<N>::smem_bytes());
+    cudaFuncSetAttribute(flux_layer_warp_kernel<N, GEN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)WCfg<N>::smem_bytes());
+  }
 }
 
 // The layer stage of `tasks` layer tasks (of each of `modes` azimuth modes).  N >= 32:
@@ -1687,7 +1672,10 @@ inline void flux_layer_launch(const FluxParams& p, long long tasks, const double
   } else {
     using C = WCfg<N>;
     const dim3 grid((unsigned)((tasks + C::TPW - 1) / C::TPW), (unsigned)modes);
-    wrap(2, [&] { flux_layer_warp_kernel<N, GEN><<<grid, 32, C::smem_bytes(), s>>>(p); });
+    wrap(2, [&] {
+      flux_layer_warp_kernel<N, GEN><<<grid, 32, C::smem_bytes(), s>>>(p);
+      flux_layer_warp_kernel<N, GEN, true><<<grid, 32, C::smem_bytes(), s>>>(p);
+    });
   }
 }
 
