@@ -81,7 +81,8 @@ dsp_status launch_flux_chunk(dsp_context ctx, const FluxParams& p, cudaStream_t 
     }
     KernelTimer kt(ctx, "flux_bvp_kernel", s);
     const int grid = (p.n + C::TPW - 1) / C::TPW;
-    if (jv) flux_bvp_kernel<N, false, SPH, C::LEAN><<<grid, 32, C::smem_bytes(), s>>>(p);
+    // (without thermal emission the Jacobians are zero and need no records)
+    if (jv && (p.flags & DSP_FLAG_THERMAL)) flux_bvp_kernel<N, false, SPH, C::LEAN><<<grid, 32, C::smem_bytes(), s>>>(p);
     else flux_bvp_kernel<N, false, SPH><<<grid, 32, C::smem_bytes(), s>>>(p);
   }
   if (jv) {
