@@ -5,7 +5,7 @@ depends on the stream count N and the layer count L of the instances:
   - flux path, N <= 16: the layer stage as two one-thread-per-task launches
     (eigensolver in registers; 64 or 128 threads per CTA) or as one team per
     layer task (eigensolver in shared memory);
-  - general path: the boundary-value kernel as one CTA or team per instance in
+  - general path: the boundary-value kernel as one team of lanes per instance in
     index order, or persistent (a resident grid taking instances from a queue
     sorted by descending layer count, the size classes).
 `tune()` times every candidate on synthetic instances of each (N, layer range)
