@@ -1397,10 +1397,11 @@ __global__ void __launch_bounds__(32, WCfg<N>::MINB) flux_layer_warp_kernel(Flux
   const long long nt = layer_tasks<GEN>(p);
   const long long task = (long long)blockIdx.x * C::TPW + threadIdx.x / TEAM;
   // a team without a task computes on the last one's inputs and writes nothing
-  const LayerTask<N, GEN> q = layer_task<N, GEN>(p, task < nt ? task : nt - 1);
-  bool act = task < nt && q.live;
   double* const mark = p.bvp_rec + mode_row<GEN>() * p.g.ms_bvp + task * brec_stride(N);
-  if constexpr (INDEF) act = act && *mark != 0.0;
+  const bool marked = INDEF && task < nt && *mark != 0.0;  // (of layers not solved: anything)
+  if (INDEF && !__any_sync(msk, marked)) return;
+  const LayerTask<N, GEN> q = layer_task<N, GEN>(p, task < nt ? task : nt - 1);
+  bool act = task < nt && q.live && (!INDEF || marked);
   if (!__any_sync(msk, act)) return;
   const double ws = q.rec[q.il.ssa_s + q.lc];
   {
