@@ -35,12 +35,13 @@
 //   phi_t = W phi_b + f,  W = 2 V G Y^T,  V = X H E,  f = X (c_t - r) + 2 V G (q - c_b),
 // and the fluxes of a level are sums w (phi +- psi), w mu (phi +- psi) with
 // psi = A phi + g, so that psi takes two vectors A w, A w mu and g.  The way down then
-// stores W, f, these two and g (106 doubles a layer at 16 streams) where the general
+// stores W, f, these two and g (108 doubles a layer at 16 streams) where the general
 // form stores G, H and r (136) and reads them and the layer record (188) again on the
 // way up; one product with W per layer, from registers, takes the place of six
 // matrix-vector products in a chain.  Two more h^3 products per layer pay for it:
 // 60,000 columns of 40 layers at 4 streams 0.80 -> 0.55 ms, 20,000 of 60 at 16 streams
-// 1.89 -> 1.51 ms, one of 60 layers 240 -> 211 us.  With 32 streams the products cost
+// 1.89 -> 1.51 ms, one of 60 layers 240 -> 211 us (now 0.56 ms, 1.40 ms, 199 us).  With 32
+// streams the products cost
 // what the way up gains (its share of a layer is 20 %, 11 % at 64).
 //
 // Mapping: lane j of a team owns column j; products read the other operand from

