@@ -1627,8 +1627,8 @@ __global__ void __launch_bounds__(32, WCfg<N>::MINB) flux_layer_warp_kernel(Flux
 }
 
 // Host side of the layer stage, launched through `wrap(kind, launch)`, which may time
-// it (kind 0: front, 1: eigensolver, 2: one kernel); `host_tab` is a host copy of the
-// (mode's) tab_* tables of N.
+// it (kind 0: front, 1: eigensolver, 2: one kernel, or either pass of the warp kernel);
+// `host_tab` is a host copy of the (mode's) tab_* tables of N.
 template <int N, bool GEN = false>
 inline void flux_layer_set_attrs() {
   if constexpr (layer_split<N>()) {
@@ -1648,7 +1648,7 @@ inline void flux_layer_set_attrs() {
 }
 
 // The layer stage of `tasks` layer tasks (of each of `modes` azimuth modes).  N >= 32:
-// the warp kernel.  N <= 16: front and eigensolver, one thread per task, with `cta`
+// the warp kernel, twice (INDEF).  N <= 16: front and eigensolver, one thread per task, with `cta`
 // threads per CTA (64 or 128), or, when a schedule of the flux path asks for it, the
 // team kernel.
 template <int N, bool GEN = false, class Wrap>
@@ -1671,10 +1671,8 @@ inline void flux_layer_launch(const FluxParams& p, long long tasks, const double
   } else {
     using C = WCfg<N>;
     const dim3 grid((unsigned)((tasks + C::TPW - 1) / C::TPW), (unsigned)modes);
-    wrap(2, [&] {
-      flux_layer_warp_kernel<N, GEN><<<grid, 32, C::smem_bytes(), s>>>(p);
-      flux_layer_warp_kernel<N, GEN, true><<<grid, 32, C::smem_bytes(), s>>>(p);
-    });
+    wrap(2, [&] { flux_layer_warp_kernel<N, GEN><<<grid, 32, C::smem_bytes(), s>>>(p); });
+    wrap(2, [&] { flux_layer_warp_kernel<N, GEN, true><<<grid, 32, C::smem_bytes(), s>>>(p); });
   }
 }
 
